@@ -99,11 +99,12 @@ __device__ void ip_bfs(const DGraph& g, const int32_t* lab, int32_t* dist, const
     __syncthreads();
 }
 
-// labels and distances live in shared memory when they fit (on_chip), else in
-// the trial's slices of the global arrays; the kept labels are written out
+// Trials of graphs too large for k_initpart_chip (coarsening that stalled
+// above 65,534 vertices, or no room for its shared-memory state): labels and
+// distances in the trial's slices of the global arrays
 __global__ void __launch_bounds__(IP_T) k_initpart(DGraph g, int32_t k, uint64_t seed, int32_t* __restrict__ labels,
                                                     int32_t* __restrict__ dists, int64_t* __restrict__ tcut,
-                                                    int64_t* __restrict__ tmaxpw, int key_iters, int on_chip) {
+                                                    int64_t* __restrict__ tmaxpw, int key_iters) {
     extern __shared__ int64_t ipsm[];
     __shared__ int flags[3];
     __shared__ int any;
@@ -119,14 +120,8 @@ __global__ void __launch_bounds__(IP_T) k_initpart(DGraph g, int32_t k, uint64_t
         int32_t* q = (int32_t*)p;
         S.cnt = q; q += k; S.cnt_d = q; q += k; S.incl = q; q += k;
     }
-    int32_t* glab = labels + (int64_t)t * n;
-    int32_t* lab = glab;
+    int32_t* lab = labels + (int64_t)t * n;
     int32_t* dist = dists + (int64_t)t * n;
-    if (on_chip) {
-        int32_t* q = (int32_t*)(ipsm + 9 * (int64_t)k) + 3 * (int64_t)k;
-        lab = q;
-        dist = q + n;
-    }
     const uint64_t ts = trial_salt(seed, t);
     for (int64_t v = threadIdx.x; v < n; v += blockDim.x) lab[v] = 0;
     for (int q = threadIdx.x; q < k; q += blockDim.x) S.cnt[q] = (q == 0) ? k : 0;
@@ -255,23 +250,399 @@ __global__ void __launch_bounds__(IP_T) k_initpart(DGraph g, int32_t k, uint64_t
         tcut[t] = s / 2;
         tmaxpw[t] = mp;
     }
-    if (on_chip)
-        for (int64_t v = threadIdx.x; v < n; v += blockDim.x) glab[v] = lab[v];
 }
 
+// ------------------------------------------------------------------ on-chip trials
+// The same trial with its whole state in shared memory (k_initpart_chip):
+// one 32-bit word per vertex (label << 16 | BFS distance, 0xFFFF: unreached),
+// a BFS queue and a work list of 16-bit ids.  What bounds it is the chain of
+// BFS levels (two barriers and the row loads of one frontier each), so the
+// work per level is the frontier's rows only, not a sweep over all vertices:
+//  - top-down levels expand the queue's frontier, a group of `tile` lanes per
+//    vertex (8, 16 or 32 by the mean degree); on graphs of a mean degree of
+//    32 and more a level whose frontier F is large runs bottom-up instead
+//    (every unreached vertex scans its row until it meets the frontier): about
+//    n / F entries per unreached vertex against F whole rows, so bottom-up
+//    when unreached * n < F * F * degree;
+//  - the second BFS sums each label's frontier weight level by level, which
+//    gives the distance at which the label's target weight is crossed, and
+//    stops there; the crossing vertex among that distance's vertices (in id
+//    order) is found by a 16-way search over ids, at most four rounds;
+//  - label weights are carried from split to split instead of summed anew.
+// CSR_SM: rows (32-bit starts, 16-bit ids) are copied to shared memory first,
+// which takes the L2 latency out of every level; taken when they fit.
+// 64 trials on a B200, this kernel against one whose BFS levels sweep every
+// vertex and whose split key takes a binary search over (distance, id):
+// 823 vertices k = 8 893 -> 143 us, random geometric 8,864 vertices k = 300
+// 44.0 -> 1.5 ms, Chung-Lu 1,789 vertices k = 64 5.4 -> 1.7 ms, R-MAT (dense)
+// 1,999 vertices k = 64 11.2 -> 3.5 ms.
+constexpr int32_t IPC_FAR = 0xFFFF;    // unreached / no crossing distance below it
+constexpr int IPC_BINS = 16;
+
+struct IpcLabels {
+    int32_t* cnt;      // parts of the label
+    int32_t* cnt_d;    // snapshot at the start of a depth
+    int32_t* W;        // weight
+    int32_t* target;   // weight wanted on the left
+    int32_t* cum;      // weight below the current distance / below the crossing vertex
+    int32_t* wlev;     // weight at the current distance
+    int32_t* crit;     // crossing distance (-1: not found yet, IPC_FAR: among the unreached)
+    int32_t* lo;       // id search range [lo, hi); lo ends as the crossing vertex
+    int32_t* hi;
+    int32_t* incl;     // crossing vertex goes left
+    uint32_t* pk;      // farthest vertex: distance << 16 | 0xFFFF - id
+    int32_t* hist;     // IPC_BINS weights
+    uint64_t* s0;      // seed: top-32 hash << 32 | id
+};
+constexpr size_t ipc_label_bytes() { return sizeof(int32_t) * (11 + IPC_BINS) + sizeof(uint64_t); }
+
+// shared counters of one trial
+struct IpcShared {
+    int32_t tail, nlist, nact, any;
+    int64_t red[32];
+};
+
+template <bool CSR_SM>
+struct IpcRows {
+    const int64_t* rp;
+    const int32_t* ci;
+    const uint32_t* srp;
+    const uint16_t* sci;
+    __device__ __forceinline__ int64_t beg(int32_t v) const { return CSR_SM ? (int64_t)srp[v] : rp[v]; }
+    __device__ __forceinline__ int32_t id(int64_t e) const { return CSR_SM ? (int32_t)sci[e] : ci[e]; }
+};
+
+// appends of the calling lanes (any subset of a warp): one shared atomic per warp
+__device__ __forceinline__ int32_t ipc_slot(int32_t* counter) {
+    const uint32_t m = __activemask();
+    const int lane = threadIdx.x & 31, lead = __ffs(m) - 1;
+    int32_t base = 0;
+    if (lane == lead) base = atomicAdd(counter, __popc(m));
+    base = __shfl_sync(m, base, lead);
+    return base + __popc(m & ((1u << lane) - 1u));
+}
+
+// BFS inside every splitting label from the sources queued at [0, tail) with
+// distance 0.  CROSS: track the crossing distances and stop once every
+// splitting label has one.  nv: vertices of splitting labels.
+template <bool CSR_SM, bool CROSS>
+__device__ void ipc_bfs(const DGraph& g, const IpcRows<CSR_SM>& R, uint32_t* state, uint16_t* queue, uint16_t* list,
+                        const IpcLabels& S, IpcShared& sh, int32_t k, int32_t nv, int tile, int64_t davg) {
+    const int32_t n = (int32_t)g.n;
+    const int lane = threadIdx.x & 31;
+    const int tl = threadIdx.x & (tile - 1);
+    const int32_t grp = threadIdx.x / tile, ngrp = blockDim.x / tile;
+    int32_t h = 0, t = sh.tail;
+    __syncthreads();
+    for (int32_t r = 0; h < t; ++r) {
+        const int64_t F = t - h, U = nv - t;
+        const bool up = davg >= 32 && U * n < F * F * davg;
+        if (up) {
+            // unreached vertices of labels still searching
+            for (int32_t v = threadIdx.x; v < n; v += blockDim.x) {
+                const uint32_t s = state[v];
+                const int32_t L = (int32_t)(s >> 16);
+                if ((s & 0xFFFFu) == (uint32_t)IPC_FAR && S.cnt_d[L] > 1 && (!CROSS || S.crit[L] < 0))
+                    list[ipc_slot(&sh.nlist)] = (uint16_t)v;
+            }
+            if (CROSS)
+                for (int32_t i = h + threadIdx.x; i < t; i += blockDim.x) {
+                    const int32_t v = queue[i];
+                    const int32_t L = (int32_t)(state[v] >> 16);
+                    if (S.crit[L] < 0) atomicAdd(&S.wlev[L], g.vw ? g.vw[v] : 1);
+                }
+            __syncthreads();
+            const int32_t nl = sh.nlist;
+            for (int32_t i = threadIdx.x >> 5; i < nl; i += blockDim.x >> 5) {
+                const int32_t v = list[i];
+                const uint32_t want = (state[v] & 0xFFFF0000u) | (uint32_t)r;
+                const int64_t end = R.beg(v + 1);
+                bool hit = false;
+                for (int64_t e0 = R.beg(v); e0 < end && !hit; e0 += 32) {
+                    const int64_t e = e0 + lane;
+                    bool f = false;
+                    if (e < end) {
+                        const int32_t u = R.id(e);
+                        f = GP_IN(u, n) && state[u] == want;
+                    }
+                    hit = __any_sync(0xffffffffu, f);
+                }
+                if (hit && lane == 0) {
+                    state[v] = want + 1u;
+                    queue[atomicAdd(&sh.tail, 1)] = (uint16_t)v;
+                }
+            }
+        } else {
+            for (int32_t i = h + grp; i < t; i += ngrp) {
+                const int32_t v = queue[i];
+                const uint32_t lab = state[v] & 0xFFFF0000u;
+                if (CROSS) {
+                    const int32_t L = (int32_t)(lab >> 16);
+                    if (S.crit[L] >= 0) continue;
+                    if (tl == 0) atomicAdd(&S.wlev[L], g.vw ? g.vw[v] : 1);
+                }
+                const uint32_t open = lab | (uint32_t)IPC_FAR;
+                const int64_t end = R.beg(v + 1);
+                for (int64_t e = R.beg(v) + tl; e < end; e += tile) {
+                    const int32_t u = R.id(e);
+                    if (GP_IN(u, n) && state[u] == open && atomicCAS(&state[u], open, lab | (uint32_t)(r + 1)) == open)
+                        queue[ipc_slot(&sh.tail)] = (uint16_t)u;
+                }
+            }
+        }
+        __syncthreads();
+        h = t;
+        t = sh.tail;
+        if (threadIdx.x == 0) sh.nlist = 0;
+        if (CROSS) {
+            for (int32_t q = threadIdx.x; q < k; q += blockDim.x) {
+                const int32_t w = S.wlev[q];
+                if (w == 0) continue;
+                S.wlev[q] = 0;
+                if (S.cum[q] + w > S.target[q]) { S.crit[q] = r; atomicSub(&sh.nact, 1); }
+                else S.cum[q] += w;
+            }
+        }
+        __syncthreads();
+        if (CROSS && sh.nact == 0) break;
+    }
+}
+
+// one trial per CTA; shared memory: ipc_smem(n, m, k, CSR_SM, lists on chip)
+template <bool CSR_SM>
+__global__ void __launch_bounds__(IP_T) k_initpart_chip(DGraph g, int32_t k, uint64_t seed, int32_t* __restrict__ labels,
+                                                        uint16_t* __restrict__ lists, int64_t* __restrict__ tcut,
+                                                        int64_t* __restrict__ tmaxpw, int tile) {
+    extern __shared__ __align__(16) unsigned char ipc_raw[];
+    __shared__ IpcShared sh;
+    const int32_t n = (int32_t)g.n;
+    const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+    IpcLabels S;
+    S.s0 = (uint64_t*)ipc_raw;
+    int32_t* p = (int32_t*)(S.s0 + k);
+    S.cnt = p; p += k; S.cnt_d = p; p += k; S.W = p; p += k; S.target = p; p += k; S.cum = p; p += k;
+    S.wlev = p; p += k; S.crit = p; p += k; S.lo = p; p += k; S.hi = p; p += k; S.incl = p; p += k;
+    S.pk = (uint32_t*)p; p += k;
+    S.hist = p; p += (int64_t)IPC_BINS * k;
+    uint32_t* state = (uint32_t*)p;
+    uint32_t* after = state + n;
+    IpcRows<CSR_SM> R{g.rp, g.ci, nullptr, nullptr};
+    if (CSR_SM) {
+        uint32_t* srp = after;
+        after += n + 1;
+        uint16_t* sci = (uint16_t*)after;
+        after += (g.m + 1) / 2;
+        for (int32_t v = threadIdx.x; v <= n; v += blockDim.x) srp[v] = (uint32_t)g.rp[v];
+        for (int32_t e = threadIdx.x; e < (int32_t)g.m; e += blockDim.x) sci[e] = (uint16_t)g.ci[e];
+        R.srp = srp; R.sci = sci;
+    }
+    // queue and list: n ids each, on chip unless the caller brings them
+    uint16_t* queue = lists ? lists + 2 * (int64_t)t * n : (uint16_t*)after;
+    uint16_t* list = queue + n;
+    const int64_t davg = g.m / (n > 0 ? n : 1);
+    const uint64_t ts = trial_salt(seed, t);
+    int64_t wsum = 0;
+    for (int32_t v = threadIdx.x; v < n; v += blockDim.x) { state[v] = 0; wsum += g.vw ? g.vw[v] : 1; }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) wsum += __shfl_xor_sync(0xffffffffu, wsum, o);
+    if (lane == 0) sh.red[warp] = wsum;
+    for (int32_t q = threadIdx.x; q < k; q += blockDim.x) {
+        S.cnt[q] = q == 0 ? k : 0;
+        S.W[q] = 0; S.wlev[q] = 0;
+    }
+    for (int32_t i = threadIdx.x; i < IPC_BINS * k; i += blockDim.x) S.hist[i] = 0;
+    if (threadIdx.x == 0) sh.nlist = 0;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int64_t s = 0;
+        for (int i = 0; i < nwarp; ++i) s += sh.red[i];
+        S.W[0] = (int32_t)s;   // the total fits in int32 (checked on input)
+    }
+    int32_t vbits = 1;   // 16-way rounds of the id search: 4 bits each
+    while ((1 << vbits) < n) ++vbits;
+    for (int d = 0;; ++d) {
+        if (threadIdx.x == 0) { sh.any = 0; sh.tail = 0; sh.nact = 0; }
+        __syncthreads();
+        int32_t mine = 0;
+        for (int32_t q = threadIdx.x; q < k; q += blockDim.x) {
+            const int32_t c = S.cnt[q];
+            S.cnt_d[q] = c;
+            S.s0[q] = ~0ull; S.pk[q] = 0;
+            if (c > 1) {
+                ++mine;
+                S.target[q] = (int32_t)((int64_t)S.W[q] * (c / 2) / c);
+                S.cum[q] = 0; S.crit[q] = -1; S.lo[q] = 0; S.hi[q] = n;
+            }
+        }
+        if (mine) atomicAdd(&sh.any, mine);
+        __syncthreads();
+        const int32_t nsplit = sh.any;
+        if (nsplit == 0) break;
+        const uint64_t ds = depth_salt(ts, d);
+        // seeds, and every vertex of a splitting label unreached.  Few labels:
+        // one 64-bit atomic per label and warp; many: a plain check keeps most
+        // lanes from the atomic
+        int32_t myv = 0;
+        for (int32_t v0 = threadIdx.x & ~31; v0 < n; v0 += blockDim.x) {
+            const int32_t v = v0 + lane;
+            int32_t L = v < n ? (int32_t)(state[v] >> 16) : -1;
+            if (L >= 0 && S.cnt_d[L] <= 1) L = -1;
+            uint64_t key = ~0ull;
+            if (L >= 0) {
+                state[v] = ((uint32_t)L << 16) | (uint32_t)IPC_FAR;
+                key = ((mix64(ds ^ (uint64_t)(uint32_t)v) >> 32) << 32) | (uint32_t)v;
+                ++myv;
+            }
+            if (nsplit <= 4) ip_label_ext<false>(S.s0, L, key);
+            else if (L >= 0 && key < S.s0[L]) atomicMin((unsigned long long*)&S.s0[L], (unsigned long long)key);
+        }
+        myv = (int32_t)__reduce_add_sync(0xffffffffu, (uint32_t)myv);
+        if (lane == 0) sh.red[warp] = myv;
+        __syncthreads();
+        int32_t nv = 0;
+        for (int i = 0; i < nwarp; ++i) nv += (int32_t)sh.red[i];
+        // BFS 1 from the seeds
+        for (int32_t q = threadIdx.x; q < k; q += blockDim.x)
+            if (S.cnt_d[q] > 1 && S.s0[q] != ~0ull) {
+                const int32_t v = (int32_t)(uint32_t)S.s0[q];
+                state[v] = (uint32_t)q << 16;
+                queue[atomicAdd(&sh.tail, 1)] = (uint16_t)v;
+            }
+        __syncthreads();
+        ipc_bfs<CSR_SM, false>(g, R, state, queue, list, S, sh, k, nv, tile, davg);
+        // pseudo-peripheral vertex: largest distance, smallest id
+        const int32_t reached = sh.tail;
+        for (int32_t i0 = threadIdx.x & ~31; i0 < reached; i0 += blockDim.x) {
+            const int32_t i = i0 + lane;
+            const int32_t v = i < reached ? (int32_t)queue[i] : 0;
+            const uint32_t s = state[v];
+            const int32_t L = i < reached ? (int32_t)(s >> 16) : -1;
+            const uint32_t key = L >= 0 ? ((s & 0xFFFFu) << 16 | (0xFFFFu - (uint32_t)v)) : 0u;
+            if (L >= 0 && key > S.pk[L]) atomicMax(&S.pk[L], key);
+        }
+        __syncthreads();
+        for (int32_t v = threadIdx.x; v < n; v += blockDim.x) state[v] |= (uint32_t)IPC_FAR;
+        if (threadIdx.x == 0) sh.tail = 0;
+        __syncthreads();
+        for (int32_t q = threadIdx.x; q < k; q += blockDim.x)
+            if (S.cnt_d[q] > 1 && S.s0[q] != ~0ull) {
+                const int32_t v = (int32_t)(0xFFFFu - (S.pk[q] & 0xFFFFu));
+                state[v] = (uint32_t)q << 16;
+                queue[atomicAdd(&sh.tail, 1)] = (uint16_t)v;
+                atomicAdd(&sh.nact, 1);
+            }
+        __syncthreads();
+        ipc_bfs<CSR_SM, true>(g, R, state, queue, list, S, sh, k, nv, tile, davg);
+        for (int32_t q = threadIdx.x; q < k; q += blockDim.x)
+            if (S.cnt_d[q] > 1 && S.crit[q] < 0) S.crit[q] = IPC_FAR;   // its component ended below the target
+        __syncthreads();
+        // crossing vertex: the first, in id order, of the crossing distance's
+        // vertices that takes the label's weight above the target
+        for (int32_t v = threadIdx.x; v < n; v += blockDim.x) {
+            const uint32_t s = state[v];
+            const int32_t L = (int32_t)(s >> 16);
+            if (S.cnt_d[L] > 1 && (int32_t)(s & 0xFFFFu) == S.crit[L]) list[ipc_slot(&sh.nlist)] = (uint16_t)v;
+        }
+        __syncthreads();
+        const int32_t nl = sh.nlist;
+        for (int32_t b = vbits; b > 0; b -= 4) {
+            for (int32_t i = threadIdx.x; i < nl; i += blockDim.x) {
+                const int32_t v = list[i];
+                const int32_t L = (int32_t)(state[v] >> 16), lo = S.lo[L], hi = S.hi[L];
+                if (v < lo || v >= hi) continue;
+                const int32_t width = (hi - lo + IPC_BINS - 1) / IPC_BINS;
+                atomicAdd(&S.hist[IPC_BINS * L + (v - lo) / width], g.vw ? g.vw[v] : 1);
+            }
+            __syncthreads();
+            if (threadIdx.x == 0) sh.nlist = 0;
+            for (int32_t q = threadIdx.x; q < k; q += blockDim.x) {
+                if (S.cnt_d[q] <= 1) continue;
+                const int32_t lo = S.lo[q], hi = S.hi[q];
+                const int32_t width = (hi - lo + IPC_BINS - 1) / IPC_BINS;
+                int32_t sum = S.cum[q], at = -1;
+                for (int i = 0; i < IPC_BINS; ++i) {
+                    const int32_t w = S.hist[IPC_BINS * q + i];
+                    S.hist[IPC_BINS * q + i] = 0;
+                    if (at < 0) { if (sum + w > S.target[q]) at = i; else sum += w; }
+                }
+                if (at >= 0) {   // always, unless the label is empty
+                    S.cum[q] = sum;
+                    S.lo[q] = lo + at * width;
+                    S.hi[q] = lo + (at + 1) * width < hi ? lo + (at + 1) * width : hi;
+                }
+            }
+            __syncthreads();
+        }
+        for (int32_t q = threadIdx.x; q < k; q += blockDim.x) {
+            const int32_t c = S.cnt_d[q];
+            if (c <= 1) continue;
+            const int32_t W = S.W[q], flo = S.cum[q];
+            const int32_t xw = W > 0 ? (g.vw ? g.vw[S.lo[q]] : 1) : 0;
+            const int32_t in = (xw > 0 && 2 * (int64_t)S.target[q] > 2 * (int64_t)flo + xw) ? 1 : 0;
+            S.incl[q] = in;
+            const int32_t left = W > 0 ? flo + (in ? xw : 0) : 0;
+            S.cnt[q] = c / 2;
+            S.cnt[q + c / 2] = c - c / 2;
+            S.W[q] = left;
+            S.W[q + c / 2] = W - left;
+        }
+        __syncthreads();
+        for (int32_t v = threadIdx.x; v < n; v += blockDim.x) {
+            const uint32_t s = state[v];
+            const int32_t L = (int32_t)(s >> 16), c = S.cnt_d[L];
+            if (c <= 1) continue;
+            const int32_t dv = (int32_t)(s & 0xFFFFu), cd = S.crit[L], x = S.lo[L];
+            const bool left = dv < cd || (dv == cd && (v < x || (v == x && S.incl[L])));
+            if (!left) state[v] = (uint32_t)(L + c / 2) << 16;
+        }
+        __syncthreads();
+    }
+    // the trial's cut and heaviest part
+    int64_t cross = 0;
+    const int tl = threadIdx.x & (tile - 1);
+    for (int32_t v = threadIdx.x / tile; v < n; v += blockDim.x / tile) {
+        const uint32_t pv = state[v] >> 16;
+        const int64_t end = R.beg(v + 1);
+        for (int64_t e = R.beg(v) + tl; e < end; e += tile) {
+            const int32_t u = R.id(e);
+            if (GP_IN(u, n) && (state[u] >> 16) != pv) cross += g.ew ? g.ew[e] : 1;
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) cross += __shfl_xor_sync(0xffffffffu, cross, o);
+    int32_t mp = 0;
+    for (int32_t q = threadIdx.x; q < k; q += blockDim.x) mp = S.W[q] > mp ? S.W[q] : mp;
+    mp = (int32_t)__reduce_max_sync(0xffffffffu, (uint32_t)mp);
+    __shared__ int32_t s_mp[32];
+    if (lane == 0) { sh.red[warp] = cross; s_mp[warp] = mp; }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int64_t s = 0;
+        for (int i = 0; i < nwarp; ++i) { s += sh.red[i]; mp = s_mp[i] > mp ? s_mp[i] : mp; }
+        tcut[t] = s / 2;
+        tmaxpw[t] = mp;
+    }
+    for (int32_t v = threadIdx.x; v < n; v += blockDim.x) labels[(int64_t)t * n + v] = (int32_t)(state[v] >> 16);
+}
+
+// the kept trial: balanced before not, then (not balanced) the smaller heaviest
+// part, then the lower cut, then the lower trial; one warp
 __global__ void k_pick_trial(int T, const int64_t* __restrict__ tcut, const int64_t* __restrict__ tmaxpw, int64_t Lmax,
                              int64_t* __restrict__ best) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    int bt = 0;
-    for (int t = 1; t < T; ++t) {
-        const bool bal = tmaxpw[t] <= Lmax, bbal = tmaxpw[bt] <= Lmax;
-        bool better;
-        if (bal != bbal) better = bal;
-        else if (!bal && tmaxpw[t] != tmaxpw[bt]) better = tmaxpw[t] < tmaxpw[bt];
-        else better = tcut[t] < tcut[bt];
-        if (better) bt = t;
+    const int lane = threadIdx.x & 31;
+    int64_t a = INT64_MAX, b = INT64_MAX;   // (max(heaviest, Lmax), cut)
+    int bt = INT32_MAX;
+    auto take = [&](int64_t a2, int64_t b2, int t2) {
+        if (a2 < a || (a2 == a && (b2 < b || (b2 == b && t2 < bt)))) { a = a2; b = b2; bt = t2; }
+    };
+    for (int t = lane; t < T; t += 32) take(tmaxpw[t] > Lmax ? tmaxpw[t] : Lmax, tcut[t], t);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const int64_t a2 = __shfl_xor_sync(0xffffffffu, a, o), b2 = __shfl_xor_sync(0xffffffffu, b, o);
+        const int t2 = __shfl_xor_sync(0xffffffffu, bt, o);
+        take(a2, b2, t2);
     }
-    best[0] = bt;
+    if (threadIdx.x == 0) best[0] = bt;
 }
 
 static int bits_for64(int64_t x) {
@@ -283,21 +654,39 @@ static int bits_for64(int64_t x) {
 size_t initpart_smem_max();
 
 int initial_partition(Ctx& c, const Level& L, const Params& P, int32_t* part_out) {
-    const int64_t n = L.g.n;
+    const int64_t n = L.g.n, m = L.g.m;
     const int T = P.o.init_trials;
     auto mk = c.tmp->save();
     int32_t* labels = c.tmp_alloc<int32_t>((int64_t)T * n);
-    int32_t* dists = c.tmp_alloc<int32_t>((int64_t)T * n);
     int64_t* tcut = c.tmp_alloc<int64_t>(T);
     int64_t* tmaxpw = c.tmp_alloc<int64_t>(T);
     int64_t* best = c.tmp_alloc<int64_t>(1);
-    const size_t base = (size_t)P.k * (9 * sizeof(int64_t) + 3 * sizeof(int32_t));
-    const size_t onchip = base + 2 * sizeof(int32_t) * (size_t)n;
-    const bool on_chip = onchip <= initpart_smem_max();
-    const size_t smem = on_chip ? onchip : base;
-    const int key_iters = bits_for64(n * (n + 1)) + 1;
-    k_initpart<<<T, IP_T, smem, c.s>>>(L.g, P.k, P.seed, labels, dists, tcut, tmaxpw, key_iters, on_chip ? 1 : 0);
-    GP_LAUNCHED(c);
+    const size_t cap = initpart_smem_max();
+    // 16-bit ids and distances, state of every vertex on chip: k_initpart_chip
+    const size_t chip = (size_t)P.k * ipc_label_bytes() + sizeof(uint32_t) * (size_t)n;
+    if (n < IPC_FAR && chip <= cap) {
+        const size_t lists = sizeof(uint16_t) * 2 * (size_t)n;
+        const size_t csr = sizeof(uint32_t) * (size_t)(n + 1) + sizeof(uint32_t) * (size_t)((m + 1) / 2);
+        const bool lists_on = chip + lists <= cap;
+        // at most half the block's shared memory for a copy of the rows: two trials stay resident per SM
+        const bool csr_on = chip + lists + csr <= cap / 2;
+        uint16_t* glists = lists_on ? nullptr : c.tmp_alloc<uint16_t>(2 * (int64_t)T * n);
+        const int64_t davg = m / std::max<int64_t>(n, 1);
+        const int tile = davg <= 8 ? 8 : (davg <= 16 ? 16 : 32);
+        const int threads = (n <= 4096 && m <= 65536) ? IP_T / 2 : IP_T;
+        const size_t smem = chip + (lists_on ? lists : 0) + (csr_on ? csr : 0);
+        if (csr_on)
+            k_initpart_chip<true><<<T, threads, smem, c.s>>>(L.g, P.k, P.seed, labels, glists, tcut, tmaxpw, tile);
+        else
+            k_initpart_chip<false><<<T, threads, smem, c.s>>>(L.g, P.k, P.seed, labels, glists, tcut, tmaxpw, tile);
+        GP_LAUNCHED(c);
+    } else {
+        int32_t* dists = c.tmp_alloc<int32_t>((int64_t)T * n);
+        const size_t base = (size_t)P.k * (9 * sizeof(int64_t) + 3 * sizeof(int32_t));
+        const int key_iters = bits_for64(n * (n + 1)) + 1;
+        k_initpart<<<T, IP_T, base, c.s>>>(L.g, P.k, P.seed, labels, dists, tcut, tmaxpw, key_iters);
+        GP_LAUNCHED(c);
+    }
     k_pick_trial<<<1, 32, 0, c.s>>>(T, tcut, tmaxpw, P.Lmax, best);
     GP_LAUNCHED(c);
     const int bt = (int)read_i64(c, best);
@@ -322,6 +711,8 @@ void initpart_smem_caps() {
     // static shared memory of the kernel (flags, reductions) stays outside the cap
     const size_t cap = std::max(need, (size_t)optin > 4096 ? (size_t)optin - 4096 : need);
     GP_CUDA(cudaFuncSetAttribute(k_initpart, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
+    GP_CUDA(cudaFuncSetAttribute(k_initpart_chip<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
+    GP_CUDA(cudaFuncSetAttribute(k_initpart_chip<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
     g_ip_smem_max = cap;
 }
 
