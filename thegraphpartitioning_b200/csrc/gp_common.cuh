@@ -170,7 +170,7 @@ inline int64_t csr_slice(int64_t m, int sm_count) {
     s = (s + 255) & ~(int64_t)255;
     return s < 256 ? 256 : (s > 16384 ? 16384 : s);
 }
-// The same argmax and a sum over aligned groups of TILE lanes (TILE a power of
+// The same argmax over aligned groups of TILE lanes (TILE a power of
 // two <= 32; every lane of the warp calls them).  A group smaller than the
 // warp reduces with butterfly shuffles inside the group: a redux.sync whose
 // member mask differs between the lanes of one warp runs once per group.
@@ -185,16 +185,6 @@ __device__ __forceinline__ void tile_argmax64(uint64_t& k, int32_t& id) {
             const int32_t i2 = __shfl_xor_sync(0xffffffffu, id, o);
             if (k2 > k || (k2 == k && (uint32_t)i2 < (uint32_t)id)) { k = k2; id = i2; }
         }
-    }
-}
-template <int TILE>
-__device__ __forceinline__ uint32_t tile_sum_u32(uint32_t x) {
-    if constexpr (TILE == 32) {
-        return __reduce_add_sync(0xffffffffu, x);
-    } else {
-#pragma unroll
-        for (int o = TILE / 2; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-        return x;
     }
 }
 #endif

@@ -55,39 +55,22 @@ __device__ __forceinline__ void group_argmax_u32(uint32_t mask, uint64_t& bk, in
     bk = mh;
     bq = mh ? (int32_t)mq : -1;
 }
-// group_argmax_u32 over aligned groups of TILE lanes (see tile_argmax64)
-template <int TILE>
-__device__ __forceinline__ void tile_argmax_u32(uint64_t& bk, int32_t& bq, uint32_t h, int32_t q) {
-    if constexpr (TILE == 32) {
-        group_argmax_u32(0xffffffffu, bk, bq, h, q);
-    } else {
-        uint32_t kq = h ? (uint32_t)q : 0xffffffffu;
-#pragma unroll
-        for (int o = TILE / 2; o > 0; o >>= 1) {
-            const uint32_t h2 = __shfl_xor_sync(0xffffffffu, h, o), q2 = __shfl_xor_sync(0xffffffffu, kq, o);
-            if (h2 > h || (h2 == h && q2 < kq)) { h = h2; kq = q2; }
-        }
-        bk = h;
-        bq = h ? (int32_t)kq : -1;
-    }
-}
 __device__ __forceinline__ void argmax_u32(uint32_t& bh, int32_t& bq, uint32_t h, int32_t q) {
     if (h > bh || (h == bh && (uint32_t)q < (uint32_t)bq)) { bh = h; bq = q; }
 }
 
-// LP candidate rule: gain >= 0, or -gain < own/den
-__device__ __forceinline__ bool lp_candidate(int64_t g, int64_t own, int32_t den) {
-    return g >= 0 || -g < own / den;
+// LP candidate rule: gain >= 0, or -gain < own/den (integer division; for
+// x = 1 - gain, x <= own/den exactly when x * den <= own: one wide multiply)
+__device__ __forceinline__ bool lp_candidate(int32_t g, int32_t own, int32_t den) {
+    return g >= 0 || (int64_t)(1 - (int64_t)g) * den <= own;
 }
 
 // ------------------------------------------------------------------ k_conn
-// One unit of work per warp: 4 rows of bucket 0 (8 lanes each), or 1 row of
-// bucket 1, or 1 row of bucket 2; rows longer than kHeavyDeg take CTAs
-// [0, nheavy).  Buckets 0/1 keep their entries in registers: a bucket-0 lane
-// sums the weights of its 8-lane tile's entries of the same part with seven
-// shuffles, a bucket-1 row adds its entries into the warp's shared-memory
-// histogram and reads its own part's bin back; bucket 2 and heavy rows build
-// the whole shared-memory histogram.
+// Light rows are taken 8 units (4 bucket-0 rows, 1 bucket-1 row or 1 bucket-2
+// row each) per warp at a time (conn_group); rows longer than kHeavyDeg take
+// CTAs [0, nheavy).  Bucket-0 rows take one thread each, bucket-1 rows 4 lanes
+// (up to 16 entries) or the warp (up to 32), bucket-2 rows the warp; bucket 2
+// and heavy rows build the whole shared-memory histogram.
 // status: [S_CROSS] += directed cross weight; [S_MAXPW], [S_MODE], [S_LIGHT]
 // written by CTA 0; LP candidates are appended to clist[bucket] (any order:
 // each is evaluated on its own), with [S_NL0..S_NL2] their counts and
@@ -99,7 +82,6 @@ struct ConnArgs {
     int64_t Lmax;
     int32_t den;
     int force_eval;
-    const int32_t* part;
     const uint8_t* lock;
     const int64_t* pw;
     const int32_t* heavy;
@@ -113,17 +95,17 @@ struct ConnArgs {
     const int64_t* wfirst;      // first light unit of each light warp, and the end (nw + 1)
     int32_t* dest;
     int32_t* gain;
-    int32_t* part_next;         // label propagation: part and cleared lock copied here for the
+    const void* pc;             // the partition: PT[n], uint8 (k <= 256), uint16 (k <= 1024) or int32
+    void* pc_next;              // label propagation: partition and cleared lock copied here for the
     uint8_t* lock_next;         // move step (nullptr: not needed)
-    const void* pc;             // the part array as gathered per neighbour: PT[n], a uint8 or uint16
-                                // copy of part (k <= 256 / k <= 1024), or part itself (int32)
-    void* pc_next;              // copy of part_next in the same type (nullptr: none kept)
     int64_t* status;
-    int32_t* clist[3];
+    int32_t* clist[3];          // nullptr: no candidate lists (the one-block loop rescans dest)
     int32_t* hhist;
     int64_t* hsum;
     int32_t* hdone;
     uint64_t* pdg;              // label propagation: pdg_pack(part, dest, gain) per row (nullptr: none)
+    int lp_dg;                  // label propagation also writes dest and gain (no pdg, or someone
+                                // else reads them)
 };
 
 // one word per vertex for the move step: part (bits 44-53), dest + 1 (bits
@@ -135,17 +117,24 @@ __device__ __forceinline__ int32_t pdg_part(uint64_t x) { return (int32_t)((x >>
 __device__ __forceinline__ int32_t pdg_dest(uint64_t x) { return (int32_t)((x >> 32) & 0xFFFu) - 1; }
 __device__ __forceinline__ int32_t pdg_gain(uint64_t x) { return (int32_t)(uint32_t)x; }
 
-// part id of neighbour u from the gather copy (read-only in the kernel)
+// part id of neighbour u (uint8 / uint16: read-only in the kernel; the int32
+// partition of the one-block loop changes within its kernel: plain loads)
 template <class PT>
 __device__ __forceinline__ int32_t gpart(const void* pc, int32_t u, int64_t n) {
-    return GP_IN(u, n) ? (int32_t)__ldg((const PT*)pc + u) : 0;
+    if (!GP_IN(u, n)) return 0;
+    if constexpr (sizeof(PT) == 4) return ((const PT*)pc)[u];
+    else return (int32_t)__ldg((const PT*)pc + u);
 }
 
-// rebalance moves keep the gather copy of part current (pcb bytes per id)
+// one part id of a partition stored in pcb bytes per vertex (1, 2 or 4)
 __device__ __forceinline__ void store_pc(void* pc, int pcb, int64_t v, int32_t d) {
-    if (!pc) return;
     if (pcb == 1) ((uint8_t*)pc)[v] = (uint8_t)d;
-    else ((uint16_t*)pc)[v] = (uint16_t)d;
+    else if (pcb == 2) ((uint16_t*)pc)[v] = (uint16_t)d;
+    else ((int32_t*)pc)[v] = d;
+}
+__device__ __forceinline__ int32_t load_pc(const void* pc, int pcb, int64_t v) {
+    return pcb == 1 ? (int32_t)((const uint8_t*)pc)[v]
+                    : (pcb == 2 ? (int32_t)((const uint16_t*)pc)[v] : ((const int32_t*)pc)[v]);
 }
 
 __device__ __forceinline__ void hist_add(int32_t* hist, int32_t q, int32_t w, bool valid, int32_t k) {
@@ -164,31 +153,28 @@ __device__ __forceinline__ void warp_push(bool take, int32_t v, int32_t* list, i
     if (take && GP_IN(idx, cap)) list[idx] = v;
 }
 
-// decision of one row from its best other part (bq, bk), own connectivity
-// and total weighted degree; returns true when an LP candidate is recorded
+// decision of one row from its best other part (bq, bk), its cross weight and
+// its total weighted degree; returns true when an LP candidate is recorded
 template <class PT>
-__device__ __forceinline__ bool conn_decide(const ConnArgs& A, int mode, bool active, int64_t v, int32_t p,
-                                            int64_t tot, int64_t cross, uint64_t bk, int32_t bq, int32_t light) {
-    if (mode == MODE_LP && A.part_next) {
-        A.part_next[v] = p; A.lock_next[v] = 0;
-        if (A.pc_next) ((PT*)A.pc_next)[v] = (PT)p;
-    }
-    const int64_t own = tot - cross;
+__device__ __forceinline__ bool conn_decide(const ConnArgs& A, int mode, bool active, int32_t v, int32_t p,
+                                            int32_t tot, int32_t cross, uint32_t bk, int32_t bq, int32_t light) {
+    const int32_t own = tot - cross;
     int32_t d = -1, gn = 0;
     bool cand = false;
     if (mode == MODE_LP) {
+        if (A.pc_next) { ((PT*)A.pc_next)[v] = (PT)p; A.lock_next[v] = 0; }
         if (active && bq >= 0) {
-            const int64_t gg = (int64_t)bk - own;
-            if (lp_candidate(gg, own, A.den)) { d = bq; gn = (int32_t)gg; cand = true; }
+            const int32_t gg = (int32_t)bk - own;
+            if (lp_candidate(gg, own, A.den)) { d = bq; gn = gg; cand = true; }
         }
+        if (A.pdg) A.pdg[v] = pdg_pack(p, d, gn);
+        if (!A.lp_dg) return cand;
     } else if (mode == MODE_RB && active) {
-        const int64_t cd = bq >= 0 ? (int64_t)bk : 0;
         d = bq >= 0 ? bq : light;
-        gn = -(int32_t)(own - cd);
+        gn = bq >= 0 ? (int32_t)bk - own : -own;
     }
     A.dest[v] = d;
     A.gain[v] = gn;
-    if (mode == MODE_LP && A.pdg) A.pdg[v] = pdg_pack(p, d, gn);
     return cand;
 }
 
@@ -199,12 +185,13 @@ struct ConnRow {
     int32_t v, p;
     bool active;
 };
-__device__ __forceinline__ ConnRow conn_row(const ConnArgs& A, int64_t v, int mode, const uint8_t* over) {
+template <class PT>
+__device__ __forceinline__ ConnRow conn_row(const ConnArgs& A, int32_t v, int mode, const uint8_t* over) {
     ConnRow r;
-    r.v = (int32_t)v; r.beg = 0; r.end = 0; r.p = -1; r.active = false;
+    r.v = v; r.beg = 0; r.end = 0; r.p = -1; r.active = false;
     if (v >= 0) {
         r.beg = A.g.rp[v]; r.end = A.g.rp[v + 1];
-        r.p = A.part[v];
+        r.p = gpart<PT>(A.pc, v, A.g.n);
         r.active = (mode == MODE_LP && !A.lock[v]) || (mode == MODE_RB && over[r.p]);
     }
     return r;
@@ -232,56 +219,142 @@ __device__ __forceinline__ int64_t* conn_list_count(const ConnArgs& A, int b) {
     return &A.status[b == 0 ? S_NL0 : (b == 1 ? S_NL1 : S_NL2)];
 }
 
-// rows of at most TILE entries, TILE lanes per row, 32/TILE rows per warp.
-// Every lane ends with the connectivity of the row to its entry's part; lanes
-// of the same part hold the same value, which the argmax (ties to the smaller
-// part) does not mind.  hist: the warp's k zeroed bins (TILE == 32 only; left
-// zeroed).  Returns true on the row's first lane when the row is an LP
-// candidate (the caller appends it).
-template <int TILE, class PT>
-__device__ __forceinline__ bool conn_tile(const ConnArgs& A, const ConnRow& R, int mode, const uint8_t* over,
-                                          int32_t light, int32_t* hist, int64_t& acc) {
-    const int lane = threadIdx.x & 31, tl = lane & (TILE - 1);
-    const int64_t v = R.v, beg = R.beg, end = R.end;
-    const int32_t p = R.p;
-    const bool active = R.active;
-    const int64_t e = beg + tl;
-    const bool has = v >= 0 && e < end;
+// what one row contributes and its best other part (bk = 0, bq = -1: none);
+// a row's weights add up to less than 2^31
+struct ConnRes {
+    int32_t tot, cross;
+    uint32_t bk;
+    int32_t bq;
+};
+
+// bucket 0 (at most 8 entries): one row per thread.  What bounds these rows is
+// the instruction count, not the loads: a warp's 32 rows are mostly consecutive
+// (the entry loads hit the lines the first of them brought in), all of a row's
+// gathers are in flight together, and the part sums are compares among the
+// thread's own registers, done only where a neighbour lies in another part.
+// Against 8 lanes per row with shuffles, 256^3 grid k = 32, one pass of level
+// 0 (16.8 M rows of 6 entries) @A0@
+template <class PT>
+__device__ __forceinline__ ConnRes conn_thread(const ConnArgs& A, const ConnRow& R, int mode, const uint8_t* over) {
+    ConnRes x{0, 0, 0u, -1};
+    const int len = (int)(R.end - R.beg);
+    const int32_t* __restrict__ row = A.g.ci + R.beg;
+    int32_t q[kTile8], w[kTile8];
+#pragma unroll
+    for (int i = 0; i < kTile8; ++i) q[i] = i < len ? __ldg(row + i) : -1;
+    if (A.g.ew) {
+        const int32_t* __restrict__ wrow = A.g.ew + R.beg;
+#pragma unroll
+        for (int i = 0; i < kTile8; ++i) w[i] = i < len ? __ldg(wrow + i) : 0;
+    } else {
+#pragma unroll
+        for (int i = 0; i < kTile8; ++i) w[i] = i < len ? 1 : 0;
+    }
+#pragma unroll
+    for (int i = 0; i < kTile8; ++i) q[i] = q[i] >= 0 ? gpart<PT>(A.pc, q[i], A.g.n) : -1;
+#pragma unroll
+    for (int i = 0; i < kTile8; ++i) { x.tot += w[i]; x.cross += q[i] != R.p ? w[i] : 0; }
+    if (R.active && x.cross > 0) {
+#pragma unroll
+        for (int i = 0; i < kTile8; ++i) {
+            int32_t h = 0;
+#pragma unroll
+            for (int j = 0; j < kTile8; ++j) h += q[j] == q[i] ? w[j] : 0;
+            if (q[i] >= 0 && q[i] != R.p && (mode != MODE_RB || !over[q[i]])) argmax_u32(x.bk, x.bq, (uint32_t)h, q[i]);
+        }
+    }
+    return x;
+}
+
+// bucket-1 rows of at most 16 entries: 4 lanes per row, 8 rows per warp, 4
+// entries per lane (entry sub + 4 i).  The part sums meet the other lanes'
+// entries by three rounds of shuffles inside the 4 lanes, skipped when no row
+// of the warp has a neighbour in another part; every lane of a row ends with
+// the row's result.  Rows of no vertex (v < 0) or longer than 16 return zeros.
+constexpr int kQuadDeg = 16;
+template <class PT>
+__device__ __forceinline__ ConnRes conn_quad(const ConnArgs& A, const ConnRow& R, int mode, const uint8_t* over) {
+    const int sub = threadIdx.x & 3;
+    const int64_t deg = R.end - R.beg;
+    const int len = deg <= kQuadDeg ? (int)deg : 0;
+    int32_t q[4], w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int e = sub + 4 * i;
+        q[i] = e < len ? __ldcs(&A.g.ci[R.beg + e]) : -1;
+        w[i] = e < len ? (A.g.ew ? __ldcs(&A.g.ew[R.beg + e]) : 1) : 0;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) q[i] = q[i] >= 0 ? gpart<PT>(A.pc, q[i], A.g.n) : -1;
+    ConnRes x{0, 0, 0u, -1};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { x.tot += w[i]; x.cross += q[i] != R.p ? w[i] : 0; }
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+        x.tot += __shfl_xor_sync(0xffffffffu, x.tot, o);
+        x.cross += __shfl_xor_sync(0xffffffffu, x.cross, o);
+    }
+    if (!__any_sync(0xffffffffu, R.active && x.cross > 0)) return x;
+    int32_t h[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        h[i] = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) h[i] += q[j] == q[i] ? w[j] : 0;
+    }
+#pragma unroll
+    for (int o = 1; o < 4; ++o)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int32_t q2 = __shfl_xor_sync(0xffffffffu, q[j], o), w2 = __shfl_xor_sync(0xffffffffu, w[j], o);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) h[i] += q2 == q[i] ? w2 : 0;
+        }
+    if (R.active) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (q[i] >= 0 && q[i] != R.p && (mode != MODE_RB || !over[q[i]])) argmax_u32(x.bk, x.bq, (uint32_t)h[i], q[i]);
+    }
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+        const uint32_t h2 = __shfl_xor_sync(0xffffffffu, x.bk, o);
+        const int32_t q2 = __shfl_xor_sync(0xffffffffu, x.bq, o);
+        argmax_u32(x.bk, x.bq, h2, q2);
+    }
+    return x;
+}
+
+// bucket-1 rows of 17 to 32 entries: one row per warp, one entry per lane; the
+// entries are added into the warp's shared-memory histogram and each lane
+// reads its own part's bin back (lanes of the same part hold the same value,
+// which the argmax, ties to the smaller part, does not mind).  hist: the
+// warp's k zeroed bins, left zeroed.
+template <class PT>
+__device__ __forceinline__ ConnRes conn_lane(const ConnArgs& A, const ConnRow& R, int mode, const uint8_t* over,
+                                             int32_t* hist) {
+    const int lane = threadIdx.x & 31;
+    const int64_t e = R.beg + lane;
+    const bool has = e < R.end;
     int32_t q = -1, w = 0;
     if (has) { q = gpart<PT>(A.pc, __ldcs(&A.g.ci[e]), A.g.n); w = A.g.ew ? __ldcs(&A.g.ew[e]) : 1; }
-    const int32_t cross = (int32_t)tile_sum_u32<TILE>((has && q != p) ? (uint32_t)w : 0u);
-    const int32_t tot = (int32_t)tile_sum_u32<TILE>((uint32_t)w);
-    uint32_t connq = 0;
-    if constexpr (TILE == 32) {
-        if (active) {  // one row per warp: uniform
-            const bool in = has && q != p && GP_IN(q, A.k);   // the own part's bin is not needed
-            if (in) atomicAdd(&hist[q], w);
-            __syncwarp();
-            if (in) connq = (uint32_t)hist[q];
-            __syncwarp();
-            if (in) hist[q] = 0;
-            __syncwarp();
-        }
-    } else {
-        const int32_t qk = has ? q : -1;
-        connq = has ? (uint32_t)w : 0u;
-#pragma unroll
-        for (int d = 1; d < TILE; ++d) {
-            const int src = (lane & ~(TILE - 1)) | ((tl + d) & (TILE - 1));
-            const int32_t q2 = __shfl_sync(0xffffffffu, qk, src);
-            const int32_t w2 = __shfl_sync(0xffffffffu, w, src);
-            if (has && q2 == q) connq += (uint32_t)w2;
-        }
+    const bool in = has && q != R.p && GP_IN(q, A.k);   // the own part's bin is not needed
+    ConnRes x;
+    x.cross = (int32_t)__reduce_add_sync(0xffffffffu, (has && q != R.p) ? (uint32_t)w : 0u);
+    x.tot = (int32_t)__reduce_add_sync(0xffffffffu, (uint32_t)w);
+    x.bk = 0; x.bq = -1;
+    if (R.active && x.cross > 0) {   // one row per warp: uniform
+        uint32_t h = 0;
+        if (in) atomicAdd(&hist[q], w);
+        __syncwarp();
+        if (in) h = (uint32_t)hist[q];
+        __syncwarp();
+        if (in) hist[q] = 0;
+        __syncwarp();
+        uint64_t bk;
+        group_argmax_u32(0xffffffffu, bk, x.bq, (in && (mode != MODE_RB || !over[q])) ? h : 0u, q);
+        x.bk = (uint32_t)bk;
     }
-    uint64_t bk;
-    int32_t bq;
-    tile_argmax_u32<TILE>(bk, bq, (active && has && q != p && (mode != MODE_RB || !over[q])) ? connq : 0u, q);
-    bool take = false;
-    if (tl == 0 && v >= 0) {
-        acc += cross;
-        take = conn_decide<PT>(A, mode, active, v, p, tot, cross, bk, bq, light);
-    }
-    return take;
+    return x;
 }
 
 // bucket 2: one row per warp, shared-memory histogram.  The row is swept
@@ -293,10 +366,10 @@ __device__ __forceinline__ bool conn_tile(const ConnArgs& A, const ConnRow& R, i
 // non-zero connection).
 constexpr int kBinsK = 256;
 template <class PT>
-__device__ __forceinline__ bool conn_warp(const ConnArgs& A, const ConnRow& R, int mode, const uint8_t* over,
-                                          int32_t light, int32_t* hist, int64_t& acc) {
+__device__ __forceinline__ ConnRes conn_warp(const ConnArgs& A, const ConnRow& R, int mode, const uint8_t* over,
+                                             int32_t* hist) {
     const int lane = threadIdx.x & 31;
-    const int64_t v = R.v, beg = R.beg, end = R.end;
+    const int64_t beg = R.beg, end = R.end;
     const int32_t p = R.p;
     const bool active = R.active;
     int32_t cross = 0, tot = 0;
@@ -351,18 +424,70 @@ __device__ __forceinline__ bool conn_warp(const ConnArgs& A, const ConnRow& R, i
         }
         __syncwarp();
     }
-    bool take = false;
-    if (lane == 0) {
-        acc += cross;
-        take = conn_decide<PT>(A, mode, active, v, p, tot, cross, bk, bq, light);
-    }
-    return take;
+    return ConnRes{tot, cross, (uint32_t)bk, bq};
 }
 
-// append a row decided by conn_tile / conn_warp to list b at once
-__device__ __forceinline__ void conn_push_now(const ConnArgs& A, bool take, const ConnRow& R, int b) {
-    if (take) atomicAdd((unsigned long long*)&A.status[S_CDEG], (unsigned long long)(R.end - R.beg));
-    warp_push(take, R.v, A.clist[b], conn_list_count(A, b), A.g.n);
+// Up to 8 light units [ub, ub + nu) by one warp (unit order: bucket 2 rows,
+// bucket 1 rows, groups of 4 bucket-0 rows).  Lane l first fetches row slot l
+// (unit l / 4; its row, or the (l % 4)-th row of a group of 4), so the list and
+// row-header loads of 8 units are in flight together; the rows' results land
+// in the lane of their slot, and the decisions of all of them are taken and
+// stored together (a warp's stores of consecutive rows coalesce), their
+// candidates appended together (one atomic per list present).  rows: the
+// warp's 32 slots in shared memory.
+template <class PT>
+__device__ __forceinline__ void conn_group(const ConnArgs& A, int64_t ub, int nu, int mode, const uint8_t* over,
+                                           int32_t light, int32_t* hist, ConnRowS* rows, int64_t& acc, int64_t& cdeg) {
+    const int lane = threadIdx.x & 31;
+    const int64_t U2 = A.nbucket[2], U21 = U2 + A.nbucket[1];
+    const int64_t u = ub + (lane >> 2);
+    const int sub = lane & 3;
+    const int lb = u < U2 ? 2 : (u < U21 ? 1 : 0);
+    int32_t v = -1;
+    if (u < ub + nu) {
+        if (lb == 2) { if (sub == 0) v = A.bucket[2][u]; }
+        else if (lb == 1) { if (sub == 0) v = A.bucket[1][u - U2]; }
+        else {
+            const int64_t i = (u - U21) * 4 + sub;
+            if (i < A.nbucket[0]) v = A.bucket[0][i];
+        }
+    }
+    const ConnRow r = conn_row<PT>(A, v, mode, over);
+    ConnRes x{0, 0, 0u, -1};
+    if (lb == 0) x = conn_thread<PT>(A, r, mode, over);
+    if (ub < U21) {   // warp or quad rows among the units
+        rows[lane] = conn_stage(r);
+        __syncwarp();
+        const int nlong = U21 - ub < nu ? (int)(U21 - ub) : nu;
+        uint32_t todo = 0;   // row slots left to whole warps
+        if (ub + nu > U2) {
+            ConnRow qr = conn_unstage(rows[lane & ~3]);
+            const bool quad = lb == 1 && qr.v >= 0 && qr.end - qr.beg <= kQuadDeg;
+            if (!quad) { qr.end = qr.beg; qr.active = false; }
+            const ConnRes y = conn_quad<PT>(A, qr, mode, over);
+            if (quad && sub == 0) x = y;
+            todo = __ballot_sync(0xffffffffu, lb == 1 && r.v >= 0 && !quad && sub == 0);
+        }
+        for (int j = 0; j < nlong; ++j) {
+            if (ub + j < U2) {
+                const ConnRes y = conn_warp<PT>(A, conn_unstage(rows[4 * j]), mode, over, hist);
+                if (lane == 4 * j) x = y;
+            } else if ((todo >> (4 * j)) & 1u) {
+                const ConnRes y = conn_lane<PT>(A, conn_unstage(rows[4 * j]), mode, over, hist);
+                if (lane == 4 * j) x = y;
+            }
+        }
+        __syncwarp();
+    }
+    bool take = false;
+    if (r.v >= 0) {
+        acc += x.cross;
+        take = conn_decide<PT>(A, mode, r.active, r.v, r.p, x.tot, x.cross, x.bk, x.bq, light);
+        if (take) cdeg += r.end - r.beg;
+    }
+    if (A.clist[0] == nullptr || !__any_sync(0xffffffffu, take)) return;
+#pragma unroll
+    for (int b = 0; b < 3; ++b) warp_push(take && lb == b, r.v, A.clist[b], conn_list_count(A, b), A.g.n);
 }
 
 template <class PT>
@@ -417,7 +542,7 @@ __global__ void __launch_bounds__(RT, 5) k_conn(ConnArgs A) {
         const int32_t h = A.item_row[blockIdx.x];
         const int64_t v = A.heavy[h];
         const int nit = A.row_items[h];
-        const int32_t p = A.part[v];
+        const int32_t p = gpart<PT>(A.pc, (int32_t)v, A.g.n);
         const bool active = (mode == MODE_LP && !A.lock[v]) || (mode == MODE_RB && over[p]);
         const int64_t beg = A.item_beg[blockIdx.x], end = A.item_end[blockIdx.x];
         int64_t cross = 0, tot = 0;
@@ -492,7 +617,7 @@ __global__ void __launch_bounds__(RT, 5) k_conn(ConnArgs A) {
             if (threadIdx.x == 0) {
                 for (int i = 1; i < RW; ++i) argmax_q(bk, bq, s_k[i], s_q[i]);
                 const int64_t rdeg = A.g.rp[v + 1] - A.g.rp[v];
-                if (conn_decide<PT>(A, mode, active, v, p, tot, cross, bk, bq, light))
+                if (conn_decide<PT>(A, mode, active, (int32_t)v, p, (int32_t)tot, (int32_t)cross, (uint32_t)bk, bq, light))
                     atomicAdd((unsigned long long*)&A.status[S_CDEG], (unsigned long long)rdeg);
             }
         }
@@ -500,58 +625,11 @@ __global__ void __launch_bounds__(RT, 5) k_conn(ConnArgs A) {
         int32_t* hist = hist_all + w * k;
         ConnRowS* rows = s_rows + w * 32;
         const int64_t wid = ((int64_t)(blockIdx.x - A.nitems) * RT + threadIdx.x) >> 5;
-        const int64_t U2 = A.nbucket[2], U1 = A.nbucket[1];
-        // contiguous units of equal total cost (k_warp_bounds), taken 8 at a
-        // time: lane l first fetches row slot l (unit l / 4; its row, or the
-        // (l % 4)-th row of a group of 4), so the list and row-header loads of
-        // 8 units are in flight together; the candidates of the 8 units are
-        // appended together afterwards (one atomic per list present)
+        // contiguous units of equal total cost (k_warp_bounds), taken 8 at a time
         const int64_t u0 = A.wfirst[wid], u1 = A.wfirst[wid + 1];
         int64_t cdeg = 0;   // degree sum of this lane's candidates
-        for (int64_t ub = u0; ub < u1; ub += 8) {
-            const int nu = (int)(u1 - ub < 8 ? u1 - ub : 8);
-            {
-                const int64_t u = ub + (lane >> 2);
-                const int sub = lane & 3;
-                int64_t v = -1;
-                if (u < ub + nu) {
-                    if (u < U2) { if (sub == 0) v = A.bucket[2][u]; }
-                    else if (u < U2 + U1) { if (sub == 0) v = A.bucket[1][u - U2]; }
-                    else {
-                        const int64_t i = (u - U2 - U1) * 4 + sub;
-                        if (i < A.nbucket[0]) v = A.bucket[0][i];
-                    }
-                }
-                rows[lane] = conn_stage(conn_row(A, v, mode, over));
-            }
-            __syncwarp();
-            uint32_t takes = 0;   // bit s: row slot s is a candidate
-            for (int j = 0; j < nu; ++j) {
-                const int64_t u = ub + j;
-                if (u < U2) {
-                    const bool t = conn_warp<PT>(A, conn_unstage(rows[4 * j]), mode, over, light, hist, acc);
-                    takes |= (__ballot_sync(0xffffffffu, t) & 1u) << (4 * j);
-                } else if (u < U2 + U1) {
-                    const bool t = conn_tile<kTile32, PT>(A, conn_unstage(rows[4 * j]), mode, over, light, hist, acc);
-                    takes |= (__ballot_sync(0xffffffffu, t) & 1u) << (4 * j);
-                } else {
-                    const bool t = conn_tile<kTile8, PT>(A, conn_unstage(rows[4 * j + (lane >> 3)]), mode, over, light,
-                                                         hist, acc);
-                    const uint32_t b = __ballot_sync(0xffffffffu, t);   // lanes 0, 8, 16, 24
-                    takes |= ((b & 1u) | ((b >> 7) & 2u) | ((b >> 14) & 4u) | ((b >> 21) & 8u)) << (4 * j);
-                }
-            }
-            {
-                const bool t = (takes >> lane) & 1u;
-                const ConnRowS rs = rows[lane];
-                const int64_t u = ub + (lane >> 2);
-                const int lb = u < U2 ? 2 : (u < U2 + U1 ? 1 : 0);
-                if (t) cdeg += rs.end - rs.beg;
-#pragma unroll
-                for (int b = 0; b < 3; ++b) warp_push(t && lb == b, rs.v, A.clist[b], conn_list_count(A, b), A.g.n);
-            }
-            __syncwarp();
-        }
+        for (int64_t ub = u0; ub < u1; ub += 8)
+            conn_group<PT>(A, ub, (int)(u1 - ub < 8 ? u1 - ub : 8), mode, over, light, hist, rows, acc, cdeg);
         cdeg = warp_sum(cdeg);
         if (lane == 0 && cdeg) atomicAdd((unsigned long long*)&A.status[S_CDEG], (unsigned long long)cdeg);
     }
@@ -590,7 +668,6 @@ __device__ __forceinline__ int32_t ab_term(const DGraph& g, int64_t e, int64_t v
 struct ApplyArgs {
     DGraph g;
     int32_t k;
-    const int32_t* part;
     const int32_t* dest;
     const int32_t* gain;
     const int32_t* heavy;
@@ -601,10 +678,9 @@ struct ApplyArgs {
     int64_t nitems;
     const int32_t* clist[3];
     const int64_t* status;
-    int32_t* part_next;
     uint8_t* lock_next;
-    const void* pc;             // gather copy of part (as in ConnArgs)
-    void* pc_next;              // its copy of part_next (nullptr: none kept)
+    const void* pc;             // the partition (as in ConnArgs)
+    void* pc_next;              // the partition after the step
     int64_t* pw;
     int64_t* moves_out;
     int64_t* hsum;
@@ -616,13 +692,23 @@ template <class PT>
 __device__ __forceinline__ void ab_commit(const ApplyArgs& A, int64_t v, int32_t p, int32_t d, int64_t* delta,
                                           int64_t& moves) {
     if (!GP_IN(d, A.k) || !GP_IN(p, A.k)) return;
-    A.part_next[v] = d;
-    if (A.pc_next) ((PT*)A.pc_next)[v] = (PT)d;
+    ((PT*)A.pc_next)[v] = (PT)d;
     A.lock_next[v] = 1;
     const int64_t wv = A.g.vw ? A.g.vw[v] : 1;
     atomicAdd((unsigned long long*)&delta[d], (unsigned long long)wv);
     atomicAdd((unsigned long long*)&delta[p], (unsigned long long)(-wv));
     ++moves;
+}
+
+// part, destination (-1: no candidate) and gain of row v
+template <class PT>
+__device__ __forceinline__ void ab_row(const ApplyArgs& A, int64_t v, int32_t& p, int32_t& d, int32_t& gv) {
+    if (A.pdg) {
+        const uint64_t x = A.pdg[v];
+        p = pdg_part(x); d = pdg_dest(x); gv = pdg_gain(x);
+    } else {
+        p = gpart<PT>(A.pc, (int32_t)v, A.g.n); d = A.dest[v]; gv = A.gain[v];
+    }
 }
 
 // candidate rows of at most TILE entries, TILE lanes each
@@ -631,8 +717,8 @@ __device__ __forceinline__ void ab_tile(const ApplyArgs& A, int64_t v, int64_t* 
     const int lane = threadIdx.x & 31, tl = lane & (TILE - 1);
     int32_t t = 0, p = -1, d = -1;
     if (v >= 0) {
-        d = A.dest[v]; p = A.part[v];
-        const int32_t gv = A.gain[v];
+        int32_t gv;
+        ab_row<PT>(A, v, p, d, gv);
         const int64_t e = A.g.rp[v] + tl;
         if (e < A.g.rp[v + 1]) t = ab_term<PT>(A.g, e, v, p, d, gv, A.pc, A.dest, A.gain, A.pdg);
     }
@@ -691,7 +777,8 @@ __device__ __forceinline__ int32_t ab_sum(const ApplyArgs& A, int64_t beg, int64
 template <class PT>
 __device__ __forceinline__ void ab_warp(const ApplyArgs& A, int64_t v, int64_t* delta, int64_t& moves) {
     const int lane = threadIdx.x & 31;
-    const int32_t d = A.dest[v], p = A.part[v], gv = A.gain[v];
+    int32_t p, d, gv;
+    ab_row<PT>(A, v, p, d, gv);
     const int32_t g2 = warp_sum(ab_sum<PT>(A, A.g.rp[v], A.g.rp[v + 1], lane, 32, v, p, d, gv));
     if (lane == 0 && g2 >= 0) ab_commit<PT>(A, v, p, d, delta, moves);
 }
@@ -707,10 +794,10 @@ __global__ void __launch_bounds__(RT) k_lp_apply(ApplyArgs A) {
     if ((int64_t)blockIdx.x < A.nitems) {
         const int32_t h = A.item_row[blockIdx.x];
         const int64_t v = A.heavy[h];
-        const int32_t d = A.dest[v];
+        int32_t p, d, gv;
+        ab_row<PT>(A, v, p, d, gv);
         if (d >= 0) {
             const int nit = A.row_items[h];
-            const int32_t p = A.part[v], gv = A.gain[v];
             int32_t g2 = ab_sum<PT>(A, A.item_beg[blockIdx.x], A.item_end[blockIdx.x], threadIdx.x, RT, v, p, d, gv);
             g2 = warp_sum(g2);
             if (lane == 0) s_red[w] = g2;
@@ -772,12 +859,12 @@ __global__ void k_rb_flags(int64_t n, const int32_t* __restrict__ dest, int32_t*
 
 // candidates in vertex order with key (source << 10 | bucket(loss))
 __global__ void k_rb_compact(int64_t n, const int32_t* __restrict__ flag, const int64_t* __restrict__ pos,
-                             const int32_t* __restrict__ part, const int32_t* __restrict__ gain,
+                             const void* __restrict__ pc, int pcb, const int32_t* __restrict__ gain,
                              uint64_t* __restrict__ keys, int32_t* __restrict__ vals) {
     for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
         if (!flag[v]) continue;
         const int64_t i = pos[v];
-        keys[i] = ((uint64_t)(uint32_t)part[v] << RB_SHIFT) | loss_bucket(-gain[v]);
+        keys[i] = ((uint64_t)(uint32_t)load_pc(pc, pcb, v) << RB_SHIFT) | loss_bucket(-gain[v]);
         vals[i] = (int32_t)v;
     }
 }
@@ -841,7 +928,7 @@ __device__ __forceinline__ void rb_delta_end(int64_t* delta, int32_t k, int64_t 
 __global__ void k_rb_weak_apply(int64_t cnt, const uint64_t* __restrict__ keys, const int64_t* __restrict__ segf,
                                 const int32_t* __restrict__ vals, const int64_t* __restrict__ pre,
                                 const int32_t* __restrict__ vw, const int64_t* __restrict__ pw_snap, int64_t Lmax,
-                                int32_t k, int32_t* __restrict__ part, void* pc, int pcb, uint8_t* __restrict__ lock,
+                                int32_t k, void* __restrict__ pc, int pcb, uint8_t* __restrict__ lock,
                                 int64_t* __restrict__ pw, int64_t* __restrict__ moves) {
     extern __shared__ int64_t rb_delta[];
     rb_delta_begin(rb_delta, k);
@@ -852,9 +939,9 @@ __global__ void k_rb_weak_apply(int64_t cnt, const uint64_t* __restrict__ keys, 
         const int32_t v = vals[i];
         const int64_t wv = vw ? vw[v] : 1;
         if ((pre[i] - pre[s]) + wv <= Lmax - pw_snap[d]) {
-            const int32_t p = part[v];
-            part[v] = (int32_t)d; lock[v] = 1;
+            const int32_t p = load_pc(pc, pcb, v);
             store_pc(pc, pcb, v, (int32_t)d);
+            lock[v] = 1;
             if (GP_IN(d, k) && GP_IN(p, k)) {
                 atomicAdd((unsigned long long*)&rb_delta[d], (unsigned long long)wv);
                 atomicAdd((unsigned long long*)&rb_delta[p], (unsigned long long)(-wv));
@@ -885,8 +972,8 @@ __global__ void k_mask_vw(int64_t cnt, const int32_t* __restrict__ flag, const i
 
 __global__ void k_rb_strong_apply(int64_t cnt, const int32_t* __restrict__ vals, const int32_t* __restrict__ flag,
                                   const int64_t* __restrict__ P, const int32_t* __restrict__ vw,
-                                  const int64_t* __restrict__ cum, int32_t k, int32_t* __restrict__ part,
-                                  void* pc, int pcb, uint8_t* __restrict__ lock, int64_t* __restrict__ pw,
+                                  const int64_t* __restrict__ cum, int32_t k, void* __restrict__ pc, int pcb,
+                                  uint8_t* __restrict__ lock, int64_t* __restrict__ pw,
                                   int64_t* __restrict__ moves) {
     extern __shared__ int64_t rb_delta[];
     rb_delta_begin(rb_delta, k);
@@ -905,9 +992,9 @@ __global__ void k_rb_strong_apply(int64_t cnt, const int32_t* __restrict__ vals,
         const int32_t v = vals[i];
         const int64_t wv = vw ? vw[v] : 1;
         if (q < k && pre + wv <= cum[q + 1]) {
-            const int32_t p = part[v];
-            part[v] = q; lock[v] = 1;
+            const int32_t p = load_pc(pc, pcb, v);
             store_pc(pc, pcb, v, q);
+            lock[v] = 1;
             if (GP_IN(p, k)) {
                 atomicAdd((unsigned long long*)&rb_delta[q], (unsigned long long)wv);
                 atomicAdd((unsigned long long*)&rb_delta[p], (unsigned long long)(-wv));
@@ -1146,8 +1233,7 @@ __device__ __forceinline__ int cta_seg_start(const uint64_t* a, int i, int shift
 // thread's move count.  Needs ncand <= kCtaMaxN.
 struct RbCta {
     const int32_t* vw;
-    int32_t* part;
-    void* pc;                   // gather copy of part to keep current (nullptr: none)
+    void* pc;                   // the partition
     int pcb;                    // its bytes per id
     uint8_t* lock;
     const int32_t* dest;
@@ -1163,14 +1249,13 @@ __device__ int64_t cta_rebalance(const RbCta& R, int mode, int64_t n, const int3
                                  int64_t* s_pw, int64_t* s_snap, int64_t* s_cum, uint64_t* s_keys, int64_t* sh) {
     const int32_t k = R.k;
     const int64_t Lmax = R.Lmax;
-    int32_t* part = R.part;
     uint8_t* lock = R.lock;
     int64_t moves = 0;
     for (int q = threadIdx.x; q < k; q += CT) s_snap[q] = s_pw[q];
     __syncthreads();
     int64_t ncand = ncand_in;
     auto key1 = [&](uint32_t v) -> uint64_t {
-        const uint64_t key = ((uint64_t)(uint32_t)part[v] << RB_SHIFT) | loss_bucket(-R.gain[v]);
+        const uint64_t key = ((uint64_t)(uint32_t)load_pc(R.pc, R.pcb, v) << RB_SHIFT) | loss_bucket(-R.gain[v]);
         return (key << 32) | v;
     };
     if (cand == nullptr) {
@@ -1218,9 +1303,9 @@ __device__ int64_t cta_rebalance(const RbCta& R, int mode, int64_t n, const int3
             const int s0 = cta_seg_start(s_keys, (int)i, 32 + 2 * RB_SHIFT);
             const int64_t wv = vwt(v);
             if ((R.pre[i] - R.pre[s0]) + wv <= Lmax - s_snap[d]) {
-                const int32_t p = part[v];
-                part[v] = d; lock[v] = 1;
+                const int32_t p = load_pc(R.pc, R.pcb, v);
                 store_pc(R.pc, R.pcb, v, d);
+                lock[v] = 1;
                 atomicAdd((unsigned long long*)&s_pw[d], (unsigned long long)wv);
                 atomicAdd((unsigned long long*)&s_pw[p], (unsigned long long)(-wv));
                 ++moves;
@@ -1249,9 +1334,9 @@ __device__ int64_t cta_rebalance(const RbCta& R, int mode, int64_t n, const int3
             const uint32_t v = (uint32_t)s_keys[i];
             const int64_t wv = vwt(v);
             if (lo < k && pre + wv <= s_cum[lo + 1]) {
-                const int32_t p = part[v];
-                part[v] = lo; lock[v] = 1;
+                const int32_t p = load_pc(R.pc, R.pcb, v);
                 store_pc(R.pc, R.pcb, v, lo);
+                lock[v] = 1;
                 atomicAdd((unsigned long long*)&s_pw[lo], (unsigned long long)wv);
                 atomicAdd((unsigned long long*)&s_pw[p], (unsigned long long)(-wv));
                 ++moves;
@@ -1300,6 +1385,7 @@ __device__ void cta_refine_level(const CtaRefineArgs& R, unsigned char* rsm) {
     __shared__ uint64_t s_lk[CW];
     __shared__ int32_t s_lq[CW];
     __shared__ int64_t s_mx[CW];
+    __shared__ ConnRowS s_rows[CT];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     int32_t* part = R.part;
     int32_t* part_next = R.part_next;
@@ -1335,29 +1421,19 @@ __device__ void cta_refine_level(const CtaRefineArgs& R, unsigned char* rsm) {
         // ---- connectivity pass
         ConnArgs CA;
         CA.g = R.g; CA.k = k; CA.Lmax = Lmax; CA.den = R.den; CA.force_eval = final_eval ? 1 : 0;
-        CA.part = part; CA.lock = lock; CA.pw = s_pw; CA.heavy = nullptr; CA.item_row = nullptr;
+        CA.lock = lock; CA.pw = s_pw; CA.heavy = nullptr; CA.item_row = nullptr;
         CA.item_beg = nullptr; CA.item_end = nullptr; CA.row_items = nullptr; CA.nitems = 0;
-        for (int b = 0; b < 3; ++b) { CA.bucket[b] = R.bucket[b]; CA.nbucket[b] = R.nbucket[b]; CA.clist[b] = R.clist[b]; }
+        for (int b = 0; b < 3; ++b) { CA.bucket[b] = R.bucket[b]; CA.nbucket[b] = R.nbucket[b]; CA.clist[b] = nullptr; }
         CA.wfirst = nullptr;
         CA.dest = R.dest; CA.gain = R.gain; CA.status = R.status;
-        CA.part_next = nullptr; CA.lock_next = nullptr;
-        CA.pc = part; CA.pc_next = nullptr; CA.pdg = nullptr;
+        CA.lock_next = nullptr;
+        CA.pc = part; CA.pc_next = nullptr; CA.pdg = nullptr; CA.lp_dg = 1;
         CA.hhist = nullptr; CA.hsum = nullptr; CA.hdone = nullptr;
-        int64_t acc = 0;
+        int64_t acc = 0, cdeg = 0;
         int32_t* hist = s_hist + w * k;
-        for (int64_t u = w; u < U2 + U1 + U0; u += CW) {
-            if (u < U2) {
-                const ConnRow r = conn_row(CA, R.bucket[2][u], dmode, s_over);
-                conn_push_now(CA, conn_warp<int32_t>(CA, r, dmode, s_over, light, hist, acc), r, 2);
-            } else if (u < U2 + U1) {
-                const ConnRow r = conn_row(CA, R.bucket[1][u - U2], dmode, s_over);
-                conn_push_now(CA, conn_tile<kTile32, int32_t>(CA, r, dmode, s_over, light, hist, acc), r, 1);
-            } else {
-                const int64_t i = (u - U2 - U1) * 4 + (lane >> 3);
-                const ConnRow r = conn_row(CA, i < R.nbucket[0] ? R.bucket[0][i] : -1, dmode, s_over);
-                conn_push_now(CA, conn_tile<kTile8, int32_t>(CA, r, dmode, s_over, light, hist, acc), r, 0);
-            }
-        }
+        for (int64_t ub = 8 * w; ub < U2 + U1 + U0; ub += 8 * CW)
+            conn_group<int32_t>(CA, ub, (int)(U2 + U1 + U0 - ub < 8 ? U2 + U1 + U0 - ub : 8), dmode, s_over, light, hist,
+                                s_rows + 32 * w, acc, cdeg);
         acc = warp_sum(acc);
         const int64_t cur_cut = cta_sum(lane == 0 ? acc : 0, sh) / 2;   // also orders the pass
         const int64_t cur_mp = maxpw;
@@ -1397,11 +1473,11 @@ __device__ void cta_refine_level(const CtaRefineArgs& R, unsigned char* rsm) {
             for (int64_t v = threadIdx.x; v < n; v += CT) { part_next[v] = part[v]; lock_next[v] = 0; }
             __syncthreads();
             ApplyArgs AA;
-            AA.g = R.g; AA.k = k; AA.part = part; AA.dest = R.dest; AA.gain = R.gain; AA.heavy = nullptr;
+            AA.g = R.g; AA.k = k; AA.dest = R.dest; AA.gain = R.gain; AA.heavy = nullptr;
             AA.item_row = nullptr; AA.item_beg = nullptr; AA.item_end = nullptr; AA.row_items = nullptr; AA.nitems = 0;
             for (int b = 0; b < 3; ++b) AA.clist[b] = R.clist[b];
-            AA.status = R.status; AA.part_next = part_next; AA.lock_next = lock_next; AA.pw = nullptr;
-            AA.pc = part; AA.pc_next = nullptr;
+            AA.status = R.status; AA.lock_next = lock_next; AA.pw = nullptr;
+            AA.pc = part; AA.pc_next = part_next;
             AA.moves_out = nullptr; AA.hsum = nullptr; AA.hdone = nullptr; AA.pdg = nullptr;
             for (int64_t u = w; u < U2 + U1 + U0; u += CW) {
                 if (u < U2) {
@@ -1423,7 +1499,7 @@ __device__ void cta_refine_level(const CtaRefineArgs& R, unsigned char* rsm) {
             for (int64_t v = threadIdx.x; v < n; v += CT) lock[v] = 0;
             __syncthreads();
             RbCta RA;
-            RA.vw = R.g.vw; RA.part = part; RA.pc = nullptr; RA.pcb = 0; RA.lock = lock; RA.dest = R.dest;
+            RA.vw = R.g.vw; RA.pc = part; RA.pcb = 4; RA.lock = lock; RA.dest = R.dest;
             RA.gain = R.gain; RA.pre = R.pre;
             RA.flag = R.flag; RA.gkeys = R.gkeys; RA.k = k; RA.Lmax = Lmax;
             moves = cta_rebalance(RA, mode, n, nullptr, 0, s_pw, s_snap, s_cum, s_keys, sh);
@@ -1662,9 +1738,22 @@ static int bits_for(int64_t x) {
     return b;
 }
 
+// the partition in 1 or 2 bytes per vertex, as a level's refinement holds it
+// (B.part is int32 between levels), and back
+__global__ void k_compact_part(int64_t n, const int32_t* __restrict__ part, void* pc, int pcb) {
+    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x)
+        store_pc(pc, pcb, v, part[v]);
+}
+__global__ void k_expand_part(int64_t n, const void* __restrict__ pc, int pcb, int32_t* __restrict__ part) {
+    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x)
+        part[v] = load_pc(pc, pcb, v);
+}
+
 static void trace_iter(Ctx& c, const RefineBufs& B, int64_t n, int64_t m, int level, int it, int mode,
                        int64_t cut_before, int64_t mp_before, const Tracer& tr) {
     std::vector<int32_t> d(n), gn(n), p(n);
+    k_expand_part<<<grid_for(n, 256), 256, 0, c.s>>>(n, B.pc, B.pcb, B.part);
+    GP_LAUNCHED(c);
     GP_CUDA(cudaMemcpyAsync(d.data(), B.dest, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, c.s));
     GP_CUDA(cudaMemcpyAsync(gn.data(), B.gain, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, c.s));
     GP_CUDA(cudaMemcpyAsync(p.data(), B.part, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, c.s));
@@ -1678,12 +1767,7 @@ static void trace_iter(Ctx& c, const RefineBufs& B, int64_t n, int64_t m, int le
     tr.emit(ev);
 }
 
-// the part array as the neighbour gathers read it: 1 or 2 bytes per vertex
-__global__ void k_compact_part(int64_t n, const int32_t* __restrict__ part, void* pc, int pcb) {
-    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x)
-        store_pc(pc, pcb, v, part[v]);
-}
-
+constexpr int64_t kConnWarpCost = 8 * (32 + 24);
 int64_t conn_max_warps(const Ctx& c) { return (int64_t)c.sm_count * c.ctas_per_sm * RW; }
 
 // light warp t of a connectivity pass over nw warps takes the units
@@ -1710,9 +1794,9 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
     const int32_t k = P.k;
     const int64_t Lmax = P.Lmax;
     memset_async(c, B.lock, 0, n);
-    // neighbour gathers read a uint8 (k <= 256) or uint16 copy of part, kept
-    // current by every step that moves vertices: a quarter or half of the
-    // bytes per gather, and of the array that has to stay in L2
+    // the level's partition is held in uint8 (k <= 256) or uint16: a quarter or
+    // half of the bytes per gather, of the array that has to stay in L2, and of
+    // every copy of it
     B.pcb = k <= 256 ? 1 : 2;
     k_compact_part<<<grid_for(n, 256), 256, 0, c.s>>>(n, B.part, B.pc, B.pcb);
     GP_LAUNCHED(c);
@@ -1720,7 +1804,12 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
     const int kpad = (k + 15) & ~15;
     const size_t conn_smem = kpad + sizeof(int32_t) * RW * k;
     // at most 1024 + 32 * GP_MAX_K bytes: below the 48 KB default, no attribute needed
-    const int light_blocks = (int)std::min<int64_t>(grid_for(n * 32, RT, c.sm_count * c.ctas_per_sm),
+    // a light warp's range costs as much as a group of 8 short units (entries
+    // + 32 each), so that its lanes have rows to work on; on levels too small
+    // for 16 such warps per SM latency counts and units are spread thinner
+    const int64_t light_warps = std::min<int64_t>(
+        L.nunits, std::max<int64_t>((g.m + 32 * L.nunits) / kConnWarpCost, (int64_t)c.sm_count * 16));
+    const int light_blocks = (int)std::min<int64_t>(grid_for(light_warps, RW, c.sm_count * c.ctas_per_sm),
                                                     (B.wfirst_cap - 1) / RW);
     const int grid = (int)L.nitems + light_blocks;
     {
@@ -1732,26 +1821,30 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
     int stall = 0, rb_streak = 0, steps = 0, last_mode = 0;
     int64_t prev_moves = -1;
     const int nb_k = bits_for(k);
+    const bool move_head = B.mp && P.gnn && gnn_has_move_head(P.gnn);
+    // with pdg, proposals and gains of a label-propagation pass are stored apart
+    // only for the move head and the trace
+    const int lp_dg = (!B.pdg || move_head || tr.on()) ? 1 : 0;
     for (int it = 0;; ++it) {
         const bool final_eval = (it == P.o.refine_max_iters);
         GP_CUDA(cudaMemsetAsync(B.status, 0, sizeof(int64_t) * S_NRESET, c.s));
         if (c.profile) GP_CUDA(cudaEventRecord(c.ev_a, c.s));
         ConnArgs CA;
         CA.g = g; CA.k = k; CA.Lmax = Lmax; CA.den = P.o.lp_filter_den; CA.force_eval = final_eval ? 1 : 0;
-        CA.part = B.part; CA.lock = B.lock; CA.pw = B.pw; CA.heavy = L.heavy;
+        CA.lock = B.lock; CA.pw = B.pw; CA.heavy = L.heavy;
         CA.item_row = L.item_row; CA.item_beg = L.item_beg; CA.item_end = L.item_end; CA.row_items = L.row_items;
         CA.nitems = L.nitems; CA.hhist = B.hhist; CA.hsum = B.hsum; CA.hdone = B.hdone;
         for (int b = 0; b < 3; ++b) { CA.bucket[b] = L.bucket[b]; CA.nbucket[b] = L.nbucket[b]; CA.clist[b] = B.clist[b]; }
         CA.wfirst = B.wfirst;
         CA.dest = B.dest; CA.gain = B.gain; CA.status = B.status;
-        CA.part_next = B.part_next; CA.lock_next = B.lock_next;   // the LP step's starting copy
-        CA.pc = B.pc; CA.pc_next = B.pc_next; CA.pdg = B.pdg;
+        CA.pc = B.pc; CA.pc_next = B.pc_next; CA.lock_next = B.lock_next;   // the LP step's starting copy
+        CA.pdg = B.pdg; CA.lp_dg = lp_dg;
         if (B.pcb == 1) k_conn<uint8_t><<<grid, RT, conn_smem, c.s>>>(CA);
         else k_conn<uint16_t><<<grid, RT, conn_smem, c.s>>>(CA);
         GP_LAUNCHED(c);
         if (c.profile) GP_CUDA(cudaEventRecord(c.ev_b, c.s));
-        // rowptr, colidx, weights, gathered part[u] (pcb bytes); part[v], lock[v] read; dest, gain written
-        const int64_t conn_bytes = L.scan_bytes() - (4 - B.pcb) * g.m + 4 * n + n + 8 * n;
+        // rowptr, colidx, weights, gathered part[u] (pcb bytes); part[v], lock[v] read; proposal and gain written
+        const int64_t conn_bytes = L.scan_bytes() - (4 - B.pcb) * g.m + B.pcb * n + n + 8 * n;
         c.bytes += conn_bytes;
         GP_CUDA(cudaMemcpyAsync(c.h_pinned, B.status, sizeof(int64_t) * S_NSLOTS, cudaMemcpyDeviceToHost, c.s));
         c.sync();
@@ -1769,7 +1862,7 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
         const int64_t cdeg = c.h_pinned[S_CDEG];
         if (it == 0) {
             best_cut = cur_cut; best_mp = cur_mp;
-            GP_CUDA(cudaMemcpyAsync(B.best, B.part, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, c.s));
+            GP_CUDA(cudaMemcpyAsync(B.best, B.pc, (size_t)B.pcb * n, cudaMemcpyDeviceToDevice, c.s));
             GP_CUDA(cudaMemcpyAsync(B.best_pw, B.pw, sizeof(int64_t) * k, cudaMemcpyDeviceToDevice, c.s));
         } else {
             const int64_t nmoves = c.h_pinned[S_STEP_MOVES];
@@ -1780,7 +1873,7 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
             else if (!cb && !bb) { better = cur_mp < best_mp || (cur_mp == best_mp && cur_cut < best_cut); signif = cur_mp < best_mp; }
             if (better) {
                 best_cut = cur_cut; best_mp = cur_mp;
-                GP_CUDA(cudaMemcpyAsync(B.best, B.part, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, c.s));
+                GP_CUDA(cudaMemcpyAsync(B.best, B.pc, (size_t)B.pcb * n, cudaMemcpyDeviceToDevice, c.s));
                 GP_CUDA(cudaMemcpyAsync(B.best_pw, B.pw, sizeof(int64_t) * k, cudaMemcpyDeviceToDevice, c.s));
             }
             stall = signif ? 0 : stall + 1;
@@ -1801,16 +1894,16 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
         int64_t* moves_d = B.status + S_STEP_MOVES;  // moves of this step, read at the next sync
         memset_async(c, moves_d, 0, sizeof(int64_t));
         if (mode == 0) {
-            // part_next / lock_next were filled by the connectivity pass
+            // pc_next / lock_next were filled by the connectivity pass
             ApplyArgs AA;
-            AA.g = g; AA.k = k; AA.part = B.part; AA.dest = B.dest; AA.gain = B.gain; AA.heavy = L.heavy;
+            AA.g = g; AA.k = k; AA.dest = B.dest; AA.gain = B.gain; AA.heavy = L.heavy;
             AA.item_row = L.item_row; AA.item_beg = L.item_beg; AA.item_end = L.item_end; AA.row_items = L.row_items;
             AA.nitems = L.nitems; AA.hsum = B.hsum; AA.hdone = B.hdone;
             for (int b = 0; b < 3; ++b) AA.clist[b] = B.clist[b];
-            AA.status = B.status; AA.part_next = B.part_next; AA.lock_next = B.lock_next; AA.pw = B.pw;
+            AA.status = B.status; AA.lock_next = B.lock_next; AA.pw = B.pw;
             AA.moves_out = moves_d;
             AA.pc = B.pc; AA.pc_next = B.pc_next; AA.pdg = B.pdg;
-            if (B.mp && P.gnn && gnn_has_move_head(P.gnn)) {
+            if (move_head) {
                 // learned order of the afterburner: (move priority, id) instead of (gain, id)
                 gnn_move_priorities(c, P.gnn, g, level, B.dest, B.gain, B.mp);
                 AA.gain = B.mp;
@@ -1831,14 +1924,13 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
             GP_LAUNCHED(c);
             // copy pass + afterburner: candidate rows with gathered part (pcb bytes), dest and gain per entry
             c.bytes += (9 + B.pcb) * n + 16 * nlist + cdeg * (4 + (g.ew ? 4 : 0) + 8 + B.pcb);
-            std::swap(B.part, B.part_next);
             std::swap(B.lock, B.lock_next);
             std::swap(B.pc, B.pc_next);
         } else if (n <= kCtaMaxN) {
             // the whole step in one thread block
             auto mk = c.tmp->save();
             RbCta RA;
-            RA.vw = g.vw; RA.part = B.part; RA.pc = B.pc; RA.pcb = B.pcb; RA.lock = B.lock; RA.dest = B.dest;
+            RA.vw = g.vw; RA.pc = B.pc; RA.pcb = B.pcb; RA.lock = B.lock; RA.dest = B.dest;
             RA.gain = B.gain;
             RA.pre = c.tmp_alloc<int64_t>(n); RA.flag = c.tmp_alloc<int32_t>(n); RA.gkeys = c.tmp_alloc<uint64_t>(n);
             RA.k = k; RA.Lmax = Lmax;
@@ -1859,10 +1951,11 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
             c.bytes += 4 * n + 12 * n;
             if (ncand > 0 && ncand <= kCtaMaxN) {
                 // few candidates: sort, select and apply in one thread block
-                k_rb_compact<<<grid_for(n, 256), 256, 0, c.s>>>(n, flag, vpos, B.part, B.gain, B.ckeys, B.cvals);
+                k_rb_compact<<<grid_for(n, 256), 256, 0, c.s>>>(n, flag, vpos, B.pc, B.pcb, B.gain, B.ckeys,
+                                                                                 B.cvals);
                 GP_LAUNCHED(c);
                 RbCta RA;
-                RA.vw = g.vw; RA.part = B.part; RA.pc = B.pc; RA.pcb = B.pcb; RA.lock = B.lock; RA.dest = B.dest;
+                RA.vw = g.vw; RA.pc = B.pc; RA.pcb = B.pcb; RA.lock = B.lock; RA.dest = B.dest;
                 RA.gain = B.gain;
                 RA.pre = c.tmp_alloc<int64_t>(ncand); RA.flag = c.tmp_alloc<int32_t>(ncand);
                 RA.gkeys = c.tmp_alloc<uint64_t>(ncand); RA.k = k; RA.Lmax = Lmax;
@@ -1870,7 +1963,8 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
                 GP_LAUNCHED(c);
                 c.bytes += 80 * ncand;
             } else if (ncand > 0) {
-                k_rb_compact<<<grid_for(n, 256), 256, 0, c.s>>>(n, flag, vpos, B.part, B.gain, B.ckeys, B.cvals);
+                k_rb_compact<<<grid_for(n, 256), 256, 0, c.s>>>(n, flag, vpos, B.pc, B.pcb, B.gain, B.ckeys,
+                                                                                 B.cvals);
                 GP_LAUNCHED(c);
                 const int bits = RB_SHIFT + nb_k;
                 radix_sort_pairs(c, B.ckeys, B.cvals, B.ckeys2, B.cvals2, ncand, bits);
@@ -1902,7 +1996,7 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
                         k_seg_first<<<grid_for(k + 1, 256), 256, 0, c.s>>>(n2, B.ckeys2, k, segf);
                         GP_LAUNCHED(c);
                         k_rb_weak_apply<<<grid_for(n2, 256), 256, sizeof(int64_t) * k, c.s>>>(
-                            n2, B.ckeys2, segf, B.cvals2, pre, g.vw, pw_snap, Lmax, k, B.part, B.pc, B.pcb, B.lock, B.pw,
+                            n2, B.ckeys2, segf, B.cvals2, pre, g.vw, pw_snap, Lmax, k, B.pc, B.pcb, B.lock, B.pw,
                             moves_d);
                         GP_LAUNCHED(c);
                     }
@@ -1915,7 +2009,7 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
                     GP_LAUNCHED(c);
                     scan_excl_i32_to_i64(c, wm, pre, ncand, nullptr);
                     k_rb_strong_apply<<<grid_for(ncand, 256), 256, sizeof(int64_t) * k, c.s>>>(
-                        ncand, B.cvals, acc, pre, g.vw, cum, k, B.part, B.pc, B.pcb, B.lock, B.pw, moves_d);
+                        ncand, B.cvals, acc, pre, g.vw, cum, k, B.pc, B.pcb, B.lock, B.pw, moves_d);
                     GP_LAUNCHED(c);
                 }
                 c.bytes += 80 * ncand;
@@ -1925,7 +2019,9 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
         ++steps;
         if (tr.on()) trace_iter(c, B, n, g.m, level, it, mode, cur_cut, cur_mp, tr);
     }
-    GP_CUDA(cudaMemcpyAsync(B.part, B.best, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, c.s));
+    k_expand_part<<<grid_for(n, 256), 256, 0, c.s>>>(n, B.best, B.pcb, B.part);
+    GP_LAUNCHED(c);
+    c.bytes += 4 * n + B.pcb * n;
     GP_CUDA(cudaMemcpyAsync(B.pw, B.best_pw, sizeof(int64_t) * k, cudaMemcpyDeviceToDevice, c.s));
     return steps;
 }
