@@ -16,30 +16,33 @@ namespace gp {
 
 // ---------------------------------------------------------------- degree buckets
 // Lists in any order (each row is processed on its own).  Appends are
-// aggregated per warp: one atomic per warp and bucket.
-__device__ __forceinline__ void warp_append(bool take, int32_t v, int32_t* list, int64_t* count, int64_t cap) {
-    const uint32_t m = __ballot_sync(0xffffffffu, take);
-    if (!m) return;
-    const int lane = threadIdx.x & 31;
-    unsigned long long base = 0;
-    if (lane == __ffs(m) - 1) base = atomicAdd((unsigned long long*)count, (unsigned long long)__popc(m));
-    base = __shfl_sync(0xffffffffu, base, __ffs(m) - 1);
-    const int64_t idx = (int64_t)base + __popc(m & ((1u << lane) - 1u));
-    if (take && GP_IN(idx, cap)) list[idx] = v;
+// aggregated per block (block_append), 4 rows per thread at a time on lists
+// long enough for that to matter.
+// Lists of under 256 K rows are appended one row per thread: there latency
+// counts (9 us against 4 us a launch), not the counter.
+constexpr int64_t kAppendMany = 262144;
+__device__ __forceinline__ int degree_bucket(int64_t d, int32_t heavy_deg) {
+    return d <= kShortDeg ? 0 : (d <= kTile32 ? 1 : (d <= heavy_deg ? 2 : 3));
 }
 
+template <int kAppendRows>
 __global__ void k_buckets(const int64_t* __restrict__ rp, int64_t n, int32_t heavy_deg, int64_t heavy_cap,
                           int32_t* __restrict__ heavy,
                           int32_t* __restrict__ b0, int32_t* __restrict__ b1, int32_t* __restrict__ b2,
                           int64_t* __restrict__ count) {
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n; base += stride) {
-        const int64_t v = base + threadIdx.x;
-        const int64_t d = v < n ? rp[v + 1] - rp[v] : -1;
-        warp_append(v < n && d <= kTile8, (int32_t)v, b0, &count[0], n);
-        warp_append(d > kTile8 && d <= kTile32, (int32_t)v, b1, &count[1], n);
-        warp_append(d > kTile32 && d <= heavy_deg, (int32_t)v, b2, &count[2], n);
-        warp_append(d > heavy_deg, (int32_t)v, heavy, &count[3], heavy_cap);
+    int32_t* const lists[4] = {b0, b1, b2, heavy};
+    const int64_t caps[4] = {n, n, n, heavy_cap};
+    const int64_t per = (int64_t)blockDim.x * kAppendRows;
+    for (int64_t base = blockIdx.x * per; base < n; base += gridDim.x * per) {
+        int b[kAppendRows];
+        int32_t vs[kAppendRows];
+#pragma unroll
+        for (int r = 0; r < kAppendRows; ++r) {
+            const int64_t v = base + (int64_t)r * blockDim.x + threadIdx.x;
+            vs[r] = (int32_t)v;
+            b[r] = v < n ? degree_bucket(rp[v + 1] - rp[v], heavy_deg) : -1;
+        }
+        block_append<4, kAppendRows>(b, vs, lists, caps, count);
     }
 }
 
@@ -57,7 +60,7 @@ __global__ void k_unit_cost(const int64_t* __restrict__ rp, const int32_t* __res
                             int64_t* __restrict__ cost) {
     const int64_t U0 = (n0 + 3) / 4, U = n2 + n1 + U0;
     for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < U; u += (int64_t)gridDim.x * blockDim.x) {
-        int64_t cst = 32;
+        int64_t cst = u < n2 + n1 ? 32 : 8;
         if (u < n2) cst += rp[b2[u] + 1] - rp[b2[u]];
         else if (u < n2 + n1) cst += rp[b1[u - n2] + 1] - rp[b1[u - n2]];
         else {
@@ -75,7 +78,8 @@ void build_heavy(Ctx& c, Level& L) {
     const int64_t heavy_cap = std::max<int64_t>(1, L.g.m / L.heavy_deg + 1);
     L.heavy = c.keep_alloc<int32_t>(heavy_cap);
     for (int b = 0; b < 3; ++b) L.bucket[b] = c.keep_alloc<int32_t>(L.g.n);
-    k_buckets<<<grid_for(L.g.n, 256), 256, 0, c.s>>>(L.g.rp, L.g.n, L.heavy_deg, heavy_cap, L.heavy, L.bucket[0], L.bucket[1], L.bucket[2],
+    const int per = L.g.n >= kAppendMany ? 4 : 1;
+    (per == 4 ? k_buckets<4> : k_buckets<1>)<<<grid_for(L.g.n, 256 * per), 256, 0, c.s>>>(L.g.rp, L.g.n, L.heavy_deg, heavy_cap, L.heavy, L.bucket[0], L.bucket[1], L.bucket[2],
                                                      d_cnt);
     GP_LAUNCHED(c);
     c.bytes += 8 * (L.g.n + 1) + 4 * L.g.n;
@@ -176,9 +180,9 @@ __device__ __forceinline__ void block_argmax(uint64_t& k, int32_t& id, uint64_t*
 // ---------------------------------------------------------------- matching
 // MODE 0: proposal to the best eligible unmatched neighbour (handshake round).
 // MODE 1: anchor = best neighbour over all neighbours (two-hop pairing).
-// Work units as in the connectivity pass: rows of the three degree buckets
-// (4 rows per warp for bucket 0, one per warp otherwise), heavy rows one per
-// CTA in blocks [0, nheavy).
+// Work units: one row of buckets 1 and 2 per warp, two rows of bucket 0 per
+// warp (k_match_short takes them when there are many), heavy rows one per CTA
+// in blocks [0, nheavy).
 struct MatchArgs {
     DGraph g;
     const int32_t* heavy;
@@ -244,11 +248,38 @@ __device__ __forceinline__ void match_emit(const MatchArgs& A, bool valid, int64
     if (take && GP_IN(idx, A.g.n)) A.keys[idx] = ((uint64_t)(uint32_t)best << A.nbits) | (uint64_t)v;
 }
 
-template <int MODE, int TILE>
-__device__ __forceinline__ void match_tile(const MatchArgs& A, int64_t v) {
-    const int lane = threadIdx.x & 31, tl = lane & (TILE - 1);
-    bool valid = v >= 0;
-    if (valid && A.match[v] != -1) valid = false;  // matched already (round 0 / anchors)
+// bucket-1 rows: one warp, an entry per lane
+template <int MODE>
+__device__ __forceinline__ void match_lane(const MatchArgs& A, int64_t v) {
+    const int lane = threadIdx.x & 31;
+    const bool valid = A.match[v] == -1;  // else matched already (round 0 / anchors)
+    uint64_t bk = 0;
+    int32_t bid = -1;
+    if (valid) {
+        const int64_t e = A.g.rp[v] + lane;
+        if (e < A.g.rp[v + 1]) {
+            const int32_t u = __ldcs(&A.g.ci[e]);
+            const int64_t vwv = A.g.vw ? A.g.vw[v] : 1;
+            if (match_ok<MODE>(A, v, u, vwv)) {
+                bk = edge_key(key_word(A, e), edge_hash(A.salt, (int32_t)v, u));
+                bid = u;
+            }
+        }
+    }
+    warp_argmax(bk, bid);
+    if (MODE == 0) {
+        if (lane == 0) A.out[v] = valid ? bid : -1;
+    } else {
+        match_emit<MODE>(A, lane == 0 && valid, v, bid);
+    }
+}
+
+// bucket-0 rows (at most 16 entries), few of them: 16 lanes per row, two rows
+// per warp (v < 0: none), the best by butterfly shuffles
+template <int MODE>
+__device__ __forceinline__ void match_half(const MatchArgs& A, int64_t v) {
+    const int tl = threadIdx.x & 15;
+    const bool valid = v >= 0 && A.match[v] == -1;
     uint64_t bk = 0;
     int32_t bid = -1;
     if (valid) {
@@ -262,12 +293,78 @@ __device__ __forceinline__ void match_tile(const MatchArgs& A, int64_t v) {
             }
         }
     }
-    tile_argmax64<TILE>(bk, bid);
-    const bool lead = tl == 0;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+        const uint64_t k2 = __shfl_xor_sync(0xffffffffu, bk, o);
+        const int32_t i2 = __shfl_xor_sync(0xffffffffu, bid, o);
+        argmax_merge(bk, bid, k2, i2);
+    }
     if (MODE == 0) {
-        if (lead && v >= 0) A.out[v] = valid ? bid : -1;
+        if (tl == 0 && v >= 0) A.out[v] = valid ? bid : -1;
     } else {
-        match_emit<MODE>(A, lead && valid, v, bid);
+        match_emit<MODE>(A, tl == 0 && valid, v, bid);
+    }
+}
+
+// bucket-0 rows, many of them: one row per lane, every lane of the warp calls
+// it; entries 4 at a time while any lane of the warp has some left, their
+// match[] and weight gathers in flight together, the best kept in registers (no
+// shuffles).  (All 16 at a time takes 80 registers: 351 -> 450 us for round 0 of
+// the 256^3 grid's level 0.)
+template <int MODE>
+__device__ __forceinline__ int32_t match_short(const MatchArgs& A, int32_t v, int64_t beg, int len, int64_t vwv) {
+    const int32_t* __restrict__ row = A.g.ci + beg;
+    const int32_t* __restrict__ kw = A.prio ? A.prio + beg : (A.g.ew ? A.g.ew + beg : nullptr);
+    uint64_t bk = 0;
+    int32_t bid = -1;
+#pragma unroll
+    for (int c = 0; c < kShortDeg; c += 4) {
+        if (!__any_sync(0xffffffffu, len > c)) break;
+        int32_t u[4], w[4], mm[4], vv[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) u[i] = c + i < len ? __ldg(row + c + i) : -1;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (u[i] == v || !GP_IN(u[i] < 0 ? 0 : u[i], A.g.n)) u[i] = -1;
+            w[i] = (kw && u[i] >= 0) ? __ldg(kw + c + i) : 1;
+            mm[i] = (MODE == 0 && A.any_matched && u[i] >= 0) ? A.match[u[i]] : -1;
+            vv[i] = (MODE == 0 && A.check_vw && A.g.vw && u[i] >= 0) ? A.g.vw[u[i]] : 1;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (u[i] < 0) continue;
+            if (MODE == 0 && (mm[i] != -1 || (A.check_vw && vwv + vv[i] > A.maxvw))) continue;
+            argmax_merge(bk, bid, edge_key(w[i], edge_hash(A.salt, v, u[i])), u[i]);
+        }
+    }
+    return bid;
+}
+// the rows of list[0], in their own launch (k_match_scan's longer rows run
+// best at 40 registers): from kMatchSplit rows on.  256^3 grid, round 0:
+// level 0 (16.8 M rows of 6 entries; 8 lanes each in one launch with the rest)
+// 1317 -> 350 us, level 1 (9.1 M rows, two thirds of 9-10 entries; a warp each) 2111 -> 293 us
+constexpr int64_t kMatchSplit = 24576;
+template <int MODE>
+__global__ void __launch_bounds__(256) k_match_short(MatchArgs A) {
+    const int64_t n0 = A.nlist[0];
+    for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); i0 < n0;
+         i0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = i0 + (threadIdx.x & 31);
+        const int32_t v = i < n0 ? A.list[0][i] : -1;
+        const bool valid = v >= 0 && A.match[v] == -1;
+        int64_t beg = 0, vwv = 1;
+        int len = 0;
+        if (valid) {
+            beg = A.g.rp[v];
+            len = (int)(A.g.rp[v + 1] - beg);
+            if (MODE == 0 && A.check_vw && A.g.vw) vwv = A.g.vw[v];
+        }
+        const int32_t best = match_short<MODE>(A, v, beg, len, vwv);
+        if (MODE == 0) {
+            if (v >= 0) A.out[v] = valid ? best : -1;
+        } else {
+            match_emit<MODE>(A, valid, v, best);
+        }
     }
 }
 
@@ -363,13 +460,14 @@ __global__ void __launch_bounds__(256, 6) k_match_scan(MatchArgs A) {
     }
     const int64_t wid = ((int64_t)(blockIdx.x - A.nitems) * blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)(gridDim.x - A.nitems) * blockDim.x) >> 5;
-    const int64_t U0 = (A.nlist[0] + 3) / 4, U1 = A.nlist[1], U2 = A.nlist[2];
+    const int64_t n0 = A.nlist[0] < kMatchSplit ? A.nlist[0] : 0;   // else k_match_short's
+    const int64_t U0 = (n0 + 1) / 2, U1 = A.nlist[1], U2 = A.nlist[2];
     for (int64_t u = wid; u < U0 + U1 + U2; u += nw) {
         if (u < U0) {
-            const int64_t i = u * 4 + (lane >> 3);
-            match_tile<MODE, kTile8>(A, i < A.nlist[0] ? A.list[0][i] : -1);
+            const int64_t i = u * 2 + (lane >> 4);
+            match_half<MODE>(A, i < n0 ? A.list[0][i] : -1);
         } else if (u < U0 + U1) {
-            match_tile<MODE, kTile32>(A, A.list[1][u - U0]);
+            match_lane<MODE>(A, A.list[1][u - U0]);
         } else {
             const int64_t v = A.list[2][u - U0 - U1];
             const bool valid = A.match[v] == -1;
@@ -444,43 +542,49 @@ __global__ void __launch_bounds__(256, 6) k_match_scan(MatchArgs A) {
 // the worklists; a heavy one is flagged in hdead instead (heavy vertices are
 // not listed: their CTAs check match[] and hdead[] directly).  next_n[3]
 // counts the heavy vertices still live.
+template <int kAppendRows>
 __global__ void k_handshake(const int64_t* __restrict__ rp, int64_t n, int32_t heavy_deg, const int32_t* l0,
                             const int32_t* l1,
                             const int32_t* l2, int64_t n0, int64_t n1, int64_t n2, const int32_t* __restrict__ heavy,
                             int64_t nheavy,
                             const int32_t* __restrict__ prop, int32_t* __restrict__ match, int64_t* __restrict__ pairs,
                             int32_t* nl0, int32_t* nl1, int32_t* nl2, int64_t* next_n, uint8_t* __restrict__ hdead) {
-    int64_t local = 0;
+    int64_t local = 0, live = 0;
     const int64_t total = n0 + n1 + n2 + nheavy;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < total; base += stride) {
-        const int64_t i = base + threadIdx.x;
-        int64_t v = -1;
-        if (i < n0) v = l0[i];
-        else if (i < n0 + n1) v = l1[i - n0];
-        else if (i < n0 + n1 + n2) v = l2[i - n0 - n1];
-        else if (i < total) v = heavy[i - n0 - n1 - n2];
-        const bool is_heavy = i >= n0 + n1 + n2;
-        bool left = false;
-        int64_t d = 0;
-        if (v >= 0 && match[v] == -1 && !(is_heavy && hdead[i - n0 - n1 - n2])) {
-            const int32_t u = prop[v];
-            if (u >= 0 && GP_IN(u, n) && prop[u] == (int32_t)v) {
-                match[v] = u;
-                if (v < u) ++local;
-            } else if (u < 0) {
-                if (is_heavy) hdead[i - n0 - n1 - n2] = 1;
-            } else if (is_heavy) {
-                atomicAdd((unsigned long long*)&next_n[3], 1ull);
-            } else {
-                left = true;
-                d = rp[v + 1] - rp[v];
+    int32_t* const lists[3] = {nl0, nl1, nl2};
+    const int64_t caps[3] = {n, n, n};
+    const int64_t per = (int64_t)blockDim.x * kAppendRows;
+    for (int64_t base = blockIdx.x * per; base < total; base += gridDim.x * per) {
+        int b[kAppendRows];
+        int32_t vs[kAppendRows];
+#pragma unroll
+        for (int r = 0; r < kAppendRows; ++r) {
+            const int64_t i = base + (int64_t)r * blockDim.x + threadIdx.x;
+            int64_t v = -1;
+            if (i < n0) v = l0[i];
+            else if (i < n0 + n1) v = l1[i - n0];
+            else if (i < n0 + n1 + n2) v = l2[i - n0 - n1];
+            else if (i < total) v = heavy[i - n0 - n1 - n2];
+            const bool is_heavy = i >= n0 + n1 + n2;
+            b[r] = -1;
+            vs[r] = (int32_t)v;
+            if (v >= 0 && match[v] == -1 && !(is_heavy && hdead[i - n0 - n1 - n2])) {
+                const int32_t u = prop[v];
+                if (u >= 0 && GP_IN(u, n) && prop[u] == (int32_t)v) {
+                    match[v] = u;
+                    if (v < u) ++local;
+                } else if (u < 0) {
+                    if (is_heavy) hdead[i - n0 - n1 - n2] = 1;
+                } else if (is_heavy) {
+                    ++live;
+                } else {
+                    b[r] = degree_bucket(rp[v + 1] - rp[v], heavy_deg);
+                }
             }
         }
-        warp_append(left && d <= kTile8, (int32_t)v, nl0, &next_n[0], n);
-        warp_append(left && d > kTile8 && d <= kTile32, (int32_t)v, nl1, &next_n[1], n);
-        warp_append(left && d > kTile32 && d <= heavy_deg, (int32_t)v, nl2, &next_n[2], n);
+        block_append<3, kAppendRows>(b, vs, lists, caps, next_n);
     }
+    if (live) atomicAdd((unsigned long long*)&next_n[3], (unsigned long long)live);
     for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
     if ((threadIdx.x & 31) == 0 && local) atomicAdd((unsigned long long*)pairs, (unsigned long long)local);
 }
@@ -521,6 +625,22 @@ __global__ void k_max_vw(int64_t n, const int32_t* __restrict__ vw, int64_t* __r
         mx = vw[v] > mx ? vw[v] : mx;
     for (int o = 16; o > 0; o >>= 1) { const int32_t y = __shfl_xor_sync(0xffffffffu, mx, o); mx = y > mx ? y : mx; }
     if ((threadIdx.x & 31) == 0 && mx) atomicMax((unsigned long long*)out, (unsigned long long)mx);
+}
+
+// one matching scan over A's lists: the short rows apart when there are many
+template <int MODE>
+static void match_scan(Ctx& c, const MatchArgs& A) {
+    const bool split = A.nlist[0] >= kMatchSplit;
+    const int64_t units = (split ? 0 : (A.nlist[0] + 1) / 2) + A.nlist[1] + A.nlist[2];
+    if (split) {
+        k_match_short<MODE><<<grid_for(A.nlist[0], 256, c.sm_count * c.ctas_per_sm), 256, 0, c.s>>>(A);
+        GP_LAUNCHED(c);
+    }
+    if (!split || units + A.nitems > 0) {
+        const int grid = (int)A.nitems + grid_for(units * 32, 256, c.sm_count * c.ctas_per_sm);
+        k_match_scan<MODE><<<grid, 256, 0, c.s>>>(A);
+        GP_LAUNCHED(c);
+    }
 }
 
 int64_t match_level(Ctx& c, const Level& L, int level, const Params& P, int32_t* match, int* rounds_out,
@@ -567,18 +687,17 @@ int64_t match_level(Ctx& c, const Level& L, int level, const Params& P, int32_t*
     int rounds = 0;
     bool anchors_ready = false;   // round 0 ran and wrote anchor0
     for (int r = 0; r < P.o.match_rounds; ++r) {
-        const int64_t units = (A.nlist[0] + 3) / 4 + A.nlist[1] + A.nlist[2];
+        const int64_t units = A.nlist[0] + A.nlist[1] + A.nlist[2];
         // nobody left who can propose: this round would add no pair
         if (units == 0 && heavy_live == 0) { rounds = r + 1; break; }
         A.any_matched = r > 0 ? 1 : 0;
-        const int grid = (int)L.nitems + grid_for(units * 32, 256, c.sm_count * c.ctas_per_sm);
         memset_async(c, d_cnt, 0, 5 * sizeof(int64_t));
-        k_match_scan<0><<<grid, 256, 0, c.s>>>(A);
-        GP_LAUNCHED(c);
+        match_scan<0>(c, A);
         if (r == 0) anchors_ready = true;
         int32_t** nxt = wl[r & 1];
         const int64_t tot = A.nlist[0] + A.nlist[1] + A.nlist[2] + L.nheavy;
-        k_handshake<<<grid_for(tot, 256), 256, 0, c.s>>>(g.rp, g.n, L.heavy_deg, A.list[0], A.list[1], A.list[2], A.nlist[0], A.nlist[1],
+        const int per = tot >= kAppendMany ? 4 : 1;
+        (per == 4 ? k_handshake<4> : k_handshake<1>)<<<grid_for(tot, 256 * per), 256, 0, c.s>>>(g.rp, g.n, L.heavy_deg, A.list[0], A.list[1], A.list[2], A.nlist[0], A.nlist[1],
                                                          A.nlist[2], L.heavy, L.nheavy, prop, match, d_cnt, nxt[0],
                                                          nxt[1], nxt[2], d_cnt + 1, hdead);
         GP_LAUNCHED(c);
@@ -608,10 +727,7 @@ int64_t match_level(Ctx& c, const Level& L, int level, const Params& P, int32_t*
         B2.any_matched = 1;
         for (int b = 0; b < 3; ++b) { B2.list[b] = L.bucket[b]; B2.nlist[b] = L.nbucket[b]; }
         B2.out = nullptr; B2.keys = keys; B2.nkeys = d_cnt + 1; B2.nbits = nb;
-        const int64_t units = (B2.nlist[0] + 3) / 4 + B2.nlist[1] + B2.nlist[2];
-        const int grid = (int)L.nitems + grid_for(units * 32, 256, c.sm_count * c.ctas_per_sm);
-        k_match_scan<1><<<grid, 256, 0, c.s>>>(B2);
-        GP_LAUNCHED(c);
+        match_scan<1>(c, B2);
         c.bytes += L.scan_bytes() + 4 * g.n;
         int64_t cnt = read_i64(c, d_cnt + 1);
         if (cnt > 1) {

@@ -170,23 +170,6 @@ inline int64_t csr_slice(int64_t m, int sm_count) {
     s = (s + 255) & ~(int64_t)255;
     return s < 256 ? 256 : (s > 16384 ? 16384 : s);
 }
-// The same argmax over aligned groups of TILE lanes (TILE a power of
-// two <= 32; every lane of the warp calls them).  A group smaller than the
-// warp reduces with butterfly shuffles inside the group: a redux.sync whose
-// member mask differs between the lanes of one warp runs once per group.
-template <int TILE>
-__device__ __forceinline__ void tile_argmax64(uint64_t& k, int32_t& id) {
-    if constexpr (TILE == 32) {
-        group_argmax64(0xffffffffu, k, id);
-    } else {
-#pragma unroll
-        for (int o = TILE / 2; o > 0; o >>= 1) {
-            const uint64_t k2 = __shfl_xor_sync(0xffffffffu, k, o);
-            const int32_t i2 = __shfl_xor_sync(0xffffffffu, id, o);
-            if (k2 > k || (k2 == k && (uint32_t)i2 < (uint32_t)id)) { k = k2; id = i2; }
-        }
-    }
-}
 #endif
 // Four consecutive entries [e, e + 4) of a row [beg, end) of a CSR array
 // (column ids, weights or per-entry priorities), e a multiple of 4: one
@@ -237,6 +220,45 @@ __device__ __forceinline__ T block_excl_scan(T x, T* sh_warp, T& total) {
     total = sh_warp[32];
     __syncthreads();
     return r;
+}
+
+// Block-aggregated append: thread t offers item v[r] to list b[r] (b[r] outside
+// [0, NB): none) for r < R; one atomic per list and block instead of one per
+// list and warp (16.8 M rows: 524 K warp atomics on one counter took 0.35 ms).
+// Every thread of the block calls it; at most 32 warps.
+template <int NB, int R>
+__device__ __forceinline__ void block_append(const int (&b)[R], const int32_t (&v)[R], int32_t* const (&list)[NB],
+                                             const int64_t (&cap)[NB], int64_t* count) {
+    __shared__ int32_t s_pre[NB][32];
+    __shared__ int64_t s_base[NB];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const uint32_t lt = (1u << lane) - 1u;
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+        int32_t c = 0;
+#pragma unroll
+        for (int r = 0; r < R; ++r) c += __popc(__ballot_sync(0xffffffffu, b[r] == q));
+        if (lane == 0) s_pre[q][w] = c;
+    }
+    __syncthreads();
+    if (threadIdx.x < NB) {
+        int32_t run = 0;
+        for (int i = 0; i < nw; ++i) { const int32_t c = s_pre[threadIdx.x][i]; s_pre[threadIdx.x][i] = run; run += c; }
+        s_base[threadIdx.x] = run ? (int64_t)atomicAdd((unsigned long long*)&count[threadIdx.x], (unsigned long long)run) : 0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+        int64_t at = s_base[q] + s_pre[q][w];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const uint32_t m = __ballot_sync(0xffffffffu, b[r] == q);
+            const int64_t idx = at + __popc(m & lt);
+            if (b[r] == q && GP_IN(idx, cap[q])) list[q][idx] = v[r];
+            at += __popc(m);
+        }
+    }
+    __syncthreads();
 }
 
 __host__ __device__ __forceinline__ uint32_t loss_bucket(int32_t loss) {

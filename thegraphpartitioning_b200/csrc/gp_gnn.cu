@@ -91,9 +91,11 @@ __device__ __forceinline__ void warp_reduce_vec(float (&x)[F]) {
 
 // ---------------------------------------------------------------- row visits
 // The level graph's rows in the degree buckets the matching uses: rows of at
-// most 8 entries four to a warp (8 lanes each), rows of 9..32 entries one
-// warp, rows of 33..2048 entries one warp looping, longer rows split into CTA
-// items of at most 16384 entries.  Every sum below adds in a fixed order (the
+// most 16 entries four to a warp (8 lanes each, entries i and i + 8 to lane i),
+// rows of 17..32 entries one warp, rows of 33..2048 entries one warp looping,
+// longer rows split into CTA items of at most 16384 entries.  (Lane sums of
+// entries i and i + 8 and the tree over 8 lanes add in the order of a tree
+// over 16 or 32 lanes with an entry each.)  Every sum below adds in a fixed order (the
 // lane layout, then a shuffle tree, then item order), so results are
 // reproducible run to run.
 struct GnnRows {
@@ -166,8 +168,9 @@ __global__ void __launch_bounds__(256) k_gnn_rowsum(GnnRows R, Val val, Fin fin,
             v = i < R.nb[0] ? R.b[0][i] : -1;
             width = 8;
             if (v >= 0) {
-                const int64_t e = R.g.rp[v] + (lane & 7);
-                if (e < R.g.rp[v + 1]) val(e, acc);
+                const int64_t e = R.g.rp[v] + (lane & 7), end = R.g.rp[v + 1];
+                if (e < end) val(e, acc);
+                if (e + 8 < end) val(e + 8, acc);
             }
         } else {
             v = u < U0 + U1 ? R.b[1][u - U0] : R.b[2][u - U0 - U1];
@@ -213,8 +216,9 @@ __global__ void __launch_bounds__(256) k_gnn_entries(GnnRows R, Op op) {
             const int64_t i = u * 4 + (lane >> 3);
             if (i < R.nb[0]) {
                 const int64_t v = R.b[0][i];
-                const int64_t e = R.g.rp[v] + (lane & 7);
-                if (e < R.g.rp[v + 1]) op(v, e);
+                const int64_t e = R.g.rp[v] + (lane & 7), end = R.g.rp[v + 1];
+                if (e < end) op(v, e);
+                if (e + 8 < end) op(v, e + 8);
             }
         } else {
             const int64_t v = u < U0 + U1 ? R.b[1][u - U0] : R.b[2][u - U0 - U1];

@@ -26,10 +26,12 @@ struct Params {
 
 // Degree classes of the rows of one level; every kernel that works row by
 // row (matching, connectivity, afterburner) schedules its units from these
-// lists: bucket 0 rows go 4 to a warp (8 lanes each), bucket 1 rows one to a
-// warp in registers, bucket 2 rows one to a warp with a shared-memory
-// histogram, heavy rows one to a CTA.
-constexpr int kTile8 = 8;         // bucket 0: degree <= 8
+// lists: bucket 0 rows take one thread each (16 lanes where they are few),
+// bucket 1 rows one warp (an entry per lane), bucket 2 rows one warp looping,
+// heavy rows whole CTAs.  16 entries per thread: the rows of 9-10 entries of a
+// once matched 256^3 grid cost the connectivity pass 5 times the rows of 8 and
+// fewer with 4 lanes each, and more with a warp each.
+constexpr int kShortDeg = 16;     // bucket 0: degree <= 16
 constexpr int kTile32 = 32;       // bucket 1: degree <= 32
 struct Level {
     DGraph g;
@@ -48,8 +50,8 @@ struct Level {
     int32_t* row_first = nullptr;  // first item of each heavy row
     int64_t nitems = 0;
     // light work units in the order bucket 2 rows, bucket 1 rows, groups of 4
-    // bucket 0 rows, with the prefix sum of their costs (entries + 32): warps
-    // take contiguous unit ranges of equal cost
+    // bucket 0 rows, with the prefix sum of their costs (entries + 32, groups of
+    // 4: entries + 8): warps take contiguous unit ranges of equal cost
     int64_t* unit_cost = nullptr;  // nunits + 1 prefix
     int64_t nunits = 0;
     // bytes of one neighbour scan: row pointers, column ids, weights, gathered per-neighbour int32 state

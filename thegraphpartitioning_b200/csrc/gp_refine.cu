@@ -68,9 +68,9 @@ __device__ __forceinline__ bool lp_candidate(int32_t g, int32_t own, int32_t den
 // ------------------------------------------------------------------ k_conn
 // Light rows are taken 8 units (4 bucket-0 rows, 1 bucket-1 row or 1 bucket-2
 // row each) per warp at a time (conn_group); rows longer than kHeavyDeg take
-// CTAs [0, nheavy).  Bucket-0 rows take one thread each, bucket-1 rows 4 lanes
-// (up to 16 entries) or the warp (up to 32), bucket-2 rows the warp; bucket 2
-// and heavy rows build the whole shared-memory histogram.
+// CTAs [0, nheavy).  Bucket-0 rows take one thread each, bucket-1 and bucket-2
+// rows the warp; bucket 2 and heavy rows build the whole shared-memory
+// histogram.
 // status: [S_CROSS] += directed cross weight; [S_MAXPW], [S_MODE], [S_LIGHT]
 // written by CTA 0; LP candidates are appended to clist[bucket] (any order:
 // each is evaluated on its own), with [S_NL0..S_NL2] their counts and
@@ -227,104 +227,60 @@ struct ConnRes {
     int32_t bq;
 };
 
-// bucket 0 (at most 8 entries): one row per thread.  What bounds these rows is
-// the instruction count, not the loads: a warp's 32 rows are mostly consecutive
-// (the entry loads hit the lines the first of them brought in), all of a row's
-// gathers are in flight together, and the part sums are compares among the
-// thread's own registers, done only where a neighbour lies in another part.
-// Against 8 lanes per row with shuffles, 256^3 grid k = 32, one pass of level
-// 0 (16.8 M rows of 6 entries) @A0@
-template <class PT>
-__device__ __forceinline__ ConnRes conn_thread(const ConnArgs& A, const ConnRow& R, int mode, const uint8_t* over) {
+// bucket 0 (at most 16 entries): one row per thread; every lane of the warp
+// calls it (rows of no vertex: no entries).  What bounds these rows is the
+// instruction count, not the loads: a warp's 32 rows are mostly consecutive
+// (the entry loads hit the lines the first of them brought in), and all of a
+// row's loads, then all its gathers, are in flight together (8 or 16 of them,
+// by the longest row of the warp).  The part sums are compares among the
+// thread's own registers, part by part in ascending order (so ties keep the
+// smaller part), done only in warps with a row that has a neighbour in another
+// part and looks for a move.
+template <int N, class PT>
+__device__ __forceinline__ ConnRes conn_thread_n(const ConnArgs& A, const ConnRow& R, int mode, const uint8_t* over) {
     ConnRes x{0, 0, 0u, -1};
     const int len = (int)(R.end - R.beg);
     const int32_t* __restrict__ row = A.g.ci + R.beg;
-    int32_t q[kTile8], w[kTile8];
+    int32_t q[N], w[N];
 #pragma unroll
-    for (int i = 0; i < kTile8; ++i) q[i] = i < len ? __ldg(row + i) : -1;
+    for (int i = 0; i < N; ++i) q[i] = i < len ? __ldg(row + i) : -1;
     if (A.g.ew) {
         const int32_t* __restrict__ wrow = A.g.ew + R.beg;
 #pragma unroll
-        for (int i = 0; i < kTile8; ++i) w[i] = i < len ? __ldg(wrow + i) : 0;
+        for (int i = 0; i < N; ++i) w[i] = i < len ? __ldg(wrow + i) : 0;
     } else {
 #pragma unroll
-        for (int i = 0; i < kTile8; ++i) w[i] = i < len ? 1 : 0;
+        for (int i = 0; i < N; ++i) w[i] = i < len ? 1 : 0;
     }
 #pragma unroll
-    for (int i = 0; i < kTile8; ++i) q[i] = q[i] >= 0 ? gpart<PT>(A.pc, q[i], A.g.n) : -1;
+    for (int i = 0; i < N; ++i) q[i] = q[i] >= 0 ? gpart<PT>(A.pc, q[i], A.g.n) : -1;
 #pragma unroll
-    for (int i = 0; i < kTile8; ++i) { x.tot += w[i]; x.cross += q[i] != R.p ? w[i] : 0; }
-    if (R.active && x.cross > 0) {
+    for (int i = 0; i < N; ++i) { x.tot += w[i]; x.cross += q[i] != R.p ? w[i] : 0; }
+    bool go = R.active && x.cross > 0;
+    int32_t cur = -1;
+    while (__any_sync(0xffffffffu, go)) {
+        int32_t nx = INT32_MAX;   // the next part above cur
 #pragma unroll
-        for (int i = 0; i < kTile8; ++i) {
+        for (int i = 0; i < N; ++i)
+            if (q[i] > cur && q[i] != R.p && q[i] < nx) nx = q[i];
+        go = go && nx != INT32_MAX;
+        if (go) {
             int32_t h = 0;
 #pragma unroll
-            for (int j = 0; j < kTile8; ++j) h += q[j] == q[i] ? w[j] : 0;
-            if (q[i] >= 0 && q[i] != R.p && (mode != MODE_RB || !over[q[i]])) argmax_u32(x.bk, x.bq, (uint32_t)h, q[i]);
+            for (int i = 0; i < N; ++i) h += q[i] == nx ? w[i] : 0;
+            if ((uint32_t)h > x.bk && (mode != MODE_RB || !over[nx])) { x.bk = (uint32_t)h; x.bq = nx; }
+            cur = nx;
         }
     }
     return x;
 }
-
-// bucket-1 rows of at most 16 entries: 4 lanes per row, 8 rows per warp, 4
-// entries per lane (entry sub + 4 i).  The part sums meet the other lanes'
-// entries by three rounds of shuffles inside the 4 lanes, skipped when no row
-// of the warp has a neighbour in another part; every lane of a row ends with
-// the row's result.  Rows of no vertex (v < 0) or longer than 16 return zeros.
-constexpr int kQuadDeg = 16;
 template <class PT>
-__device__ __forceinline__ ConnRes conn_quad(const ConnArgs& A, const ConnRow& R, int mode, const uint8_t* over) {
-    const int sub = threadIdx.x & 3;
-    const int64_t deg = R.end - R.beg;
-    const int len = deg <= kQuadDeg ? (int)deg : 0;
-    int32_t q[4], w[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int e = sub + 4 * i;
-        q[i] = e < len ? __ldcs(&A.g.ci[R.beg + e]) : -1;
-        w[i] = e < len ? (A.g.ew ? __ldcs(&A.g.ew[R.beg + e]) : 1) : 0;
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) q[i] = q[i] >= 0 ? gpart<PT>(A.pc, q[i], A.g.n) : -1;
-    ConnRes x{0, 0, 0u, -1};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { x.tot += w[i]; x.cross += q[i] != R.p ? w[i] : 0; }
-#pragma unroll
-    for (int o = 1; o < 4; o <<= 1) {
-        x.tot += __shfl_xor_sync(0xffffffffu, x.tot, o);
-        x.cross += __shfl_xor_sync(0xffffffffu, x.cross, o);
-    }
-    if (!__any_sync(0xffffffffu, R.active && x.cross > 0)) return x;
-    int32_t h[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        h[i] = 0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) h[i] += q[j] == q[i] ? w[j] : 0;
-    }
-#pragma unroll
-    for (int o = 1; o < 4; ++o)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int32_t q2 = __shfl_xor_sync(0xffffffffu, q[j], o), w2 = __shfl_xor_sync(0xffffffffu, w[j], o);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) h[i] += q2 == q[i] ? w2 : 0;
-        }
-    if (R.active) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-            if (q[i] >= 0 && q[i] != R.p && (mode != MODE_RB || !over[q[i]])) argmax_u32(x.bk, x.bq, (uint32_t)h[i], q[i]);
-    }
-#pragma unroll
-    for (int o = 1; o < 4; o <<= 1) {
-        const uint32_t h2 = __shfl_xor_sync(0xffffffffu, x.bk, o);
-        const int32_t q2 = __shfl_xor_sync(0xffffffffu, x.bq, o);
-        argmax_u32(x.bk, x.bq, h2, q2);
-    }
-    return x;
+__device__ __forceinline__ ConnRes conn_thread(const ConnArgs& A, const ConnRow& R, int mode, const uint8_t* over) {
+    const uint32_t most = __reduce_max_sync(0xffffffffu, (uint32_t)(R.end - R.beg));
+    return most <= 8 ? conn_thread_n<8, PT>(A, R, mode, over) : conn_thread_n<kShortDeg, PT>(A, R, mode, over);
 }
 
-// bucket-1 rows of 17 to 32 entries: one row per warp, one entry per lane; the
+// bucket 1 (17 to 32 entries): one row per warp, one entry per lane; the
 // entries are added into the warp's shared-memory histogram and each lane
 // reads its own part's bin back (lanes of the same part hold the same value,
 // which the argmax, ties to the smaller part, does not mind).  hist: the
@@ -434,15 +390,15 @@ __device__ __forceinline__ ConnRes conn_warp(const ConnArgs& A, const ConnRow& R
 // in the lane of their slot, and the decisions of all of them are taken and
 // stored together (a warp's stores of consecutive rows coalesce), their
 // candidates appended together (one atomic per list present).  rows: the
-// warp's 32 slots in shared memory.
-template <class PT>
+// warp's 32 slots in shared memory.  SHORT: there may be bucket-0 units.
+template <class PT, bool SHORT>
 __device__ __forceinline__ void conn_group(const ConnArgs& A, int64_t ub, int nu, int mode, const uint8_t* over,
                                            int32_t light, int32_t* hist, ConnRowS* rows, int64_t& acc, int64_t& cdeg) {
     const int lane = threadIdx.x & 31;
     const int64_t U2 = A.nbucket[2], U21 = U2 + A.nbucket[1];
     const int64_t u = ub + (lane >> 2);
     const int sub = lane & 3;
-    const int lb = u < U2 ? 2 : (u < U21 ? 1 : 0);
+    const int lb = u < U2 ? 2 : (!SHORT || u < U21 ? 1 : 0);
     int32_t v = -1;
     if (u < ub + nu) {
         if (lb == 2) { if (sub == 0) v = A.bucket[2][u]; }
@@ -454,28 +410,20 @@ __device__ __forceinline__ void conn_group(const ConnArgs& A, int64_t ub, int nu
     }
     const ConnRow r = conn_row<PT>(A, v, mode, over);
     ConnRes x{0, 0, 0u, -1};
-    if (lb == 0) x = conn_thread<PT>(A, r, mode, over);
-    if (ub < U21) {   // warp or quad rows among the units
+    if (SHORT && ub + nu > U21) {
+        ConnRow tr = r;
+        if (lb != 0) { tr.end = tr.beg; tr.active = false; }
+        x = conn_thread<PT>(A, tr, mode, over);
+    }
+    if (ub < U21) {   // warp rows among the units
         rows[lane] = conn_stage(r);
         __syncwarp();
         const int nlong = U21 - ub < nu ? (int)(U21 - ub) : nu;
-        uint32_t todo = 0;   // row slots left to whole warps
-        if (ub + nu > U2) {
-            ConnRow qr = conn_unstage(rows[lane & ~3]);
-            const bool quad = lb == 1 && qr.v >= 0 && qr.end - qr.beg <= kQuadDeg;
-            if (!quad) { qr.end = qr.beg; qr.active = false; }
-            const ConnRes y = conn_quad<PT>(A, qr, mode, over);
-            if (quad && sub == 0) x = y;
-            todo = __ballot_sync(0xffffffffu, lb == 1 && r.v >= 0 && !quad && sub == 0);
-        }
         for (int j = 0; j < nlong; ++j) {
-            if (ub + j < U2) {
-                const ConnRes y = conn_warp<PT>(A, conn_unstage(rows[4 * j]), mode, over, hist);
-                if (lane == 4 * j) x = y;
-            } else if ((todo >> (4 * j)) & 1u) {
-                const ConnRes y = conn_lane<PT>(A, conn_unstage(rows[4 * j]), mode, over, hist);
-                if (lane == 4 * j) x = y;
-            }
+            const ConnRow wr = conn_unstage(rows[4 * j]);
+            const ConnRes y = ub + j < U2 ? conn_warp<PT>(A, wr, mode, over, hist)
+                                          : conn_lane<PT>(A, wr, mode, over, hist);
+            if (lane == 4 * j) x = y;
         }
         __syncwarp();
     }
@@ -487,52 +435,115 @@ __device__ __forceinline__ void conn_group(const ConnArgs& A, int64_t ub, int nu
     }
     if (A.clist[0] == nullptr || !__any_sync(0xffffffffu, take)) return;
 #pragma unroll
-    for (int b = 0; b < 3; ++b) warp_push(take && lb == b, r.v, A.clist[b], conn_list_count(A, b), A.g.n);
+    for (int b = SHORT ? 0 : 1; b < 3; ++b) warp_push(take && lb == b, r.v, A.clist[b], conn_list_count(A, b), A.g.n);
 }
 
-template <class PT>
-__global__ void __launch_bounds__(RT, 5) k_conn(ConnArgs A) {
-    extern __shared__ int32_t csm[];
-    const int32_t k = A.k;
-    const int64_t Lmax = A.Lmax;
-    const int kpad = (k + 15) & ~15;
-    uint8_t* over = (uint8_t*)csm;
-    int32_t* hist_all = csm + kpad / 4;
-    __shared__ int64_t s_red[RW];
-    __shared__ uint64_t s_k[RW];
-    __shared__ int32_t s_q[RW];
-    __shared__ int64_t s_maxpw;
-    __shared__ int32_t s_light;
-    __shared__ ConnRowS s_rows[RT];   // light warps: 32 staged rows each
+// part-weight summary every block of a connectivity pass starts from: over
+// flags, the heaviest part, the lightest part within Lmax (ties: lower id) and
+// the mode they imply; block 0 writes the summary to the status block
+struct ConnHead {
+    int64_t red[RW];
+    uint64_t k[RW];
+    int32_t q[RW];
+    int64_t maxpw;
+    int32_t light;
+};
+__device__ __forceinline__ int conn_head(const ConnArgs& A, uint8_t* over, ConnHead& sh, int32_t& light) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-
-    // over flags, heaviest part, lightest non-overweight part (ties: lower id)
+    const int64_t Lmax = A.Lmax;
     int64_t mx = 0;
     uint64_t lk = 0; int32_t lq = -1;  // argmax of (~pw) == argmin pw
-    for (int q = threadIdx.x; q < k; q += RT) {
+    for (int q = threadIdx.x; q < A.k; q += RT) {
         const int64_t x = A.pw[q];
         over[q] = x > Lmax;
         mx = x > mx ? x : mx;
         if (x <= Lmax) argmax_q(lk, lq, ~(uint64_t)x, q);
     }
-    for (int i = threadIdx.x; i < RW * k; i += RT) hist_all[i] = 0;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) { int64_t y = __shfl_xor_sync(0xffffffffu, mx, o); mx = y > mx ? y : mx; }
     warp_argmax_q(lk, lq);
-    if (lane == 0) { s_red[w] = mx; s_k[w] = lk; s_q[w] = lq; }
+    if (lane == 0) { sh.red[w] = mx; sh.k[w] = lk; sh.q[w] = lq; }
     __syncthreads();
     if (threadIdx.x == 0) {
         int64_t m2 = 0; uint64_t k2 = 0; int32_t q2 = -1;
-        for (int i = 0; i < RW; ++i) { m2 = s_red[i] > m2 ? s_red[i] : m2; argmax_q(k2, q2, s_k[i], s_q[i]); }
-        s_maxpw = m2; s_light = q2;
+        for (int i = 0; i < RW; ++i) { m2 = sh.red[i] > m2 ? sh.red[i] : m2; argmax_q(k2, q2, sh.k[i], sh.q[i]); }
+        sh.maxpw = m2; sh.light = q2;
     }
     __syncthreads();
-    const int64_t maxpw = s_maxpw;
-    const int32_t light = s_light;
+    const int64_t maxpw = sh.maxpw;
+    light = sh.light;
     const int mode = A.force_eval ? MODE_EVAL : (maxpw > Lmax ? MODE_RB : MODE_LP);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         A.status[S_MAXPW] = maxpw; A.status[S_MODE] = mode; A.status[S_LIGHT] = light;
     }
+    return mode;
+}
+// adds every thread's cross weight to the status block, one atomic per block
+__device__ __forceinline__ void conn_tail(const ConnArgs& A, int64_t acc, int64_t* s_red) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    acc = warp_sum(acc);
+    __syncthreads();
+    if (lane == 0) s_red[w] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int64_t s = 0;
+        for (int i = 0; i < RW; ++i) s += s_red[i];
+        if (s) atomicAdd((unsigned long long*)&A.status[S_CROSS], (unsigned long long)s);
+    }
+}
+
+// Bucket-0 rows of a large level: one row per lane, 32 listed rows per warp at
+// a time, grid-stride.  Its own kernel because a thread's 16 entries, weights
+// and gathers take 64 registers, while the longer rows (k_conn) run best at
+// 48: with them in k_conn its R-MAT 24 passes took 138 ms in all (spills),
+// apart 125.  256^3 grid, k = 32, one pass, against 8 lanes per row of up to 8
+// entries and a warp per row above: level 0 (16.8 M rows of 6 entries) 1860 ->
+// 330 us; all 270 passes of its V-cycle 182 -> 44 ms.
+template <class PT>
+__global__ void __launch_bounds__(RT, 4) k_conn_short(ConnArgs A) {
+    extern __shared__ int32_t csm[];
+    uint8_t* over = (uint8_t*)csm;
+    __shared__ ConnHead sh;
+    int32_t light;
+    const int mode = conn_head(A, over, sh, light);
+    const int lane = threadIdx.x & 31;
+    int64_t acc = 0, cdeg = 0;
+    const int64_t n0 = A.nbucket[0];
+    for (int64_t i0 = (int64_t)blockIdx.x * RT + (threadIdx.x & ~31); i0 < n0; i0 += (int64_t)gridDim.x * RT) {
+        const int64_t i = i0 + lane;
+        const ConnRow r = conn_row<PT>(A, i < n0 ? A.bucket[0][i] : -1, mode, over);
+        const ConnRes x = conn_thread<PT>(A, r, mode, over);
+        bool take = false;
+        if (r.v >= 0) {
+            acc += x.cross;
+            take = conn_decide<PT>(A, mode, r.active, r.v, r.p, x.tot, x.cross, x.bk, x.bq, light);
+            if (take) cdeg += r.end - r.beg;
+        }
+        warp_push(take, r.v, A.clist[0], conn_list_count(A, 0), A.g.n);
+    }
+    cdeg = warp_sum(cdeg);
+    if (lane == 0 && cdeg) atomicAdd((unsigned long long*)&A.status[S_CDEG], (unsigned long long)cdeg);
+    conn_tail(A, acc, sh.red);
+}
+
+// SHORT: the light units include the bucket-0 rows (small levels: one launch);
+// else they are left to k_conn_short
+template <class PT, bool SHORT>
+__global__ void __launch_bounds__(RT, SHORT ? 4 : 5) k_conn(ConnArgs A) {
+    extern __shared__ int32_t csm[];
+    const int32_t k = A.k;
+    const int kpad = (k + 15) & ~15;
+    uint8_t* over = (uint8_t*)csm;
+    int32_t* hist_all = csm + kpad / 4;
+    __shared__ ConnHead sh;
+    __shared__ ConnRowS s_rows[RT];   // light warps: 32 staged rows each
+    int64_t* s_red = sh.red;
+    uint64_t* s_k = sh.k;
+    int32_t* s_q = sh.q;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int i = threadIdx.x; i < RW * k; i += RT) hist_all[i] = 0;
+    int32_t light;
+    const int mode = conn_head(A, over, sh, light);
     int64_t acc = 0;  // directed cross weight (this thread)
 
     if ((int64_t)blockIdx.x < A.nitems) {
@@ -629,19 +640,11 @@ __global__ void __launch_bounds__(RT, 5) k_conn(ConnArgs A) {
         const int64_t u0 = A.wfirst[wid], u1 = A.wfirst[wid + 1];
         int64_t cdeg = 0;   // degree sum of this lane's candidates
         for (int64_t ub = u0; ub < u1; ub += 8)
-            conn_group<PT>(A, ub, (int)(u1 - ub < 8 ? u1 - ub : 8), mode, over, light, hist, rows, acc, cdeg);
+            conn_group<PT, SHORT>(A, ub, (int)(u1 - ub < 8 ? u1 - ub : 8), mode, over, light, hist, rows, acc, cdeg);
         cdeg = warp_sum(cdeg);
         if (lane == 0 && cdeg) atomicAdd((unsigned long long*)&A.status[S_CDEG], (unsigned long long)cdeg);
     }
-    acc = warp_sum(acc);
-    __syncthreads();
-    if (lane == 0) s_red[w] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int64_t s = 0;
-        for (int i = 0; i < RW; ++i) s += s_red[i];
-        if (s) atomicAdd((unsigned long long*)&A.status[S_CROSS], (unsigned long long)s);
-    }
+    conn_tail(A, acc, s_red);
 }
 
 // ------------------------------------------------------------------ LP apply
@@ -711,7 +714,52 @@ __device__ __forceinline__ void ab_row(const ApplyArgs& A, int64_t v, int32_t& p
     }
 }
 
-// candidate rows of at most TILE entries, TILE lanes each
+// candidate rows of bucket 0, many of them: one row per lane (v < 0: none),
+// every lane of the warp calls it; all of a row's entries are in flight
+// together (8 or 16 of them, by the longest row of the warp)
+template <int N, class PT>
+__device__ __forceinline__ int32_t ab_short_n(const ApplyArgs& A, int64_t v, int32_t p, int32_t d, int32_t gv,
+                                              int64_t beg, int len) {
+    const int32_t* __restrict__ row = A.g.ci + beg;
+    int32_t u[N], t = 0;
+    uint64_t x[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) u[i] = i < len ? __ldg(row + i) : -1;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        x[i] = 0;
+        if (u[i] < 0 || !GP_IN(u[i], A.g.n)) { u[i] = -1; continue; }
+        if (A.pdg) x[i] = A.pdg[u[i]];
+        else x[i] = pdg_pack(gpart<PT>(A.pc, u[i], A.g.n), A.dest[u[i]], A.dest[u[i]] >= 0 ? A.gain[u[i]] : 0);
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        if (u[i] < 0) continue;
+        int32_t q = pdg_part(x[i]);
+        const int32_t du = pdg_dest(x[i]), gu = pdg_gain(x[i]);
+        if (du >= 0 && (gu > gv || (gu == gv && u[i] < (int32_t)v))) q = du;
+        const int32_t w = A.g.ew ? __ldg(A.g.ew + beg + i) : 1;
+        t += q == d ? w : (q == p ? -w : 0);
+    }
+    return t;
+}
+template <class PT>
+__device__ __forceinline__ void ab_short(const ApplyArgs& A, int64_t v, int64_t* delta, int64_t& moves) {
+    int32_t p = -1, d = -1, gv = 0;
+    int64_t beg = 0;
+    int len = 0;
+    if (v >= 0) {
+        ab_row<PT>(A, v, p, d, gv);
+        beg = A.g.rp[v];
+        len = (int)(A.g.rp[v + 1] - beg);
+    }
+    const uint32_t most = __reduce_max_sync(0xffffffffu, (uint32_t)len);
+    const int32_t t = most <= 8 ? ab_short_n<8, PT>(A, v, p, d, gv, beg, len)
+                                : ab_short_n<kShortDeg, PT>(A, v, p, d, gv, beg, len);
+    if (v >= 0 && t >= 0) ab_commit<PT>(A, v, p, d, delta, moves);
+}
+
+// candidate rows of at most TILE entries, TILE lanes each (v < 0: none)
 template <int TILE, class PT>
 __device__ __forceinline__ void ab_tile(const ApplyArgs& A, int64_t v, int64_t* delta, int64_t& moves) {
     const int lane = threadIdx.x & 31, tl = lane & (TILE - 1);
@@ -784,7 +832,7 @@ __device__ __forceinline__ void ab_warp(const ApplyArgs& A, int64_t v, int64_t* 
 }
 
 template <class PT>
-__global__ void __launch_bounds__(RT) k_lp_apply(ApplyArgs A) {
+__global__ void __launch_bounds__(RT, 4) k_lp_apply(ApplyArgs A) {
     extern __shared__ int64_t delta[];
     __shared__ int64_t s_red[RW];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -822,13 +870,18 @@ __global__ void __launch_bounds__(RT) k_lp_apply(ApplyArgs A) {
         }
     } else {
         const int64_t n0 = A.status[S_NL0], n1 = A.status[S_NL1], n2 = A.status[S_NL2];
-        const int64_t U0 = (n0 + 3) / 4;
         const int64_t wid = ((int64_t)(blockIdx.x - A.nitems) * RT + threadIdx.x) >> 5;
         const int64_t nw = ((int64_t)(gridDim.x - A.nitems) * RT) >> 5;
+        // short rows: one per lane when that still fills the launch's warps, else
+        // 16 lanes each (fewer rows one after another per warp)
+        const int rpw = n0 >= 32 * nw ? 32 : 2;
+        const int64_t U0 = (n0 + rpw - 1) / rpw;
         for (int64_t u = wid; u < U0 + n1 + n2; u += nw) {
             if (u < U0) {
-                const int64_t i = u * 4 + (lane >> 3);
-                ab_tile<kTile8, PT>(A, i < n0 ? A.clist[0][i] : -1, delta, moves);
+                const int64_t i = u * rpw + (rpw == 32 ? lane : lane >> 4);
+                const int64_t v = i < n0 ? A.clist[0][i] : -1;
+                if (rpw == 32) ab_short<PT>(A, v, delta, moves);
+                else ab_tile<16, PT>(A, v, delta, moves);
             } else if (u < U0 + n1) {
                 ab_tile<kTile32, PT>(A, A.clist[1][u - U0], delta, moves);
             } else {
@@ -1432,7 +1485,7 @@ __device__ void cta_refine_level(const CtaRefineArgs& R, unsigned char* rsm) {
         int64_t acc = 0, cdeg = 0;
         int32_t* hist = s_hist + w * k;
         for (int64_t ub = 8 * w; ub < U2 + U1 + U0; ub += 8 * CW)
-            conn_group<int32_t>(CA, ub, (int)(U2 + U1 + U0 - ub < 8 ? U2 + U1 + U0 - ub : 8), dmode, s_over, light, hist,
+            conn_group<int32_t, true>(CA, ub, (int)(U2 + U1 + U0 - ub < 8 ? U2 + U1 + U0 - ub : 8), dmode, s_over, light, hist,
                                 s_rows + 32 * w, acc, cdeg);
         acc = warp_sum(acc);
         const int64_t cur_cut = cta_sum(lane == 0 ? acc : 0, sh) / 2;   // also orders the pass
@@ -1479,18 +1532,15 @@ __device__ void cta_refine_level(const CtaRefineArgs& R, unsigned char* rsm) {
             AA.status = R.status; AA.lock_next = lock_next; AA.pw = nullptr;
             AA.pc = part; AA.pc_next = part_next;
             AA.moves_out = nullptr; AA.hsum = nullptr; AA.hdone = nullptr; AA.pdg = nullptr;
-            for (int64_t u = w; u < U2 + U1 + U0; u += CW) {
-                if (u < U2) {
-                    const int64_t v = R.bucket[2][u];
-                    if (R.dest[v] >= 0) ab_warp<int32_t>(AA, v, s_pw, moves);
-                } else if (u < U2 + U1) {
-                    const int64_t v = R.bucket[1][u - U2];
-                    ab_tile<kTile32, int32_t>(AA, R.dest[v] >= 0 ? v : -1, s_pw, moves);
-                } else {
-                    const int64_t i = (u - U2 - U1) * 4 + (lane >> 3);
-                    const int64_t v = i < R.nbucket[0] ? R.bucket[0][i] : -1;
-                    ab_tile<kTile8, int32_t>(AA, (v >= 0 && R.dest[v] >= 0) ? v : -1, s_pw, moves);
-                }
+            for (int64_t u = w; u < U2 + U1; u += CW) {
+                const int64_t v = u < U2 ? R.bucket[2][u] : R.bucket[1][u - U2];
+                if (R.dest[v] < 0) continue;
+                if (u < U2) ab_warp<int32_t>(AA, v, s_pw, moves);
+                else ab_tile<kTile32, int32_t>(AA, v, s_pw, moves);
+            }
+            for (int64_t i0 = 32 * w; i0 < R.nbucket[0]; i0 += 32 * CW) {
+                const int64_t v = i0 + lane < R.nbucket[0] ? R.bucket[0][i0 + lane] : -1;
+                ab_short<int32_t>(AA, v >= 0 && R.dest[v] >= 0 ? v : -1, s_pw, moves);
             }
             nmoves = cta_sum(moves, sh);
             int32_t* tp = part; part = part_next; part_next = tp;
@@ -1767,7 +1817,10 @@ static void trace_iter(Ctx& c, const RefineBufs& B, int64_t n, int64_t m, int le
     tr.emit(ev);
 }
 
-constexpr int64_t kConnWarpCost = 8 * (32 + 24);
+constexpr int64_t kConnWarpCost = 8 * (8 + 28);
+// bucket-0 rows from which they take their own launch: below, a second launch
+// (about 3 us a pass) costs more than the registers
+constexpr int64_t kConnSplit = 32768;
 int64_t conn_max_warps(const Ctx& c) { return (int64_t)c.sm_count * c.ctas_per_sm * RW; }
 
 // light warp t of a connectivity pass over nw warps takes the units
@@ -1804,17 +1857,26 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
     const int kpad = (k + 15) & ~15;
     const size_t conn_smem = kpad + sizeof(int32_t) * RW * k;
     // at most 1024 + 32 * GP_MAX_K bytes: below the 48 KB default, no attribute needed
-    // a light warp's range costs as much as a group of 8 short units (entries
-    // + 32 each), so that its lanes have rows to work on; on levels too small
-    // for 16 such warps per SM latency counts and units are spread thinner
+    // bucket-0 rows: their own launch on large levels
+    const bool split = L.nbucket[0] >= kConnSplit;
+    const bool long_rows = !split || L.nitems + L.nbucket[1] + L.nbucket[2] > 0;
+    const int64_t nunits = split ? L.nbucket[2] + L.nbucket[1] : L.nunits;
+    const int64_t short_cost = split ? 0 : 2 * L.nbucket[0];
+    // a light warp's range costs as much as a group of 8 units of short rows,
+    // so that its lanes have rows to work on; on levels too small for 16 such
+    // warps per SM latency counts and units are spread thinner
     const int64_t light_warps = std::min<int64_t>(
-        L.nunits, std::max<int64_t>((g.m + 32 * L.nunits) / kConnWarpCost, (int64_t)c.sm_count * 16));
+        nunits, std::max<int64_t>((g.m + 32 * (L.nbucket[2] + L.nbucket[1]) + short_cost) / kConnWarpCost,
+                                  (int64_t)c.sm_count * 16));
     const int light_blocks = (int)std::min<int64_t>(grid_for(light_warps, RW, c.sm_count * c.ctas_per_sm),
                                                     (B.wfirst_cap - 1) / RW);
     const int grid = (int)L.nitems + light_blocks;
-    {
+    const int short_grid = grid_for(L.nbucket[0], RT, c.sm_count * std::min(c.ctas_per_sm, 32));
+    // label propagation moves candidates of every bucket in one launch
+    const int lp_grid = split ? (int)L.nitems + std::max(light_blocks, grid_for(L.nbucket[0], 4 * RT, c.sm_count * 8)) : grid;
+    if (long_rows) {
         const int64_t nw = (int64_t)light_blocks * RW;
-        k_warp_bounds<<<grid_for(nw + 1, 256), 256, 0, c.s>>>(L.unit_cost, L.nunits, nw, B.wfirst);
+        k_warp_bounds<<<grid_for(nw + 1, 256), 256, 0, c.s>>>(L.unit_cost, nunits, nw, B.wfirst);
         GP_LAUNCHED(c);
     }
     int64_t best_cut = 0, best_mp = 0;
@@ -1839,9 +1901,17 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
         CA.dest = B.dest; CA.gain = B.gain; CA.status = B.status;
         CA.pc = B.pc; CA.pc_next = B.pc_next; CA.lock_next = B.lock_next;   // the LP step's starting copy
         CA.pdg = B.pdg; CA.lp_dg = lp_dg;
-        if (B.pcb == 1) k_conn<uint8_t><<<grid, RT, conn_smem, c.s>>>(CA);
-        else k_conn<uint16_t><<<grid, RT, conn_smem, c.s>>>(CA);
-        GP_LAUNCHED(c);
+        if (long_rows) {
+            auto kc = B.pcb == 1 ? (split ? k_conn<uint8_t, false> : k_conn<uint8_t, true>)
+                                 : (split ? k_conn<uint16_t, false> : k_conn<uint16_t, true>);
+            kc<<<grid, RT, conn_smem, c.s>>>(CA);
+            GP_LAUNCHED(c);
+        }
+        if (split) {
+            auto ks = B.pcb == 1 ? k_conn_short<uint8_t> : k_conn_short<uint16_t>;
+            ks<<<short_grid, RT, kpad, c.s>>>(CA);
+            GP_LAUNCHED(c);
+        }
         if (c.profile) GP_CUDA(cudaEventRecord(c.ev_b, c.s));
         // rowptr, colidx, weights, gathered part[u] (pcb bytes); part[v], lock[v] read; proposal and gain written
         const int64_t conn_bytes = L.scan_bytes() - (4 - B.pcb) * g.m + B.pcb * n + n + 8 * n;
@@ -1919,8 +1989,8 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
                     tr.emit(ev);
                 }
             }
-            if (B.pcb == 1) k_lp_apply<uint8_t><<<grid, RT, sizeof(int64_t) * k, c.s>>>(AA);
-            else k_lp_apply<uint16_t><<<grid, RT, sizeof(int64_t) * k, c.s>>>(AA);
+            if (B.pcb == 1) k_lp_apply<uint8_t><<<lp_grid, RT, sizeof(int64_t) * k, c.s>>>(AA);
+            else k_lp_apply<uint16_t><<<lp_grid, RT, sizeof(int64_t) * k, c.s>>>(AA);
             GP_LAUNCHED(c);
             // copy pass + afterburner: candidate rows with gathered part (pcb bytes), dest and gain per entry
             c.bytes += (9 + B.pcb) * n + 16 * nlist + cdeg * (4 + (g.ew ? 4 : 0) + 8 + B.pcb);
