@@ -338,10 +338,14 @@ constexpr int kLearnedItemLen = 16384;
 // exclusive scan; out may alias in; returns total on the host if total_out != nullptr
 void scan_excl_i32_to_i64(Ctx& c, const int32_t* in, int64_t* out, int64_t n, int64_t* d_total);
 void scan_excl_i64(Ctx& c, const int64_t* in, int64_t* out, int64_t n, int64_t* d_total);
+// exclusive scan of the weights vw[list[i]] (1 without weights), i < n; n_dev
+// (may be nullptr): the length in device memory, n being a bound on it
+void scan_list_weights(Ctx& c, const int32_t* list, const int32_t* vw, int64_t* out, int64_t n, const int64_t* n_dev,
+                       int64_t* d_total);
 // LSD radix sort of (key, val) pairs by the low `bits` bits of key.  Result in
-// keys/vals (ping-pong through the provided temporaries).
+// keys/vals (ping-pong through the provided temporaries); n_dev as above.
 void radix_sort_pairs(Ctx& c, uint64_t* keys, int32_t* vals, uint64_t* keys_tmp, int32_t* vals_tmp,
-                      int64_t n, int bits);
+                      int64_t n, int bits, const int64_t* n_dev = nullptr);
 int64_t read_i64(Ctx& c, const int64_t* d);   // synchronous small read
 void memset_async(Ctx& c, void* p, int value, size_t bytes);
 

@@ -112,7 +112,7 @@ struct RefineBufs {
     uint8_t* lock_next = nullptr;
     int64_t* pw = nullptr;        // k
     int64_t* best_pw = nullptr;   // k
-    int64_t* status = nullptr;    // 16
+    int64_t* status = nullptr;    // kStatusRing blocks of S_NSLOTS
     int32_t* clist[3] = {nullptr, nullptr, nullptr};   // LP candidates by degree bucket
     int64_t* wfirst = nullptr;    // first light unit of each warp of the connectivity pass (+ end)
     int64_t wfirst_cap = 0;       // its length
@@ -126,10 +126,12 @@ struct RefineBufs {
     int32_t* cvals2 = nullptr;
 };
 
-// device status block of the refinement loop; slots [0, S_NRESET) are cleared
-// before every connectivity pass, S_STEP_MOVES before every move step
+// device status block of one refinement iteration: the connectivity pass's
+// slots [0, S_NRESET), the move step's S_STEP_MOVES, and S_DONE, the pass's
+// finished blocks.  A level uses a ring of blocks, cleared half a ring at a time.
 enum StatusSlot { S_CROSS = 0, S_MAXPW = 1, S_MODE = 2, S_NL0 = 3, S_NL1 = 4, S_LIGHT = 5, S_NL2 = 6, S_CDEG = 7,
-                  S_NRESET = 8, S_STEP_MOVES = 8, S_NSLOTS = 16 };
+                  S_NRESET = 8, S_STEP_MOVES = 8, S_DONE = 9, S_NSLOTS = 16 };
+constexpr int kStatusRing = 64;
 
 // CUDA events of the phases of one V-cycle
 struct Timer {

@@ -1,11 +1,15 @@
 // gp_prims.cu -- arena, prefix scans and the LSD radix sort.
 //
-// Scans are three-phase (tile reduce -> scan of tile sums -> tile scan), each
-// tile 256 threads x 8 items.  The radix sort is a stable LSD sort of 64-bit
-// keys with 32-bit payloads, 8-bit digits: per pass a tile histogram kernel, a
-// scan of the digit-major (digit, tile) count table, and a scatter kernel that
-// ranks items stably inside the tile with warp match/ballot and per-warp digit
-// counters in shared memory.
+// Scans reduce tiles of 256 threads x 8 items, then scan every tile from the
+// sums of the tiles before it; few tiles are summed by each tile's own block
+// (two launches), many by a kernel in between (three), and short arrays take
+// one block and one launch.  The radix sort is a stable LSD sort of 64-bit keys
+// with 32-bit payloads, 8-bit digits: per pass a tile histogram kernel, a
+// kernel that scans each digit's tile counts (one block per digit), and a
+// scatter kernel that adds the digits' bases and ranks items stably inside the
+// tile with warp match/ballot and per-warp digit counters in shared memory.
+// Sorts and weight scans take their length from device memory when the caller
+// has it only there.
 #define GP_TU_ID 1   // site ids of the bounds-checked build
 #include "gp_common.cuh"
 
@@ -105,52 +109,74 @@ constexpr int SCAN_T = 256;
 constexpr int SCAN_I = 8;
 constexpr int SCAN_TILE = SCAN_T * SCAN_I;
 
-template <class TI, class TO>
-__global__ void k_tile_reduce(const TI* __restrict__ in, int64_t n, TO* __restrict__ tile_sums) {
-    __shared__ TO sh[33];
+// scan inputs: an array; the vertex weights of a list of vertices (1 without weights)
+template <class T>
+struct InArray {
+    const T* p;
+    __device__ __forceinline__ int64_t operator()(int64_t i) const { return (int64_t)p[i]; }
+};
+struct InListWeight {
+    const int32_t* list;
+    const int32_t* vw;
+    __device__ __forceinline__ int64_t operator()(int64_t i) const { return vw ? (int64_t)vw[list[i]] : 1; }
+};
+
+template <class In>
+__global__ void k_tile_reduce(In in, int64_t n, const int64_t* __restrict__ n_dev, int64_t* __restrict__ tile_sums) {
+    __shared__ int64_t sh[33];
+    if (n_dev) n = *n_dev;
     const int64_t base = (int64_t)blockIdx.x * SCAN_TILE;
-    TO s = 0;
+    int64_t s = 0;
 #pragma unroll
     for (int i = 0; i < SCAN_I; ++i) {
         int64_t idx = base + (int64_t)i * SCAN_T + threadIdx.x;
-        if (idx < n) s += (TO)in[idx];
+        if (idx < n) s += in(idx);
     }
-    TO tot;
-    block_excl_scan<TO>(s, sh, tot);
+    int64_t tot;
+    block_excl_scan<int64_t>(s, sh, tot);
     if (threadIdx.x == 0) tile_sums[blockIdx.x] = tot;
 }
 
-// single block: exclusive scan of the tile sums, in place; writes the grand total
-template <class T>
-__global__ void k_scan_small(T* __restrict__ a, int64_t n, T* __restrict__ total) {
-    __shared__ T sh[33];
-    T carry = 0;
+// single block: exclusive scan of the tile sums, in place
+__global__ void k_scan_small(int64_t* __restrict__ a, int64_t n) {
+    __shared__ int64_t sh[33];
+    int64_t carry = 0;
     for (int64_t base = 0; base < n; base += blockDim.x) {
         int64_t idx = base + threadIdx.x;
-        T x = idx < n ? a[idx] : T(0);
-        T tot;
-        T e = block_excl_scan<T>(x, sh, tot);
+        int64_t x = idx < n ? a[idx] : 0;
+        int64_t tot;
+        int64_t e = block_excl_scan<int64_t>(x, sh, tot);
         if (idx < n) a[idx] = carry + e;
         carry += tot;
     }
-    if (threadIdx.x == 0 && total) *total = carry;
 }
 
-template <class TI, class TO>
-__global__ void k_tile_scan(const TI* __restrict__ in, TO* __restrict__ out, int64_t n,
-                            const TO* __restrict__ tile_offs) {
-    __shared__ TO sh[33];
+// SUMMED: tile_offs holds the tiles' exclusive offsets; else their sums, and
+// each block adds up those before it.  The last tile writes the total.
+template <class In, bool SUMMED>
+__global__ void k_tile_scan(In in, int64_t* __restrict__ out, int64_t n, const int64_t* __restrict__ n_dev,
+                            const int64_t* __restrict__ tile_offs, int64_t* __restrict__ total) {
+    __shared__ int64_t sh[33];
+    if (n_dev) n = *n_dev;
+    int64_t off;
+    if (SUMMED) off = tile_offs[blockIdx.x];
+    else {
+        int64_t s = 0;
+        for (int64_t t = threadIdx.x; t < blockIdx.x; t += SCAN_T) s += tile_offs[t];
+        block_excl_scan<int64_t>(s, sh, off);
+    }
     const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_I;
-    TO v[SCAN_I];
-    TO s = 0;
+    int64_t v[SCAN_I];
+    int64_t s = 0;
 #pragma unroll
     for (int i = 0; i < SCAN_I; ++i) {
         int64_t idx = base + i;
-        v[i] = idx < n ? (TO)in[idx] : TO(0);
+        v[i] = idx < n ? in(idx) : 0;
         s += v[i];
     }
-    TO tot;
-    TO e = block_excl_scan<TO>(s, sh, tot) + tile_offs[blockIdx.x];
+    int64_t tot;
+    int64_t e = block_excl_scan<int64_t>(s, sh, tot) + off;
+    if (total && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *total = off + tot;
 #pragma unroll
     for (int i = 0; i < SCAN_I; ++i) {
         int64_t idx = base + i;
@@ -159,30 +185,76 @@ __global__ void k_tile_scan(const TI* __restrict__ in, TO* __restrict__ out, int
     }
 }
 
-template <class TI, class TO>
-static void scan_excl(Ctx& c, const TI* in, TO* out, int64_t n, TO* d_total) {
+// short arrays: one block, one launch
+constexpr int SCAN_ONE_T = 1024;
+template <class In>
+__global__ void __launch_bounds__(SCAN_ONE_T) k_scan_one(In in, int64_t* __restrict__ out, int64_t n,
+                                                         const int64_t* __restrict__ n_dev, int64_t* __restrict__ total) {
+    __shared__ int64_t sh[33];
+    if (n_dev) n = *n_dev;
+    int64_t carry = 0;
+    for (int64_t base = 0; base < n; base += SCAN_ONE_T * SCAN_I) {
+        const int64_t b = base + (int64_t)threadIdx.x * SCAN_I;
+        int64_t v[SCAN_I];
+        int64_t s = 0;
+#pragma unroll
+        for (int i = 0; i < SCAN_I; ++i) {
+            v[i] = b + i < n ? in(b + i) : 0;
+            s += v[i];
+        }
+        int64_t tot;
+        int64_t e = carry + block_excl_scan<int64_t>(s, sh, tot);
+#pragma unroll
+        for (int i = 0; i < SCAN_I; ++i) {
+            if (b + i < n) out[b + i] = e;
+            e += v[i];
+        }
+        carry += tot;
+    }
+    if (total && threadIdx.x == 0) *total = carry;
+}
+
+// n: the length, or a bound on *n_dev
+constexpr int64_t SCAN_ONE = 16384;      // one block up to here: two passes of 8192
+constexpr int64_t SCAN_TWO_TILES = 2048; // a block adds up at most 8 sums per thread
+template <class In>
+static void scan_excl(Ctx& c, In in, int64_t* out, int64_t n, const int64_t* n_dev, int64_t* d_total) {
     if (n <= 0) {
-        if (d_total) GP_CUDA(cudaMemsetAsync(d_total, 0, sizeof(TO), c.s));
+        if (d_total) GP_CUDA(cudaMemsetAsync(d_total, 0, sizeof(int64_t), c.s));
+        return;
+    }
+    c.bytes += (int64_t)(2 * sizeof(int32_t) + sizeof(int64_t)) * n;
+    if (n <= SCAN_ONE) {
+        k_scan_one<In><<<1, SCAN_ONE_T, 0, c.s>>>(in, out, n, n_dev, d_total);
+        GP_LAUNCHED(c);
         return;
     }
     auto m = c.tmp->save();
-    int64_t nt = (n + SCAN_TILE - 1) / SCAN_TILE;
-    TO* sums = c.tmp_alloc<TO>(nt);
-    k_tile_reduce<TI, TO><<<(unsigned)nt, SCAN_T, 0, c.s>>>(in, n, sums);
+    const int64_t nt = (n + SCAN_TILE - 1) / SCAN_TILE;
+    int64_t* sums = c.tmp_alloc<int64_t>(nt);
+    k_tile_reduce<In><<<(unsigned)nt, SCAN_T, 0, c.s>>>(in, n, n_dev, sums);
     GP_LAUNCHED(c);
-    k_scan_small<TO><<<1, 1024, 0, c.s>>>(sums, nt, d_total);
-    GP_LAUNCHED(c);
-    k_tile_scan<TI, TO><<<(unsigned)nt, SCAN_T, 0, c.s>>>(in, out, n, sums);
-    GP_LAUNCHED(c);
-    c.bytes += (int64_t)(2 * sizeof(TI) + sizeof(TO)) * n;
+    if (nt <= SCAN_TWO_TILES) {
+        k_tile_scan<In, false><<<(unsigned)nt, SCAN_T, 0, c.s>>>(in, out, n, n_dev, sums, d_total);
+        GP_LAUNCHED(c);
+    } else {
+        k_scan_small<<<1, 1024, 0, c.s>>>(sums, nt);
+        GP_LAUNCHED(c);
+        k_tile_scan<In, true><<<(unsigned)nt, SCAN_T, 0, c.s>>>(in, out, n, n_dev, sums, d_total);
+        GP_LAUNCHED(c);
+    }
     c.tmp->restore(m);
 }
 
 void scan_excl_i32_to_i64(Ctx& c, const int32_t* in, int64_t* out, int64_t n, int64_t* d_total) {
-    scan_excl<int32_t, int64_t>(c, in, out, n, d_total);
+    scan_excl(c, InArray<int32_t>{in}, out, n, nullptr, d_total);
 }
 void scan_excl_i64(Ctx& c, const int64_t* in, int64_t* out, int64_t n, int64_t* d_total) {
-    scan_excl<int64_t, int64_t>(c, in, out, n, d_total);
+    scan_excl(c, InArray<int64_t>{in}, out, n, nullptr, d_total);
+}
+void scan_list_weights(Ctx& c, const int32_t* list, const int32_t* vw, int64_t* out, int64_t n, const int64_t* n_dev,
+                       int64_t* d_total) {
+    scan_excl(c, InListWeight{list, vw}, out, n, n_dev, d_total);
 }
 
 // ================================================================ radix sort
@@ -193,9 +265,10 @@ constexpr int RS_W = RS_T / 32;           // warps per tile
 constexpr int RS_WITEMS = 32 * RS_I;      // items per warp (contiguous)
 
 // digit-major counts: counts[d * ntiles + tile]
-__global__ void k_rs_hist(const uint64_t* __restrict__ keys, int64_t n, int shift,
+__global__ void k_rs_hist(const uint64_t* __restrict__ keys, int64_t n, const int64_t* __restrict__ n_dev, int shift,
                           int32_t* __restrict__ counts, int64_t ntiles) {
     __shared__ int32_t h[256];
+    if (n_dev) n = *n_dev;
     h[threadIdx.x] = 0;
     __syncthreads();
     const int64_t base = (int64_t)blockIdx.x * RS_TILE;
@@ -208,10 +281,31 @@ __global__ void k_rs_hist(const uint64_t* __restrict__ keys, int64_t n, int shif
     counts[(int64_t)threadIdx.x * ntiles + blockIdx.x] = h[threadIdx.x];
 }
 
+// one block per digit: exclusive scan of its tile counts in place, its total apart
+__global__ void __launch_bounds__(RS_T) k_rs_scan(int32_t* __restrict__ counts, int64_t ntiles,
+                                                  int32_t* __restrict__ totals) {
+    __shared__ int32_t sh[33];
+    int32_t* row = counts + (int64_t)blockIdx.x * ntiles;
+    int32_t carry = 0;
+    for (int64_t base = 0; base < ntiles; base += RS_T) {
+        const int64_t i = base + threadIdx.x;
+        const int32_t x = i < ntiles ? row[i] : 0;
+        int32_t tot;
+        const int32_t e = block_excl_scan<int32_t>(x, sh, tot);
+        if (i < ntiles) row[i] = carry + e;
+        carry += tot;
+    }
+    if (threadIdx.x == 0) totals[blockIdx.x] = carry;
+}
+
 __global__ void __launch_bounds__(RS_T) k_rs_scatter(const uint64_t* __restrict__ kin, const int32_t* __restrict__ vin,
                              uint64_t* __restrict__ kout, int32_t* __restrict__ vout,
-                             int64_t n, int shift, const int64_t* __restrict__ offs, int64_t ntiles) {
+                             int64_t n, const int64_t* __restrict__ n_dev, int shift,
+                             const int32_t* __restrict__ offs, const int32_t* __restrict__ totals, int64_t ntiles) {
     __shared__ int32_t wcnt[RS_W][256];
+    __shared__ int32_t dbase[256];
+    __shared__ int32_t sh[33];
+    if (n_dev) n = *n_dev;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (int i = threadIdx.x; i < RS_W * 256; i += RS_T) (&wcnt[0][0])[i] = 0;
     __syncthreads();
@@ -237,7 +331,9 @@ __global__ void __launch_bounds__(RS_T) k_rs_scatter(const uint64_t* __restrict_
     // exclusive prefix over warps per digit, plus the global tile offset
     {
         int d = threadIdx.x;  // RS_T == 256 digits
-        int64_t off = offs[(int64_t)d * ntiles + blockIdx.x];
+        int32_t all;
+        const int32_t first = block_excl_scan<int32_t>(totals[d], sh, all);   // the digit's base
+        const int32_t off = first + offs[(int64_t)d * ntiles + blockIdx.x];
         int32_t run = 0;
 #pragma unroll
         for (int ww = 0; ww < RS_W; ++ww) {
@@ -245,9 +341,6 @@ __global__ void __launch_bounds__(RS_T) k_rs_scatter(const uint64_t* __restrict_
             wcnt[ww][d] = run;
             run += cnt;
         }
-        // store the 64-bit base split: tile offsets fit int64; keep it in a
-        // second table indexed by digit
-        __shared__ int64_t dbase[256];
         dbase[d] = off;
         __syncthreads();
         // pass B: positions
@@ -260,7 +353,7 @@ __global__ void __launch_bounds__(RS_T) k_rs_scatter(const uint64_t* __restrict_
             int32_t basecnt = ok ? wcnt[w][dg[i]] : 0;
             __syncwarp();
             if (ok) {
-                int64_t pos = dbase[dg[i]] + basecnt + __popc(peers & lt);
+                const int64_t pos = (int64_t)dbase[dg[i]] + basecnt + __popc(peers & lt);
                 if (GP_IN(pos, n)) {
                     kout[pos] = k[i];
                     vout[pos] = v[i];
@@ -273,21 +366,23 @@ __global__ void __launch_bounds__(RS_T) k_rs_scatter(const uint64_t* __restrict_
 }
 
 void radix_sort_pairs(Ctx& c, uint64_t* keys, int32_t* vals, uint64_t* keys_tmp, int32_t* vals_tmp,
-                      int64_t n, int bits) {
+                      int64_t n, int bits, const int64_t* n_dev) {
     if (n <= 1 || bits <= 0) return;
+    if (n > INT32_MAX) throw GpError(GP_EINTERNAL, "radix sort of more than 2^31 - 1 items");
     auto m = c.tmp->save();
     const int64_t ntiles = (n + RS_TILE - 1) / RS_TILE;
     int32_t* counts = c.tmp_alloc<int32_t>(256 * ntiles);
-    int64_t* offs = c.tmp_alloc<int64_t>(256 * ntiles);
+    int32_t* totals = c.tmp_alloc<int32_t>(256);
     int passes = (bits + 7) / 8;
     uint64_t* ka = keys; int32_t* va = vals;
     uint64_t* kb = keys_tmp; int32_t* vb = vals_tmp;
     for (int p = 0; p < passes; ++p) {
         int shift = 8 * p;
-        k_rs_hist<<<(unsigned)ntiles, RS_T, 0, c.s>>>(ka, n, shift, counts, ntiles);
+        k_rs_hist<<<(unsigned)ntiles, RS_T, 0, c.s>>>(ka, n, n_dev, shift, counts, ntiles);
         GP_LAUNCHED(c);
-        scan_excl_i32_to_i64(c, counts, offs, 256 * ntiles, nullptr);
-        k_rs_scatter<<<(unsigned)ntiles, RS_T, 0, c.s>>>(ka, va, kb, vb, n, shift, offs, ntiles);
+        k_rs_scan<<<256, RS_T, 0, c.s>>>(counts, ntiles, totals);
+        GP_LAUNCHED(c);
+        k_rs_scatter<<<(unsigned)ntiles, RS_T, 0, c.s>>>(ka, va, kb, vb, n, n_dev, shift, counts, totals, ntiles);
         GP_LAUNCHED(c);
         c.bytes += n * (8 + 2 * 12);
         std::swap(ka, kb);

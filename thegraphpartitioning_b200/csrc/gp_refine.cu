@@ -75,7 +75,8 @@ __device__ __forceinline__ bool lp_candidate(int32_t g, int32_t own, int32_t den
 // written by CTA 0; LP candidates are appended to clist[bucket] (any order:
 // each is evaluated on its own), with [S_NL0..S_NL2] their counts and
 // [S_CDEG] the sum of their degrees.  Rebalance candidates are the vertices
-// with dest >= 0; they are compacted in vertex order afterwards.
+// with dest >= 0, [S_CDEG] their number; they are collected in vertex order
+// afterwards.
 struct ConnArgs {
     DGraph g;
     int32_t k;
@@ -104,6 +105,9 @@ struct ConnArgs {
     int64_t* hsum;
     int32_t* hdone;
     uint64_t* pdg;              // label propagation: pdg_pack(part, dest, gain) per row (nullptr: none)
+    const int64_t* prev_moves;  // moves of the step before (nullptr: none)
+    int64_t* host;              // host-resident copy of the status block, written by the pass's last
+    int nblocks;                // block out of nblocks (over all its launches)
     int lp_dg;                  // label propagation also writes dest and gain (no pdg, or someone
                                 // else reads them)
 };
@@ -432,6 +436,7 @@ __device__ __forceinline__ void conn_group(const ConnArgs& A, int64_t ub, int nu
         acc += x.cross;
         take = conn_decide<PT>(A, mode, r.active, r.v, r.p, x.tot, x.cross, x.bk, x.bq, light);
         if (take) cdeg += r.end - r.beg;
+        else if (mode == MODE_RB && r.active) ++cdeg;
     }
     if (A.clist[0] == nullptr || !__any_sync(0xffffffffu, take)) return;
 #pragma unroll
@@ -478,17 +483,31 @@ __device__ __forceinline__ int conn_head(const ConnArgs& A, uint8_t* over, ConnH
     }
     return mode;
 }
-// adds every thread's cross weight to the status block, one atomic per block
+// adds every thread's cross weight to the status block, one atomic per block;
+// the pass's last block then writes the block to the host (pinned, mapped
+// memory: no copy operation between the pass and the host's wait)
 __device__ __forceinline__ void conn_tail(const ConnArgs& A, int64_t acc, int64_t* s_red) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     acc = warp_sum(acc);
     __syncthreads();
     if (lane == 0) s_red[w] = acc;
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (w != 0) return;
+    uint32_t last = 0;
+    if (lane == 0) {
         int64_t s = 0;
         for (int i = 0; i < RW; ++i) s += s_red[i];
         if (s) atomicAdd((unsigned long long*)&A.status[S_CROSS], (unsigned long long)s);
+        __threadfence();
+        last = atomicAdd((unsigned long long*)&A.status[S_DONE], 1ull) == (unsigned long long)A.nblocks - 1ull;
+    }
+    if (!__shfl_sync(0xffffffffu, last, 0)) return;
+    __threadfence();
+    // one 72-byte store of the warp: the status slots and the last step's moves
+    static_assert(S_STEP_MOVES == S_NRESET, "slots written together");
+    if (lane <= S_NRESET) {
+        const int64_t* from = lane < S_NRESET ? A.status + lane : A.prev_moves;
+        A.host[lane] = from ? (int64_t)__ldcg((const unsigned long long*)from) : 0;
     }
 }
 
@@ -518,6 +537,7 @@ __global__ void __launch_bounds__(RT, 4) k_conn_short(ConnArgs A) {
             acc += x.cross;
             take = conn_decide<PT>(A, mode, r.active, r.v, r.p, x.tot, x.cross, x.bk, x.bq, light);
             if (take) cdeg += r.end - r.beg;
+            else if (mode == MODE_RB && r.active) ++cdeg;
         }
         warp_push(take, r.v, A.clist[0], conn_list_count(A, 0), A.g.n);
     }
@@ -630,6 +650,7 @@ __global__ void __launch_bounds__(RT, SHORT ? 4 : 5) k_conn(ConnArgs A) {
                 const int64_t rdeg = A.g.rp[v + 1] - A.g.rp[v];
                 if (conn_decide<PT>(A, mode, active, (int32_t)v, p, (int32_t)tot, (int32_t)cross, (uint32_t)bk, bq, light))
                     atomicAdd((unsigned long long*)&A.status[S_CDEG], (unsigned long long)rdeg);
+                else if (mode == MODE_RB && active) atomicAdd((unsigned long long*)&A.status[S_CDEG], 1ull);
             }
         }
     } else {
@@ -692,14 +713,14 @@ struct ApplyArgs {
 };
 
 template <class PT>
-__device__ __forceinline__ void ab_commit(const ApplyArgs& A, int64_t v, int32_t p, int32_t d, int64_t* delta,
+__device__ __forceinline__ void ab_commit(const ApplyArgs& A, int64_t v, int32_t p, int32_t d, int32_t* delta,
                                           int64_t& moves) {
     if (!GP_IN(d, A.k) || !GP_IN(p, A.k)) return;
     ((PT*)A.pc_next)[v] = (PT)d;
     A.lock_next[v] = 1;
-    const int64_t wv = A.g.vw ? A.g.vw[v] : 1;
-    atomicAdd((unsigned long long*)&delta[d], (unsigned long long)wv);
-    atomicAdd((unsigned long long*)&delta[p], (unsigned long long)(-wv));
+    const int32_t wv = A.g.vw ? A.g.vw[v] : 1;
+    atomicAdd(&delta[d], wv);
+    atomicAdd(&delta[p], -wv);
     ++moves;
 }
 
@@ -744,7 +765,7 @@ __device__ __forceinline__ int32_t ab_short_n(const ApplyArgs& A, int64_t v, int
     return t;
 }
 template <class PT>
-__device__ __forceinline__ void ab_short(const ApplyArgs& A, int64_t v, int64_t* delta, int64_t& moves) {
+__device__ __forceinline__ void ab_short(const ApplyArgs& A, int64_t v, int32_t* delta, int64_t& moves) {
     int32_t p = -1, d = -1, gv = 0;
     int64_t beg = 0;
     int len = 0;
@@ -761,7 +782,7 @@ __device__ __forceinline__ void ab_short(const ApplyArgs& A, int64_t v, int64_t*
 
 // candidate rows of at most TILE entries, TILE lanes each (v < 0: none)
 template <int TILE, class PT>
-__device__ __forceinline__ void ab_tile(const ApplyArgs& A, int64_t v, int64_t* delta, int64_t& moves) {
+__device__ __forceinline__ void ab_tile(const ApplyArgs& A, int64_t v, int32_t* delta, int64_t& moves) {
     const int lane = threadIdx.x & 31, tl = lane & (TILE - 1);
     int32_t t = 0, p = -1, d = -1;
     if (v >= 0) {
@@ -823,7 +844,7 @@ __device__ __forceinline__ int32_t ab_sum(const ApplyArgs& A, int64_t beg, int64
 
 // one candidate row of 33..heavy_deg entries per warp, 128 entries per sweep
 template <class PT>
-__device__ __forceinline__ void ab_warp(const ApplyArgs& A, int64_t v, int64_t* delta, int64_t& moves) {
+__device__ __forceinline__ void ab_warp(const ApplyArgs& A, int64_t v, int32_t* delta, int64_t& moves) {
     const int lane = threadIdx.x & 31;
     int32_t p, d, gv;
     ab_row<PT>(A, v, p, d, gv);
@@ -833,7 +854,7 @@ __device__ __forceinline__ void ab_warp(const ApplyArgs& A, int64_t v, int64_t* 
 
 template <class PT>
 __global__ void __launch_bounds__(RT, 4) k_lp_apply(ApplyArgs A) {
-    extern __shared__ int64_t delta[];
+    extern __shared__ int32_t delta[];   // part-weight changes (32-bit shared atomics, see rb_delta_begin)
     __shared__ int64_t s_red[RW];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (int q = threadIdx.x; q < A.k; q += RT) delta[q] = 0;
@@ -893,32 +914,74 @@ __global__ void __launch_bounds__(RT, 4) k_lp_apply(ApplyArgs A) {
     __syncthreads();
     if (lane == 0 && moves) atomicAdd((unsigned long long*)A.moves_out, (unsigned long long)moves);
     for (int q = threadIdx.x; q < A.k; q += RT)
-        if (delta[q]) atomicAdd((unsigned long long*)&A.pw[q], (unsigned long long)delta[q]);
+        if (delta[q]) atomicAdd((unsigned long long*)&A.pw[q], (unsigned long long)(int64_t)delta[q]);
 }
 
 // ------------------------------------------------------------------ rebalance
-__global__ void k_gather_vw(int64_t cnt, const int32_t* __restrict__ vidx, const int32_t* __restrict__ vw,
-                            int32_t* __restrict__ out) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += (int64_t)gridDim.x * blockDim.x)
-        out[i] = vw ? vw[vidx[i]] : 1;
-}
-
 constexpr int RB_SHIFT = 10;   // key = segment << 10 | loss bucket
 
-__global__ void k_rb_flags(int64_t n, const int32_t* __restrict__ dest, int32_t* __restrict__ flag) {
-    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x)
-        flag[v] = dest[v] >= 0 ? 1 : 0;
+// Candidates (dest >= 0) in vertex order with key (source << 10 | bucket(loss)):
+// k_rb_count counts those of every tile of 8192 vertices, k_rb_collect adds up
+// the counts of the tiles before its own and writes them (each warp 1024
+// vertices: one ballot per 32, then the offsets of the warps before), clearing
+// the locks on the way.  dest is read twice and nothing but the candidates
+// written: 256^3 grid, level 0 (16.8 M vertices, one overweight part in 32)
+// 15 + 55 us against 200 us for flags, a scan of them and a gather.
+constexpr int RB_TILE = 32 * 32 * RW;
+__global__ void __launch_bounds__(RT) k_rb_count(int64_t n, const int32_t* __restrict__ dest, int32_t* __restrict__ cnt) {
+    __shared__ int32_t s_cnt[RW];
+    const int64_t base = (int64_t)blockIdx.x * RB_TILE;
+    int32_t c = 0;
+#pragma unroll 8
+    for (int i = 0; i < RB_TILE / RT; ++i) {
+        const int64_t v = base + (int64_t)i * RT + threadIdx.x;
+        c += v < n && dest[v] >= 0 ? 1 : 0;
+    }
+    c = (int32_t)__reduce_add_sync(0xffffffffu, (uint32_t)c);
+    if ((threadIdx.x & 31) == 0) s_cnt[threadIdx.x >> 5] = c;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int32_t t = 0;
+        for (int i = 0; i < RW; ++i) t += s_cnt[i];
+        cnt[blockIdx.x] = t;
+    }
 }
-
-// candidates in vertex order with key (source << 10 | bucket(loss))
-__global__ void k_rb_compact(int64_t n, const int32_t* __restrict__ flag, const int64_t* __restrict__ pos,
-                             const void* __restrict__ pc, int pcb, const int32_t* __restrict__ gain,
-                             uint64_t* __restrict__ keys, int32_t* __restrict__ vals) {
-    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
-        if (!flag[v]) continue;
-        const int64_t i = pos[v];
-        keys[i] = ((uint64_t)(uint32_t)load_pc(pc, pcb, v) << RB_SHIFT) | loss_bucket(-gain[v]);
-        vals[i] = (int32_t)v;
+__global__ void __launch_bounds__(RT) k_rb_collect(int64_t n, const int32_t* __restrict__ dest,
+                                                   const int32_t* __restrict__ cnt, int64_t ncand,
+                                                   const void* __restrict__ pc, int pcb,
+                                                   const int32_t* __restrict__ gain, uint8_t* __restrict__ lock,
+                                                   uint64_t* __restrict__ keys, int32_t* __restrict__ vals) {
+    __shared__ int64_t sh[33];
+    __shared__ int32_t s_cnt[RW];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t lt = (1u << lane) - 1u;
+    int64_t before = 0, s = 0;
+    for (int64_t t = threadIdx.x; t < blockIdx.x; t += RT) s += cnt[t];
+    block_excl_scan<int64_t>(s, sh, before);
+    const int64_t base = (int64_t)blockIdx.x * RB_TILE + (int64_t)w * 1024;
+    uint32_t mine = 0;   // the ballot of step lane
+    int32_t total = 0;
+#pragma unroll 8
+    for (int i = 0; i < 32; ++i) {
+        const int64_t v = base + 32 * i + lane;
+        const uint32_t m = __ballot_sync(0xffffffffu, v < n && dest[v] >= 0);
+        if (v < n) lock[v] = 0;
+        if (lane == i) mine = m;
+        total += __popc(m);
+    }
+    if (lane == 0) s_cnt[w] = total;
+    __syncthreads();
+    int64_t pos = before;
+    for (int i = 0; i < w; ++i) pos += s_cnt[i];
+    for (int i = 0; i < 32; ++i) {
+        const uint32_t m = __shfl_sync(0xffffffffu, mine, i);
+        const int64_t at = pos + __popc(m & lt);
+        if (((m >> lane) & 1u) && GP_IN(at, ncand)) {
+            const int64_t v = base + 32 * i + lane;
+            keys[at] = ((uint64_t)(uint32_t)load_pc(pc, pcb, v) << RB_SHIFT) | loss_bucket(-gain[v]);
+            vals[at] = (int32_t)v;
+        }
+        pos += __popc(m);
     }
 }
 
@@ -933,59 +996,100 @@ __device__ __forceinline__ int64_t seg_start(const uint64_t* keys, int64_t i, ui
 
 // first index of every key segment (key >> RB_SHIFT = d, d = 0..k) of a
 // sorted candidate list: k + 1 searches instead of one per candidate
-__global__ void k_seg_first(int64_t cnt, const uint64_t* __restrict__ keys, int32_t k, int64_t* __restrict__ first) {
+__global__ void k_seg_first(const int64_t* __restrict__ cnt, const uint64_t* __restrict__ keys, int32_t k,
+                            int64_t* __restrict__ first) {
     for (int64_t d = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; d <= k; d += (int64_t)gridDim.x * blockDim.x)
-        first[d] = seg_start(keys, cnt, (uint64_t)d);
+        first[d] = seg_start(keys, *cnt, (uint64_t)d);
 }
 
-// flag[i] = 1 when the move keeps its source within the excess prefix
-__global__ void k_rb_source(int64_t cnt, const uint64_t* __restrict__ keys, const int64_t* __restrict__ segf,
-                            const int64_t* __restrict__ pre, const int64_t* __restrict__ pw, int64_t Lmax,
-                            int32_t* __restrict__ flag) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += (int64_t)gridDim.x * blockDim.x) {
-        const uint64_t src = keys[i] >> RB_SHIFT;
-        const int64_t s = segf[src];
-        flag[i] = (pre[i] - pre[s]) < (pw[src] - Lmax) ? 1 : 0;
+// What the sorted candidates let each source part give up, in one block: a
+// source keeps the prefix of its candidates whose weight before the candidate
+// is below its excess.  Also the part weights before the step and the
+// concatenated free capacities (strong).  pre: exclusive weight prefix of the
+// list (pre[ncand] = total).
+struct RbPlan {
+    int64_t* seg;      // first candidate of the source
+    int64_t* acc;      // candidates it keeps
+    int64_t* off;      // kept candidates of the sources before it
+    int64_t* woff;     // and their weight
+    int64_t* cum;      // k + 1: free capacity of the parts before
+    int64_t* snap;     // part weights before the step
+    int64_t* n2;       // kept candidates in all
+};
+__global__ void __launch_bounds__(GP_MAX_K) k_rb_plan(int64_t ncand, const uint64_t* __restrict__ keys,
+                                                      const int64_t* __restrict__ pre, const int64_t* __restrict__ pw,
+                                                      int64_t Lmax, int32_t k, RbPlan P) {
+    __shared__ int64_t sh[33];
+    const int q = threadIdx.x;
+    const int64_t x = q < k ? pw[q] : 0;
+    int64_t a = 0, wa = 0;
+    if (q < k) {
+        const int64_t s = seg_start(keys, ncand, (uint64_t)q), e = x > Lmax ? seg_start(keys, ncand, (uint64_t)q + 1) : s;
+        int64_t lo = s, hi = e;   // first candidate whose weight before reaches the excess
+        const int64_t p0 = s < ncand ? pre[s] : 0;
+        while (lo < hi) {
+            const int64_t mid = (lo + hi) >> 1;
+            if (pre[mid] - p0 < x - Lmax) lo = mid + 1; else hi = mid;
+        }
+        a = lo - s;
+        wa = a > 0 ? pre[lo] - p0 : 0;
+        P.seg[q] = s; P.acc[q] = a; P.snap[q] = x;
     }
+    int64_t tot;
+    int64_t e = block_excl_scan<int64_t>(a, sh, tot);
+    if (q < k) P.off[q] = e;
+    if (q == 0) *P.n2 = tot;
+    e = block_excl_scan<int64_t>(wa, sh, tot);
+    if (q < k) P.woff[q] = e;
+    e = block_excl_scan<int64_t>(q < k && x <= Lmax ? Lmax - x : 0, sh, tot);
+    if (q < k) P.cum[q] = e;
+    if (q == 0) P.cum[k] = tot;
 }
 
-// weak: accepted moves, in list order, re-keyed by (dest << 10 | bucket)
-__global__ void k_rb_rekey(int64_t cnt, const uint64_t* __restrict__ keys, const int32_t* __restrict__ vals,
-                           const int32_t* __restrict__ flag, const int64_t* __restrict__ pos,
+// weak: kept candidates, in list order, re-keyed by (dest << 10 | bucket)
+__global__ void k_rb_rekey(int64_t cnt, const uint64_t* __restrict__ keys, const int32_t* __restrict__ vals, RbPlan P,
                            const int32_t* __restrict__ dest, uint64_t* __restrict__ keys2, int32_t* __restrict__ vals2) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += (int64_t)gridDim.x * blockDim.x) {
-        if (!flag[i]) continue;
+        const uint64_t key = keys[i];
+        const int64_t q = (int64_t)(key >> RB_SHIFT), r = i - P.seg[q];
+        if (r >= P.acc[q]) continue;
         const int32_t v = vals[i];
-        const int64_t j = pos[i];
-        keys2[j] = ((uint64_t)(uint32_t)dest[v] << RB_SHIFT) | (keys[i] & ((1ull << RB_SHIFT) - 1));
+        const int64_t j = P.off[q] + r;
+        if (!GP_IN(j, cnt)) continue;
+        keys2[j] = ((uint64_t)(uint32_t)dest[v] << RB_SHIFT) | (key & ((1ull << RB_SHIFT) - 1));
         vals2[j] = v;
     }
 }
 
 // part-weight changes and moves of a block, added to the global totals once
-// per part (dynamic shared memory: k int64)
-__device__ __forceinline__ void rb_delta_begin(int64_t* delta, int32_t k) {
+// per part (dynamic shared memory: k int32).  The vertex weights add up to less
+// than 2^31, so every partial sum fits in 32 bits; a 64-bit shared add is a
+// compare-and-swap loop, which a rebalance step (most moves leave one part)
+// drives into full contention: k_rb_step_cta on R-MAT 20 (k = 64), longest launch 757 -> 123 us
+__device__ __forceinline__ void rb_delta_begin(int32_t* delta, int32_t k) {
     for (int q = threadIdx.x; q < k; q += blockDim.x) delta[q] = 0;
     __syncthreads();
 }
-__device__ __forceinline__ void rb_delta_end(int64_t* delta, int32_t k, int64_t nmoves, int64_t* __restrict__ pw,
+__device__ __forceinline__ void rb_delta_end(int32_t* delta, int32_t k, int64_t nmoves, int64_t* __restrict__ pw,
                                              int64_t* __restrict__ moves) {
     for (int o = 16; o > 0; o >>= 1) nmoves += __shfl_xor_sync(0xffffffffu, nmoves, o);
     if ((threadIdx.x & 31) == 0 && nmoves) atomicAdd((unsigned long long*)moves, (unsigned long long)nmoves);
     __syncthreads();
     for (int q = threadIdx.x; q < k; q += blockDim.x)
-        if (delta[q]) atomicAdd((unsigned long long*)&pw[q], (unsigned long long)delta[q]);
+        if (delta[q]) atomicAdd((unsigned long long*)&pw[q], (unsigned long long)(int64_t)delta[q]);
 }
 
 // weak: keep moves whose destination prefix fits the capacity; apply
-__global__ void k_rb_weak_apply(int64_t cnt, const uint64_t* __restrict__ keys, const int64_t* __restrict__ segf,
+__global__ void k_rb_weak_apply(const int64_t* __restrict__ cnt_dev, const uint64_t* __restrict__ keys,
+                                const int64_t* __restrict__ segf,
                                 const int32_t* __restrict__ vals, const int64_t* __restrict__ pre,
                                 const int32_t* __restrict__ vw, const int64_t* __restrict__ pw_snap, int64_t Lmax,
                                 int32_t k, void* __restrict__ pc, int pcb, uint8_t* __restrict__ lock,
                                 int64_t* __restrict__ pw, int64_t* __restrict__ moves) {
-    extern __shared__ int64_t rb_delta[];
+    extern __shared__ int32_t rb_delta[];
     rb_delta_begin(rb_delta, k);
     int64_t nm = 0;
+    const int64_t cnt = *cnt_dev;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += (int64_t)gridDim.x * blockDim.x) {
         const uint64_t d = keys[i] >> RB_SHIFT;
         const int64_t s = segf[d];
@@ -996,8 +1100,8 @@ __global__ void k_rb_weak_apply(int64_t cnt, const uint64_t* __restrict__ keys, 
             store_pc(pc, pcb, v, (int32_t)d);
             lock[v] = 1;
             if (GP_IN(d, k) && GP_IN(p, k)) {
-                atomicAdd((unsigned long long*)&rb_delta[d], (unsigned long long)wv);
-                atomicAdd((unsigned long long*)&rb_delta[p], (unsigned long long)(-wv));
+                atomicAdd(&rb_delta[d], (int32_t)wv);
+                atomicAdd(&rb_delta[p], -(int32_t)wv);
             }
             ++nm;
         }
@@ -1005,35 +1109,20 @@ __global__ void k_rb_weak_apply(int64_t cnt, const uint64_t* __restrict__ keys, 
     rb_delta_end(rb_delta, k, nm, pw, moves);
 }
 
-// strong: cumulative free capacity of non-overweight parts
-__global__ void k_cumfree(int32_t k, const int64_t* __restrict__ pw, int64_t Lmax, int64_t* __restrict__ cum) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    int64_t s = 0;
-    cum[0] = 0;
-    for (int q = 0; q < k; ++q) {
-        const int64_t x = pw[q];
-        s += (x > Lmax) ? 0 : (Lmax - x);
-        cum[q + 1] = s;
-    }
-}
-
-__global__ void k_mask_vw(int64_t cnt, const int32_t* __restrict__ flag, const int32_t* __restrict__ wvals,
-                          int32_t* __restrict__ out) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += (int64_t)gridDim.x * blockDim.x)
-        out[i] = flag[i] ? wvals[i] : 0;
-}
-
-__global__ void k_rb_strong_apply(int64_t cnt, const int32_t* __restrict__ vals, const int32_t* __restrict__ flag,
-                                  const int64_t* __restrict__ P, const int32_t* __restrict__ vw,
-                                  const int64_t* __restrict__ cum, int32_t k, void* __restrict__ pc, int pcb,
+// strong: kept candidates laid over the concatenated free capacities
+__global__ void k_rb_strong_apply(int64_t cnt, const uint64_t* __restrict__ keys, const int32_t* __restrict__ vals,
+                                  const int64_t* __restrict__ P, RbPlan plan, const int32_t* __restrict__ vw,
+                                  int32_t k, void* __restrict__ pc, int pcb,
                                   uint8_t* __restrict__ lock, int64_t* __restrict__ pw,
                                   int64_t* __restrict__ moves) {
-    extern __shared__ int64_t rb_delta[];
+    const int64_t* __restrict__ cum = plan.cum;
+    extern __shared__ int32_t rb_delta[];
     rb_delta_begin(rb_delta, k);
     int64_t nm = 0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += (int64_t)gridDim.x * blockDim.x) {
-        if (!flag[i]) continue;
-        const int64_t pre = P[i];
+        const int64_t src = (int64_t)(keys[i] >> RB_SHIFT), s = plan.seg[src];
+        if (i - s >= plan.acc[src]) continue;
+        const int64_t pre = plan.woff[src] + (P[i] - P[s]);
         if (pre >= cum[k]) continue;
         // q with cum[q] <= pre < cum[q+1]: last index with cum <= pre
         int lo = 0, hi = k;  // search in cum[0..k]
@@ -1049,8 +1138,8 @@ __global__ void k_rb_strong_apply(int64_t cnt, const int32_t* __restrict__ vals,
             store_pc(pc, pcb, v, q);
             lock[v] = 1;
             if (GP_IN(p, k)) {
-                atomicAdd((unsigned long long*)&rb_delta[q], (unsigned long long)wv);
-                atomicAdd((unsigned long long*)&rb_delta[p], (unsigned long long)(-wv));
+                atomicAdd(&rb_delta[q], (int32_t)wv);
+                atomicAdd(&rb_delta[p], -(int32_t)wv);
             }
             ++nm;
         }
@@ -1065,16 +1154,23 @@ __global__ void k_project(int64_t n, const int32_t* __restrict__ cmap, const int
         pf[v] = pc[cmap[v]];
 }
 
+// unit weights: 32-bit shared counts; given weights: 64-bit sums (an edge-cut
+// call takes weights whose total is not checked against 2^31)
 __global__ void k_part_weights(int64_t n, const int32_t* __restrict__ part, const int32_t* __restrict__ vw, int32_t k,
                                int64_t* __restrict__ pw) {
     extern __shared__ int64_t spw[];
+    int32_t* cnt = (int32_t*)spw;
     for (int q = threadIdx.x; q < k; q += blockDim.x) spw[q] = 0;
     __syncthreads();
-    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x)
-        atomicAdd((unsigned long long*)&spw[part[v]], (unsigned long long)(vw ? vw[v] : 1));
+    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
+        if (vw) atomicAdd((unsigned long long*)&spw[part[v]], (unsigned long long)vw[v]);
+        else atomicAdd(&cnt[part[v]], 1);
+    }
     __syncthreads();
-    for (int q = threadIdx.x; q < k; q += blockDim.x)
-        if (spw[q]) atomicAdd((unsigned long long*)&pw[q], (unsigned long long)spw[q]);
+    for (int q = threadIdx.x; q < k; q += blockDim.x) {
+        const int64_t x = vw ? spw[q] : (int64_t)cnt[q];
+        if (x) atomicAdd((unsigned long long*)&pw[q], (unsigned long long)x);
+    }
 }
 
 // warp per row: directed cross weight (d_cross2 accumulates 2*cut)
@@ -1175,6 +1271,11 @@ void cut_and_weights(Ctx& c, const DGraph& g, const int32_t* part, int32_t k, in
 // (source, loss bucket, id), then (destination, loss bucket, source, id).
 constexpr int CT = 1024, CW = CT / 32;
 constexpr int64_t kCtaMaxN = 16384;                 // candidates sorted in shared memory (8 B each)
+// A rebalance step of at most this many candidates is taken by one block
+// (k_rb_step_cta), of more by about 20 launches over the whole chip.  1024, 2048,
+// 4096, 16384: weighted RGG 150k k = 300 7.8 / 7.2 / 7.0 / 7.0 ms, R-MAT 20 k = 64
+// 44.8 / 44.1 / 44.2 / 45.5 ms, Chung-Lu 262k k = 64 17.4 / 16.8 / 16.6 / 17.3 ms.
+constexpr int64_t kRbCta = 4096;
 
 struct CtaRefineArgs {
     DGraph g;
@@ -1299,7 +1400,7 @@ struct RbCta {
 };
 
 __device__ int64_t cta_rebalance(const RbCta& R, int mode, int64_t n, const int32_t* cand, int64_t ncand_in,
-                                 int64_t* s_pw, int64_t* s_snap, int64_t* s_cum, uint64_t* s_keys, int64_t* sh) {
+                                 int32_t* s_pw, int32_t* s_snap, int64_t* s_cum, uint64_t* s_keys, int64_t* sh) {
     const int32_t k = R.k;
     const int64_t Lmax = R.Lmax;
     uint8_t* lock = R.lock;
@@ -1359,8 +1460,8 @@ __device__ int64_t cta_rebalance(const RbCta& R, int mode, int64_t n, const int3
                 const int32_t p = load_pc(R.pc, R.pcb, v);
                 store_pc(R.pc, R.pcb, v, d);
                 lock[v] = 1;
-                atomicAdd((unsigned long long*)&s_pw[d], (unsigned long long)wv);
-                atomicAdd((unsigned long long*)&s_pw[p], (unsigned long long)(-wv));
+                atomicAdd(&s_pw[d], (int32_t)wv);
+                atomicAdd(&s_pw[p], -(int32_t)wv);
                 ++moves;
             }
         }
@@ -1390,8 +1491,8 @@ __device__ int64_t cta_rebalance(const RbCta& R, int mode, int64_t n, const int3
                 const int32_t p = load_pc(R.pc, R.pcb, v);
                 store_pc(R.pc, R.pcb, v, lo);
                 lock[v] = 1;
-                atomicAdd((unsigned long long*)&s_pw[lo], (unsigned long long)wv);
-                atomicAdd((unsigned long long*)&s_pw[p], (unsigned long long)(-wv));
+                atomicAdd(&s_pw[lo], (int32_t)wv);
+                atomicAdd(&s_pw[p], -(int32_t)wv);
                 ++moves;
             }
         }
@@ -1407,12 +1508,12 @@ __global__ void __launch_bounds__(CT, 1) k_rb_step_cta(RbCta R, int mode, int64_
                                                         int64_t ncand, int64_t* pw, int64_t* moves_out) {
     extern __shared__ __align__(16) unsigned char rsm[];
     const int32_t k = R.k;
-    int64_t* s_pw = (int64_t*)rsm;
-    int64_t* s_snap = s_pw + k;
-    int64_t* s_cum = s_snap + 2 * k;
+    int32_t* s_pw = (int32_t*)rsm;               // part weights fit in 32 bits (rb_delta_begin)
+    int32_t* s_snap = s_pw + 2 * k;
+    int64_t* s_cum = (int64_t*)rsm + 3 * k;
     uint64_t* s_keys = (uint64_t*)(rsm + (((size_t)(4 * k + 1) * 8 + k + 15) & ~(size_t)15));
     __shared__ int64_t sh[33];
-    for (int q = threadIdx.x; q < k; q += CT) s_pw[q] = pw[q];
+    for (int q = threadIdx.x; q < k; q += CT) s_pw[q] = (int32_t)pw[q];
     if (cand == nullptr)
         for (int64_t v = threadIdx.x; v < n; v += CT) R.lock[v] = 0;
     __syncthreads();
@@ -1426,10 +1527,10 @@ __global__ void __launch_bounds__(CT, 1) k_rb_step_cta(RbCta R, int mode, int64_
 __device__ void cta_refine_level(const CtaRefineArgs& R, unsigned char* rsm) {
     const int32_t k = R.k;
     const int64_t Lmax = R.Lmax, n = R.g.n;
-    int64_t* s_pw = (int64_t*)rsm;               // k: current part weights
-    int64_t* s_snap = s_pw + k;                  // k: weights at the start of a rebalance step
-    int64_t* s_best = s_snap + k;                // k: weights of the kept state
-    int64_t* s_cum = s_best + k;                 // k + 1: free capacity prefix (strong)
+    int32_t* s_pw = (int32_t*)rsm;               // k: current part weights (32 bits: rb_delta_begin)
+    int32_t* s_snap = s_pw + 2 * k;              // k: weights at the start of a rebalance step
+    int32_t* s_best = s_snap + 2 * k;            // k: weights of the kept state
+    int64_t* s_cum = (int64_t*)rsm + 3 * k;      // k + 1: free capacity prefix (strong)
     uint8_t* s_over = (uint8_t*)(s_cum + k + 1); // k
     unsigned char* big = rsm + (((size_t)(4 * k + 1) * 8 + k + 15) & ~(size_t)15);
     int32_t* s_hist = (int32_t*)big;             // CW * k connectivity histograms, or
@@ -1444,7 +1545,7 @@ __device__ void cta_refine_level(const CtaRefineArgs& R, unsigned char* rsm) {
     int32_t* part_next = R.part_next;
     uint8_t* lock = R.lock;
     uint8_t* lock_next = R.lock_next;
-    for (int q = threadIdx.x; q < k; q += CT) s_pw[q] = R.pw[q];
+    for (int q = threadIdx.x; q < k; q += CT) s_pw[q] = (int32_t)R.pw[q];
     for (int64_t v = threadIdx.x; v < n; v += CT) lock[v] = 0;
     __syncthreads();
     int64_t best_cut = 0, best_mp = 0, prev_moves = -1, nmoves = 0;
@@ -1474,12 +1575,12 @@ __device__ void cta_refine_level(const CtaRefineArgs& R, unsigned char* rsm) {
         // ---- connectivity pass
         ConnArgs CA;
         CA.g = R.g; CA.k = k; CA.Lmax = Lmax; CA.den = R.den; CA.force_eval = final_eval ? 1 : 0;
-        CA.lock = lock; CA.pw = s_pw; CA.heavy = nullptr; CA.item_row = nullptr;
+        CA.lock = lock; CA.pw = nullptr; CA.heavy = nullptr; CA.item_row = nullptr;
         CA.item_beg = nullptr; CA.item_end = nullptr; CA.row_items = nullptr; CA.nitems = 0;
         for (int b = 0; b < 3; ++b) { CA.bucket[b] = R.bucket[b]; CA.nbucket[b] = R.nbucket[b]; CA.clist[b] = nullptr; }
         CA.wfirst = nullptr;
         CA.dest = R.dest; CA.gain = R.gain; CA.status = R.status;
-        CA.lock_next = nullptr;
+        CA.lock_next = nullptr; CA.prev_moves = nullptr; CA.host = nullptr; CA.nblocks = 0;
         CA.pc = part; CA.pc_next = nullptr; CA.pdg = nullptr; CA.lp_dg = 1;
         CA.hhist = nullptr; CA.hsum = nullptr; CA.hdone = nullptr;
         int64_t acc = 0, cdeg = 0;
@@ -1799,7 +1900,7 @@ __global__ void k_expand_part(int64_t n, const void* __restrict__ pc, int pcb, i
         part[v] = load_pc(pc, pcb, v);
 }
 
-static void trace_iter(Ctx& c, const RefineBufs& B, int64_t n, int64_t m, int level, int it, int mode,
+static void trace_iter(Ctx& c, const RefineBufs& B, const int64_t* moves_d, int64_t n, int64_t m, int level, int it, int mode,
                        int64_t cut_before, int64_t mp_before, const Tracer& tr) {
     std::vector<int32_t> d(n), gn(n), p(n);
     k_expand_part<<<grid_for(n, 256), 256, 0, c.s>>>(n, B.pc, B.pcb, B.part);
@@ -1807,7 +1908,7 @@ static void trace_iter(Ctx& c, const RefineBufs& B, int64_t n, int64_t m, int le
     GP_CUDA(cudaMemcpyAsync(d.data(), B.dest, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, c.s));
     GP_CUDA(cudaMemcpyAsync(gn.data(), B.gain, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, c.s));
     GP_CUDA(cudaMemcpyAsync(p.data(), B.part, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, c.s));
-    GP_CUDA(cudaMemcpyAsync(c.h_pinned, B.status + S_STEP_MOVES, sizeof(int64_t), cudaMemcpyDeviceToHost, c.s));
+    GP_CUDA(cudaMemcpyAsync(c.h_pinned, moves_d, sizeof(int64_t), cudaMemcpyDeviceToHost, c.s));
     c.sync();
     gp_trace_event ev;
     memset(&ev, 0, sizeof ev);
@@ -1871,7 +1972,7 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
     const int light_blocks = (int)std::min<int64_t>(grid_for(light_warps, RW, c.sm_count * c.ctas_per_sm),
                                                     (B.wfirst_cap - 1) / RW);
     const int grid = (int)L.nitems + light_blocks;
-    const int short_grid = grid_for(L.nbucket[0], RT, c.sm_count * std::min(c.ctas_per_sm, 32));
+    const int short_grid = grid_for(L.nbucket[0], RT, c.sm_count * std::min(c.ctas_per_sm, 8));
     // label propagation moves candidates of every bucket in one launch
     const int lp_grid = split ? (int)L.nitems + std::max(light_blocks, grid_for(L.nbucket[0], 4 * RT, c.sm_count * 8)) : grid;
     if (long_rows) {
@@ -1883,13 +1984,20 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
     int stall = 0, rb_streak = 0, steps = 0, last_mode = 0;
     int64_t prev_moves = -1;
     const int nb_k = bits_for(k);
+    int64_t* moves_d = nullptr;   // moves of the last step (its iteration's status block)
     const bool move_head = B.mp && P.gnn && gnn_has_move_head(P.gnn);
     // with pdg, proposals and gains of a label-propagation pass are stored apart
     // only for the move head and the trace
     const int lp_dg = (!B.pdg || move_head || tr.on()) ? 1 : 0;
     for (int it = 0;; ++it) {
         const bool final_eval = (it == P.o.refine_max_iters);
-        GP_CUDA(cudaMemsetAsync(B.status, 0, sizeof(int64_t) * S_NRESET, c.s));
+        // this iteration's status block; the half of the ring that is not in use
+        // is cleared ahead
+        constexpr int half = kStatusRing / 2;
+        int64_t* status = B.status + (int64_t)(it % kStatusRing) * S_NSLOTS;
+        if (it == 0) memset_async(c, B.status, 0, sizeof(int64_t) * S_NSLOTS * kStatusRing);
+        else if (it % kStatusRing == half / 2) memset_async(c, B.status + half * S_NSLOTS, 0, sizeof(int64_t) * S_NSLOTS * half);
+        else if (it % kStatusRing == half + half / 2) memset_async(c, B.status, 0, sizeof(int64_t) * S_NSLOTS * half);
         if (c.profile) GP_CUDA(cudaEventRecord(c.ev_a, c.s));
         ConnArgs CA;
         CA.g = g; CA.k = k; CA.Lmax = Lmax; CA.den = P.o.lp_filter_den; CA.force_eval = final_eval ? 1 : 0;
@@ -1898,7 +2006,8 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
         CA.nitems = L.nitems; CA.hhist = B.hhist; CA.hsum = B.hsum; CA.hdone = B.hdone;
         for (int b = 0; b < 3; ++b) { CA.bucket[b] = L.bucket[b]; CA.nbucket[b] = L.nbucket[b]; CA.clist[b] = B.clist[b]; }
         CA.wfirst = B.wfirst;
-        CA.dest = B.dest; CA.gain = B.gain; CA.status = B.status;
+        CA.dest = B.dest; CA.gain = B.gain; CA.status = status;
+        CA.prev_moves = moves_d; CA.host = c.h_pinned; CA.nblocks = (long_rows ? grid : 0) + (split ? short_grid : 0);
         CA.pc = B.pc; CA.pc_next = B.pc_next; CA.lock_next = B.lock_next;   // the LP step's starting copy
         CA.pdg = B.pdg; CA.lp_dg = lp_dg;
         if (long_rows) {
@@ -1916,8 +2025,7 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
         // rowptr, colidx, weights, gathered part[u] (pcb bytes); part[v], lock[v] read; proposal and gain written
         const int64_t conn_bytes = L.scan_bytes() - (4 - B.pcb) * g.m + B.pcb * n + n + 8 * n;
         c.bytes += conn_bytes;
-        GP_CUDA(cudaMemcpyAsync(c.h_pinned, B.status, sizeof(int64_t) * S_NSLOTS, cudaMemcpyDeviceToHost, c.s));
-        c.sync();
+        c.sync();   // the pass wrote its status block to c.h_pinned
         if (c.profile) {
             float t = 0;
             GP_CUDA(cudaEventElapsedTime(&t, c.ev_a, c.ev_b));
@@ -1961,8 +2069,7 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
         if (dev_mode == MODE_RB) { mode = (rb_streak >= P.o.strong_after) ? 2 : 1; ++rb_streak; }
         else { mode = 0; rb_streak = 0; }
         last_mode = mode;
-        int64_t* moves_d = B.status + S_STEP_MOVES;  // moves of this step, read at the next sync
-        memset_async(c, moves_d, 0, sizeof(int64_t));
+        moves_d = status + S_STEP_MOVES;  // moves of this step, read at the next sync
         if (mode == 0) {
             // pc_next / lock_next were filled by the connectivity pass
             ApplyArgs AA;
@@ -1970,7 +2077,7 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
             AA.item_row = L.item_row; AA.item_beg = L.item_beg; AA.item_end = L.item_end; AA.row_items = L.row_items;
             AA.nitems = L.nitems; AA.hsum = B.hsum; AA.hdone = B.hdone;
             for (int b = 0; b < 3; ++b) AA.clist[b] = B.clist[b];
-            AA.status = B.status; AA.lock_next = B.lock_next; AA.pw = B.pw;
+            AA.status = status; AA.lock_next = B.lock_next; AA.pw = B.pw;
             AA.moves_out = moves_d;
             AA.pc = B.pc; AA.pc_next = B.pc_next; AA.pdg = B.pdg;
             if (move_head) {
@@ -1989,41 +2096,39 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
                     tr.emit(ev);
                 }
             }
-            if (B.pcb == 1) k_lp_apply<uint8_t><<<lp_grid, RT, sizeof(int64_t) * k, c.s>>>(AA);
-            else k_lp_apply<uint16_t><<<lp_grid, RT, sizeof(int64_t) * k, c.s>>>(AA);
+            if (B.pcb == 1) k_lp_apply<uint8_t><<<lp_grid, RT, sizeof(int32_t) * k, c.s>>>(AA);
+            else k_lp_apply<uint16_t><<<lp_grid, RT, sizeof(int32_t) * k, c.s>>>(AA);
             GP_LAUNCHED(c);
             // copy pass + afterburner: candidate rows with gathered part (pcb bytes), dest and gain per entry
             c.bytes += (9 + B.pcb) * n + 16 * nlist + cdeg * (4 + (g.ew ? 4 : 0) + 8 + B.pcb);
             std::swap(B.lock, B.lock_next);
             std::swap(B.pc, B.pc_next);
-        } else if (n <= kCtaMaxN) {
+        } else if (n <= kCtaMaxN && cdeg <= kRbCta) {
             // the whole step in one thread block
             auto mk = c.tmp->save();
             RbCta RA;
             RA.vw = g.vw; RA.pc = B.pc; RA.pcb = B.pcb; RA.lock = B.lock; RA.dest = B.dest;
             RA.gain = B.gain;
-            RA.pre = c.tmp_alloc<int64_t>(n); RA.flag = c.tmp_alloc<int32_t>(n); RA.gkeys = c.tmp_alloc<uint64_t>(n);
-            RA.k = k; RA.Lmax = Lmax;
+            RA.pre = c.tmp_alloc<int64_t>(n); RA.flag = c.tmp_alloc<int32_t>(n);
+            RA.gkeys = c.tmp_alloc<uint64_t>(n); RA.k = k; RA.Lmax = Lmax;
             k_rb_step_cta<<<1, CT, cta_refine_smem(k), c.s>>>(RA, mode, n, nullptr, 0, B.pw, moves_d);
             GP_LAUNCHED(c);
             c.bytes += 4 * n + 12 * n + 80 * n;
             c.tmp->restore(mk);
         } else {
-            memset_async(c, B.lock, 0, n);
+            // candidates in vertex order; stable sort -> (source, bucket, id)
+            const int64_t ncand = cdeg;
             auto mk = c.tmp->save();
-            // candidates (dest >= 0) in vertex order, keyed (source, bucket); stable sort -> (source, bucket, id)
-            int32_t* flag = c.tmp_alloc<int32_t>(n);
-            int64_t* vpos = c.tmp_alloc<int64_t>(n + 1);
-            k_rb_flags<<<grid_for(n, 256), 256, 0, c.s>>>(n, B.dest, flag);
+            const int64_t ntile = (n + RB_TILE - 1) / RB_TILE;
+            int32_t* tcnt = c.tmp_alloc<int32_t>(ntile);
+            k_rb_count<<<(unsigned)ntile, RT, 0, c.s>>>(n, B.dest, tcnt);
             GP_LAUNCHED(c);
-            scan_excl_i32_to_i64(c, flag, vpos, n, vpos + n);
-            const int64_t ncand = read_i64(c, vpos + n);
-            c.bytes += 4 * n + 12 * n;
-            if (ncand > 0 && ncand <= kCtaMaxN) {
+            k_rb_collect<<<(unsigned)ntile, RT, 0, c.s>>>(n, B.dest, tcnt, ncand, B.pc, B.pcb, B.gain, B.lock, B.ckeys,
+                                                          B.cvals);
+            GP_LAUNCHED(c);
+            c.bytes += 9 * n;
+            if (ncand > 0 && ncand <= kRbCta) {
                 // few candidates: sort, select and apply in one thread block
-                k_rb_compact<<<grid_for(n, 256), 256, 0, c.s>>>(n, flag, vpos, B.pc, B.pcb, B.gain, B.ckeys,
-                                                                                 B.cvals);
-                GP_LAUNCHED(c);
                 RbCta RA;
                 RA.vw = g.vw; RA.pc = B.pc; RA.pcb = B.pcb; RA.lock = B.lock; RA.dest = B.dest;
                 RA.gain = B.gain;
@@ -2033,53 +2138,32 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
                 GP_LAUNCHED(c);
                 c.bytes += 80 * ncand;
             } else if (ncand > 0) {
-                k_rb_compact<<<grid_for(n, 256), 256, 0, c.s>>>(n, flag, vpos, B.pc, B.pcb, B.gain, B.ckeys,
-                                                                                 B.cvals);
-                GP_LAUNCHED(c);
                 const int bits = RB_SHIFT + nb_k;
                 radix_sort_pairs(c, B.ckeys, B.cvals, B.ckeys2, B.cvals2, ncand, bits);
-                int32_t* wv = c.tmp_alloc<int32_t>(ncand);
                 int64_t* pre = c.tmp_alloc<int64_t>(ncand + 1);
-                int32_t* acc = c.tmp_alloc<int32_t>(ncand);
-                int64_t* pw_snap = c.tmp_alloc<int64_t>(k);
-                GP_CUDA(cudaMemcpyAsync(pw_snap, B.pw, sizeof(int64_t) * k, cudaMemcpyDeviceToDevice, c.s));
-                k_gather_vw<<<grid_for(ncand, 256), 256, 0, c.s>>>(ncand, B.cvals, g.vw, wv);
-                GP_LAUNCHED(c);
-                scan_excl_i32_to_i64(c, wv, pre, ncand, nullptr);
-                int64_t* segf = c.tmp_alloc<int64_t>(k + 1);
-                k_seg_first<<<grid_for(k + 1, 256), 256, 0, c.s>>>(ncand, B.ckeys, k, segf);
-                GP_LAUNCHED(c);
-                k_rb_source<<<grid_for(ncand, 256), 256, 0, c.s>>>(ncand, B.ckeys, segf, pre, B.pw, Lmax, acc);
+                scan_list_weights(c, B.cvals, g.vw, pre, ncand, nullptr, pre + ncand);
+                RbPlan plan;
+                int64_t* pl = c.tmp_alloc<int64_t>(6 * (int64_t)k + 2);
+                plan.seg = pl; plan.acc = pl + k; plan.off = pl + 2 * k; plan.woff = pl + 3 * k; plan.snap = pl + 4 * k;
+                plan.cum = pl + 5 * k; plan.n2 = pl + 6 * k + 1;
+                k_rb_plan<<<1, (k + 31) & ~31, 0, c.s>>>(ncand, B.ckeys, pre, B.pw, Lmax, k, plan);
                 GP_LAUNCHED(c);
                 if (mode == 1) {
-                    int64_t* apos = c.tmp_alloc<int64_t>(ncand + 1);
-                    scan_excl_i32_to_i64(c, acc, apos, ncand, apos + ncand);
-                    const int64_t n2 = read_i64(c, apos + ncand);
-                    if (n2 > 0) {
-                        k_rb_rekey<<<grid_for(ncand, 256), 256, 0, c.s>>>(ncand, B.ckeys, B.cvals, acc, apos, B.dest,
-                                                                        B.ckeys2, B.cvals2);
-                        GP_LAUNCHED(c);
-                        radix_sort_pairs(c, B.ckeys2, B.cvals2, B.ckeys, B.cvals, n2, bits);
-                        k_gather_vw<<<grid_for(n2, 256), 256, 0, c.s>>>(n2, B.cvals2, g.vw, wv);
-                        GP_LAUNCHED(c);
-                        scan_excl_i32_to_i64(c, wv, pre, n2, nullptr);
-                        k_seg_first<<<grid_for(k + 1, 256), 256, 0, c.s>>>(n2, B.ckeys2, k, segf);
-                        GP_LAUNCHED(c);
-                        k_rb_weak_apply<<<grid_for(n2, 256), 256, sizeof(int64_t) * k, c.s>>>(
-                            n2, B.ckeys2, segf, B.cvals2, pre, g.vw, pw_snap, Lmax, k, B.pc, B.pcb, B.lock, B.pw,
-                            moves_d);
-                        GP_LAUNCHED(c);
-                    }
+                    k_rb_rekey<<<grid_for(ncand, 256), 256, 0, c.s>>>(ncand, B.ckeys, B.cvals, plan, B.dest, B.ckeys2,
+                                                                      B.cvals2);
+                    GP_LAUNCHED(c);
+                    radix_sort_pairs(c, B.ckeys2, B.cvals2, B.ckeys, B.cvals, ncand, bits, plan.n2);
+                    scan_list_weights(c, B.cvals2, g.vw, pre, ncand, plan.n2, nullptr);
+                    int64_t* segf = c.tmp_alloc<int64_t>(k + 1);
+                    k_seg_first<<<grid_for(k + 1, 256), 256, 0, c.s>>>(plan.n2, B.ckeys2, k, segf);
+                    GP_LAUNCHED(c);
+                    k_rb_weak_apply<<<grid_for(ncand, 256, c.sm_count * 8), 256, sizeof(int32_t) * k, c.s>>>(
+                        plan.n2, B.ckeys2, segf, B.cvals2, pre, g.vw, plan.snap, Lmax, k, B.pc, B.pcb, B.lock, B.pw,
+                        moves_d);
+                    GP_LAUNCHED(c);
                 } else {
-                    int64_t* cum = c.tmp_alloc<int64_t>(k + 1);
-                    int32_t* wm = c.tmp_alloc<int32_t>(ncand);
-                    k_cumfree<<<1, 32, 0, c.s>>>(k, B.pw, Lmax, cum);
-                    GP_LAUNCHED(c);
-                    k_mask_vw<<<grid_for(ncand, 256), 256, 0, c.s>>>(ncand, acc, wv, wm);
-                    GP_LAUNCHED(c);
-                    scan_excl_i32_to_i64(c, wm, pre, ncand, nullptr);
-                    k_rb_strong_apply<<<grid_for(ncand, 256), 256, sizeof(int64_t) * k, c.s>>>(
-                        ncand, B.cvals, acc, pre, g.vw, cum, k, B.pc, B.pcb, B.lock, B.pw, moves_d);
+                    k_rb_strong_apply<<<grid_for(ncand, 256, c.sm_count * 8), 256, sizeof(int32_t) * k, c.s>>>(
+                        ncand, B.ckeys, B.cvals, pre, plan, g.vw, k, B.pc, B.pcb, B.lock, B.pw, moves_d);
                     GP_LAUNCHED(c);
                 }
                 c.bytes += 80 * ncand;
@@ -2087,7 +2171,7 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
             c.tmp->restore(mk);
         }
         ++steps;
-        if (tr.on()) trace_iter(c, B, n, g.m, level, it, mode, cur_cut, cur_mp, tr);
+        if (tr.on()) trace_iter(c, B, moves_d, n, g.m, level, it, mode, cur_cut, cur_mp, tr);
     }
     k_expand_part<<<grid_for(n, 256), 256, 0, c.s>>>(n, B.best, B.pcb, B.part);
     GP_LAUNCHED(c);
