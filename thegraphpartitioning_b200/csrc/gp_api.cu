@@ -88,13 +88,24 @@ __global__ void k_check_rowptr(int64_t n, int64_t m, const int64_t* __restrict__
 
 // one entry: weight >= 1, column id in range, no self loop (the smallest
 // (code, index) reported wins, whatever the order of the checks)
+// and the symmetry fingerprint: the sum over entries of w times a 64-bit hash of
+// the unordered pair, positive for v < u and negative for v > u (mod 2^64).
+// Zero for every symmetric graph; an asymmetric one has weights whose signed
+// sums per pair are not all zero, and a random hash of the pairs then cancels
+// with probability about 2^-64.
 __device__ __forceinline__ void check_entry(int64_t n, int64_t e, int64_t v, int32_t u, int32_t w, int check,
-                                            unsigned long long* err, int64_t& local) {
+                                            unsigned long long* err, int64_t& local, uint64_t& finger) {
     if (w < 1) report(err, V_EWGT, e);
     local += w;
     if (check >= 1) {
         if (u < 0 || u >= n) report(err, V_COLIDX, e);
         else if (u == v) report(err, V_SELF, v);
+        const uint32_t a = (uint32_t)v < (uint32_t)u ? (uint32_t)v : (uint32_t)u;
+        const uint32_t b = (uint32_t)v < (uint32_t)u ? (uint32_t)u : (uint32_t)v;
+        uint32_t x = a * 0x9E3779B1u + b * 0x85EBCA77u, y = a * 0xC2B2AE3Du + b * 0x27D4EB2Fu;
+        x ^= x >> 15; y ^= y >> 13;
+        const uint64_t h = ((uint64_t)(x * 0x85EBCA6Bu ^ y) * (y | 1u) + x) * (uint64_t)(uint32_t)w;
+        finger += (uint32_t)v < (uint32_t)u ? h : 0ull - h;
     }
 }
 // entries of a row-pointer-checked CSR, entry-sliced (csr_row_of /
@@ -107,6 +118,7 @@ __global__ void k_check_rows(int64_t n, int64_t m, int64_t slice, const int64_t*
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const int64_t nslice = (m + slice - 1) / slice;
     int64_t local = 0;
+    uint64_t finger = 0;
     for (int64_t sl = wid; sl < nslice; sl += nw) {
         const int64_t o0 = sl * slice, o1 = o0 + slice < m ? o0 + slice : m;
         int64_t cb = csr_row_of(rp, n, o0), s = 0, wend = 0;
@@ -129,12 +141,12 @@ __global__ void k_check_rows(int64_t n, int64_t m, int64_t slice, const int64_t*
                     w[q] = ew ? __ldcs(&ew[oi]) : 1;
                 }
 #pragma unroll
-                for (int q = 0; q < 8; ++q) check_entry(n, o + 32 * q + lane, v[q], u[q], w[q], check, err, local);
+                for (int q = 0; q < 8; ++q) check_entry(n, o + 32 * q + lane, v[q], u[q], w[q], check, err, local, finger);
                 o += 256;
             } else if (o < lim) {
                 const int64_t oi = o + lane;
                 const int64_t v = cb + csr_window_lane(s, oi);
-                if (oi < lim) check_entry(n, oi, v, check >= 1 ? ci[oi] : 0, ew ? ew[oi] : 1, check, err, local);
+                if (oi < lim) check_entry(n, oi, v, check >= 1 ? ci[oi] : 0, ew ? ew[oi] : 1, check, err, local, finger);
                 o = o + 32 < lim ? o + 32 : lim;
             } else {
                 cb += 32;   // o >= wend: o lies in a later row
@@ -142,8 +154,14 @@ __global__ void k_check_rows(int64_t n, int64_t m, int64_t slice, const int64_t*
             }
         }
     }
-    for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
-    if (lane == 0) atomicAdd((unsigned long long*)&sums[1], (unsigned long long)local);
+    for (int o = 16; o > 0; o >>= 1) {
+        local += __shfl_xor_sync(0xffffffffu, local, o);
+        finger += __shfl_xor_sync(0xffffffffu, finger, o);
+    }
+    if (lane == 0) {
+        atomicAdd((unsigned long long*)&sums[1], (unsigned long long)local);
+        atomicAdd((unsigned long long*)&sums[2], (unsigned long long)finger);
+    }
 }
 
 // symmetry: every entry (v,u,w) has a partner (u,v,w).  Both directions are
@@ -199,13 +217,13 @@ static int bits_for(int64_t x) {
     return b;
 }
 
-// returns total vertex weight
-static int64_t validate(Ctx& c, const DGraph& g, int check) {
+// returns total vertex weight; symmetric: the entries were checked and passed the fingerprint
+static int64_t validate(Ctx& c, const DGraph& g, int check, bool& symmetric) {
     auto mk = c.tmp->save();
     unsigned long long* err = (unsigned long long*)c.tmp_alloc<int64_t>(4);
-    int64_t* sums = c.tmp_alloc<int64_t>(2);
+    int64_t* sums = c.tmp_alloc<int64_t>(3);
     GP_CUDA(cudaMemsetAsync(err, 0xff, 8, c.s));
-    memset_async(c, sums, 0, 16);
+    memset_async(c, sums, 0, 24);
     k_check_rowptr<<<grid_for(g.n, 256), 256, 0, c.s>>>(g.n, g.m, g.rp, g.vw, err, sums);
     GP_LAUNCHED(c);
     GP_CUDA(cudaMemcpyAsync(c.h_pinned, err, 8, cudaMemcpyDeviceToHost, c.s));
@@ -218,11 +236,12 @@ static int64_t validate(Ctx& c, const DGraph& g, int check) {
     GP_LAUNCHED(c);
     c.bytes += 8 * (g.n + 1) + (g.vw ? 4 * g.n : 0) + (check >= 1 ? 4 * g.m : 0) + (g.ew ? 4 * g.m : 0);
     GP_CUDA(cudaMemcpyAsync(c.h_pinned, err, 8, cudaMemcpyDeviceToHost, c.s));
-    GP_CUDA(cudaMemcpyAsync(c.h_pinned + 1, sums, 16, cudaMemcpyDeviceToHost, c.s));
+    GP_CUDA(cudaMemcpyAsync(c.h_pinned + 1, sums, 24, cudaMemcpyDeviceToHost, c.s));
     c.sync();
     e0 = (uint64_t)c.h_pinned[0];
     if (e0 != ~0ull) throw GpError(GP_EINVAL, verr((int)(e0 >> 48), (int64_t)(e0 & ((1ull << 48) - 1))));
     const int64_t W = c.h_pinned[1], EW = c.h_pinned[2];
+    symmetric = check >= 1 && c.h_pinned[3] == 0;
     if (W > INT32_MAX) throw GpError(GP_EINVAL, "sum of vertex weights exceeds int32");
     if (EW > INT32_MAX) throw GpError(GP_EINVAL, "sum of edge weights exceeds int32");
     if (check >= 2 && g.m > 0) {
@@ -277,7 +296,7 @@ void vc_begin(Ctx& c, const DGraph& g0, int32_t k, float imbalance, uint64_t see
     c.profile = P.o.profile > 0;
     if (c.profile) { c.ev_a = tm.e[6]; c.ev_b = tm.e[7]; }
     GP_CUDA(cudaEventRecord(tm.e[0], c.s));
-    P.W = validate(c, g0, P.o.check_input);
+    P.W = validate(c, g0, P.o.check_input, P.symmetric);
     P.Lmax = compute_lmax(P.W, k, imbalance);
     P.maxvw = std::max<int64_t>(1, (3 * P.W) / (2 * (int64_t)P.o.coarsen_to));
     S.g0 = g0;

@@ -19,6 +19,7 @@ struct Params {
     int64_t W = 0;        // total vertex weight
     int64_t Lmax = 0;     // max allowed part weight
     int64_t maxvw = 0;    // coarse vertex weight cap
+    bool symmetric = false;   // the input's entries passed the symmetry fingerprint (checked input only)
     uint64_t seed = 0;
     float imbalance = 0.03f;
     gp_options o{};
@@ -127,11 +128,16 @@ struct RefineBufs {
 };
 
 // device status block of one refinement iteration: the connectivity pass's
-// slots [0, S_NRESET), the move step's S_STEP_MOVES, and S_DONE, the pass's
-// finished blocks.  A level uses a ring of blocks, cleared half a ring at a time.
+// slots [0, S_NRESET), the move step's S_STEP_MOVES (moves), S_MVDEG (entries of
+// the moved rows) and S_DELTA (the step's change of the directed cross weight,
+// k_track), and S_DONE, the pass's finished blocks.  A level uses a ring of
+// blocks, cleared half a ring at a time.
 enum StatusSlot { S_CROSS = 0, S_MAXPW = 1, S_MODE = 2, S_NL0 = 3, S_NL1 = 4, S_LIGHT = 5, S_NL2 = 6, S_CDEG = 7,
-                  S_NRESET = 8, S_STEP_MOVES = 8, S_DONE = 9, S_NSLOTS = 16 };
+                  S_NRESET = 8, S_STEP_MOVES = 8, S_DONE = 9, S_MVDEG = 10, S_DELTA = 11, S_NSLOTS = 16 };
 constexpr int kStatusRing = 64;
+// host copy: slots [0, S_NRESET), then of the step before its moves and delta,
+// and whether the pass summed the cross weight over every row
+enum HostSlot { H_MOVES = 8, H_DELTA = 9, H_FULL = 10, H_NSLOTS = 11 };
 
 // CUDA events of the phases of one V-cycle
 struct Timer {

@@ -105,7 +105,10 @@ struct ConnArgs {
     int64_t* hsum;
     int32_t* hdone;
     uint64_t* pdg;              // label propagation: pdg_pack(part, dest, gain) per row (nullptr: none)
-    const int64_t* prev_moves;  // moves of the step before (nullptr: none)
+    const int64_t* prev;        // status block of the iteration before (nullptr: none)
+    int64_t track_deg;          // its step's cross-weight change is known (k_track) when the moved rows
+                                // had at most this many entries (-1: never)
+    int rb_all;                 // rebalancing passes store proposals of every row (trace)
     int64_t* host;              // host-resident copy of the status block, written by the pass's last
     int nblocks;                // block out of nblocks (over all its launches)
     int lp_dg;                  // label propagation also writes dest and gain (no pdg, or someone
@@ -165,6 +168,7 @@ __device__ __forceinline__ bool conn_decide(const ConnArgs& A, int mode, bool ac
     const int32_t own = tot - cross;
     int32_t d = -1, gn = 0;
     bool cand = false;
+    if (mode == MODE_EVAL || (mode == MODE_RB && !active && !A.rb_all)) return false;
     if (mode == MODE_LP) {
         if (A.pc_next) { ((PT*)A.pc_next)[v] = (PT)p; A.lock_next[v] = 0; }
         if (active && bq >= 0) {
@@ -189,14 +193,16 @@ struct ConnRow {
     int32_t v, p;
     bool active;
 };
+// full: the pass sums the cross weight over every row; else only active rows
+// are swept (the others read as empty)
 template <class PT>
-__device__ __forceinline__ ConnRow conn_row(const ConnArgs& A, int32_t v, int mode, const uint8_t* over) {
+__device__ __forceinline__ ConnRow conn_row(const ConnArgs& A, int32_t v, int mode, bool full, const uint8_t* over) {
     ConnRow r;
     r.v = v; r.beg = 0; r.end = 0; r.p = -1; r.active = false;
     if (v >= 0) {
-        r.beg = A.g.rp[v]; r.end = A.g.rp[v + 1];
         r.p = gpart<PT>(A.pc, v, A.g.n);
         r.active = (mode == MODE_LP && !A.lock[v]) || (mode == MODE_RB && over[r.p]);
+        if (full || r.active) { r.beg = A.g.rp[v]; r.end = A.g.rp[v + 1]; }
     }
     return r;
 }
@@ -396,7 +402,7 @@ __device__ __forceinline__ ConnRes conn_warp(const ConnArgs& A, const ConnRow& R
 // candidates appended together (one atomic per list present).  rows: the
 // warp's 32 slots in shared memory.  SHORT: there may be bucket-0 units.
 template <class PT, bool SHORT>
-__device__ __forceinline__ void conn_group(const ConnArgs& A, int64_t ub, int nu, int mode, const uint8_t* over,
+__device__ __forceinline__ void conn_group(const ConnArgs& A, int64_t ub, int nu, int mode, bool full, const uint8_t* over,
                                            int32_t light, int32_t* hist, ConnRowS* rows, int64_t& acc, int64_t& cdeg) {
     const int lane = threadIdx.x & 31;
     const int64_t U2 = A.nbucket[2], U21 = U2 + A.nbucket[1];
@@ -412,9 +418,9 @@ __device__ __forceinline__ void conn_group(const ConnArgs& A, int64_t ub, int nu
             if (i < A.nbucket[0]) v = A.bucket[0][i];
         }
     }
-    const ConnRow r = conn_row<PT>(A, v, mode, over);
+    const ConnRow r = conn_row<PT>(A, v, mode, full, over);
     ConnRes x{0, 0, 0u, -1};
-    if (SHORT && ub + nu > U21) {
+    if (SHORT && ub + nu > U21 && __any_sync(0xffffffffu, r.end > r.beg)) {
         ConnRow tr = r;
         if (lb != 0) { tr.end = tr.beg; tr.active = false; }
         x = conn_thread<PT>(A, tr, mode, over);
@@ -423,7 +429,9 @@ __device__ __forceinline__ void conn_group(const ConnArgs& A, int64_t ub, int nu
         rows[lane] = conn_stage(r);
         __syncwarp();
         const int nlong = U21 - ub < nu ? (int)(U21 - ub) : nu;
+        const uint32_t todo = __ballot_sync(0xffffffffu, r.end > r.beg);   // rows to sweep
         for (int j = 0; j < nlong; ++j) {
+            if (!((todo >> (4 * j)) & 1u)) continue;
             const ConnRow wr = conn_unstage(rows[4 * j]);
             const ConnRes y = ub + j < U2 ? conn_warp<PT>(A, wr, mode, over, hist)
                                           : conn_lane<PT>(A, wr, mode, over, hist);
@@ -453,7 +461,7 @@ struct ConnHead {
     int64_t maxpw;
     int32_t light;
 };
-__device__ __forceinline__ int conn_head(const ConnArgs& A, uint8_t* over, ConnHead& sh, int32_t& light) {
+__device__ __forceinline__ int conn_head(const ConnArgs& A, uint8_t* over, ConnHead& sh, int32_t& light, bool& full) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t Lmax = A.Lmax;
     int64_t mx = 0;
@@ -478,6 +486,9 @@ __device__ __forceinline__ int conn_head(const ConnArgs& A, uint8_t* over, ConnH
     const int64_t maxpw = sh.maxpw;
     light = sh.light;
     const int mode = A.force_eval ? MODE_EVAL : (maxpw > Lmax ? MODE_RB : MODE_LP);
+    // a rebalancing pass sweeps only the rows of overweight parts when k_track
+    // has the last step's change of the cut (the same test there)
+    full = mode != MODE_RB || !A.prev || A.prev[S_MVDEG] > A.track_deg;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         A.status[S_MAXPW] = maxpw; A.status[S_MODE] = mode; A.status[S_LIGHT] = light;
     }
@@ -486,7 +497,7 @@ __device__ __forceinline__ int conn_head(const ConnArgs& A, uint8_t* over, ConnH
 // adds every thread's cross weight to the status block, one atomic per block;
 // the pass's last block then writes the block to the host (pinned, mapped
 // memory: no copy operation between the pass and the host's wait)
-__device__ __forceinline__ void conn_tail(const ConnArgs& A, int64_t acc, int64_t* s_red) {
+__device__ __forceinline__ void conn_tail(const ConnArgs& A, int64_t acc, int64_t* s_red, bool full) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     acc = warp_sum(acc);
     __syncthreads();
@@ -503,11 +514,13 @@ __device__ __forceinline__ void conn_tail(const ConnArgs& A, int64_t acc, int64_
     }
     if (!__shfl_sync(0xffffffffu, last, 0)) return;
     __threadfence();
-    // one 72-byte store of the warp: the status slots and the last step's moves
-    static_assert(S_STEP_MOVES == S_NRESET, "slots written together");
-    if (lane <= S_NRESET) {
-        const int64_t* from = lane < S_NRESET ? A.status + lane : A.prev_moves;
-        A.host[lane] = from ? (int64_t)__ldcg((const unsigned long long*)from) : 0;
+    // one store of the warp (HostSlot)
+    if (lane < H_NSLOTS) {
+        const int64_t* from = lane < S_NRESET ? A.status + lane : nullptr;
+        if (A.prev && lane == H_MOVES) from = A.prev + S_STEP_MOVES;
+        if (A.prev && lane == H_DELTA) from = A.prev + S_DELTA;
+        const int64_t x = from ? (int64_t)__ldcg((const unsigned long long*)from) : 0;
+        A.host[lane] = lane == H_FULL ? (full ? 1 : 0) : x;
     }
 }
 
@@ -524,13 +537,15 @@ __global__ void __launch_bounds__(RT, 4) k_conn_short(ConnArgs A) {
     uint8_t* over = (uint8_t*)csm;
     __shared__ ConnHead sh;
     int32_t light;
-    const int mode = conn_head(A, over, sh, light);
+    bool full;
+    const int mode = conn_head(A, over, sh, light, full);
     const int lane = threadIdx.x & 31;
     int64_t acc = 0, cdeg = 0;
     const int64_t n0 = A.nbucket[0];
     for (int64_t i0 = (int64_t)blockIdx.x * RT + (threadIdx.x & ~31); i0 < n0; i0 += (int64_t)gridDim.x * RT) {
         const int64_t i = i0 + lane;
-        const ConnRow r = conn_row<PT>(A, i < n0 ? A.bucket[0][i] : -1, mode, over);
+        const ConnRow r = conn_row<PT>(A, i < n0 ? A.bucket[0][i] : -1, mode, full, over);
+        if (!full && !A.rb_all && !__any_sync(0xffffffffu, r.active)) continue;
         const ConnRes x = conn_thread<PT>(A, r, mode, over);
         bool take = false;
         if (r.v >= 0) {
@@ -543,7 +558,7 @@ __global__ void __launch_bounds__(RT, 4) k_conn_short(ConnArgs A) {
     }
     cdeg = warp_sum(cdeg);
     if (lane == 0 && cdeg) atomicAdd((unsigned long long*)&A.status[S_CDEG], (unsigned long long)cdeg);
-    conn_tail(A, acc, sh.red);
+    conn_tail(A, acc, sh.red, full);
 }
 
 // SHORT: the light units include the bucket-0 rows (small levels: one launch);
@@ -563,7 +578,8 @@ __global__ void __launch_bounds__(RT, SHORT ? 4 : 5) k_conn(ConnArgs A) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (int i = threadIdx.x; i < RW * k; i += RT) hist_all[i] = 0;
     int32_t light;
-    const int mode = conn_head(A, over, sh, light);
+    bool full;
+    const int mode = conn_head(A, over, sh, light, full);
     int64_t acc = 0;  // directed cross weight (this thread)
 
     if ((int64_t)blockIdx.x < A.nitems) {
@@ -575,7 +591,9 @@ __global__ void __launch_bounds__(RT, SHORT ? 4 : 5) k_conn(ConnArgs A) {
         const int nit = A.row_items[h];
         const int32_t p = gpart<PT>(A.pc, (int32_t)v, A.g.n);
         const bool active = (mode == MODE_LP && !A.lock[v]) || (mode == MODE_RB && over[p]);
-        const int64_t beg = A.item_beg[blockIdx.x], end = A.item_end[blockIdx.x];
+        const bool sweep = full || active;   // the same for every piece of the row
+        if (!sweep && A.rb_all && threadIdx.x == 0) { A.dest[v] = -1; A.gain[v] = 0; }
+        const int64_t beg = sweep ? A.item_beg[blockIdx.x] : 0, end = sweep ? A.item_end[blockIdx.x] : 0;
         int64_t cross = 0, tot = 0;
         const bool v4 = aligned16(A.g.ci) && aligned16(A.g.ew);
         for (int64_t base = beg & ~(int64_t)3; base < end; base += 4 * RT) {
@@ -606,10 +624,10 @@ __global__ void __launch_bounds__(RT, SHORT ? 4 : 5) k_conn(ConnArgs A) {
             int64_t c2 = 0, t2 = 0;
             for (int i = 0; i < RW; ++i) { c2 += s_red[i]; t2 += (int64_t)s_k[i]; }
             s_red[0] = c2; s_k[0] = (uint64_t)t2;
-            s_last = 1;
+            s_last = sweep ? 1 : 0;
         }
         __syncthreads();
-        if (nit > 1) {
+        if (sweep && nit > 1) {
             if (active)
                 for (int q = threadIdx.x; q < k; q += RT)
                     if (hist[q]) atomicAdd(&A.hhist[(int64_t)h * k + q], hist[q]);
@@ -661,11 +679,11 @@ __global__ void __launch_bounds__(RT, SHORT ? 4 : 5) k_conn(ConnArgs A) {
         const int64_t u0 = A.wfirst[wid], u1 = A.wfirst[wid + 1];
         int64_t cdeg = 0;   // degree sum of this lane's candidates
         for (int64_t ub = u0; ub < u1; ub += 8)
-            conn_group<PT, SHORT>(A, ub, (int)(u1 - ub < 8 ? u1 - ub : 8), mode, over, light, hist, rows, acc, cdeg);
+            conn_group<PT, SHORT>(A, ub, (int)(u1 - ub < 8 ? u1 - ub : 8), mode, full, over, light, hist, rows, acc, cdeg);
         cdeg = warp_sum(cdeg);
         if (lane == 0 && cdeg) atomicAdd((unsigned long long*)&A.status[S_CDEG], (unsigned long long)cdeg);
     }
-    conn_tail(A, acc, s_red);
+    conn_tail(A, acc, s_red, full);
 }
 
 // ------------------------------------------------------------------ LP apply
@@ -706,22 +724,27 @@ struct ApplyArgs {
     const void* pc;             // the partition (as in ConnArgs)
     void* pc_next;              // the partition after the step
     int64_t* pw;
-    int64_t* moves_out;
+    int64_t* step;              // status block the step's moves and moved entries are added to
     int64_t* hsum;
     int32_t* hdone;
     const uint64_t* pdg;        // packed part / dest / gain of every vertex (nullptr: gather them apart)
 };
 
+// a thread's moves and the entries of their rows
+struct AbCount {
+    int64_t moves = 0, deg = 0;
+};
 template <class PT>
-__device__ __forceinline__ void ab_commit(const ApplyArgs& A, int64_t v, int32_t p, int32_t d, int32_t* delta,
-                                          int64_t& moves) {
+__device__ __forceinline__ void ab_commit(const ApplyArgs& A, int64_t v, int32_t p, int32_t d, int64_t deg,
+                                          int32_t* delta, AbCount& cnt) {
     if (!GP_IN(d, A.k) || !GP_IN(p, A.k)) return;
     ((PT*)A.pc_next)[v] = (PT)d;
     A.lock_next[v] = 1;
     const int32_t wv = A.g.vw ? A.g.vw[v] : 1;
     atomicAdd(&delta[d], wv);
     atomicAdd(&delta[p], -wv);
-    ++moves;
+    ++cnt.moves;
+    cnt.deg += deg;
 }
 
 // part, destination (-1: no candidate) and gain of row v
@@ -765,7 +788,7 @@ __device__ __forceinline__ int32_t ab_short_n(const ApplyArgs& A, int64_t v, int
     return t;
 }
 template <class PT>
-__device__ __forceinline__ void ab_short(const ApplyArgs& A, int64_t v, int32_t* delta, int64_t& moves) {
+__device__ __forceinline__ void ab_short(const ApplyArgs& A, int64_t v, int32_t* delta, AbCount& cnt) {
     int32_t p = -1, d = -1, gv = 0;
     int64_t beg = 0;
     int len = 0;
@@ -777,23 +800,24 @@ __device__ __forceinline__ void ab_short(const ApplyArgs& A, int64_t v, int32_t*
     const uint32_t most = __reduce_max_sync(0xffffffffu, (uint32_t)len);
     const int32_t t = most <= 8 ? ab_short_n<8, PT>(A, v, p, d, gv, beg, len)
                                 : ab_short_n<kShortDeg, PT>(A, v, p, d, gv, beg, len);
-    if (v >= 0 && t >= 0) ab_commit<PT>(A, v, p, d, delta, moves);
+    if (v >= 0 && t >= 0) ab_commit<PT>(A, v, p, d, len, delta, cnt);
 }
 
 // candidate rows of at most TILE entries, TILE lanes each (v < 0: none)
 template <int TILE, class PT>
-__device__ __forceinline__ void ab_tile(const ApplyArgs& A, int64_t v, int32_t* delta, int64_t& moves) {
+__device__ __forceinline__ void ab_tile(const ApplyArgs& A, int64_t v, int32_t* delta, AbCount& cnt) {
     const int lane = threadIdx.x & 31, tl = lane & (TILE - 1);
     int32_t t = 0, p = -1, d = -1;
+    int64_t beg = 0, end = 0;
     if (v >= 0) {
         int32_t gv;
         ab_row<PT>(A, v, p, d, gv);
-        const int64_t e = A.g.rp[v] + tl;
-        if (e < A.g.rp[v + 1]) t = ab_term<PT>(A.g, e, v, p, d, gv, A.pc, A.dest, A.gain, A.pdg);
+        beg = A.g.rp[v]; end = A.g.rp[v + 1];
+        if (beg + tl < end) t = ab_term<PT>(A.g, beg + tl, v, p, d, gv, A.pc, A.dest, A.gain, A.pdg);
     }
 #pragma unroll
     for (int o = TILE / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (tl == 0 && v >= 0 && t >= 0) ab_commit<PT>(A, v, p, d, delta, moves);
+    if (tl == 0 && v >= 0 && t >= 0) ab_commit<PT>(A, v, p, d, end - beg, delta, cnt);
 }
 
 // this thread's part (thread t of nt) of the ab_term sum over entries
@@ -844,12 +868,13 @@ __device__ __forceinline__ int32_t ab_sum(const ApplyArgs& A, int64_t beg, int64
 
 // one candidate row of 33..heavy_deg entries per warp, 128 entries per sweep
 template <class PT>
-__device__ __forceinline__ void ab_warp(const ApplyArgs& A, int64_t v, int32_t* delta, int64_t& moves) {
+__device__ __forceinline__ void ab_warp(const ApplyArgs& A, int64_t v, int32_t* delta, AbCount& cnt) {
     const int lane = threadIdx.x & 31;
     int32_t p, d, gv;
     ab_row<PT>(A, v, p, d, gv);
-    const int32_t g2 = warp_sum(ab_sum<PT>(A, A.g.rp[v], A.g.rp[v + 1], lane, 32, v, p, d, gv));
-    if (lane == 0 && g2 >= 0) ab_commit<PT>(A, v, p, d, delta, moves);
+    const int64_t beg = A.g.rp[v], end = A.g.rp[v + 1];
+    const int32_t g2 = warp_sum(ab_sum<PT>(A, beg, end, lane, 32, v, p, d, gv));
+    if (lane == 0 && g2 >= 0) ab_commit<PT>(A, v, p, d, end - beg, delta, cnt);
 }
 
 template <class PT>
@@ -859,7 +884,7 @@ __global__ void __launch_bounds__(RT, 4) k_lp_apply(ApplyArgs A) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (int q = threadIdx.x; q < A.k; q += RT) delta[q] = 0;
     __syncthreads();
-    int64_t moves = 0;
+    AbCount cnt;
     if ((int64_t)blockIdx.x < A.nitems) {
         const int32_t h = A.item_row[blockIdx.x];
         const int64_t v = A.heavy[h];
@@ -886,7 +911,7 @@ __global__ void __launch_bounds__(RT, 4) k_lp_apply(ApplyArgs A) {
                         A.hdone[h] = 0;
                     }
                 }
-                if (last && sum >= 0) ab_commit<PT>(A, v, p, d, delta, moves);
+                if (last && sum >= 0) ab_commit<PT>(A, v, p, d, A.g.rp[v + 1] - A.g.rp[v], delta, cnt);
             }
         }
     } else {
@@ -901,18 +926,22 @@ __global__ void __launch_bounds__(RT, 4) k_lp_apply(ApplyArgs A) {
             if (u < U0) {
                 const int64_t i = u * rpw + (rpw == 32 ? lane : lane >> 4);
                 const int64_t v = i < n0 ? A.clist[0][i] : -1;
-                if (rpw == 32) ab_short<PT>(A, v, delta, moves);
-                else ab_tile<16, PT>(A, v, delta, moves);
+                if (rpw == 32) ab_short<PT>(A, v, delta, cnt);
+                else ab_tile<16, PT>(A, v, delta, cnt);
             } else if (u < U0 + n1) {
-                ab_tile<kTile32, PT>(A, A.clist[1][u - U0], delta, moves);
+                ab_tile<kTile32, PT>(A, A.clist[1][u - U0], delta, cnt);
             } else {
-                ab_warp<PT>(A, A.clist[2][u - U0 - n1], delta, moves);
+                ab_warp<PT>(A, A.clist[2][u - U0 - n1], delta, cnt);
             }
         }
     }
-    moves = warp_sum(moves);
+    cnt.moves = warp_sum(cnt.moves);
+    cnt.deg = warp_sum(cnt.deg);
     __syncthreads();
-    if (lane == 0 && moves) atomicAdd((unsigned long long*)A.moves_out, (unsigned long long)moves);
+    if (lane == 0 && cnt.moves) {
+        atomicAdd((unsigned long long*)&A.step[S_STEP_MOVES], (unsigned long long)cnt.moves);
+        atomicAdd((unsigned long long*)&A.step[S_MVDEG], (unsigned long long)cnt.deg);
+    }
     for (int q = threadIdx.x; q < A.k; q += RT)
         if (delta[q]) atomicAdd((unsigned long long*)&A.pw[q], (unsigned long long)(int64_t)delta[q]);
 }
@@ -920,23 +949,66 @@ __global__ void __launch_bounds__(RT, 4) k_lp_apply(ApplyArgs A) {
 // ------------------------------------------------------------------ rebalance
 constexpr int RB_SHIFT = 10;   // key = segment << 10 | loss bucket
 
-// Candidates (dest >= 0) in vertex order with key (source << 10 | bucket(loss)):
-// k_rb_count counts those of every tile of 8192 vertices, k_rb_collect adds up
-// the counts of the tiles before its own and writes them (each warp 1024
-// vertices: one ballot per 32, then the offsets of the warps before), clearing
-// the locks on the way.  dest is read twice and nothing but the candidates
-// written: 256^3 grid, level 0 (16.8 M vertices, one overweight part in 32)
-// 15 + 55 us against 200 us for flags, a scan of them and a gather.
-constexpr int RB_TILE = 32 * 32 * RW;
-__global__ void __launch_bounds__(RT) k_rb_count(int64_t n, const int32_t* __restrict__ dest, int32_t* __restrict__ cnt) {
-    __shared__ int32_t s_cnt[RW];
-    const int64_t base = (int64_t)blockIdx.x * RB_TILE;
-    int32_t c = 0;
-#pragma unroll 8
-    for (int i = 0; i < RB_TILE / RT; ++i) {
-        const int64_t v = base + (int64_t)i * RT + threadIdx.x;
-        c += v < n && dest[v] >= 0 ? 1 : 0;
+// Candidates (vertices of overweight parts) in vertex order with key (source <<
+// 10 | bucket(loss)): k_rb_count counts those of every tile of PER * 256
+// vertices, k_rb_collect adds up the counts of the tiles before its own and
+// writes them, clearing the locks and copying the partition (the state before
+// the step) on the way.  From kRbWide vertices on a thread takes 32 consecutive
+// ones in 16-byte loads and stores (256^3 grid, level 0, one overweight part in
+// 32: 8 + 48 us against 200 us for flags, a scan of them and a gather); below, one
+// (a warp's 32 rounds of writes are a chain of load latencies: 26 us on 250 K
+// vertices).
+constexpr int64_t kRbWide = 1 << 20;
+constexpr int RB_PER = 32;             // vertices per thread on large levels
+// over flags of the parts in dynamic shared memory (k bytes)
+__device__ __forceinline__ void rb_over(const int64_t* __restrict__ pw, int64_t Lmax, int32_t k, uint8_t* over) {
+    for (int q = threadIdx.x; q < k; q += blockDim.x) over[q] = pw[q] > Lmax;
+    __syncthreads();
+}
+// a thread's 32 vertices from v0 on (v0 a multiple of 32): bit i of the result
+// says whether vertex v0 + i lies in an overweight part; copy (may be nullptr)
+// and lock receive the parts and zeros
+template <class PT>
+__device__ __forceinline__ uint32_t rb_mask(int64_t v0, int64_t n, const PT* __restrict__ pc, const uint8_t* over,
+                                            PT* __restrict__ copy, uint8_t* __restrict__ lock) {
+    constexpr int V = 16 / sizeof(PT), NV = RB_PER / V;
+    uint32_t m = 0;
+    if (v0 + RB_PER <= n) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const uint4 x = *reinterpret_cast<const uint4*>(pc + v0 + i * V);
+            if (copy) *reinterpret_cast<uint4*>(copy + v0 + i * V) = x;
+            const uint32_t word[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int j = 0; j < V; ++j) {
+                const uint32_t p = (word[j * sizeof(PT) / 4] >> (8 * (j * sizeof(PT) % 4))) & (uint32_t)(PT)~(PT)0;
+                m |= (over[p] ? 1u : 0u) << (i * V + j);
+            }
+        }
+        if (lock) {
+            reinterpret_cast<uint4*>(lock + v0)[0] = make_uint4(0, 0, 0, 0);
+            reinterpret_cast<uint4*>(lock + v0)[1] = make_uint4(0, 0, 0, 0);
+        }
+    } else {
+        for (int i = 0; i < RB_PER && v0 + i < n; ++i) {
+            const PT p = pc[v0 + i];
+            if (copy) copy[v0 + i] = p;
+            if (lock) lock[v0 + i] = 0;
+            m |= (over[p] ? 1u : 0u) << i;
+        }
     }
+    return m;
+}
+template <class PT, int PER>
+__global__ void __launch_bounds__(RT) k_rb_count(int64_t n, const PT* __restrict__ pc, const int64_t* __restrict__ pw,
+                                                 int64_t Lmax, int32_t k, int32_t* __restrict__ cnt) {
+    extern __shared__ uint8_t rb_ov[];
+    __shared__ int32_t s_cnt[RW];
+    rb_over(pw, Lmax, k, rb_ov);
+    const int64_t v0 = ((int64_t)blockIdx.x * RT + threadIdx.x) * PER;
+    int32_t c;
+    if (PER == 1) c = v0 < n && rb_ov[pc[v0]] ? 1 : 0;
+    else c = __popc(rb_mask<PT>(v0, n, pc, rb_ov, nullptr, nullptr));
     c = (int32_t)__reduce_add_sync(0xffffffffu, (uint32_t)c);
     if ((threadIdx.x & 31) == 0) s_cnt[threadIdx.x >> 5] = c;
     __syncthreads();
@@ -946,60 +1018,59 @@ __global__ void __launch_bounds__(RT) k_rb_count(int64_t n, const int32_t* __res
         cnt[blockIdx.x] = t;
     }
 }
-__global__ void __launch_bounds__(RT) k_rb_collect(int64_t n, const int32_t* __restrict__ dest,
-                                                   const int32_t* __restrict__ cnt, int64_t ncand,
-                                                   const void* __restrict__ pc, int pcb,
-                                                   const int32_t* __restrict__ gain, uint8_t* __restrict__ lock,
+template <class PT, int PER>
+__global__ void __launch_bounds__(RT) k_rb_collect(int64_t n, const PT* __restrict__ pc, const int64_t* __restrict__ pw,
+                                                   int64_t Lmax, int32_t k, const int32_t* __restrict__ cnt,
+                                                   int64_t ncand, const int32_t* __restrict__ gain,
+                                                   PT* __restrict__ pc_old, uint8_t* __restrict__ lock,
                                                    uint64_t* __restrict__ keys, int32_t* __restrict__ vals) {
+    extern __shared__ uint8_t rb_ov[];
     __shared__ int64_t sh[33];
-    __shared__ int32_t s_cnt[RW];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint32_t lt = (1u << lane) - 1u;
-    int64_t before = 0, s = 0;
+    rb_over(pw, Lmax, k, rb_ov);
+    const int lane = threadIdx.x & 31;
+    int64_t before = 0, s = 0, all;
     for (int64_t t = threadIdx.x; t < blockIdx.x; t += RT) s += cnt[t];
     block_excl_scan<int64_t>(s, sh, before);
-    const int64_t base = (int64_t)blockIdx.x * RB_TILE + (int64_t)w * 1024;
-    uint32_t mine = 0;   // the ballot of step lane
-    int32_t total = 0;
-#pragma unroll 8
-    for (int i = 0; i < 32; ++i) {
-        const int64_t v = base + 32 * i + lane;
-        const uint32_t m = __ballot_sync(0xffffffffu, v < n && dest[v] >= 0);
-        if (v < n) lock[v] = 0;
-        if (lane == i) mine = m;
-        total += __popc(m);
+    const int64_t v0 = ((int64_t)blockIdx.x * RT + threadIdx.x) * PER;
+    if (PER == 1) {
+        const int32_t p = v0 < n ? (int32_t)pc[v0] : -1;
+        const bool take = p >= 0 && rb_ov[p];
+        if (p >= 0) { pc_old[v0] = (PT)p; lock[v0] = 0; }
+        const int64_t at = before + block_excl_scan<int64_t>(take ? 1 : 0, sh, all);
+        if (take && GP_IN(at, ncand)) {
+            keys[at] = ((uint64_t)(uint32_t)p << RB_SHIFT) | loss_bucket(-gain[v0]);
+            vals[at] = (int32_t)v0;
+        }
+        return;
     }
-    if (lane == 0) s_cnt[w] = total;
-    __syncthreads();
-    int64_t pos = before;
-    for (int i = 0; i < w; ++i) pos += s_cnt[i];
+    const uint32_t mine = rb_mask<PT>(v0, n, pc, rb_ov, pc_old, lock);
+    const int64_t at0 = before + block_excl_scan<int64_t>(__popc(mine), sh, all);
+    // the warp writes the 32 vertices of each lane together
     for (int i = 0; i < 32; ++i) {
         const uint32_t m = __shfl_sync(0xffffffffu, mine, i);
-        const int64_t at = pos + __popc(m & lt);
+        if (!m) continue;
+        const int64_t at = __shfl_sync(0xffffffffu, at0, i) + __popc(m & ((1u << lane) - 1u));
         if (((m >> lane) & 1u) && GP_IN(at, ncand)) {
-            const int64_t v = base + 32 * i + lane;
-            keys[at] = ((uint64_t)(uint32_t)load_pc(pc, pcb, v) << RB_SHIFT) | loss_bucket(-gain[v]);
+            const int64_t v = v0 + (int64_t)(i - lane) * RB_PER + lane;
+            keys[at] = ((uint64_t)(uint32_t)pc[v] << RB_SHIFT) | loss_bucket(-gain[v]);
             vals[at] = (int32_t)v;
         }
-        pos += __popc(m);
     }
-}
-
-__device__ __forceinline__ int64_t seg_start(const uint64_t* keys, int64_t i, uint64_t seg) {
-    int64_t lo = 0, hi = i;
-    while (lo < hi) {
-        int64_t mid = (lo + hi) >> 1;
-        if ((keys[mid] >> RB_SHIFT) < seg) lo = mid + 1; else hi = mid;
-    }
-    return lo;
 }
 
 // first index of every key segment (key >> RB_SHIFT = d, d = 0..k) of a
 // sorted candidate list: k + 1 searches instead of one per candidate
+// (a warp per segment, 32 probes at a time)
+template <class F>
+__device__ __forceinline__ int64_t warp_first(int64_t lo, int64_t hi, F below);
 __global__ void k_seg_first(const int64_t* __restrict__ cnt, const uint64_t* __restrict__ keys, int32_t k,
                             int64_t* __restrict__ first) {
-    for (int64_t d = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; d <= k; d += (int64_t)gridDim.x * blockDim.x)
-        first[d] = seg_start(keys, *cnt, (uint64_t)d);
+    const int64_t n = *cnt;
+    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+    for (int d = w; d <= k; d += nw) {
+        const int64_t f = warp_first(0, n, [&](int64_t i) { return (int64_t)(keys[i] >> RB_SHIFT) < d; });
+        if ((threadIdx.x & 31) == 0) first[d] = f;
+    }
 }
 
 // What the sorted candidates let each source part give up, in one block: a
@@ -1016,30 +1087,52 @@ struct RbPlan {
     int64_t* snap;     // part weights before the step
     int64_t* n2;       // kept candidates in all
 };
+// First index in [lo, hi) where below(i) turns false (below is true up to
+// there), by a warp: 32 probes at a time.
+template <class F>
+__device__ __forceinline__ int64_t warp_first(int64_t lo, int64_t hi, F below) {
+    const int lane = threadIdx.x & 31;
+    while (lo < hi) {
+        const int64_t step = (hi - lo + 31) / 32;
+        const int64_t i = lo + (int64_t)lane * step;
+        const uint32_t m = __ballot_sync(0xffffffffu, i < hi && below(i));   // a run of low lanes
+        const int t = __popc(m);
+        if (t == 0) return lo;
+        hi = lo + (int64_t)t * step < hi ? lo + (int64_t)t * step : hi;   // probe t (if any) is not below
+        lo = lo + (int64_t)(t - 1) * step + 1;                             // probe t - 1 is
+    }
+    return lo;
+}
 __global__ void __launch_bounds__(GP_MAX_K) k_rb_plan(int64_t ncand, const uint64_t* __restrict__ keys,
                                                       const int64_t* __restrict__ pre, const int64_t* __restrict__ pw,
                                                       int64_t Lmax, int32_t k, RbPlan P) {
     __shared__ int64_t sh[33];
+    __shared__ int64_t s_a[GP_MAX_K], s_w[GP_MAX_K];
+    // a warp per part: its segment, and the prefix that covers its excess
+    for (int q = threadIdx.x >> 5; q < k; q += blockDim.x >> 5) {
+        const int64_t x = pw[q];
+        int64_t s = 0, a = 0, wa = 0;
+        if (x > Lmax) {
+            s = warp_first(0, ncand, [&](int64_t i) { return (int64_t)(keys[i] >> RB_SHIFT) < q; });
+            const int64_t e = warp_first(s, ncand, [&](int64_t i) { return (int64_t)(keys[i] >> RB_SHIFT) <= q; });
+            const int64_t p0 = s < ncand ? pre[s] : 0;
+            const int64_t f = warp_first(s, e, [&](int64_t i) { return pre[i] - p0 < x - Lmax; });
+            a = f - s;
+            wa = a > 0 ? pre[f] - p0 : 0;
+        }
+        if ((threadIdx.x & 31) == 0) {
+            s_a[q] = a; s_w[q] = wa;
+            P.seg[q] = s; P.acc[q] = a; P.snap[q] = x;
+        }
+    }
+    __syncthreads();
     const int q = threadIdx.x;
     const int64_t x = q < k ? pw[q] : 0;
-    int64_t a = 0, wa = 0;
-    if (q < k) {
-        const int64_t s = seg_start(keys, ncand, (uint64_t)q), e = x > Lmax ? seg_start(keys, ncand, (uint64_t)q + 1) : s;
-        int64_t lo = s, hi = e;   // first candidate whose weight before reaches the excess
-        const int64_t p0 = s < ncand ? pre[s] : 0;
-        while (lo < hi) {
-            const int64_t mid = (lo + hi) >> 1;
-            if (pre[mid] - p0 < x - Lmax) lo = mid + 1; else hi = mid;
-        }
-        a = lo - s;
-        wa = a > 0 ? pre[lo] - p0 : 0;
-        P.seg[q] = s; P.acc[q] = a; P.snap[q] = x;
-    }
     int64_t tot;
-    int64_t e = block_excl_scan<int64_t>(a, sh, tot);
+    int64_t e = block_excl_scan<int64_t>(q < k ? s_a[q] : 0, sh, tot);
     if (q < k) P.off[q] = e;
     if (q == 0) *P.n2 = tot;
-    e = block_excl_scan<int64_t>(wa, sh, tot);
+    e = block_excl_scan<int64_t>(q < k ? s_w[q] : 0, sh, tot);
     if (q < k) P.woff[q] = e;
     e = block_excl_scan<int64_t>(q < k && x <= Lmax ? Lmax - x : 0, sh, tot);
     if (q < k) P.cum[q] = e;
@@ -1070,10 +1163,14 @@ __device__ __forceinline__ void rb_delta_begin(int32_t* delta, int32_t k) {
     for (int q = threadIdx.x; q < k; q += blockDim.x) delta[q] = 0;
     __syncthreads();
 }
-__device__ __forceinline__ void rb_delta_end(int32_t* delta, int32_t k, int64_t nmoves, int64_t* __restrict__ pw,
-                                             int64_t* __restrict__ moves) {
-    for (int o = 16; o > 0; o >>= 1) nmoves += __shfl_xor_sync(0xffffffffu, nmoves, o);
-    if ((threadIdx.x & 31) == 0 && nmoves) atomicAdd((unsigned long long*)moves, (unsigned long long)nmoves);
+__device__ __forceinline__ void rb_delta_end(int32_t* delta, int32_t k, AbCount cnt, int64_t* __restrict__ pw,
+                                             int64_t* __restrict__ step) {
+    cnt.moves = warp_sum(cnt.moves);
+    cnt.deg = warp_sum(cnt.deg);
+    if ((threadIdx.x & 31) == 0 && cnt.moves) {
+        atomicAdd((unsigned long long*)&step[S_STEP_MOVES], (unsigned long long)cnt.moves);
+        atomicAdd((unsigned long long*)&step[S_MVDEG], (unsigned long long)cnt.deg);
+    }
     __syncthreads();
     for (int q = threadIdx.x; q < k; q += blockDim.x)
         if (delta[q]) atomicAdd((unsigned long long*)&pw[q], (unsigned long long)(int64_t)delta[q]);
@@ -1085,10 +1182,10 @@ __global__ void k_rb_weak_apply(const int64_t* __restrict__ cnt_dev, const uint6
                                 const int32_t* __restrict__ vals, const int64_t* __restrict__ pre,
                                 const int32_t* __restrict__ vw, const int64_t* __restrict__ pw_snap, int64_t Lmax,
                                 int32_t k, void* __restrict__ pc, int pcb, uint8_t* __restrict__ lock,
-                                int64_t* __restrict__ pw, int64_t* __restrict__ moves) {
+                                int64_t* __restrict__ pw, const int64_t* __restrict__ rp, int64_t* __restrict__ step) {
     extern __shared__ int32_t rb_delta[];
     rb_delta_begin(rb_delta, k);
-    int64_t nm = 0;
+    AbCount nm;
     const int64_t cnt = *cnt_dev;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += (int64_t)gridDim.x * blockDim.x) {
         const uint64_t d = keys[i] >> RB_SHIFT;
@@ -1103,10 +1200,11 @@ __global__ void k_rb_weak_apply(const int64_t* __restrict__ cnt_dev, const uint6
                 atomicAdd(&rb_delta[d], (int32_t)wv);
                 atomicAdd(&rb_delta[p], -(int32_t)wv);
             }
-            ++nm;
+            ++nm.moves;
+            nm.deg += rp[v + 1] - rp[v];
         }
     }
-    rb_delta_end(rb_delta, k, nm, pw, moves);
+    rb_delta_end(rb_delta, k, nm, pw, step);
 }
 
 // strong: kept candidates laid over the concatenated free capacities
@@ -1114,11 +1212,11 @@ __global__ void k_rb_strong_apply(int64_t cnt, const uint64_t* __restrict__ keys
                                   const int64_t* __restrict__ P, RbPlan plan, const int32_t* __restrict__ vw,
                                   int32_t k, void* __restrict__ pc, int pcb,
                                   uint8_t* __restrict__ lock, int64_t* __restrict__ pw,
-                                  int64_t* __restrict__ moves) {
+                                  const int64_t* __restrict__ rp, int64_t* __restrict__ step) {
     const int64_t* __restrict__ cum = plan.cum;
     extern __shared__ int32_t rb_delta[];
     rb_delta_begin(rb_delta, k);
-    int64_t nm = 0;
+    AbCount nm;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t src = (int64_t)(keys[i] >> RB_SHIFT), s = plan.seg[src];
         if (i - s >= plan.acc[src]) continue;
@@ -1141,10 +1239,131 @@ __global__ void k_rb_strong_apply(int64_t cnt, const uint64_t* __restrict__ keys
                 atomicAdd(&rb_delta[q], (int32_t)wv);
                 atomicAdd(&rb_delta[p], -(int32_t)wv);
             }
-            ++nm;
+            ++nm.moves;
+            nm.deg += rp[v + 1] - rp[v];
         }
     }
-    rb_delta_end(rb_delta, k, nm, pw, moves);
+    rb_delta_end(rb_delta, k, nm, pw, step);
+}
+
+// ------------------------------------------------------------------ cut change of a step
+// After a move step whose next pass will rebalance: the change of the directed
+// cross weight, from the rows of the moved vertices alone (those whose part
+// differs between the partition before and after).  An entry (v, u) of a moved
+// v changes by w ([new v != new u] - [old v != old u]); its mirror (u, v), the
+// same weight on a symmetric graph, is counted with it when u did not move.
+// Exact integers, so that the pass after it need not sweep the rows it looks
+// for no move in: on the 256^3 grid (k = 32) the rebalancing passes, two thirds
+// of all, sweep one part in 32 instead of every row: all its passes take 47 ->
+// 32 ms, k_track 2.5 ms.  Left out when the
+// next pass sweeps every row anyway: no overweight part, or moved rows of more
+// than track_deg entries.  A block compares the partitions over its range of
+// vertices, 4 bytes per lane, and queues the moved ones; its threads take the
+// short rows of the queue, its warps the longer ones (a shared ticket: their
+// lengths differ widely); blocks [0, nitems) take the pieces of the heavy rows.
+struct TrackArgs {
+    DGraph g;
+    int32_t k;
+    int64_t Lmax;
+    const int64_t* pw;
+    const void* pc;             // after the step
+    const void* pc_old;         // before it
+    int64_t* step;              // its status block
+    int64_t track_deg;
+    int32_t heavy_deg;
+    int32_t range;              // vertices per block, a multiple of 4 * RT up to kTrackRange
+    const int32_t* heavy;
+    const int32_t* item_row;
+    const int64_t* item_beg;
+    const int64_t* item_end;
+    int64_t nitems;
+};
+constexpr int kTrackRange = 8192;
+template <class PT>
+__device__ __forceinline__ int32_t track_term(const TrackArgs& T, int64_t e, int32_t po, int32_t pn) {
+    const int32_t u = __ldcs(&T.g.ci[e]);
+    if (!GP_IN(u, T.g.n)) return 0;
+    const int32_t uo = __ldg((const PT*)T.pc_old + u), un = __ldg((const PT*)T.pc + u);
+    const int32_t c = (pn != un ? 1 : 0) - (po != uo ? 1 : 0);
+    const int32_t w = T.g.ew ? __ldcs(&T.g.ew[e]) : 1;
+    return uo == un ? 2 * c * w : c * w;
+}
+template <class PT>
+__global__ void __launch_bounds__(RT) k_track(TrackArgs T) {
+    __shared__ int32_t s_queue[kTrackRange];
+    __shared__ int32_t s_cnt, s_ticket;
+    __shared__ int64_t s_red[RW];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (threadIdx.x == 0) { s_cnt = 0; s_ticket = 0; }
+    int over = 0;
+    for (int q = threadIdx.x; q < T.k; q += RT) over |= T.pw[q] > T.Lmax ? 1 : 0;
+    if (!__syncthreads_or(over)) return;
+    if (T.step[S_STEP_MOVES] == 0 || T.step[S_MVDEG] > T.track_deg) return;
+    int64_t acc = 0;
+    if ((int64_t)blockIdx.x < T.nitems) {
+        const int32_t v = T.heavy[T.item_row[blockIdx.x]];
+        const int32_t po = ((const PT*)T.pc_old)[v], pn = ((const PT*)T.pc)[v];
+        if (po != pn)
+            for (int64_t e = T.item_beg[blockIdx.x] + threadIdx.x; e < T.item_end[blockIdx.x]; e += RT)
+                acc += track_term<PT>(T, e, po, pn);
+    } else {
+        constexpr int per = 4 / sizeof(PT);   // ids per 4-byte word
+        const int64_t v0 = (int64_t)(blockIdx.x - T.nitems) * T.range;
+        for (int32_t i = threadIdx.x * per; i < T.range; i += RT * per) {
+            const int64_t v = v0 + i;
+            uint32_t a = 0, b = 0;
+            if (v + per <= T.g.n) {
+                a = ((const uint32_t*)T.pc_old)[v / per];
+                b = ((const uint32_t*)T.pc)[v / per];
+            } else {
+                for (int j = 0; j < per && v + j < T.g.n; ++j) {
+                    a |= (uint32_t)((const PT*)T.pc_old)[v + j] << (8 * sizeof(PT) * j);
+                    b |= (uint32_t)((const PT*)T.pc)[v + j] << (8 * sizeof(PT) * j);
+                }
+            }
+            const uint32_t x = a ^ b;
+            if (!__any_sync(0xffffffffu, x != 0)) continue;
+#pragma unroll
+            for (int j = 0; j < per; ++j) {
+                const bool mv = ((x >> (8 * sizeof(PT) * j)) & (PT)~(PT)0) != 0;
+                const uint32_t m = __ballot_sync(0xffffffffu, mv);
+                if (!m) continue;
+                int32_t at = 0;
+                if (lane == __ffs(m) - 1) at = atomicAdd(&s_cnt, __popc(m));
+                at = __shfl_sync(0xffffffffu, at, __ffs(m) - 1) + __popc(m & ((1u << lane) - 1u));
+                if (mv && GP_IN(at, kTrackRange)) s_queue[at] = (int32_t)(v + j);
+            }
+        }
+        __syncthreads();
+        const int32_t cnt = s_cnt;
+        for (int32_t i = threadIdx.x; i < cnt; i += RT) {
+            const int32_t v = s_queue[i];
+            const int64_t beg = T.g.rp[v], end = T.g.rp[v + 1];
+            if (end - beg > kShortDeg) continue;
+            const int32_t po = ((const PT*)T.pc_old)[v], pn = ((const PT*)T.pc)[v];
+            for (int64_t e = beg; e < end; ++e) acc += track_term<PT>(T, e, po, pn);
+        }
+        for (;;) {
+            int32_t i = 0;
+            if (lane == 0) i = atomicAdd(&s_ticket, 1);
+            i = __shfl_sync(0xffffffffu, i, 0);
+            if (i >= cnt) break;
+            const int32_t v = s_queue[i];
+            const int64_t beg = T.g.rp[v], end = T.g.rp[v + 1];
+            if (end - beg <= kShortDeg || end - beg > T.heavy_deg) continue;
+            const int32_t po = ((const PT*)T.pc_old)[v], pn = ((const PT*)T.pc)[v];
+#pragma unroll 4
+            for (int64_t e = beg + lane; e < end; e += 32) acc += track_term<PT>(T, e, po, pn);
+        }
+    }
+    acc = warp_sum(acc);
+    if (lane == 0) s_red[w] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int64_t s = 0;
+        for (int i = 0; i < RW; ++i) s += s_red[i];
+        if (s) atomicAdd((unsigned long long*)&T.step[S_DELTA], (unsigned long long)s);
+    }
 }
 
 // ------------------------------------------------------------------ projection, weights, cut
@@ -1383,12 +1602,15 @@ __device__ __forceinline__ int cta_seg_start(const uint64_t* a, int i, int shift
 // (destination, loss bucket, source, id), moves that fit the remaining
 // capacity; strong: kept moves laid over the concatenated free capacities).
 // cand: the candidates in vertex order (ncand of them), or nullptr to take
-// every v < n with dest[v] >= 0.  s_pw (shared) is updated; returns this
-// thread's move count.  Needs ncand <= kCtaMaxN.
+// every v < n of an overweight part.  s_pw (shared) is updated; returns this
+// thread's moves.  Needs ncand <= kCtaMaxN.
 struct RbCta {
     const int32_t* vw;
     void* pc;                   // the partition
     int pcb;                    // its bytes per id
+    void* pc_old;               // receives the partition before the step (nullptr, or a candidate list:
+                                // not wanted / copied already)
+    const int64_t* rp;          // row pointers (nullptr: entries of moved rows not wanted)
     uint8_t* lock;
     const int32_t* dest;
     const int32_t* gain;
@@ -1399,12 +1621,16 @@ struct RbCta {
     int64_t Lmax;
 };
 
-__device__ int64_t cta_rebalance(const RbCta& R, int mode, int64_t n, const int32_t* cand, int64_t ncand_in,
+__device__ AbCount cta_rebalance(const RbCta& R, int mode, int64_t n, const int32_t* cand, int64_t ncand_in,
                                  int32_t* s_pw, int32_t* s_snap, int64_t* s_cum, uint64_t* s_keys, int64_t* sh) {
     const int32_t k = R.k;
     const int64_t Lmax = R.Lmax;
     uint8_t* lock = R.lock;
-    int64_t moves = 0;
+    AbCount cnt;
+    auto moved = [&](uint32_t v) {
+        ++cnt.moves;
+        if (R.rp) cnt.deg += R.rp[v + 1] - R.rp[v];
+    };
     for (int q = threadIdx.x; q < k; q += CT) s_snap[q] = s_pw[q];
     __syncthreads();
     int64_t ncand = ncand_in;
@@ -1414,9 +1640,10 @@ __device__ int64_t cta_rebalance(const RbCta& R, int mode, int64_t n, const int3
     };
     if (cand == nullptr) {
         // candidates in vertex order, then sorted by (source, loss bucket, id)
-        ncand = cta_scan(n, [&](int64_t v) -> int64_t { return R.dest[v] >= 0 ? 1 : 0; }, R.pre, sh);
+        auto over = [&](int64_t v) -> int64_t { return s_snap[load_pc(R.pc, R.pcb, v)] > Lmax ? 1 : 0; };
+        ncand = cta_scan(n, over, R.pre, sh);
         for (int64_t v = threadIdx.x; v < n; v += CT)
-            if (R.dest[v] >= 0) s_keys[R.pre[v]] = key1((uint32_t)v);
+            if (over(v)) s_keys[R.pre[v]] = key1((uint32_t)v);
     } else {
         for (int64_t i = threadIdx.x; i < ncand; i += CT) s_keys[i] = key1((uint32_t)cand[i]);
     }
@@ -1462,7 +1689,7 @@ __device__ int64_t cta_rebalance(const RbCta& R, int mode, int64_t n, const int3
                 lock[v] = 1;
                 atomicAdd(&s_pw[d], (int32_t)wv);
                 atomicAdd(&s_pw[p], -(int32_t)wv);
-                ++moves;
+                moved(v);
             }
         }
     } else {
@@ -1493,19 +1720,19 @@ __device__ int64_t cta_rebalance(const RbCta& R, int mode, int64_t n, const int3
                 lock[v] = 1;
                 atomicAdd(&s_pw[lo], (int32_t)wv);
                 atomicAdd(&s_pw[p], -(int32_t)wv);
-                ++moves;
+                moved(v);
             }
         }
     }
     __syncthreads();
-    return moves;
+    return cnt;
 }
 
 // one rebalance step of the multi-kernel loop in one launch: candidates from
 // dest (n <= kCtaMaxN, locks cleared here) or from a compacted list; part
 // weights in and out of global memory; the step's moves added to *moves_out
 __global__ void __launch_bounds__(CT, 1) k_rb_step_cta(RbCta R, int mode, int64_t n, const int32_t* cand,
-                                                        int64_t ncand, int64_t* pw, int64_t* moves_out) {
+                                                        int64_t ncand, int64_t* pw, int64_t* step) {
     extern __shared__ __align__(16) unsigned char rsm[];
     const int32_t k = R.k;
     int32_t* s_pw = (int32_t*)rsm;               // part weights fit in 32 bits (rb_delta_begin)
@@ -1515,11 +1742,15 @@ __global__ void __launch_bounds__(CT, 1) k_rb_step_cta(RbCta R, int mode, int64_
     __shared__ int64_t sh[33];
     for (int q = threadIdx.x; q < k; q += CT) s_pw[q] = (int32_t)pw[q];
     if (cand == nullptr)
-        for (int64_t v = threadIdx.x; v < n; v += CT) R.lock[v] = 0;
+        for (int64_t v = threadIdx.x; v < n; v += CT) {
+            R.lock[v] = 0;
+            store_pc(R.pc_old, R.pcb, v, load_pc(R.pc, R.pcb, v));
+        }
     __syncthreads();
-    const int64_t moves = cta_sum(cta_rebalance(R, mode, n, cand, ncand, s_pw, s_snap, s_cum, s_keys, sh), sh);
+    const AbCount cnt = cta_rebalance(R, mode, n, cand, ncand, s_pw, s_snap, s_cum, s_keys, sh);
+    const int64_t moves = cta_sum(cnt.moves, sh), deg = cta_sum(cnt.deg, sh);
     for (int q = threadIdx.x; q < k; q += CT) pw[q] = s_pw[q];
-    if (threadIdx.x == 0) *moves_out += moves;
+    if (threadIdx.x == 0) { step[S_STEP_MOVES] += moves; step[S_MVDEG] += deg; }
 }
 
 // the whole refinement loop of one level by one block of CT threads; rsm:
@@ -1580,13 +1811,14 @@ __device__ void cta_refine_level(const CtaRefineArgs& R, unsigned char* rsm) {
         for (int b = 0; b < 3; ++b) { CA.bucket[b] = R.bucket[b]; CA.nbucket[b] = R.nbucket[b]; CA.clist[b] = nullptr; }
         CA.wfirst = nullptr;
         CA.dest = R.dest; CA.gain = R.gain; CA.status = R.status;
-        CA.lock_next = nullptr; CA.prev_moves = nullptr; CA.host = nullptr; CA.nblocks = 0;
+        CA.lock_next = nullptr; CA.prev = nullptr; CA.track_deg = -1; CA.host = nullptr; CA.nblocks = 0;
+        CA.rb_all = R.tr_arrays ? 1 : 0;
         CA.pc = part; CA.pc_next = nullptr; CA.pdg = nullptr; CA.lp_dg = 1;
         CA.hhist = nullptr; CA.hsum = nullptr; CA.hdone = nullptr;
         int64_t acc = 0, cdeg = 0;
         int32_t* hist = s_hist + w * k;
         for (int64_t ub = 8 * w; ub < U2 + U1 + U0; ub += 8 * CW)
-            conn_group<int32_t, true>(CA, ub, (int)(U2 + U1 + U0 - ub < 8 ? U2 + U1 + U0 - ub : 8), dmode, s_over, light, hist,
+            conn_group<int32_t, true>(CA, ub, (int)(U2 + U1 + U0 - ub < 8 ? U2 + U1 + U0 - ub : 8), dmode, true, s_over, light, hist,
                                 s_rows + 32 * w, acc, cdeg);
         acc = warp_sum(acc);
         const int64_t cur_cut = cta_sum(lane == 0 ? acc : 0, sh) / 2;   // also orders the pass
@@ -1621,7 +1853,6 @@ __device__ void cta_refine_level(const CtaRefineArgs& R, unsigned char* rsm) {
         if (dmode == MODE_RB) { mode = (rb_streak >= R.strong_after) ? 2 : 1; ++rb_streak; }
         else { mode = 0; rb_streak = 0; }
         last_mode = mode;
-        int64_t moves = 0;
         __syncthreads();
         if (mode == 0) {
             for (int64_t v = threadIdx.x; v < n; v += CT) { part_next[v] = part[v]; lock_next[v] = 0; }
@@ -1632,29 +1863,29 @@ __device__ void cta_refine_level(const CtaRefineArgs& R, unsigned char* rsm) {
             for (int b = 0; b < 3; ++b) AA.clist[b] = R.clist[b];
             AA.status = R.status; AA.lock_next = lock_next; AA.pw = nullptr;
             AA.pc = part; AA.pc_next = part_next;
-            AA.moves_out = nullptr; AA.hsum = nullptr; AA.hdone = nullptr; AA.pdg = nullptr;
+            AA.step = nullptr; AA.hsum = nullptr; AA.hdone = nullptr; AA.pdg = nullptr;
+            AbCount cnt;
             for (int64_t u = w; u < U2 + U1; u += CW) {
                 const int64_t v = u < U2 ? R.bucket[2][u] : R.bucket[1][u - U2];
                 if (R.dest[v] < 0) continue;
-                if (u < U2) ab_warp<int32_t>(AA, v, s_pw, moves);
-                else ab_tile<kTile32, int32_t>(AA, v, s_pw, moves);
+                if (u < U2) ab_warp<int32_t>(AA, v, s_pw, cnt);
+                else ab_tile<kTile32, int32_t>(AA, v, s_pw, cnt);
             }
             for (int64_t i0 = 32 * w; i0 < R.nbucket[0]; i0 += 32 * CW) {
                 const int64_t v = i0 + lane < R.nbucket[0] ? R.bucket[0][i0 + lane] : -1;
-                ab_short<int32_t>(AA, v >= 0 && R.dest[v] >= 0 ? v : -1, s_pw, moves);
+                ab_short<int32_t>(AA, v >= 0 && R.dest[v] >= 0 ? v : -1, s_pw, cnt);
             }
-            nmoves = cta_sum(moves, sh);
+            nmoves = cta_sum(cnt.moves, sh);
             int32_t* tp = part; part = part_next; part_next = tp;
             uint8_t* tl = lock; lock = lock_next; lock_next = tl;
         } else {
             for (int64_t v = threadIdx.x; v < n; v += CT) lock[v] = 0;
             __syncthreads();
             RbCta RA;
-            RA.vw = R.g.vw; RA.pc = part; RA.pcb = 4; RA.lock = lock; RA.dest = R.dest;
+            RA.vw = R.g.vw; RA.pc = part; RA.pcb = 4; RA.pc_old = nullptr; RA.rp = nullptr; RA.lock = lock; RA.dest = R.dest;
             RA.gain = R.gain; RA.pre = R.pre;
             RA.flag = R.flag; RA.gkeys = R.gkeys; RA.k = k; RA.Lmax = Lmax;
-            moves = cta_rebalance(RA, mode, n, nullptr, 0, s_pw, s_snap, s_cum, s_keys, sh);
-            nmoves = cta_sum(moves, sh);
+            nmoves = cta_sum(cta_rebalance(RA, mode, n, nullptr, 0, s_pw, s_snap, s_cum, s_keys, sh).moves, sh);
         }
         if (R.tr_arrays) {
             int32_t* t = R.tr_arrays + (int64_t)steps * 3 * n;
@@ -1900,7 +2131,7 @@ __global__ void k_expand_part(int64_t n, const void* __restrict__ pc, int pcb, i
         part[v] = load_pc(pc, pcb, v);
 }
 
-static void trace_iter(Ctx& c, const RefineBufs& B, const int64_t* moves_d, int64_t n, int64_t m, int level, int it, int mode,
+static void trace_iter(Ctx& c, const RefineBufs& B, const int64_t* step_d, int64_t n, int64_t m, int level, int it, int mode,
                        int64_t cut_before, int64_t mp_before, const Tracer& tr) {
     std::vector<int32_t> d(n), gn(n), p(n);
     k_expand_part<<<grid_for(n, 256), 256, 0, c.s>>>(n, B.pc, B.pcb, B.part);
@@ -1908,7 +2139,7 @@ static void trace_iter(Ctx& c, const RefineBufs& B, const int64_t* moves_d, int6
     GP_CUDA(cudaMemcpyAsync(d.data(), B.dest, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, c.s));
     GP_CUDA(cudaMemcpyAsync(gn.data(), B.gain, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, c.s));
     GP_CUDA(cudaMemcpyAsync(p.data(), B.part, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, c.s));
-    GP_CUDA(cudaMemcpyAsync(c.h_pinned, moves_d, sizeof(int64_t), cudaMemcpyDeviceToHost, c.s));
+    GP_CUDA(cudaMemcpyAsync(c.h_pinned, step_d + S_STEP_MOVES, sizeof(int64_t), cudaMemcpyDeviceToHost, c.s));
     c.sync();
     gp_trace_event ev;
     memset(&ev, 0, sizeof ev);
@@ -1922,6 +2153,8 @@ constexpr int64_t kConnWarpCost = 8 * (8 + 28);
 // bucket-0 rows from which they take their own launch: below, a second launch
 // (about 3 us a pass) costs more than the registers
 constexpr int64_t kConnSplit = 32768;
+constexpr int64_t kTrackShare = 32;
+constexpr int64_t kTrackMin = 1 << 22;   // entries from which the cut's change is tracked
 int64_t conn_max_warps(const Ctx& c) { return (int64_t)c.sm_count * c.ctas_per_sm * RW; }
 
 // light warp t of a connectivity pass over nw warps takes the units
@@ -1984,7 +2217,15 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
     int stall = 0, rb_streak = 0, steps = 0, last_mode = 0;
     int64_t prev_moves = -1;
     const int nb_k = bits_for(k);
-    int64_t* moves_d = nullptr;   // moves of the last step (its iteration's status block)
+    int64_t* step_d = nullptr;   // status block of the last step
+    int64_t cross2 = 0;          // directed cross weight of the current state
+    // the cut's change over a step is taken from the moved rows when they hold
+    // few of the entries (two gathers each, unbalanced; a pass over every row one
+    // gather each), on levels whose passes cost more than k_track's launch; an
+    // input that is not symmetric has no mirror entries
+    const int64_t track_deg = P.symmetric && g.m >= kTrackMin ? g.m / kTrackShare : -1;
+    int32_t track_range = 4 * RT;   // about 8 blocks per SM
+    while (track_range < kTrackRange && n > (int64_t)track_range * c.sm_count * 8) track_range *= 2;
     const bool move_head = B.mp && P.gnn && gnn_has_move_head(P.gnn);
     // with pdg, proposals and gains of a label-propagation pass are stored apart
     // only for the move head and the trace
@@ -2007,7 +2248,7 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
         for (int b = 0; b < 3; ++b) { CA.bucket[b] = L.bucket[b]; CA.nbucket[b] = L.nbucket[b]; CA.clist[b] = B.clist[b]; }
         CA.wfirst = B.wfirst;
         CA.dest = B.dest; CA.gain = B.gain; CA.status = status;
-        CA.prev_moves = moves_d; CA.host = c.h_pinned; CA.nblocks = (long_rows ? grid : 0) + (split ? short_grid : 0);
+        CA.prev = step_d; CA.track_deg = track_deg; CA.rb_all = tr.on() ? 1 : 0; CA.host = c.h_pinned; CA.nblocks = (long_rows ? grid : 0) + (split ? short_grid : 0);
         CA.pc = B.pc; CA.pc_next = B.pc_next; CA.lock_next = B.lock_next;   // the LP step's starting copy
         CA.pdg = B.pdg; CA.lp_dg = lp_dg;
         if (long_rows) {
@@ -2033,7 +2274,8 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
             c.conn_launches += 1;
             c.conn_bytes += conn_bytes;
         }
-        const int64_t cur_cut = c.h_pinned[S_CROSS] / 2;
+        cross2 = c.h_pinned[H_FULL] ? c.h_pinned[S_CROSS] : cross2 + c.h_pinned[H_DELTA];
+        const int64_t cur_cut = cross2 / 2;
         const int64_t cur_mp = c.h_pinned[S_MAXPW];
         const int dev_mode = (int)c.h_pinned[S_MODE];
         const int64_t nlist = c.h_pinned[S_NL0] + c.h_pinned[S_NL1] + c.h_pinned[S_NL2];
@@ -2043,7 +2285,7 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
             GP_CUDA(cudaMemcpyAsync(B.best, B.pc, (size_t)B.pcb * n, cudaMemcpyDeviceToDevice, c.s));
             GP_CUDA(cudaMemcpyAsync(B.best_pw, B.pw, sizeof(int64_t) * k, cudaMemcpyDeviceToDevice, c.s));
         } else {
-            const int64_t nmoves = c.h_pinned[S_STEP_MOVES];
+            const int64_t nmoves = c.h_pinned[H_MOVES];
             const bool cb = cur_mp <= Lmax, bb = best_mp <= Lmax;
             bool better = false, signif = false;
             if (cb && !bb) { better = true; signif = true; }
@@ -2069,7 +2311,7 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
         if (dev_mode == MODE_RB) { mode = (rb_streak >= P.o.strong_after) ? 2 : 1; ++rb_streak; }
         else { mode = 0; rb_streak = 0; }
         last_mode = mode;
-        moves_d = status + S_STEP_MOVES;  // moves of this step, read at the next sync
+        step_d = status;   // moves of this step, read at the next sync
         if (mode == 0) {
             // pc_next / lock_next were filled by the connectivity pass
             ApplyArgs AA;
@@ -2078,7 +2320,7 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
             AA.nitems = L.nitems; AA.hsum = B.hsum; AA.hdone = B.hdone;
             for (int b = 0; b < 3; ++b) AA.clist[b] = B.clist[b];
             AA.status = status; AA.lock_next = B.lock_next; AA.pw = B.pw;
-            AA.moves_out = moves_d;
+            AA.step = step_d;
             AA.pc = B.pc; AA.pc_next = B.pc_next; AA.pdg = B.pdg;
             if (move_head) {
                 // learned order of the afterburner: (move priority, id) instead of (gain, id)
@@ -2103,15 +2345,16 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
             c.bytes += (9 + B.pcb) * n + 16 * nlist + cdeg * (4 + (g.ew ? 4 : 0) + 8 + B.pcb);
             std::swap(B.lock, B.lock_next);
             std::swap(B.pc, B.pc_next);
+            // label propagation leaves the state before the step in pc_next (swapped)
         } else if (n <= kCtaMaxN && cdeg <= kRbCta) {
             // the whole step in one thread block
             auto mk = c.tmp->save();
             RbCta RA;
-            RA.vw = g.vw; RA.pc = B.pc; RA.pcb = B.pcb; RA.lock = B.lock; RA.dest = B.dest;
+            RA.vw = g.vw; RA.pc = B.pc; RA.pcb = B.pcb; RA.pc_old = B.pc_next; RA.rp = g.rp; RA.lock = B.lock; RA.dest = B.dest;
             RA.gain = B.gain;
             RA.pre = c.tmp_alloc<int64_t>(n); RA.flag = c.tmp_alloc<int32_t>(n);
             RA.gkeys = c.tmp_alloc<uint64_t>(n); RA.k = k; RA.Lmax = Lmax;
-            k_rb_step_cta<<<1, CT, cta_refine_smem(k), c.s>>>(RA, mode, n, nullptr, 0, B.pw, moves_d);
+            k_rb_step_cta<<<1, CT, cta_refine_smem(k), c.s>>>(RA, mode, n, nullptr, 0, B.pw, step_d);
             GP_LAUNCHED(c);
             c.bytes += 4 * n + 12 * n + 80 * n;
             c.tmp->restore(mk);
@@ -2119,22 +2362,33 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
             // candidates in vertex order; stable sort -> (source, bucket, id)
             const int64_t ncand = cdeg;
             auto mk = c.tmp->save();
-            const int64_t ntile = (n + RB_TILE - 1) / RB_TILE;
+            const int per = n >= kRbWide ? RB_PER : 1;
+            const int64_t ntile = (n + (int64_t)per * RT - 1) / ((int64_t)per * RT);
             int32_t* tcnt = c.tmp_alloc<int32_t>(ntile);
-            k_rb_count<<<(unsigned)ntile, RT, 0, c.s>>>(n, B.dest, tcnt);
-            GP_LAUNCHED(c);
-            k_rb_collect<<<(unsigned)ntile, RT, 0, c.s>>>(n, B.dest, tcnt, ncand, B.pc, B.pcb, B.gain, B.lock, B.ckeys,
-                                                          B.cvals);
-            GP_LAUNCHED(c);
+            auto collect = [&](auto* pc, auto* pc_old, auto kcount, auto kcollect) {
+                kcount<<<(unsigned)ntile, RT, kpad, c.s>>>(n, pc, B.pw, Lmax, k, tcnt);
+                GP_LAUNCHED(c);
+                kcollect<<<(unsigned)ntile, RT, kpad, c.s>>>(n, pc, B.pw, Lmax, k, tcnt, ncand, B.gain, pc_old, B.lock,
+                                                             B.ckeys, B.cvals);
+                GP_LAUNCHED(c);
+            };
+            if (B.pcb == 1 && per > 1)
+                collect((uint8_t*)B.pc, (uint8_t*)B.pc_next, k_rb_count<uint8_t, RB_PER>, k_rb_collect<uint8_t, RB_PER>);
+            else if (B.pcb == 1)
+                collect((uint8_t*)B.pc, (uint8_t*)B.pc_next, k_rb_count<uint8_t, 1>, k_rb_collect<uint8_t, 1>);
+            else if (per > 1)
+                collect((uint16_t*)B.pc, (uint16_t*)B.pc_next, k_rb_count<uint16_t, RB_PER>, k_rb_collect<uint16_t, RB_PER>);
+            else
+                collect((uint16_t*)B.pc, (uint16_t*)B.pc_next, k_rb_count<uint16_t, 1>, k_rb_collect<uint16_t, 1>);
             c.bytes += 9 * n;
             if (ncand > 0 && ncand <= kRbCta) {
                 // few candidates: sort, select and apply in one thread block
                 RbCta RA;
-                RA.vw = g.vw; RA.pc = B.pc; RA.pcb = B.pcb; RA.lock = B.lock; RA.dest = B.dest;
+                RA.vw = g.vw; RA.pc = B.pc; RA.pcb = B.pcb; RA.pc_old = B.pc_next; RA.rp = g.rp; RA.lock = B.lock; RA.dest = B.dest;
                 RA.gain = B.gain;
                 RA.pre = c.tmp_alloc<int64_t>(ncand); RA.flag = c.tmp_alloc<int32_t>(ncand);
                 RA.gkeys = c.tmp_alloc<uint64_t>(ncand); RA.k = k; RA.Lmax = Lmax;
-                k_rb_step_cta<<<1, CT, cta_refine_smem(k), c.s>>>(RA, mode, n, B.cvals, ncand, B.pw, moves_d);
+                k_rb_step_cta<<<1, CT, cta_refine_smem(k), c.s>>>(RA, mode, n, B.cvals, ncand, B.pw, step_d);
                 GP_LAUNCHED(c);
                 c.bytes += 80 * ncand;
             } else if (ncand > 0) {
@@ -2146,7 +2400,7 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
                 int64_t* pl = c.tmp_alloc<int64_t>(6 * (int64_t)k + 2);
                 plan.seg = pl; plan.acc = pl + k; plan.off = pl + 2 * k; plan.woff = pl + 3 * k; plan.snap = pl + 4 * k;
                 plan.cum = pl + 5 * k; plan.n2 = pl + 6 * k + 1;
-                k_rb_plan<<<1, (k + 31) & ~31, 0, c.s>>>(ncand, B.ckeys, pre, B.pw, Lmax, k, plan);
+                k_rb_plan<<<1, GP_MAX_K, 0, c.s>>>(ncand, B.ckeys, pre, B.pw, Lmax, k, plan);
                 GP_LAUNCHED(c);
                 if (mode == 1) {
                     k_rb_rekey<<<grid_for(ncand, 256), 256, 0, c.s>>>(ncand, B.ckeys, B.cvals, plan, B.dest, B.ckeys2,
@@ -2155,23 +2409,33 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
                     radix_sort_pairs(c, B.ckeys2, B.cvals2, B.ckeys, B.cvals, ncand, bits, plan.n2);
                     scan_list_weights(c, B.cvals2, g.vw, pre, ncand, plan.n2, nullptr);
                     int64_t* segf = c.tmp_alloc<int64_t>(k + 1);
-                    k_seg_first<<<grid_for(k + 1, 256), 256, 0, c.s>>>(plan.n2, B.ckeys2, k, segf);
+                    k_seg_first<<<grid_for(k + 1, 8), 256, 0, c.s>>>(plan.n2, B.ckeys2, k, segf);
                     GP_LAUNCHED(c);
                     k_rb_weak_apply<<<grid_for(ncand, 256, c.sm_count * 8), 256, sizeof(int32_t) * k, c.s>>>(
                         plan.n2, B.ckeys2, segf, B.cvals2, pre, g.vw, plan.snap, Lmax, k, B.pc, B.pcb, B.lock, B.pw,
-                        moves_d);
+                        g.rp, step_d);
                     GP_LAUNCHED(c);
                 } else {
                     k_rb_strong_apply<<<grid_for(ncand, 256, c.sm_count * 8), 256, sizeof(int32_t) * k, c.s>>>(
-                        ncand, B.ckeys, B.cvals, pre, plan, g.vw, k, B.pc, B.pcb, B.lock, B.pw, moves_d);
+                        ncand, B.ckeys, B.cvals, pre, plan, g.vw, k, B.pc, B.pcb, B.lock, B.pw, g.rp, step_d);
                     GP_LAUNCHED(c);
                 }
                 c.bytes += 80 * ncand;
             }
             c.tmp->restore(mk);
         }
+        if (track_deg >= 0) {
+            TrackArgs T;
+            T.g = g; T.k = k; T.Lmax = Lmax; T.pw = B.pw; T.pc = B.pc; T.pc_old = B.pc_next; T.step = step_d;
+            T.track_deg = track_deg; T.heavy_deg = L.heavy_deg; T.heavy = L.heavy; T.item_row = L.item_row;
+            T.item_beg = L.item_beg; T.item_end = L.item_end; T.nitems = L.nitems;
+            T.range = track_range;
+            const int tg = (int)(L.nitems + (n + track_range - 1) / track_range);
+            (B.pcb == 1 ? k_track<uint8_t> : k_track<uint16_t>)<<<tg, RT, 0, c.s>>>(T);
+            GP_LAUNCHED(c);
+        }
         ++steps;
-        if (tr.on()) trace_iter(c, B, moves_d, n, g.m, level, it, mode, cur_cut, cur_mp, tr);
+        if (tr.on()) trace_iter(c, B, step_d, n, g.m, level, it, mode, cur_cut, cur_mp, tr);
     }
     k_expand_part<<<grid_for(n, 256), 256, 0, c.s>>>(n, B.best, B.pcb, B.part);
     GP_LAUNCHED(c);
