@@ -349,7 +349,9 @@ void vc_begin(Ctx& c, const DGraph& g0, int32_t k, float imbalance, uint64_t see
         }
         if (20 * (n - pairs) > 19 * n) { c.tmp->restore(mk); break; }
         Level cl;
-        contract_level(c, lv.back(), cl, match);
+        cl.heavy_deg = P.o.heavy_deg;
+        cl.item_len = P.o.item_len;
+        contract_level(c, lv.back(), cl, match, pairs);
         c.tmp->restore(mk);
         if (tr.on()) {
             auto cm = to_host(c, lv.back().cmap, n);
@@ -362,9 +364,6 @@ void vc_begin(Ctx& c, const DGraph& g0, int32_t k, float imbalance, uint64_t see
             ev.a0 = cm.data(); ev.rowptr = rp.data(); ev.colidx = ci.data(); ev.ewgt = ew.data(); ev.vwgt = vw.data();
             tr.emit(ev);
         }
-        cl.heavy_deg = P.o.heavy_deg;
-        cl.item_len = P.o.item_len;
-        build_heavy(c, cl);
         lv.push_back(cl);
     }
     GP_CUDA(cudaEventRecord(tm.e[1], c.s));

@@ -15,6 +15,19 @@
 namespace gp {
 
 // ---------------------------------------------------------------- degree buckets
+// Control block of one level (device): what the host reads of it comes in one
+// copy at the end of the level's contraction.
+enum LevelCtl { C_BUCKETS = 0 /* 4: bucket and heavy counts */, C_MAXDEG = 4, C_MAXVW = 5, C_MC = 6, C_ERR = 7,
+                C_LONG = 8 /* 6: long-row tiers */, C_NCTL = 16 };
+
+// raise *out to the warp's largest x (the plain read keeps most warps from the atomic)
+__device__ __forceinline__ void warp_max_to(int64_t x, int64_t* out) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) { const int64_t y = __shfl_xor_sync(0xffffffffu, x, o); x = y > x ? y : x; }
+    if ((threadIdx.x & 31) == 0 && x > *(volatile int64_t*)out)
+        atomicMax((unsigned long long*)out, (unsigned long long)x);
+}
+
 // Lists in any order (each row is processed on its own).  Appends are
 // aggregated per block (block_append), 4 rows per thread at a time on lists
 // long enough for that to matter.
@@ -33,6 +46,7 @@ __global__ void k_buckets(const int64_t* __restrict__ rp, int64_t n, int32_t hea
     int32_t* const lists[4] = {b0, b1, b2, heavy};
     const int64_t caps[4] = {n, n, n, heavy_cap};
     const int64_t per = (int64_t)blockDim.x * kAppendRows;
+    int64_t most = 0;
     for (int64_t base = blockIdx.x * per; base < n; base += gridDim.x * per) {
         int b[kAppendRows];
         int32_t vs[kAppendRows];
@@ -40,10 +54,13 @@ __global__ void k_buckets(const int64_t* __restrict__ rp, int64_t n, int32_t hea
         for (int r = 0; r < kAppendRows; ++r) {
             const int64_t v = base + (int64_t)r * blockDim.x + threadIdx.x;
             vs[r] = (int32_t)v;
-            b[r] = v < n ? degree_bucket(rp[v + 1] - rp[v], heavy_deg) : -1;
+            const int64_t d = v < n ? rp[v + 1] - rp[v] : -1;
+            b[r] = v < n ? degree_bucket(d, heavy_deg) : -1;
+            most = d > most ? d : most;
         }
         block_append<4, kAppendRows>(b, vs, lists, caps, count);
     }
+    warp_max_to(most, &count[C_MAXDEG]);
 }
 
 __global__ void k_heavy_bounds(const int64_t* __restrict__ rp, const int32_t* __restrict__ heavy, int64_t nh,
@@ -71,23 +88,22 @@ __global__ void k_unit_cost(const int64_t* __restrict__ rp, const int32_t* __res
     }
 }
 
-void build_heavy(Ctx& c, Level& L) {
-    auto mk = c.tmp->save();
-    int64_t* d_cnt = c.tmp_alloc<int64_t>(4);
-    memset_async(c, d_cnt, 0, 4 * sizeof(int64_t));
-    const int64_t heavy_cap = std::max<int64_t>(1, L.g.m / L.heavy_deg + 1);
+// enqueue the bucket lists of L (counts and the longest row into ctl), then take
+// what the host read of ctl into L
+static void buckets_begin(Ctx& c, Level& L, int64_t heavy_cap, int64_t* ctl) {
     L.heavy = c.keep_alloc<int32_t>(heavy_cap);
     for (int b = 0; b < 3; ++b) L.bucket[b] = c.keep_alloc<int32_t>(L.g.n);
     const int per = L.g.n >= kAppendMany ? 4 : 1;
-    (per == 4 ? k_buckets<4> : k_buckets<1>)<<<grid_for(L.g.n, 256 * per), 256, 0, c.s>>>(L.g.rp, L.g.n, L.heavy_deg, heavy_cap, L.heavy, L.bucket[0], L.bucket[1], L.bucket[2],
-                                                     d_cnt);
+    (per == 4 ? k_buckets<4> : k_buckets<1>)<<<grid_for(L.g.n, 256 * per), 256, 0, c.s>>>(
+        L.g.rp, L.g.n, L.heavy_deg, heavy_cap, L.heavy, L.bucket[0], L.bucket[1], L.bucket[2], ctl);
     GP_LAUNCHED(c);
     c.bytes += 8 * (L.g.n + 1) + 4 * L.g.n;
-    GP_CUDA(cudaMemcpyAsync(c.h_pinned, d_cnt, 4 * sizeof(int64_t), cudaMemcpyDeviceToHost, c.s));
-    c.sync();
-    for (int b = 0; b < 3; ++b) L.nbucket[b] = c.h_pinned[b];
-    L.nheavy = c.h_pinned[3];
-    c.tmp->restore(mk);
+}
+static void buckets_end(Ctx& c, Level& L, const int64_t* h) {
+    for (int b = 0; b < 3; ++b) L.nbucket[b] = h[C_BUCKETS + b];
+    L.nheavy = h[C_BUCKETS + 3];
+    L.max_deg = h[C_MAXDEG];
+    auto mk = c.tmp->save();
     // items: heavy row h covers [rp[v], rp[v+1]) in pieces of at most item_len
     std::vector<int64_t> rb((size_t)std::max<int64_t>(L.nheavy, 1)), re((size_t)std::max<int64_t>(L.nheavy, 1));
     if (L.nheavy > 0) {
@@ -138,6 +154,31 @@ void build_heavy(Ctx& c, Level& L) {
         GP_CUDA(cudaMemcpyAsync(L.row_first, rows_first.data(), sizeof(int32_t) * L.nheavy, cudaMemcpyHostToDevice, c.s));
         c.sync();  // host vectors go out of scope
     }
+}
+
+__global__ void k_max_vw(int64_t n, const int32_t* __restrict__ vw, int64_t* __restrict__ out) {
+    int64_t mx = 0;
+    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x)
+        mx = vw[v] > mx ? vw[v] : mx;
+    warp_max_to(mx, out);
+}
+
+void build_heavy(Ctx& c, Level& L) {
+    auto mk = c.tmp->save();
+    int64_t* ctl = c.tmp_alloc<int64_t>(C_NCTL);
+    memset_async(c, ctl, 0, C_NCTL * sizeof(int64_t));
+    buckets_begin(c, L, std::max<int64_t>(1, L.g.m / L.heavy_deg + 1), ctl);
+    if (L.g.vw) {
+        k_max_vw<<<grid_for(L.g.n, 256, c.sm_count * 4), 256, 0, c.s>>>(L.g.n, L.g.vw, ctl + C_MAXVW);
+        GP_LAUNCHED(c);
+    }
+    GP_CUDA(cudaMemcpyAsync(c.h_pinned, ctl, C_NCTL * sizeof(int64_t), cudaMemcpyDeviceToHost, c.s));
+    c.sync();
+    int64_t h[C_NCTL];
+    std::copy(c.h_pinned, c.h_pinned + C_NCTL, h);
+    c.tmp->restore(mk);
+    L.max_vw = L.g.vw ? h[C_MAXVW] : 1;
+    buckets_end(c, L, h);
 }
 
 // ---------------------------------------------------------------- argmax helpers
@@ -197,7 +238,10 @@ struct MatchArgs {
     int32_t* iid;
     int32_t* hdone;            // per heavy row: items finished (reset by the last)
     const int32_t* list[3];   // rows to process, by degree bucket
-    int64_t nlist[3];
+    int64_t nlist[3];         // their counts, or bounds on them when
+    const int64_t* dlist;     // the counts are in device memory (nullptr: they are not)
+    int split;                // list[0] is k_match_short's
+    __device__ __forceinline__ int64_t count(int b) const { return dlist ? dlist[b] : nlist[b]; }
     const int32_t* match;
     int32_t* out;             // MODE 0: proposals
     uint32_t salt;
@@ -346,7 +390,7 @@ __device__ __forceinline__ int32_t match_short(const MatchArgs& A, int32_t v, in
 constexpr int64_t kMatchSplit = 24576;
 template <int MODE>
 __global__ void __launch_bounds__(256) k_match_short(MatchArgs A) {
-    const int64_t n0 = A.nlist[0];
+    const int64_t n0 = A.count(0);
     for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); i0 < n0;
          i0 += (int64_t)gridDim.x * blockDim.x) {
         const int64_t i = i0 + (threadIdx.x & 31);
@@ -460,8 +504,8 @@ __global__ void __launch_bounds__(256, 6) k_match_scan(MatchArgs A) {
     }
     const int64_t wid = ((int64_t)(blockIdx.x - A.nitems) * blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)(gridDim.x - A.nitems) * blockDim.x) >> 5;
-    const int64_t n0 = A.nlist[0] < kMatchSplit ? A.nlist[0] : 0;   // else k_match_short's
-    const int64_t U0 = (n0 + 1) / 2, U1 = A.nlist[1], U2 = A.nlist[2];
+    const int64_t n0 = A.split ? 0 : A.count(0);
+    const int64_t U0 = (n0 + 1) / 2, U1 = A.count(1), U2 = A.count(2);
     for (int64_t u = wid; u < U0 + U1 + U2; u += nw) {
         if (u < U0) {
             const int64_t i = u * 2 + (lane >> 4);
@@ -545,10 +589,12 @@ __global__ void __launch_bounds__(256, 6) k_match_scan(MatchArgs A) {
 template <int kAppendRows>
 __global__ void k_handshake(const int64_t* __restrict__ rp, int64_t n, int32_t heavy_deg, const int32_t* l0,
                             const int32_t* l1,
-                            const int32_t* l2, int64_t n0, int64_t n1, int64_t n2, const int32_t* __restrict__ heavy,
+                            const int32_t* l2, int64_t n0, int64_t n1, int64_t n2,
+                            const int64_t* __restrict__ dlist, const int32_t* __restrict__ heavy,
                             int64_t nheavy,
                             const int32_t* __restrict__ prop, int32_t* __restrict__ match, int64_t* __restrict__ pairs,
                             int32_t* nl0, int32_t* nl1, int32_t* nl2, int64_t* next_n, uint8_t* __restrict__ hdead) {
+    if (dlist) { n0 = dlist[0]; n1 = dlist[1]; n2 = dlist[2]; }
     int64_t local = 0, live = 0;
     const int64_t total = n0 + n1 + n2 + nheavy;
     int32_t* const lists[3] = {nl0, nl1, nl2};
@@ -590,10 +636,11 @@ __global__ void k_handshake(const int64_t* __restrict__ rp, int64_t n, int32_t h
 }
 
 // sorted (anchor << nbits | v) keys: pair ranks (0,1), (2,3), ... of each anchor group
-__global__ void k_twohop_pair(const uint64_t* __restrict__ keys, int64_t cnt, int64_t n, int nbits,
+__global__ void k_twohop_pair(const uint64_t* __restrict__ keys, const int64_t* __restrict__ cnt_dev, int64_t n, int nbits,
                               const int32_t* __restrict__ vw,
                               int64_t maxvw, int32_t* __restrict__ match, int64_t* __restrict__ pairs) {
     int64_t local = 0;
+    const int64_t cnt = *cnt_dev;
     const uint64_t lowmask = (1ull << nbits) - 1;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += (int64_t)gridDim.x * blockDim.x) {
         const uint64_t a = keys[i] >> nbits;
@@ -619,24 +666,15 @@ static int bits_for(int64_t x) {  // bits to represent values in [0, x)
     return b;
 }
 
-__global__ void k_max_vw(int64_t n, const int32_t* __restrict__ vw, int64_t* __restrict__ out) {
-    int32_t mx = 0;
-    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x)
-        mx = vw[v] > mx ? vw[v] : mx;
-    for (int o = 16; o > 0; o >>= 1) { const int32_t y = __shfl_xor_sync(0xffffffffu, mx, o); mx = y > mx ? y : mx; }
-    if ((threadIdx.x & 31) == 0 && mx) atomicMax((unsigned long long*)out, (unsigned long long)mx);
-}
-
 // one matching scan over A's lists: the short rows apart when there are many
 template <int MODE>
 static void match_scan(Ctx& c, const MatchArgs& A) {
-    const bool split = A.nlist[0] >= kMatchSplit;
-    const int64_t units = (split ? 0 : (A.nlist[0] + 1) / 2) + A.nlist[1] + A.nlist[2];
-    if (split) {
+    const int64_t units = (A.split ? 0 : (A.nlist[0] + 1) / 2) + A.nlist[1] + A.nlist[2];
+    if (A.split) {
         k_match_short<MODE><<<grid_for(A.nlist[0], 256, c.sm_count * c.ctas_per_sm), 256, 0, c.s>>>(A);
         GP_LAUNCHED(c);
     }
-    if (!split || units + A.nitems > 0) {
+    if (!A.split || units + A.nitems > 0) {
         const int grid = (int)A.nitems + grid_for(units * 32, 256, c.sm_count * c.ctas_per_sm);
         k_match_scan<MODE><<<grid, 256, 0, c.s>>>(A);
         GP_LAUNCHED(c);
@@ -652,7 +690,9 @@ int64_t match_level(Ctx& c, const Level& L, int level, const Params& P, int32_t*
     int32_t* wl[2][3];
     for (int s2 = 0; s2 < 2; ++s2)
         for (int b = 0; b < 3; ++b) wl[s2][b] = c.tmp_alloc<int32_t>(std::max<int64_t>(L.nbucket[b], 1));
-    int64_t* d_cnt = c.tmp_alloc<int64_t>(8);
+    // counters of a batch of rounds: pairs, the next lists' three counts, live heavy rows
+    constexpr int kBatch = 4, kCnt = 8;
+    int64_t* d_cnt = c.tmp_alloc<int64_t>(kBatch * kCnt);
     GP_CUDA(cudaMemsetAsync(match, 0xff, sizeof(int32_t) * g.n, c.s));
     MatchArgs A;
     A.g = g; A.heavy = L.heavy; A.nheavy = L.nheavy; A.match = match; A.out = prop; A.salt = salt;
@@ -669,48 +709,58 @@ int64_t match_level(Ctx& c, const Level& L, int level, const Params& P, int32_t*
     A.anchor0 = c.tmp_alloc<int32_t>(g.n);
     // weight cap: skip the per-neighbour weight check when the two heaviest
     // vertices of the level together stay within maxvw
-    A.check_vw = 0;
-    if (g.vw) {
-        int64_t* d_mx = c.tmp_alloc<int64_t>(1);
-        memset_async(c, d_mx, 0, sizeof(int64_t));
-        k_max_vw<<<grid_for(g.n, 256, c.sm_count * 4), 256, 0, c.s>>>(g.n, g.vw, d_mx);
-        GP_LAUNCHED(c);
-        A.check_vw = 2 * read_i64(c, d_mx) > P.maxvw ? 1 : 0;
-    } else {
-        A.check_vw = 2 > P.maxvw ? 1 : 0;
-    }
+    A.check_vw = 2 * L.max_vw > P.maxvw ? 1 : 0;
     uint8_t* hdead = c.tmp_alloc<uint8_t>(std::max<int64_t>(L.nheavy, 1));
     memset_async(c, hdead, 0, std::max<int64_t>(L.nheavy, 1));
     A.hdead = hdead;
     for (int b = 0; b < 3; ++b) { A.list[b] = L.bucket[b]; A.nlist[b] = L.nbucket[b]; }
-    int64_t pairs = 0, heavy_live = L.nheavy;
+    A.dlist = nullptr;
+    A.split = L.nbucket[0] >= kMatchSplit ? 1 : 0;
+    int64_t pairs = 0;
     int rounds = 0;
     bool anchors_ready = false;   // round 0 ran and wrote anchor0
-    for (int r = 0; r < P.o.match_rounds; ++r) {
-        const int64_t units = A.nlist[0] + A.nlist[1] + A.nlist[2];
-        // nobody left who can propose: this round would add no pair
-        if (units == 0 && heavy_live == 0) { rounds = r + 1; break; }
-        A.any_matched = r > 0 ? 1 : 0;
-        memset_async(c, d_cnt, 0, 5 * sizeof(int64_t));
-        match_scan<0>(c, A);
-        if (r == 0) anchors_ready = true;
-        int32_t** nxt = wl[r & 1];
-        const int64_t tot = A.nlist[0] + A.nlist[1] + A.nlist[2] + L.nheavy;
-        const int per = tot >= kAppendMany ? 4 : 1;
-        (per == 4 ? k_handshake<4> : k_handshake<1>)<<<grid_for(tot, 256 * per), 256, 0, c.s>>>(g.rp, g.n, L.heavy_deg, A.list[0], A.list[1], A.list[2], A.nlist[0], A.nlist[1],
-                                                         A.nlist[2], L.heavy, L.nheavy, prop, match, d_cnt, nxt[0],
-                                                         nxt[1], nxt[2], d_cnt + 1, hdead);
-        GP_LAUNCHED(c);
-        const int64_t share = g.n ? (tot * 1000) / g.n : 0;
-        c.bytes += (L.scan_bytes() + 4 * g.m) * share / 1000 + 16 * tot;
-        GP_CUDA(cudaMemcpyAsync(c.h_pinned, d_cnt, 5 * sizeof(int64_t), cudaMemcpyDeviceToHost, c.s));
+    const int64_t tot0 = A.nlist[0] + A.nlist[1] + A.nlist[2] + L.nheavy;
+    // Rounds are enqueued four at a time, each taking its lists' counts from
+    // device memory (the level's counts bound them), and read together.  A round
+    // that adds no pair ends the matching: the rounds after it add none either,
+    // since nothing they look at has changed.
+    bool done = tot0 == 0;
+    if (done && P.o.match_rounds > 0) rounds = 1;
+    int64_t left = tot0;
+    for (int r0 = 0; r0 < P.o.match_rounds && !done; r0 += kBatch) {
+        const int nr = std::min(kBatch, P.o.match_rounds - r0);
+        memset_async(c, d_cnt, 0, kBatch * kCnt * sizeof(int64_t));
+        for (int i = 0; i < nr; ++i) {
+            const int r = r0 + i;
+            int64_t* cnt = d_cnt + i * kCnt;
+            A.any_matched = r > 0 ? 1 : 0;
+            match_scan<0>(c, A);
+            anchors_ready = true;
+            int32_t** nxt = wl[r & 1];
+            const int per = tot0 >= kAppendMany ? 4 : 1;
+            (per == 4 ? k_handshake<4> : k_handshake<1>)<<<grid_for(tot0, 256 * per), 256, 0, c.s>>>(
+                g.rp, g.n, L.heavy_deg, A.list[0], A.list[1], A.list[2], A.nlist[0], A.nlist[1], A.nlist[2], A.dlist,
+                L.heavy, L.nheavy, prop, match, cnt, nxt[0], nxt[1], nxt[2], cnt + 1, hdead);
+            GP_LAUNCHED(c);
+            for (int b = 0; b < 3; ++b) A.list[b] = nxt[b];
+            A.dlist = cnt + 1;
+        }
+        GP_CUDA(cudaMemcpyAsync(c.h_pinned, d_cnt, kBatch * kCnt * sizeof(int64_t), cudaMemcpyDeviceToHost, c.s));
         c.sync();
-        const int64_t newp = c.h_pinned[0];
-        heavy_live = c.h_pinned[4];
-        rounds = r + 1;
-        pairs += newp;
-        for (int b = 0; b < 3; ++b) { A.list[b] = nxt[b]; A.nlist[b] = c.h_pinned[1 + b]; }
-        if (newp == 0) break;
+        for (int i = 0; i < nr && !done; ++i) {
+            const int64_t* h = c.h_pinned + i * kCnt;
+            const int64_t share = g.n ? (left * 1000) / g.n : 0;
+            c.bytes += (L.scan_bytes() + 4 * g.m) * share / 1000 + 16 * left;
+            rounds = r0 + i + 1;
+            pairs += h[0];
+            left = h[1] + h[2] + h[3] + L.nheavy;
+            if (h[0] == 0) done = true;
+        }
+        if (r0 + kBatch < P.o.match_rounds) {   // the counters are cleared: the counts move to the host
+            for (int b = 0; b < 3; ++b) A.nlist[b] = c.h_pinned[(nr - 1) * kCnt + 1 + b];
+            A.dlist = nullptr;
+            A.split = A.nlist[0] >= kMatchSplit ? 1 : 0;
+        }
     }
     if (P.o.two_hop > 0 && 4 * (g.n - pairs) > 3 * g.n) {
         const int nb = bits_for(g.n);
@@ -720,6 +770,8 @@ int64_t match_level(Ctx& c, const Level& L, int level, const Params& P, int32_t*
         int32_t* vals2 = c.tmp_alloc<int32_t>(g.n);
         memset_async(c, d_cnt, 0, 2 * sizeof(int64_t));
         MatchArgs B2 = A;
+        B2.dlist = nullptr;
+        B2.split = L.nbucket[0] >= kMatchSplit ? 1 : 0;
         B2.hdead = nullptr;   // anchors: the top neighbour over all neighbours
         B2.cand = nullptr; B2.cmore = nullptr;
         // round 0 saw every neighbour but v itself when no pair can exceed the weight cap
@@ -729,13 +781,13 @@ int64_t match_level(Ctx& c, const Level& L, int level, const Params& P, int32_t*
         B2.out = nullptr; B2.keys = keys; B2.nkeys = d_cnt + 1; B2.nbits = nb;
         match_scan<1>(c, B2);
         c.bytes += L.scan_bytes() + 4 * g.n;
-        int64_t cnt = read_i64(c, d_cnt + 1);
-        if (cnt > 1) {
-            GP_CUDA(cudaMemsetAsync(vals, 0, sizeof(int32_t) * cnt, c.s));
-            radix_sort_pairs(c, keys, vals, keys2, vals2, cnt, 2 * nb);
-            k_twohop_pair<<<grid_for(cnt, 256), 256, 0, c.s>>>(keys, cnt, g.n, nb, g.vw, P.maxvw, match, d_cnt);
+        // at most the unmatched vertices have an anchor; vals is payload nobody reads
+        const int64_t most = g.n - 2 * pairs;
+        if (most > 1) {
+            radix_sort_pairs(c, keys, vals, keys2, vals2, most, 2 * nb, d_cnt + 1);
+            k_twohop_pair<<<grid_for(most, 256), 256, 0, c.s>>>(keys, d_cnt + 1, g.n, nb, g.vw, P.maxvw, match, d_cnt);
             GP_LAUNCHED(c);
-            c.bytes += 24 * cnt;
+            c.bytes += 24 * most;
             pairs += read_i64(c, d_cnt);
         }
     }
@@ -745,17 +797,11 @@ int64_t match_level(Ctx& c, const Level& L, int level, const Params& P, int32_t*
 }
 
 // ---------------------------------------------------------------- contraction
-__global__ void k_rep_flags(int64_t n, const int32_t* __restrict__ match, int32_t* __restrict__ flag) {
-    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t u = match[v];
-        flag[v] = (u < 0 || v < u) ? 1 : 0;
-    }
-}
-
 // cmap for every fine vertex; members, weight and row-length bound per coarse vertex
 __global__ void k_cmap(DGraph g, const int32_t* __restrict__ match, const int64_t* __restrict__ cid,
                        int32_t* __restrict__ cmap, int32_t* __restrict__ mem, int32_t* __restrict__ cvw,
-                       int64_t* __restrict__ cdeg) {
+                       int64_t* __restrict__ cdeg, int64_t* __restrict__ max_vw) {
+    int64_t most = 0;
     for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < g.n; v += (int64_t)gridDim.x * blockDim.x) {
         const int32_t u = match[v];
         const bool rep = (u < 0 || v < u);
@@ -771,8 +817,10 @@ __global__ void k_cmap(DGraph g, const int32_t* __restrict__ match, const int64_
             if (u >= 0) { w += g.vw ? g.vw[u] : 1; d += g.rp[u + 1] - g.rp[u]; }
             cvw[cc] = (int32_t)w;
             cdeg[cc] = d;
+            most = w > most ? w : most;
         }
     }
+    warp_max_to(most, max_vw);
 }
 
 // ---- row dedup in first-occurrence order
@@ -786,6 +834,7 @@ __global__ void k_cmap(DGraph g, const int32_t* __restrict__ match, const int64_
 // three times, so k_fill_walk_d first writes those rows, mapped, into a walk
 // layout (row c at off[c]).  Every tier writes its unique entries at off[c]
 // (a bound on the row) and k_contract_copy packs them.  Tiers by row length d:
+//   S  d <= 32         one thread, 16 or 32 entries in registers
 //   A  d <= 128        one warp, 256-slot table in shared memory
 //   A2 d <= 256        one warp, 512-slot table
 //   B  d <= 512        one warp, 1024-slot table (11 KB per warp: 20 warps per SM)
@@ -893,6 +942,58 @@ __device__ __forceinline__ int32_t warp_dedup(const DGraph& g, const int32_t* __
         __syncwarp();
     }
     return count;
+}
+
+// Tier S: a row of at most N walk entries by one thread.  The entries' loads,
+// then their cmap gathers, are in flight together; a later copy of a key adds
+// its weight to the first one's register and drops out, so the keys that remain
+// are in first-occurrence order.  A warp per row spent most of its issue slots
+// on rows of a dozen entries (256^3 grid, level 0: 9.1 M coarse rows of at most
+// 12 walk entries, 3.3 -> 0.9 ms).
+template <int N>
+__device__ __forceinline__ int32_t thread_dedup(const DGraph& g, const int32_t* __restrict__ cmap, const Walk& W,
+                                                int32_t deg, int32_t self, int32_t* __restrict__ tci,
+                                                int32_t* __restrict__ tew) {
+    int32_t key[N], w[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) key[i] = i < deg ? __ldg(&g.ci[W.entry(i)]) : -1;
+    if (g.ew) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) w[i] = i < deg ? __ldg(&g.ew[W.entry(i)]) : 0;
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; ++i) w[i] = 1;
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+        if (key[i] >= 0) key[i] = GP_IN(key[i], g.n) ? cmap[key[i]] : -1;
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+        if (key[i] == self) key[i] = -1;
+#pragma unroll
+    for (int j = 1; j < N; ++j)
+#pragma unroll
+        for (int i = 0; i < j; ++i)
+            if (key[j] >= 0 && key[i] == key[j]) { w[i] += w[j]; key[j] = -1; }
+    int32_t r = 0;
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+        if (key[i] >= 0) { tci[r] = key[i]; tew[r] = w[i]; ++r; }
+    return r;
+}
+constexpr int TS_ROW = 32;
+template <int N>
+__global__ void __launch_bounds__(128) k_dedup_thread(DGraph g, const int32_t* __restrict__ cmap,
+                                                      const int32_t* __restrict__ mem, int64_t nc, int64_t minrow,
+                                                      const int64_t* __restrict__ off, const int64_t* __restrict__ cdeg,
+                                                      int32_t* __restrict__ tci, int32_t* __restrict__ tew,
+                                                      int32_t* __restrict__ cnt) {
+    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t deg = cdeg[c];
+        if (deg > N || deg < minrow) continue;
+        const int64_t o = off[c];
+        cnt[c] = thread_dedup<N>(g, cmap, walk_of(g, mem, c), (int32_t)deg, (int32_t)c, tci + o, tew + o);
+    }
 }
 
 template <int MAXROW, int SLOTS, class IdxT>
@@ -1492,24 +1593,26 @@ __global__ void __launch_bounds__(256) k_contract_copy(int64_t nc, int64_t cm, i
     }
 }
 
-void contract_level(Ctx& c, Level& fine, Level& coarse, const int32_t* match) {
+void contract_level(Ctx& c, Level& fine, Level& coarse, const int32_t* match, int64_t pairs) {
     const DGraph& g = fine.g;
-    auto mk = c.tmp->save();
-    int32_t* flag = c.tmp_alloc<int32_t>(g.n);
-    int64_t* cid = c.tmp_alloc<int64_t>(g.n);
-    int64_t* d_tot = c.tmp_alloc<int64_t>(4);
-    k_rep_flags<<<grid_for(g.n, 256), 256, 0, c.s>>>(g.n, match, flag);
-    GP_LAUNCHED(c);
-    scan_excl_i32_to_i64(c, flag, cid, g.n, d_tot);
-    const int64_t nc = read_i64(c, d_tot);
+    const int64_t nc = g.n - pairs;
     fine.cmap = c.keep_alloc<int32_t>(g.n);
-    int32_t* mem = c.tmp_alloc<int32_t>(2 * nc);
     int32_t* cvw = c.keep_alloc<int32_t>(nc);
+    int64_t* crp = c.keep_alloc<int64_t>(nc + 1);
+    coarse.g.n = nc;
+    coarse.g.rp = crp;
+    coarse.g.vw = cvw;
+    auto mk = c.tmp->save();
+    int64_t* cid = c.tmp_alloc<int64_t>(g.n);
+    int64_t* ctl = c.tmp_alloc<int64_t>(C_NCTL);
+    memset_async(c, ctl, 0, C_NCTL * sizeof(int64_t));
+    scan_representatives(c, match, cid, g.n);
+    int32_t* mem = c.tmp_alloc<int32_t>(2 * nc);
     int64_t* cdeg = c.tmp_alloc<int64_t>(nc);
-    k_cmap<<<grid_for(g.n, 256), 256, 0, c.s>>>(g, match, cid, fine.cmap, mem, cvw, cdeg);
+    k_cmap<<<grid_for(g.n, 256), 256, 0, c.s>>>(g, match, cid, fine.cmap, mem, cvw, cdeg, ctl + C_MAXVW);
     GP_LAUNCHED(c);
     int64_t* off = c.tmp_alloc<int64_t>(nc + 1);
-    scan_excl_i64(c, cdeg, off, nc, off + nc);
+    scan_excl_i64(c, cdeg, off, nc, nullptr);
     const int64_t T = g.m;
     int32_t* mapped = c.tmp_alloc<int32_t>(T);
     int32_t* mw = c.tmp_alloc<int32_t>(T);
@@ -1521,10 +1624,9 @@ void contract_level(Ctx& c, Level& fine, Level& coarse, const int32_t* match) {
     int32_t* listC2 = c.tmp_alloc<int32_t>(nc);
     int32_t* listC3 = c.tmp_alloc<int32_t>(nc);
     int32_t* listD = c.tmp_alloc<int32_t>(nc);
-    int64_t* lcount = c.tmp_alloc<int64_t>(6);
-    int32_t* err = c.tmp_alloc<int32_t>(1);
-    memset_async(c, lcount, 0, 6 * sizeof(int64_t));
-    memset_async(c, err, 0, sizeof(int32_t));
+    int64_t* lcount = ctl + C_LONG;
+    int32_t* err = (int32_t*)(ctl + C_ERR);
+    const int64_t most = 2 * fine.max_deg;   // no coarse row has a longer walk
     {
         constexpr size_t smA = 8 * warp_dedup_smem<TA_ROW, TA_SLOTS, int32_t>();
         constexpr size_t smA2 = 8 * warp_dedup_smem<TA2_ROW, TA2_SLOTS, int16_t>();
@@ -1532,22 +1634,38 @@ void contract_level(Ctx& c, Level& fine, Level& coarse, const int32_t* match) {
         auto kA = k_dedup_warp<TA_ROW, TA_SLOTS, 8, int32_t>;
         auto kA2 = k_dedup_warp<TA2_ROW, TA2_SLOTS, 8, int16_t>;
         auto kB = k_dedup_warp<TB_ROW, TB_SLOTS, TB_WARPS, int16_t>;
-        kA<<<grid_for(nc * 32, 256, c.sm_count * c.ctas_per_sm), 256, smA, c.s>>>(g, fine.cmap, mem, nc, 0, off, cdeg,
-                                                                                  tci, tew, rowcnt);
+        k_dedup_thread<16><<<grid_for(nc, 128, c.sm_count * c.ctas_per_sm), 128, 0, c.s>>>(g, fine.cmap, mem, nc, 0, off,
+                                                                                         cdeg, tci, tew, rowcnt);
         GP_LAUNCHED(c);
-        kA2<<<grid_for(nc * 32, 256, c.sm_count * c.ctas_per_sm), 256, smA2, c.s>>>(g, fine.cmap, mem, nc, TA_ROW + 1,
-                                                                                    off, cdeg, tci, tew, rowcnt);
-        GP_LAUNCHED(c);
-        kB<<<grid_for(nc * 32, TB_WARPS * 32, c.sm_count * c.ctas_per_sm), TB_WARPS * 32, smB, c.s>>>(
-            g, fine.cmap, mem, nc, TA2_ROW + 1, off, cdeg, tci, tew, rowcnt);
-        GP_LAUNCHED(c);
+        if (most > 16) {
+            k_dedup_thread<TS_ROW><<<grid_for(nc, 128, c.sm_count * c.ctas_per_sm), 128, 0, c.s>>>(
+                g, fine.cmap, mem, nc, 17, off, cdeg, tci, tew, rowcnt);
+            GP_LAUNCHED(c);
+        }
+        if (most > TS_ROW) {
+            kA<<<grid_for(nc * 32, 256, c.sm_count * c.ctas_per_sm), 256, smA, c.s>>>(g, fine.cmap, mem, nc, TS_ROW + 1, off,
+                                                                                      cdeg, tci, tew, rowcnt);
+            GP_LAUNCHED(c);
+        }
+        if (most > TA_ROW) {
+            kA2<<<grid_for(nc * 32, 256, c.sm_count * c.ctas_per_sm), 256, smA2, c.s>>>(
+                g, fine.cmap, mem, nc, TA_ROW + 1, off, cdeg, tci, tew, rowcnt);
+            GP_LAUNCHED(c);
+        }
+        if (most > TA2_ROW) {
+            kB<<<grid_for(nc * 32, TB_WARPS * 32, c.sm_count * c.ctas_per_sm), TB_WARPS * 32, smB, c.s>>>(
+                g, fine.cmap, mem, nc, TA2_ROW + 1, off, cdeg, tci, tew, rowcnt);
+            GP_LAUNCHED(c);
+        }
     }
-    k_long_rows<<<grid_for(nc, 256), 256, 0, c.s>>>(nc, cdeg, listC1, listC, listC2, listC3, listD, lcount);
-    GP_LAUNCHED(c);
-    GP_CUDA(cudaMemcpyAsync(c.h_pinned, lcount, 6 * sizeof(int64_t), cudaMemcpyDeviceToHost, c.s));
-    c.sync();
-    const int64_t nC = c.h_pinned[0], nD = c.h_pinned[1], maxD = c.h_pinned[2], nC2 = c.h_pinned[3];
-    const int64_t nC3 = c.h_pinned[4], nC1 = c.h_pinned[5];
+    int64_t nC = 0, nD = 0, nC2 = 0, nC3 = 0, nC1 = 0;
+    if (most > TB_ROW) {
+        k_long_rows<<<grid_for(nc, 256), 256, 0, c.s>>>(nc, cdeg, listC1, listC, listC2, listC3, listD, lcount);
+        GP_LAUNCHED(c);
+        GP_CUDA(cudaMemcpyAsync(c.h_pinned, lcount, 6 * sizeof(int64_t), cudaMemcpyDeviceToHost, c.s));
+        c.sync();
+        nC = c.h_pinned[0]; nD = c.h_pinned[1]; nC2 = c.h_pinned[3]; nC3 = c.h_pinned[4]; nC1 = c.h_pinned[5];
+    }
     if (nC1 > 0) {
         k_dedup_cta_smem<TC1_T, TC1_SLOTS, TC1_ROW>
             <<<(unsigned)std::min<int64_t>(nC1, (int64_t)c.sm_count * c.ctas_per_sm), TC1_T,
@@ -1580,7 +1698,6 @@ void contract_level(Ctx& c, Level& fine, Level& coarse, const int32_t* match) {
         GP_LAUNCHED(c);
     }
     if (nD > 0) {
-        (void)maxD;
         // row lengths to the host: tables, word ranges and pieces
         int64_t* d_deg = c.tmp_alloc<int64_t>(nD);
         k_td_rows<<<grid_for(nD, 256), 256, 0, c.s>>>(listD, nD, cdeg, d_deg);
@@ -1642,13 +1759,16 @@ void contract_level(Ctx& c, Level& fine, Level& coarse, const int32_t* match) {
         k_td_write<<<(unsigned)np, TD_T, 0, c.s>>>(D, off, cdeg, mapped, tci, tew, rowcnt);
         GP_LAUNCHED(c);
     }
-    int64_t* crp = c.keep_alloc<int64_t>(nc + 1);
     scan_excl_i32_to_i64(c, rowcnt, crp, nc, crp + nc);
-    GP_CUDA(cudaMemcpyAsync(c.h_pinned, crp + nc, sizeof(int64_t), cudaMemcpyDeviceToHost, c.s));
-    GP_CUDA(cudaMemcpyAsync(c.h_pinned + 1, err, sizeof(int32_t), cudaMemcpyDeviceToHost, c.s));
+    GP_CUDA(cudaMemcpyAsync(ctl + C_MC, crp + nc, sizeof(int64_t), cudaMemcpyDeviceToDevice, c.s));
+    // the coarse rows' buckets, then everything the host needs in one read
+    buckets_begin(c, coarse, std::max<int64_t>(1, g.m / coarse.heavy_deg + 1), ctl);
+    GP_CUDA(cudaMemcpyAsync(c.h_pinned, ctl, C_NCTL * sizeof(int64_t), cudaMemcpyDeviceToHost, c.s));
     c.sync();
-    const int64_t mc = c.h_pinned[0];
-    if ((int32_t)c.h_pinned[1] != 0) throw GpError(GP_EINTERNAL, "contraction hash table overflow");
+    int64_t h[C_NCTL];
+    std::copy(c.h_pinned, c.h_pinned + C_NCTL, h);
+    const int64_t mc = h[C_MC];
+    if ((int32_t)h[C_ERR] != 0) throw GpError(GP_EINTERNAL, "contraction hash table overflow");
     int32_t* cci = c.keep_alloc<int32_t>(mc);
     int32_t* cew = c.keep_alloc<int32_t>(mc);
     const int64_t cslice = csr_slice(mc, c.sm_count);
@@ -1658,13 +1778,12 @@ void contract_level(Ctx& c, Level& fine, Level& coarse, const int32_t* match) {
     // rows read twice (count and rank for long rows), cmap gathered per entry,
     // unique entries written to the temporary and copied once
     c.bytes += 2 * (8 * (g.n + 1) + 8 * g.m) + 4 * g.m + 8 * (nc + 1) + 4 * nc + 24 * mc + 24 * nc;
-    coarse.g.n = nc;
     coarse.g.m = mc;
-    coarse.g.rp = crp;
     coarse.g.ci = cci;
     coarse.g.ew = cew;
-    coarse.g.vw = cvw;
+    coarse.max_vw = h[C_MAXVW];
     c.tmp->restore(mk);
+    buckets_end(c, coarse, h);
 }
 
 // shared-memory caps of the contraction kernels above 48 KB; set once per

@@ -338,6 +338,8 @@ constexpr int kLearnedItemLen = 16384;
 // exclusive scan; out may alias in; returns total on the host if total_out != nullptr
 void scan_excl_i32_to_i64(Ctx& c, const int32_t* in, int64_t* out, int64_t n, int64_t* d_total);
 void scan_excl_i64(Ctx& c, const int64_t* in, int64_t* out, int64_t n, int64_t* d_total);
+// exclusive scan of the flags "vertex i represents its matched pair, or is unmatched"
+void scan_representatives(Ctx& c, const int32_t* match, int64_t* out, int64_t n);
 // exclusive scan of the weights vw[list[i]] (1 without weights), i < n; n_dev
 // (may be nullptr): the length in device memory, n being a bound on it
 void scan_list_weights(Ctx& c, const int32_t* list, const int32_t* vw, int64_t* out, int64_t n, const int64_t* n_dev,

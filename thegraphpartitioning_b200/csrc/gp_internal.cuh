@@ -43,6 +43,8 @@ struct Level {
     int64_t nheavy = 0;
     int32_t* bucket[3] = {nullptr, nullptr, nullptr};
     int64_t nbucket[3] = {0, 0, 0};
+    int64_t max_deg = 0;          // longest row
+    int64_t max_vw = 1;           // heaviest vertex
     // heavy rows split into items of at most item_len entries, one CTA each
     int32_t* item_row = nullptr;   // index into heavy[]
     int64_t* item_beg = nullptr;   // entry range of the item
@@ -207,11 +209,13 @@ void gnn_move_priorities(Ctx& c, const gp_gnn* G, const DGraph& g, int level, co
                          const int32_t* gain, int32_t* mp);
 
 // gp_coarsen.cu
+// the row buckets of a level (a coarse level of contract_level has them)
 void build_heavy(Ctx& c, Level& L);
 // prio: per-entry matching priority replacing the edge weight (nullptr: weights)
 int64_t match_level(Ctx& c, const Level& L, int level, const Params& P, int32_t* match, int* rounds_out,
                     const int32_t* prio = nullptr);
-void contract_level(Ctx& c, Level& fine, Level& coarse, const int32_t* match);
+// pairs: matched pairs; coarse.heavy_deg and coarse.item_len are set by the caller
+void contract_level(Ctx& c, Level& fine, Level& coarse, const int32_t* match, int64_t pairs);
 
 // gp_initpart.cu
 int initial_partition(Ctx& c, const Level& L, const Params& P, int32_t* part_out);

@@ -115,6 +115,13 @@ struct InArray {
     const T* p;
     __device__ __forceinline__ int64_t operator()(int64_t i) const { return (int64_t)p[i]; }
 };
+struct InRep {                 // 1 for the representative of a matched pair and for unmatched vertices
+    const int32_t* match;
+    __device__ __forceinline__ int64_t operator()(int64_t i) const {
+        const int32_t u = match[i];
+        return u < 0 || i < u ? 1 : 0;
+    }
+};
 struct InListWeight {
     const int32_t* list;
     const int32_t* vw;
@@ -251,6 +258,9 @@ void scan_excl_i32_to_i64(Ctx& c, const int32_t* in, int64_t* out, int64_t n, in
 }
 void scan_excl_i64(Ctx& c, const int64_t* in, int64_t* out, int64_t n, int64_t* d_total) {
     scan_excl(c, InArray<int64_t>{in}, out, n, nullptr, d_total);
+}
+void scan_representatives(Ctx& c, const int32_t* match, int64_t* out, int64_t n) {
+    scan_excl(c, InRep{match}, out, n, nullptr, nullptr);
 }
 void scan_list_weights(Ctx& c, const int32_t* list, const int32_t* vw, int64_t* out, int64_t n, const int64_t* n_dev,
                        int64_t* d_total) {
