@@ -40,6 +40,7 @@
 
 #include <cuda_bf16.h>
 #include <mutex>
+#include <type_traits>
 
 namespace gp {
 
@@ -129,6 +130,9 @@ __device__ __forceinline__ void tile_reduce(float (&x)[F], int width) {
         for (int j = 0; j < F; ++j) x[j] += __shfl_xor_sync(0xffffffffu, x[j], o);
 }
 
+// bucket-0 rows from which they take a launch of their own, one thread per row
+constexpr int64_t kGnnSplit = 24576;
+
 // out_v = fin(v, sum over entries e of row v of val(e)) for every vertex v.
 // CTAs [0, nitems) each sum one item of a long row into ipart[item]; the
 // long rows are finished by k_gnn_rowsum_heavy.
@@ -156,7 +160,8 @@ __global__ void __launch_bounds__(256) k_gnn_rowsum(GnnRows R, Val val, Fin fin,
     }
     const int64_t wid = ((int64_t)(blockIdx.x - R.nitems) * blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)(gridDim.x - R.nitems) * blockDim.x) >> 5;
-    const int64_t U0 = (R.nb[0] + 3) / 4, U1 = R.nb[1], U2 = R.nb[2];
+    const int64_t U0 = R.nb[0] < kGnnSplit ? (R.nb[0] + 3) / 4 : 0;   // else k_gnn_rowsum_short's
+    const int64_t U1 = R.nb[1], U2 = R.nb[2];
     for (int64_t u = wid; u < U0 + U1 + U2; u += nw) {
         float acc[F];
 #pragma unroll
@@ -198,32 +203,88 @@ __global__ void k_gnn_rowsum_heavy(GnnRows R, Fin fin, const float* __restrict__
     }
 }
 
-// op(v, e) for every entry e of every row v, in the same row layout
-template <class Op>
-__global__ void __launch_bounds__(256) k_gnn_entries(GnnRows R, Op op) {
-    const int lane = threadIdx.x & 31;
-    if ((int64_t)blockIdx.x < R.nitems) {
-        const int64_t v = R.heavy[R.item_row[blockIdx.x]];
-        const int64_t end = R.item_end[blockIdx.x];
-        for (int64_t e = R.item_beg[blockIdx.x] + threadIdx.x; e < end; e += blockDim.x) op(v, e);
-        return;
+// The bucket-0 rows of k_gnn_rowsum, one per thread: the entries' values (parts
+// of Val::G floats) in registers, added in the order of the 8-lane layout
+// (entries i and i + 8, then the tree over 8), so the sums are the same bits.
+// 8 lanes per row left lanes idle and spent a shuffle per float and step: 128^3
+// grid (2.1 M rows of 6 entries), 8 floats 267 -> 100 us, 4 floats 126 -> 61 us.
+template <int N, int F, class Val>
+__device__ __forceinline__ void rowsum_thread(const Val& val, int64_t beg, int len, float (&acc)[F]) {
+    constexpr int G = Val::G;
+    int32_t u[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) u[i] = i < len ? val.id(beg + i) : 0;
+#pragma unroll
+    for (int p = 0; p < F; p += G) {
+        float x[N][G];
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+#pragma unroll
+            for (int j = 0; j < G; ++j) x[i][j] = 0.f;
+            if (i < len) val.part(u[i], p / G, x[i]);
+        }
+#pragma unroll
+        for (int s = N / 2; s > 0; s >>= 1)
+#pragma unroll
+            for (int i = 0; i < s; ++i)
+#pragma unroll
+                for (int j = 0; j < G; ++j) x[i][j] += x[i + s][j];
+#pragma unroll
+        for (int j = 0; j < G; ++j) acc[p + j] = x[0][j];
     }
-    const int64_t wid = ((int64_t)(blockIdx.x - R.nitems) * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nw = ((int64_t)(gridDim.x - R.nitems) * blockDim.x) >> 5;
-    const int64_t U0 = (R.nb[0] + 3) / 4, U1 = R.nb[1], U2 = R.nb[2];
-    for (int64_t u = wid; u < U0 + U1 + U2; u += nw) {
-        if (u < U0) {
-            const int64_t i = u * 4 + (lane >> 3);
-            if (i < R.nb[0]) {
-                const int64_t v = R.b[0][i];
-                const int64_t e = R.g.rp[v] + (lane & 7), end = R.g.rp[v + 1];
-                if (e < end) op(v, e);
-                if (e + 8 < end) op(v, e + 8);
+}
+template <int F, class Val, class Fin>
+__global__ void __launch_bounds__(256) k_gnn_rowsum_short(GnnRows R, Val val, Fin fin) {
+    const int64_t n0 = R.nb[0];
+    for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); i0 < n0;
+         i0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = i0 + (threadIdx.x & 31);
+        const int64_t v = i < n0 ? R.b[0][i] : -1;
+        int64_t beg = 0;
+        int len = 0;
+        if (v >= 0) { beg = R.g.rp[v]; len = (int)(R.g.rp[v + 1] - beg); }
+        const uint32_t most = __reduce_max_sync(0xffffffffu, (uint32_t)len);
+        float acc[F];
+        if (most <= 8) rowsum_thread<8, F>(val, beg, len, acc);
+        else rowsum_thread<kShortDeg, F>(val, beg, len, acc);
+        if (v >= 0) fin(v, acc);
+    }
+}
+
+// op(v, e) for every entry e of every row v: a warp per slice of entries, the
+// rows of 32 consecutive vertices in its lanes (csr_row_of, csr_window_lane),
+// so that loads and stores of the entries coalesce whatever the row lengths
+template <class Op>
+__global__ void __launch_bounds__(256) k_gnn_entries(DGraph g, int64_t slice, Op op) {
+    const int lane = threadIdx.x & 31;
+    const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const int64_t nslice = (g.m + slice - 1) / slice;
+    for (int64_t sl = wid; sl < nslice; sl += nw) {
+        const int64_t o1 = (sl + 1) * slice < g.m ? (sl + 1) * slice : g.m;
+        int64_t o = sl * slice;
+        int64_t cb = csr_row_of(g.rp, g.n, o), s = 0, wend = 0;
+        auto window = [&]() {
+            s = cb + lane < g.n ? g.rp[cb + lane] : g.m;
+            wend = g.rp[cb + 32 < g.n ? cb + 32 : g.n];
+        };
+        window();
+        while (o < o1) {
+            const int64_t lim = o1 < wend ? o1 : wend;
+            if (o + 64 <= lim) {   // two groups' loads in flight
+                const int64_t e = o + lane;
+                const int64_t v = cb + csr_window_lane(s, e), v2 = cb + csr_window_lane(s, e + 32);
+                op(v, e, v2, e + 32);
+                o += 64;
+            } else if (o < lim) {
+                const int64_t e = o + lane;
+                const int64_t v = cb + csr_window_lane(s, e);
+                if (e < lim) op(v, e);
+                o = o + 32 < lim ? o + 32 : lim;
+            } else {
+                cb += 32;   // o >= wend: o lies in a later row
+                window();
             }
-        } else {
-            const int64_t v = u < U0 + U1 ? R.b[1][u - U0] : R.b[2][u - U0 - U1];
-            const int64_t end = R.g.rp[v + 1];
-            for (int64_t e = R.g.rp[v] + lane; e < end; e += 32) op(v, e);
         }
     }
 }
@@ -231,10 +292,19 @@ __global__ void __launch_bounds__(256) k_gnn_entries(GnnRows R, Op op) {
 // entry values and row finishers
 struct ValWeight {          // edge weight
     const int32_t* ew;
+    static constexpr int G = 1;
+    __device__ int32_t id(int64_t e) const { return __ldg(&ew[e]); }
+    __device__ void part(int32_t w, int, float (&a)[1]) const { a[0] += (float)w; }
     __device__ void operator()(int64_t e, float (&a)[1]) const { a[0] += (float)__ldcs(&ew[e]); }
 };
 struct ValRow4 {            // the neighbour's 4-float row
     const int32_t* ci; const float4* in;
+    static constexpr int G = 4;
+    __device__ int32_t id(int64_t e) const { return __ldg(&ci[e]); }
+    __device__ void part(int32_t u, int, float (&a)[4]) const {
+        const float4 x = in[u];
+        a[0] += x.x; a[1] += x.y; a[2] += x.z; a[3] += x.w;
+    }
     __device__ void operator()(int64_t e, float (&a)[4]) const {
         const float4 x = in[__ldcs(&ci[e])];
         a[0] += x.x; a[1] += x.y; a[2] += x.z; a[3] += x.w;
@@ -242,6 +312,12 @@ struct ValRow4 {            // the neighbour's 4-float row
 };
 struct ValRow8 {            // the neighbour's 8-float row
     const int32_t* ci; const float4* in;
+    static constexpr int G = 4;
+    __device__ int32_t id(int64_t e) const { return __ldg(&ci[e]); }
+    __device__ void part(int32_t u, int p, float (&a)[4]) const {
+        const float4 x = in[2 * (int64_t)u + p];
+        a[0] += x.x; a[1] += x.y; a[2] += x.z; a[3] += x.w;
+    }
     __device__ void operator()(int64_t e, float (&a)[8]) const {
         const int64_t u = __ldcs(&ci[e]);
         const float4 x = in[2 * u], y = in[2 * u + 1];
@@ -279,113 +355,240 @@ __global__ void k_gnn_vfeat(int64_t n, const int64_t* __restrict__ rp, const int
     }
 }
 
-// h1 = ReLU(W1 [x; a] + b1), m = P h1; thread per vertex, weights in shared memory
+// two FP32 fused multiply-adds in one instruction, each rounded as the scalar one
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 p, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(p));
+}
+__device__ __forceinline__ void fma2(f32x2& acc, f32x2 a, f32x2 b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+
+// The dense layers run on packed FMAs (fma.rn.f32x2) against weights staged in
+// shared memory; every sum adds its terms in input order.  What bounds them is
+// the shared loads' return path (a 16-byte load of a warp brings 512 bytes to
+// registers even when all lanes read the same address), so the weights a thread
+// loads serve several vertices.  128^3 grid (2.1 M vertices), l1 169 -> 108 us
+// with two vertices per thread (V = 2, from kGnnWide vertices on: below, the chip
+// has more use for the blocks).
+constexpr int64_t kGnnWide = 131072;
+
+// h1 = ReLU(W1 [x; a] + b1), m = P h1
+template <int V>
 __global__ void __launch_bounds__(128) k_gnn_l1(int64_t n, const __nv_bfloat16* __restrict__ w,
                                                 const float* __restrict__ x, const float* __restrict__ a,
                                                 float* __restrict__ m, float* __restrict__ h1_out) {
-    __shared__ float sW1[H * 2 * F0], sB1[H], sP[MSG * H];
+    __shared__ __align__(16) float sW1[H * 2 * F0], sB1[H], sPT[H * MSG];
     for (int i = threadIdx.x; i < H * 2 * F0; i += blockDim.x) sW1[i] = wload(w, O_W1 + i);
     for (int i = threadIdx.x; i < H; i += blockDim.x) sB1[i] = wload(w, O_B1 + i);
-    for (int i = threadIdx.x; i < MSG * H; i += blockDim.x) sP[i] = wload(w, O_P + i);
+    for (int i = threadIdx.x; i < MSG * H; i += blockDim.x) sPT[(i % H) * MSG + i / H] = wload(w, O_P + i);
     __syncthreads();
-    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
-        float in[2 * F0];
+    const int64_t step = (int64_t)blockDim.x * V;
+    for (int64_t v0 = blockIdx.x * step + threadIdx.x; v0 < n; v0 += gridDim.x * step) {
+        float in[V][2 * F0];
+        f32x2 mm[V][MSG / 2];
 #pragma unroll
-        for (int j = 0; j < F0; ++j) { in[j] = x[F0 * v + j]; in[F0 + j] = a[F0 * v + j]; }
-        float mm[MSG];
+        for (int t = 0; t < V; ++t) {
+            const int64_t v = v0 + t * blockDim.x;
+            const float4 p = v < n ? reinterpret_cast<const float4*>(x)[v] : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 q = v < n ? reinterpret_cast<const float4*>(a)[v] : make_float4(0.f, 0.f, 0.f, 0.f);
+            in[t][0] = p.x; in[t][1] = p.y; in[t][2] = p.z; in[t][3] = p.w;
+            in[t][4] = q.x; in[t][5] = q.y; in[t][6] = q.z; in[t][7] = q.w;
 #pragma unroll
-        for (int j = 0; j < MSG; ++j) mm[j] = 0.f;
+            for (int j = 0; j < MSG / 2; ++j) mm[t][j] = 0ull;
+        }
+        asm volatile("" ::: "memory");   // the weights stay in shared memory
+#pragma unroll 2
         for (int i = 0; i < H; ++i) {
-            float s = sB1[i];
+            const float4 w0 = reinterpret_cast<const float4*>(sW1)[2 * i], w1 = reinterpret_cast<const float4*>(sW1)[2 * i + 1];
+            const float wr[2 * F0] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+            const f32x2* pt = reinterpret_cast<const f32x2*>(sPT + i * MSG);
 #pragma unroll
-            for (int j = 0; j < 2 * F0; ++j) s += sW1[i * 2 * F0 + j] * in[j];
-            s = s > 0.f ? s : 0.f;
-            if (h1_out) h1_out[H * v + i] = s;
+            for (int t = 0; t < V; ++t) {
+                float s = sB1[i];
 #pragma unroll
-            for (int j = 0; j < MSG; ++j) mm[j] += sP[j * H + i] * s;
+                for (int j = 0; j < 2 * F0; ++j) s += wr[j] * in[t][j];
+                s = s > 0.f ? s : 0.f;
+                if (h1_out && v0 + t * blockDim.x < n) h1_out[H * (v0 + t * blockDim.x) + i] = s;
+                const f32x2 ss = pack2(s, s);
+#pragma unroll
+                for (int j = 0; j < MSG / 2; ++j) fma2(mm[t][j], pt[j], ss);
+            }
         }
 #pragma unroll
-        for (int j = 0; j < MSG; ++j) m[MSG * v + j] = mm[j];
+        for (int t = 0; t < V; ++t) {
+            const int64_t v = v0 + t * blockDim.x;
+            if (v >= n) continue;
+            float o[MSG];
+#pragma unroll
+            for (int j = 0; j < MSG / 2; ++j) unpack2(mm[t][j], o[2 * j], o[2 * j + 1]);
+            reinterpret_cast<float4*>(m)[2 * v] = make_float4(o[0], o[1], o[2], o[3]);
+            reinterpret_cast<float4*>(m)[2 * v + 1] = make_float4(o[4], o[5], o[6], o[7]);
+        }
     }
 }
 
-// h2 = ReLU(W2 [h1; c] + b2), z = Z h2 (h1 recomputed from x, a); thread per vertex.
-// W2 is staged transposed so that one h1 (or c) component updates all 64
-// accumulators from one contiguous shared-memory row; each h2 sum still adds
-// its terms in input order.
-__global__ void __launch_bounds__(128) k_gnn_l2(int64_t n, const __nv_bfloat16* __restrict__ w,
-                                                const float* __restrict__ x, const float* __restrict__ a,
-                                                const float* __restrict__ c, float* __restrict__ z,
-                                                float* __restrict__ h2_out) {
-    __shared__ float sW1[H * 2 * F0], sB1[H], sW2T[(H + MSG) * H], sB2[H], sZ[ZD * H];
+// h2 = ReLU(W2 [h1; c] + b2), z = Z h2 (h1 recomputed from x, a).  A warp takes
+// 32 vertices, a lane an 8 x 8 tile of their outputs (vertices 8 (lane % 4) + t,
+// outputs 8 (lane / 4) + i): per input component 8 weights and 8 components, four
+// 16-byte shared loads, feed 32 packed FMAs, which balances the loads' return path
+// (16 floats per lane) against the FMA pipe.  The components of 16 inputs at a
+// time are computed by their vertex's lane and shared through the warp's buffer,
+// the outputs come back through it, 32 at a time, to their vertex's lane, which
+// sums z in input order.  2.1 M vertices: a vertex per thread 728 us (16 loads per
+// 32 packed FMAs), 4 vertices x 16 outputs with shuffled components 631, this 543.
+// W2 is staged transposed.
+constexpr int L2_T = 128, L2_PITCH = 36;
+__global__ void __launch_bounds__(L2_T, 4) k_gnn_l2(int64_t n, const __nv_bfloat16* __restrict__ w,
+                                                    const float* __restrict__ x, const float* __restrict__ a,
+                                                    const float* __restrict__ c, float* __restrict__ z,
+                                                    float* __restrict__ h2_out) {
+    __shared__ __align__(16) float sW1[H * 2 * F0], sB1[H], sW2T[(H + MSG) * H], sB2[H], sZ[ZD * H];
+    __shared__ __align__(16) float s_out[L2_T / 32][32 * L2_PITCH];
     for (int i = threadIdx.x; i < H * 2 * F0; i += blockDim.x) sW1[i] = wload(w, O_W1 + i);
     for (int i = threadIdx.x; i < H; i += blockDim.x) { sB1[i] = wload(w, O_B1 + i); sB2[i] = wload(w, O_B2 + i); }
     for (int i = threadIdx.x; i < H * (H + MSG); i += blockDim.x) {
-        const int r = i / (H + MSG), q = i % (H + MSG);
-        sW2T[q * H + r] = wload(w, O_W2 + i);
+        const int r = i % H, q = i / H;
+        sW2T[i] = wload(w, O_W2 + r * (H + MSG) + q);
     }
     for (int i = threadIdx.x; i < ZD * H; i += blockDim.x) sZ[i] = wload(w, O_Z + i);
     __syncthreads();
-    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
-        float in[2 * F0];
-#pragma unroll
-        for (int j = 0; j < F0; ++j) { in[j] = x[F0 * v + j]; in[F0 + j] = a[F0 * v + j]; }
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, vg = lane & 3, og = lane >> 2;
+    float* out = s_out[wp];
+    for (int64_t base = ((int64_t)blockIdx.x * (L2_T / 32) + wp) * 32; base < n; base += (int64_t)gridDim.x * L2_T) {
+        const int64_t v = base + lane;
+        const bool valid = v < n;
+        const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 x4 = valid ? reinterpret_cast<const float4*>(x)[v] : zero;
+        const float4 a4 = valid ? reinterpret_cast<const float4*>(a)[v] : zero;
+        const float in[2 * F0] = {x4.x, x4.y, x4.z, x4.w, a4.x, a4.y, a4.z, a4.w};
         // keep the staged weights in shared memory: without this barrier the
-        // compiler hoists every constant-indexed weight read out of the vertex
-        // loop and spills them
+        // compiler hoists constant-indexed weight reads out of the vertex loop
         asm volatile("" ::: "memory");
-        float acc[H];
+        f32x2 acc[8][4];
+        {
+            const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(sB2 + 8 * og);
+            const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(sB2 + 8 * og + 4);
 #pragma unroll
-        for (int i = 0; i < H; ++i) acc[i] = sB2[i];
-#pragma unroll 1
-        for (int q = 0; q < H; ++q) {
-            float s = sB1[q];
-#pragma unroll
-            for (int j = 0; j < 2 * F0; ++j) s += sW1[q * 2 * F0 + j] * in[j];
-            s = s > 0.f ? s : 0.f;
-            const float* col = sW2T + q * H;
-#pragma unroll
-            for (int i = 0; i < H; ++i) acc[i] += col[i] * s;
+            for (int t = 0; t < 8; ++t) { acc[t][0] = b0.x; acc[t][1] = b0.y; acc[t][2] = b1.x; acc[t][3] = b1.y; }
         }
-#pragma unroll 1
-        for (int q = 0; q < MSG; ++q) {
-            const float s = c[MSG * v + q];
-            const float* col = sW2T + (H + q) * H;
+        // inputs [q0, q0 + cnt), their components at the warp's vertices in out[i * 32 + vertex]
+        auto columns = [&](int q0, int cnt) {
+            __syncwarp();
+#pragma unroll 2
+            for (int i = 0; i < cnt; ++i) {
+                float s[8];
+                *reinterpret_cast<float4*>(s) = *reinterpret_cast<const float4*>(out + i * 32 + 8 * vg);
+                *reinterpret_cast<float4*>(s + 4) = *reinterpret_cast<const float4*>(out + i * 32 + 8 * vg + 4);
+                const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(sW2T + (q0 + i) * H + 8 * og);
+                const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(sW2T + (q0 + i) * H + 8 * og + 4);
 #pragma unroll
-            for (int i = 0; i < H; ++i) acc[i] += col[i] * s;
+                for (int t = 0; t < 8; ++t) {
+                    const f32x2 ss = pack2(s[t], s[t]);
+                    fma2(acc[t][0], b0.x, ss);
+                    fma2(acc[t][1], b0.y, ss);
+                    fma2(acc[t][2], b1.x, ss);
+                    fma2(acc[t][3], b1.y, ss);
+                }
+            }
+            __syncwarp();
+        };
+#pragma unroll 1
+        for (int q0 = 0; q0 < H; q0 += 16) {
+#pragma unroll 4
+            for (int i = 0; i < 16; ++i) {
+                const int q = q0 + i;
+                const float4 w0 = reinterpret_cast<const float4*>(sW1)[2 * q], w1 = reinterpret_cast<const float4*>(sW1)[2 * q + 1];
+                const float wr[2 * F0] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+                float s = sB1[q];
+#pragma unroll
+                for (int j = 0; j < 2 * F0; ++j) s += wr[j] * in[j];
+                out[i * 32 + lane] = s > 0.f ? s : 0.f;
+            }
+            columns(q0, 16);
+        }
+        {
+            const float4 c0 = valid ? reinterpret_cast<const float4*>(c)[2 * v] : zero;
+            const float4 c1 = valid ? reinterpret_cast<const float4*>(c)[2 * v + 1] : zero;
+            const float cc[MSG] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+#pragma unroll
+            for (int q = 0; q < MSG; ++q) out[q * 32 + lane] = cc[q];
+            columns(H, MSG);
         }
         float zz[ZD];
 #pragma unroll
         for (int j = 0; j < ZD; ++j) zz[j] = 0.f;
 #pragma unroll
-        for (int i = 0; i < H; ++i) {
-            const float s = acc[i] > 0.f ? acc[i] : 0.f;
-            if (h2_out) h2_out[H * v + i] = s;
+        for (int half = 0; half < 2; ++half) {
+            __syncwarp();
+            if ((og >> 2) == half) {
 #pragma unroll
-            for (int j = 0; j < ZD; ++j) zz[j] += sZ[j * H + i] * s;
+                for (int t = 0; t < 8; ++t)
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        float4 o;
+                        unpack2(acc[t][2 * k], o.x, o.y);
+                        unpack2(acc[t][2 * k + 1], o.z, o.w);
+                        o.x = o.x > 0.f ? o.x : 0.f; o.y = o.y > 0.f ? o.y : 0.f;
+                        o.z = o.z > 0.f ? o.z : 0.f; o.w = o.w > 0.f ? o.w : 0.f;
+                        *reinterpret_cast<float4*>(out + (8 * vg + t) * L2_PITCH + 8 * (og & 3) + 4 * k) = o;
+                        if (h2_out && base + 8 * vg + t < n)
+                            *reinterpret_cast<float4*>(h2_out + H * (base + 8 * vg + t) + 8 * og + 4 * k) = o;
+                    }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) {
+                const float4 o = *reinterpret_cast<const float4*>(out + lane * L2_PITCH + i);
+                const float ov[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+#pragma unroll
+                    for (int j = 0; j < ZD; ++j) zz[j] += sZ[j * H + 32 * half + i + e] * ov[e];
+            }
         }
-#pragma unroll
-        for (int j = 0; j < ZD; ++j) z[ZD * v + j] = zz[j];
+        if (valid) reinterpret_cast<float4*>(z)[v] = make_float4(zz[0], zz[1], zz[2], zz[3]);
     }
 }
 
 // signature bit of vertex x (0..127)
 __host__ __device__ __forceinline__ uint32_t nb_bit(int32_t x) { return fmix32((uint32_t)x * 0x9E3779B1u) >> 25; }
 
-// 128-bit neighbour signature of every vertex, one warp per row
+// 128-bit neighbour signature of every vertex: 32 vertices per warp, rows of at
+// most 32 entries by their lane, longer ones by the warp one after another
+__device__ __forceinline__ void sig_add(int32_t u, uint32_t (&w)[4]) {
+    const uint32_t b = nb_bit(u), m = 1u << (b & 31), q = b >> 5;
+    w[0] |= q == 0 ? m : 0u; w[1] |= q == 1 ? m : 0u; w[2] |= q == 2 ? m : 0u; w[3] |= q == 3 ? m : 0u;
+}
 __global__ void k_gnn_sig(DGraph g, uint4* __restrict__ sig) {
     const int lane = threadIdx.x & 31;
     const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t v = wid; v < g.n; v += nw) {
-        uint32_t w0 = 0, w1 = 0, w2 = 0, w3 = 0;
-        for (int64_t e = g.rp[v] + lane; e < g.rp[v + 1]; e += 32) {
-            const uint32_t b = nb_bit(__ldcs(&g.ci[e])), m = 1u << (b & 31), q = b >> 5;
-            w0 |= q == 0 ? m : 0u; w1 |= q == 1 ? m : 0u; w2 |= q == 2 ? m : 0u; w3 |= q == 3 ? m : 0u;
+    for (int64_t v0 = wid * 32; v0 < g.n; v0 += nw * 32) {
+        const int64_t v = v0 + lane;
+        const int64_t beg = v < g.n ? g.rp[v] : 0, end = v < g.n ? g.rp[v + 1] : 0;
+        const bool is_long = end - beg > 32;
+        if (v < g.n && !is_long) {
+            uint32_t w[4] = {0, 0, 0, 0};
+#pragma unroll 4
+            for (int64_t e = beg; e < end; ++e) sig_add(__ldg(&g.ci[e]), w);
+            sig[v] = make_uint4(w[0], w[1], w[2], w[3]);
         }
-        w0 = __reduce_or_sync(0xffffffffu, w0); w1 = __reduce_or_sync(0xffffffffu, w1);
-        w2 = __reduce_or_sync(0xffffffffu, w2); w3 = __reduce_or_sync(0xffffffffu, w3);
-        if (lane == 0) sig[v] = make_uint4(w0, w1, w2, w3);
+        for (uint32_t todo = __ballot_sync(0xffffffffu, is_long); todo; todo &= todo - 1) {
+            const int src = __ffs(todo) - 1;
+            const int64_t b2 = __shfl_sync(0xffffffffu, beg, src), e2 = __shfl_sync(0xffffffffu, end, src);
+            uint32_t w[4] = {0, 0, 0, 0};
+#pragma unroll 4
+            for (int64_t e = b2 + lane; e < e2; e += 32) sig_add(__ldcs(&g.ci[e]), w);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) w[q] = __reduce_or_sync(0xffffffffu, w[q]);
+            if (lane == 0) sig[v0 + src] = make_uint4(w[0], w[1], w[2], w[3]);
+        }
     }
 }
 
@@ -432,15 +635,24 @@ struct EdgeOp {
     const float* z; const float* wdeg; const uint4* sig;
     float A[ZD]; float beta, gamma, delta, eta, pscale;
     int32_t* prio; float* logit;
-    __device__ void operator()(int64_t v, int64_t e) const {
+    __device__ void operator()(int64_t v, int64_t e) const { store(e, logit_of(v, e)); }
+    __device__ float logit_of(int64_t v, int64_t e) const {
         const int64_t u = __ldcs(&g.ci[e]);
         float zv[ZD];
         const float4 q = reinterpret_cast<const float4*>(z)[v];
         zv[0] = q.x; zv[1] = q.y; zv[2] = q.z; zv[3] = q.w;
-        const float t = edge_logit(A, beta, gamma, delta, eta, cn_feat(sig, v, u), zv, z, u,
-                                   g.ew ? (float)__ldcs(&g.ew[e]) : 1.f, wdeg[v], wdeg[u]);
+        return edge_logit(A, beta, gamma, delta, eta, cn_feat(sig, v, u), zv, z, u,
+                          g.ew ? (float)__ldcs(&g.ew[e]) : 1.f, wdeg[v], wdeg[u]);
+    }
+    __device__ void store(int64_t e, float t) const {
         if (prio) prio[e] = logit_prio(t, pscale);
         if (logit) logit[e] = t;
+    }
+    // two entries, their loads in flight together
+    __device__ void operator()(int64_t v, int64_t e, int64_t v2, int64_t e2) const {
+        const float t = logit_of(v, e), t2 = logit_of(v2, e2);
+        store(e, t);
+        store(e2, t2);
     }
 };
 
@@ -678,29 +890,31 @@ static void gnn_forward(Ctx& c, const gp_gnn* G, const Level& L, int level, bool
     A.h1 = keep ? c.tmp_alloc<float>(H * n) : nullptr;
     A.h2 = keep ? c.tmp_alloc<float>(H * n) : nullptr;
     float* ipart = c.tmp_alloc<float>(MSG * std::max<int64_t>(L.nitems, 1));
-    const int64_t U = (L.nbucket[0] + 3) / 4 + L.nbucket[1] + L.nbucket[2];
+    const bool split = L.nbucket[0] >= kGnnSplit;
+    const int64_t U = (split ? 0 : (L.nbucket[0] + 3) / 4) + L.nbucket[1] + L.nbucket[2];
     const int rg = (int)(L.nitems + grid_for(U * 32, 256, c.sm_count * 16));
-    const int vg = grid_for(n, 256, c.sm_count * 8), tg = grid_for(n, 128, c.sm_count * 8);
+    const int sg = grid_for(L.nbucket[0], 256, c.sm_count * 16);
+    const int vg = grid_for(n, 256, c.sm_count * 8);
     const int hg = grid_for(std::max<int64_t>(L.nheavy, 1), 128);
-    if (g.ew) {
-        k_gnn_rowsum<1><<<rg, 256, 0, c.s>>>(R, ValWeight{g.ew}, FinStore1{A.wdeg}, ipart);
-        GP_LAUNCHED(c);
-        if (L.nheavy) { k_gnn_rowsum_heavy<1><<<hg, 128, 0, c.s>>>(R, FinStore1{A.wdeg}, ipart); GP_LAUNCHED(c); }
-    }
+    auto rowsum = [&](auto val, auto fin, auto f) {
+        constexpr int F = decltype(f)::value;
+        if (split) { k_gnn_rowsum_short<F><<<sg, 256, 0, c.s>>>(R, val, fin); GP_LAUNCHED(c); }
+        if (U + L.nitems > 0) { k_gnn_rowsum<F><<<rg, 256, 0, c.s>>>(R, val, fin, ipart); GP_LAUNCHED(c); }
+        if (L.nheavy) { k_gnn_rowsum_heavy<F><<<hg, 128, 0, c.s>>>(R, fin, ipart); GP_LAUNCHED(c); }
+    };
+    if (g.ew) rowsum(ValWeight{g.ew}, FinStore1{A.wdeg}, std::integral_constant<int, 1>());
     k_gnn_vfeat<<<vg, 256, 0, c.s>>>(n, g.rp, g.vw, (float)level, g.ew ? 0 : 1, (float4*)A.x, A.wdeg);
     GP_LAUNCHED(c);
     A.sig = (uint4*)c.tmp->alloc(sizeof(uint4) * (size_t)std::max<int64_t>(n, 1));
-    k_gnn_sig<<<grid_for(n * 32, 256, c.sm_count * 16), 256, 0, c.s>>>(g, A.sig);
+    k_gnn_sig<<<grid_for(n, 256, c.sm_count * 32), 256, 0, c.s>>>(g, A.sig);
     GP_LAUNCHED(c);
-    k_gnn_rowsum<F0><<<rg, 256, 0, c.s>>>(R, ValRow4{g.ci, (const float4*)A.x}, FinMean<F0>{g.rp, A.a}, ipart);
+    rowsum(ValRow4{g.ci, (const float4*)A.x}, FinMean<F0>{g.rp, A.a}, std::integral_constant<int, F0>());
+    const bool wide = n >= kGnnWide;
+    const int tg = grid_for(n, wide ? 256 : 128, c.sm_count * 8);
+    (wide ? k_gnn_l1<2> : k_gnn_l1<1>)<<<tg, 128, 0, c.s>>>(n, G->w16, A.x, A.a, A.m, A.h1);
     GP_LAUNCHED(c);
-    if (L.nheavy) { k_gnn_rowsum_heavy<F0><<<hg, 128, 0, c.s>>>(R, FinMean<F0>{g.rp, A.a}, ipart); GP_LAUNCHED(c); }
-    k_gnn_l1<<<tg, 128, 0, c.s>>>(n, G->w16, A.x, A.a, A.m, A.h1);
-    GP_LAUNCHED(c);
-    k_gnn_rowsum<MSG><<<rg, 256, 0, c.s>>>(R, ValRow8{g.ci, (const float4*)A.m}, FinMean<MSG>{g.rp, A.c}, ipart);
-    GP_LAUNCHED(c);
-    if (L.nheavy) { k_gnn_rowsum_heavy<MSG><<<hg, 128, 0, c.s>>>(R, FinMean<MSG>{g.rp, A.c}, ipart); GP_LAUNCHED(c); }
-    k_gnn_l2<<<tg, 128, 0, c.s>>>(n, G->w16, A.x, A.a, A.c, A.z, A.h2);
+    rowsum(ValRow8{g.ci, (const float4*)A.m}, FinMean<MSG>{g.rp, A.c}, std::integral_constant<int, MSG>());
+    k_gnn_l2<<<grid_for(n, L2_T, c.sm_count * 8), L2_T, 0, c.s>>>(n, G->w16, A.x, A.a, A.c, A.z, A.h2);
     GP_LAUNCHED(c);
     // row sums: rowptr, column ids (+ weights), gathered neighbour rows; per-vertex arrays
     c.bytes += 3 * (8 * (n + 1) + 4 * g.m) + (g.ew ? 8 * g.m : 0) + 4 * g.m * (F0 + MSG) +
@@ -719,9 +933,9 @@ static EdgeOp edge_op(const gp_gnn* G, const DGraph& g, const GnnActs& A, int32_
 }
 
 static void gnn_edges(Ctx& c, const gp_gnn* G, const Level& L, const GnnActs& A, int32_t* prio, float* logit) {
-    const int64_t U = (L.nbucket[0] + 3) / 4 + L.nbucket[1] + L.nbucket[2];
-    const int rg = (int)(L.nitems + grid_for(U * 32, 256, c.sm_count * 16));
-    k_gnn_entries<<<rg, 256, 0, c.s>>>(gnn_rows(L), edge_op(G, L.g, A, prio, logit));
+    const int64_t slice = csr_slice(L.g.m, 4 * c.sm_count);   // short slices: latency-bound gathers want warps
+    k_gnn_entries<<<grid_for((L.g.m + slice - 1) / slice * 32, 256, c.sm_count * 32), 256, 0, c.s>>>(
+        L.g, slice, edge_op(G, L.g, A, prio, logit));
     GP_LAUNCHED(c);
     c.bytes += 8 * (L.g.n + 1) + 4 * L.g.m * (2 + ZD + 1) + (L.g.ew ? 4 * L.g.m : 0) + 4 * L.g.n * (ZD + 1);
 }
