@@ -99,7 +99,7 @@ static void buckets_begin(Ctx& c, Level& L, int64_t heavy_cap, int64_t* ctl) {
     GP_LAUNCHED(c);
     c.bytes += 8 * (L.g.n + 1) + 4 * L.g.n;
 }
-static void buckets_end(Ctx& c, Level& L, const int64_t* h) {
+static void buckets_end(Ctx& c, Level& L, const int64_t* h, bool units) {
     for (int b = 0; b < 3; ++b) L.nbucket[b] = h[C_BUCKETS + b];
     L.nheavy = h[C_BUCKETS + 3];
     L.max_deg = h[C_MAXDEG];
@@ -131,7 +131,7 @@ static void buckets_end(Ctx& c, Level& L, const int64_t* h) {
         rows_items[h] = cnt;
     }
     L.nitems = (int64_t)irow.size();
-    {
+    if (units) {
         L.nunits = L.nbucket[2] + L.nbucket[1] + (L.nbucket[0] + 3) / 4;
         int64_t* cost = c.tmp_alloc<int64_t>(L.nunits + 1);
         L.unit_cost = c.keep_alloc<int64_t>(L.nunits + 1);
@@ -163,7 +163,7 @@ __global__ void k_max_vw(int64_t n, const int32_t* __restrict__ vw, int64_t* __r
     warp_max_to(mx, out);
 }
 
-void build_heavy(Ctx& c, Level& L) {
+void build_heavy(Ctx& c, Level& L, bool units) {
     auto mk = c.tmp->save();
     int64_t* ctl = c.tmp_alloc<int64_t>(C_NCTL);
     memset_async(c, ctl, 0, C_NCTL * sizeof(int64_t));
@@ -178,7 +178,7 @@ void build_heavy(Ctx& c, Level& L) {
     std::copy(c.h_pinned, c.h_pinned + C_NCTL, h);
     c.tmp->restore(mk);
     L.max_vw = L.g.vw ? h[C_MAXVW] : 1;
-    buckets_end(c, L, h);
+    buckets_end(c, L, h, units);
 }
 
 // ---------------------------------------------------------------- argmax helpers
@@ -1783,7 +1783,7 @@ void contract_level(Ctx& c, Level& fine, Level& coarse, const int32_t* match, in
     coarse.g.ew = cew;
     coarse.max_vw = h[C_MAXVW];
     c.tmp->restore(mk);
-    buckets_end(c, coarse, h);
+    buckets_end(c, coarse, h, true);
 }
 
 // shared-memory caps of the contraction kernels above 48 KB; set once per

@@ -59,7 +59,7 @@ constexpr int MO_W1 = 0, MO_B1 = MO_W1 + MH * MF, MO_W2 = MO_B1 + MH, MO_B2 = MO
 struct gp_gnn {
     float* master = nullptr;          // FP32 master weights (device)
     __nv_bfloat16* w16 = nullptr;     // BF16 weights used by every kernel (device)
-    float* grad = nullptr;            // gradients (device)
+    float* grad = nullptr;            // gradients (device), then the loss (double)
     float* adam_m = nullptr;
     float* adam_v = nullptr;
     int64_t step = 0;
@@ -583,7 +583,7 @@ __global__ void k_gnn_sig(DGraph g, uint4* __restrict__ sig) {
             const int src = __ffs(todo) - 1;
             const int64_t b2 = __shfl_sync(0xffffffffu, beg, src), e2 = __shfl_sync(0xffffffffu, end, src);
             uint32_t w[4] = {0, 0, 0, 0};
-#pragma unroll 4
+#pragma unroll 16
             for (int64_t e = b2 + lane; e < e2; e += 32) sig_add(__ldcs(&g.ci[e]), w);
 #pragma unroll
             for (int q = 0; q < 4; ++q) w[q] = __reduce_or_sync(0xffffffffu, w[q]);
@@ -657,11 +657,62 @@ struct EdgeOp {
 };
 
 // ------------------------------------------------------------------ training
+// Rows of the backward passes over entries: body(e, width lanes' accumulators)
+// for every entry, fin(v, sums) per row.  Rows of 33 entries and more take a
+// block each (a hub row of an R-MAT training graph by one warp was the whole
+// launch's tail: 221 -> 52 us for the loss pass, 157 -> 34 for the message pass on
+// a 16,384-vertex R-MAT graph),
+// bucket-1 rows a warp, bucket-0 rows 8 lanes.  blockDim 256.
+template <int F, class Pre, class Body, class Fin>
+__device__ __forceinline__ void rows_bwd(const GnnRows& R, Pre pre, Body body, Fin fin) {
+    __shared__ float s_part[8][F];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t nlong = R.nb[2] + R.nheavy;
+    float acc[F];
+    for (int64_t i = blockIdx.x; i < nlong; i += gridDim.x) {
+        const int64_t v = i < R.nheavy ? R.heavy[i] : R.b[2][i - R.nheavy];   // the longest first
+#pragma unroll
+        for (int j = 0; j < F; ++j) acc[j] = 0.f;
+        pre(v);
+        const int64_t end = R.g.rp[v + 1];
+        for (int64_t e = R.g.rp[v] + threadIdx.x; e < end; e += blockDim.x) body(v, e, acc);
+        tile_reduce<F>(acc, 32);
+        if (lane == 0)
+#pragma unroll
+            for (int j = 0; j < F; ++j) s_part[w][j] = acc[j];
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int t = 1; t < 8; ++t)
+#pragma unroll
+                for (int j = 0; j < F; ++j) acc[j] += s_part[t][j];
+            fin(v, acc);
+        }
+        __syncthreads();
+    }
+    const int64_t U0 = (R.nb[0] + 3) / 4, nw = (int64_t)gridDim.x * 8;
+    for (int64_t u = (int64_t)blockIdx.x * 8 + w; u < U0 + R.nb[1]; u += nw) {
+#pragma unroll
+        for (int j = 0; j < F; ++j) acc[j] = 0.f;
+        const bool tile = u < U0;
+        const int width = tile ? 8 : 32, tl = lane & (width - 1);
+        const int64_t i = tile ? u * 4 + (lane >> 3) : u - U0;
+        const int64_t v = tile ? (i < R.nb[0] ? R.b[0][i] : -1) : R.b[1][i];
+        if (v >= 0) {
+            pre(v);
+            const int64_t e = R.g.rp[v] + tl, end = R.g.rp[v + 1];
+            if (e < end) body(v, e, acc);
+            if (tile && e + 8 < end) body(v, e + 8, acc);
+        }
+        tile_reduce<F>(acc, width);
+        if (v >= 0 && tl == 0) fin(v, acc);
+    }
+}
+
 // loss and dt per entry; dz_v = 2 sum_u dt_vu A (.) z_u; gradients of A, beta, gamma, delta
-__global__ void k_gnn_edge_bwd(DGraph g, const __nv_bfloat16* __restrict__ w, const float* __restrict__ z,
+__global__ void __launch_bounds__(256) k_gnn_edge_bwd(GnnRows R, const __nv_bfloat16* __restrict__ w, const float* __restrict__ z,
                                const float* __restrict__ wdeg, const uint4* __restrict__ sig,
                                const uint8_t* __restrict__ label, float inv_e, float* __restrict__ dz,
-                               float* __restrict__ grad, float* __restrict__ loss) {
+                               float* __restrict__ grad, double* __restrict__ loss) {
     __shared__ float sA[ZD];
     __shared__ float sc[4];
     __shared__ float sg[ZD + 5];
@@ -669,44 +720,41 @@ __global__ void k_gnn_edge_bwd(DGraph g, const __nv_bfloat16* __restrict__ w, co
     if (threadIdx.x < 4) sc[threadIdx.x] = wload(w, O_BETA + threadIdx.x);
     if (threadIdx.x < ZD + 5) sg[threadIdx.x] = 0.f;
     __syncthreads();
+    const DGraph& g = R.g;
     const int lane = threadIdx.x & 31;
-    const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
     float gA[ZD] = {0.f, 0.f, 0.f, 0.f}, gb = 0.f, gg = 0.f, gd = 0.f, ge = 0.f, ls = 0.f;
-    for (int64_t v = wid; v < g.n; v += nw) {
-        float zv[ZD], dzv[ZD];
+    float zv[ZD], wdv = 0.f;
+    auto pre = [&](int64_t v) {
+        const float4 q = reinterpret_cast<const float4*>(z)[v];
+        zv[0] = q.x; zv[1] = q.y; zv[2] = q.z; zv[3] = q.w;
+        wdv = wdeg[v];
+    };
+    auto body = [&](int64_t v, int64_t e, float (&dzv)[ZD]) {
+        const int64_t u = g.ci[e];
+        const float we = g.ew ? (float)g.ew[e] : 1.f;
+        const float fcn = cn_feat(sig, v, u), wdu = wdeg[u];
+        const float t = edge_logit(sA, sc[0], sc[1], sc[2], sc[3], fcn, zv, z, u, we, wdv, wdu);
+        const float y = label[e] ? 1.f : 0.f;
+        const float s = 1.f / (1.f + expf(-t));
+        // BCE with logits, stable form
+        ls += (fmaxf(t, 0.f) - t * y + log1pf(expf(-fabsf(t)))) * inv_e;
+        const float dt = (s - y) * inv_e;
+        const float4 q = reinterpret_cast<const float4*>(z)[u];
+        const float zu[ZD] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-        for (int j = 0; j < ZD; ++j) { zv[j] = z[ZD * v + j]; dzv[j] = 0.f; }
-        const float wdv = wdeg[v];
-        for (int64_t e = g.rp[v] + lane; e < g.rp[v + 1]; e += 32) {
-            const int64_t u = g.ci[e];
-            const float we = g.ew ? (float)g.ew[e] : 1.f;
-            const float fcn = cn_feat(sig, v, u);
-            const float t = edge_logit(sA, sc[0], sc[1], sc[2], sc[3], fcn, zv, z, u, we, wdv, wdeg[u]);
-            const float y = label[e] ? 1.f : 0.f;
-            const float s = 1.f / (1.f + expf(-t));
-            // BCE with logits, stable form
-            ls += (fmaxf(t, 0.f) - t * y + log1pf(expf(-fabsf(t)))) * inv_e;
-            const float dt = (s - y) * inv_e;
-#pragma unroll
-            for (int j = 0; j < ZD; ++j) {
-                const float zu = z[ZD * u + j];
-                gA[j] += dt * zv[j] * zu;
-                dzv[j] += 2.f * dt * sA[j] * zu;
-            }
-            gb += dt * (log2f(1.f + we) * 0.125f);
-            gg += dt * (we / wdv + we / wdeg[u]);
-            gd += dt;
-            ge += dt * fcn;
+        for (int j = 0; j < ZD; ++j) {
+            gA[j] += dt * zv[j] * zu[j];
+            dzv[j] += 2.f * dt * sA[j] * zu[j];
         }
-        warp_reduce_vec<ZD>(dzv);
-        if (lane < ZD) {
-            float r = 0.f;
-#pragma unroll
-            for (int j = 0; j < ZD; ++j) if (j == lane) r = dzv[j];
-            dz[ZD * v + lane] = r;
-        }
-    }
+        gb += dt * (log2f(1.f + we) * 0.125f);
+        gg += dt * (we / wdv + we / wdu);
+        gd += dt;
+        ge += dt * fcn;
+    };
+    auto fin = [&](int64_t v, float (&dzv)[ZD]) {
+        reinterpret_cast<float4*>(dz)[v] = make_float4(dzv[0], dzv[1], dzv[2], dzv[3]);
+    };
+    rows_bwd<ZD>(R, pre, body, fin);
     float part[ZD + 5] = {gA[0], gA[1], gA[2], gA[3], gb, gg, gd, ls, ge};
     warp_reduce_vec<ZD + 5>(part);
     if (lane == 0)
@@ -716,7 +764,7 @@ __global__ void k_gnn_edge_bwd(DGraph g, const __nv_bfloat16* __restrict__ w, co
     if (threadIdx.x == ZD) atomicAdd(&grad[O_BETA], sg[ZD]);
     if (threadIdx.x == ZD + 1) atomicAdd(&grad[O_GAMMA], sg[ZD + 1]);
     if (threadIdx.x == ZD + 2) atomicAdd(&grad[O_DELTA], sg[ZD + 2]);
-    if (threadIdx.x == ZD + 3) atomicAdd(loss, sg[ZD + 3]);
+    if (threadIdx.x == ZD + 3) atomicAdd(loss, (double)sg[ZD + 3]);   // the blocks' sums in 64 bits
     if (threadIdx.x == ZD + 4) atomicAdd(&grad[O_ETA], sg[ZD + 4]);
 }
 
@@ -755,28 +803,20 @@ __global__ void __launch_bounds__(128) k_gnn_l2_bwd(int64_t n, const __nv_bfloat
 }
 
 // dm_u = sum_{v in N(u)} dc_v / deg_v (symmetric graph: the row owner gathers)
-__global__ void k_gnn_msg_bwd(DGraph g, const float* __restrict__ dc, float* __restrict__ dm) {
-    const int lane = threadIdx.x & 31;
-    const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t u = wid; u < g.n; u += nw) {
-        float acc[MSG];
-#pragma unroll
-        for (int j = 0; j < MSG; ++j) acc[j] = 0.f;
-        for (int64_t e = g.rp[u] + lane; e < g.rp[u + 1]; e += 32) {
-            const int64_t v = g.ci[e];
-            const float inv = 1.f / (float)(g.rp[v + 1] - g.rp[v]);
-#pragma unroll
-            for (int j = 0; j < MSG; ++j) acc[j] += dc[MSG * v + j] * inv;
-        }
-        warp_reduce_vec<MSG>(acc);
-        if (lane < MSG) {
-            float r = 0.f;
-#pragma unroll
-            for (int j = 0; j < MSG; ++j) if (j == lane) r = acc[j];
-            dm[MSG * u + lane] = r;
-        }
-    }
+__global__ void __launch_bounds__(256) k_gnn_msg_bwd(GnnRows R, const float* __restrict__ dc, float* __restrict__ dm) {
+    const DGraph& g = R.g;
+    auto body = [&](int64_t, int64_t e, float (&acc)[MSG]) {
+        const int64_t v = g.ci[e];
+        const float inv = 1.f / (float)(g.rp[v + 1] - g.rp[v]);
+        const float4 p = reinterpret_cast<const float4*>(dc)[2 * v], q = reinterpret_cast<const float4*>(dc)[2 * v + 1];
+        acc[0] += p.x * inv; acc[1] += p.y * inv; acc[2] += p.z * inv; acc[3] += p.w * inv;
+        acc[4] += q.x * inv; acc[5] += q.y * inv; acc[6] += q.z * inv; acc[7] += q.w * inv;
+    };
+    auto fin = [&](int64_t u, float (&acc)[MSG]) {
+        reinterpret_cast<float4*>(dm)[2 * u] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        reinterpret_cast<float4*>(dm)[2 * u + 1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+    };
+    rows_bwd<MSG>(R, [](int64_t) {}, body, fin);
 }
 
 // dpre1 = (dh1 + P^T dm) * [h1 > 0]; thread per vertex
@@ -799,59 +839,85 @@ __global__ void __launch_bounds__(128) k_gnn_l1_bwd(int64_t n, const __nv_bfloat
     }
 }
 
-// grad[o + i*C + j] += sum_v A[v*ra + i] * B[v*rb + j]  (i < R, j < C; B == nullptr: ones)
-// CTA per chunk of 64 vertices, rows staged in shared memory; each thread
-// keeps its (up to OP_PER_THREAD) output sums in registers across all of its
-// CTA's chunks and adds them to grad once at the end.
-constexpr int OP_CHUNK = 64, OP_THREADS = 256, OP_PER_THREAD = 18;   // R*C <= 256*18 (W2: 64*72)
-__global__ void __launch_bounds__(OP_THREADS) k_gnn_outer(int64_t n, const float* __restrict__ A, int ra, int R,
-                                                          const float* __restrict__ B, int rb, int C,
-                                                          float* __restrict__ grad, int o) {
-    extern __shared__ float sm[];
+// Weight gradients: grad[w + i*C + j] += sum_v A[v][i] B[v][j] (i < R, j < C) and,
+// with a bias, grad[b + i] += sum_v A[v][i]; B is the concatenation of two arrays
+// (b2 may be nullptr).  A block takes chunks of 64 vertices, staged in shared
+// memory; each thread keeps a tile of TR rows (consecutive) by TC columns
+// (strided) of the sums in registers over all of its block's chunks, the sums of
+// a chunk apart, and adds them to grad once at the end.  What bounds it is the
+// shared loads: one output per load pair took 889 us, tiles 311 (all four gradients
+// of 8 training graphs, the concatenated copies of B included before).
+struct OuterJob {
+    const float* A;
+    const float *b1, *b2;
+    int R, c1, c2;
+    int w, b;        // offsets in grad (b < 0: no bias)
+};
+constexpr int OP_CHUNK = 64, OP_THREADS = 256;
+template <int TR, int TC>
+__device__ __forceinline__ void outer_job(int64_t n, const OuterJob& J, float* __restrict__ grad, float* sm) {
+    const int R = J.R, C = J.c1 + J.c2, CB = C + 1;   // the bias is a column of ones
     float* sa = sm;                       // OP_CHUNK * R
-    float* sb = sm + OP_CHUNK * R;        // OP_CHUNK * C
-    float acc[OP_PER_THREAD];
+    float* sb = sm + OP_CHUNK * R;        // OP_CHUNK * CB
+    const int tr = (R + TR - 1) / TR, tc = OP_THREADS / tr;   // threads along rows and columns
+    const int i0 = (int)(threadIdx.x % tr) * TR, j0 = threadIdx.x / tr;
+    float acc[TR][TC];
 #pragma unroll
-    for (int q = 0; q < OP_PER_THREAD; ++q) acc[q] = 0.f;
+    for (int p = 0; p < TR; ++p)
+#pragma unroll
+        for (int q = 0; q < TC; ++q) acc[p][q] = 0.f;
     for (int64_t base = (int64_t)blockIdx.x * OP_CHUNK; base < n; base += (int64_t)gridDim.x * OP_CHUNK) {
         const int cnt = (int)((n - base) < OP_CHUNK ? (n - base) : OP_CHUNK);
-        for (int i = threadIdx.x; i < OP_CHUNK * R; i += blockDim.x) {
-            const int v = i / R, r = i % R;
-            sa[i] = v < cnt ? A[(base + v) * ra + r] : 0.f;
-        }
-        for (int i = threadIdx.x; i < OP_CHUNK * C; i += blockDim.x) {
-            const int v = i / C, cc = i % C;
-            sb[i] = v < cnt ? (B ? B[(base + v) * rb + cc] : 1.f) : 0.f;
-        }
+        for (int i = threadIdx.x; i < cnt * R; i += OP_THREADS) sa[i] = J.A[base * R + i];
+        for (int i = threadIdx.x; i < cnt * J.c1; i += OP_THREADS)
+            sb[(i / J.c1) * CB + i % J.c1] = J.b1[base * J.c1 + i];
+        if (J.b2)
+            for (int i = threadIdx.x; i < cnt * J.c2; i += OP_THREADS)
+                sb[(i / J.c2) * CB + J.c1 + i % J.c2] = J.b2[base * J.c2 + i];
+        for (int i = threadIdx.x; i < cnt; i += OP_THREADS) sb[i * CB + C] = 1.f;
         __syncthreads();
+        float part[TR][TC];
 #pragma unroll
-        for (int q = 0; q < OP_PER_THREAD; ++q) {
-            const int idx = threadIdx.x + q * OP_THREADS;
-            if (idx < R * C) {
-                const int i = idx / C, j = idx % C;
-                float s = 0.f;
-                for (int v = 0; v < cnt; ++v) s += sa[v * R + i] * sb[v * C + j];
-                acc[q] += s;
-            }
+        for (int p = 0; p < TR; ++p)
+#pragma unroll
+            for (int q = 0; q < TC; ++q) part[p][q] = 0.f;
+        for (int v = 0; v < cnt; ++v) {
+            float a[TR], b[TC];
+#pragma unroll
+            for (int p = 0; p < TR; ++p) a[p] = i0 + p < R ? sa[v * R + i0 + p] : 0.f;
+#pragma unroll
+            for (int q = 0; q < TC; ++q) b[q] = j0 + q * tc < CB ? sb[v * CB + j0 + q * tc] : 0.f;
+#pragma unroll
+            for (int p = 0; p < TR; ++p)
+#pragma unroll
+                for (int q = 0; q < TC; ++q) part[p][q] += a[p] * b[q];
         }
+#pragma unroll
+        for (int p = 0; p < TR; ++p)
+#pragma unroll
+            for (int q = 0; q < TC; ++q) acc[p][q] += part[p][q];
         __syncthreads();
     }
 #pragma unroll
-    for (int q = 0; q < OP_PER_THREAD; ++q) {
-        const int idx = threadIdx.x + q * OP_THREADS;
-        if (idx < R * C && acc[q] != 0.f) atomicAdd(&grad[o + idx], acc[q]);
-    }
+    for (int p = 0; p < TR; ++p)
+#pragma unroll
+        for (int q = 0; q < TC; ++q) {
+            const int i = i0 + p, j = j0 + q * tc;
+            if (i >= R || j >= CB || acc[p][q] == 0.f) continue;
+            if (j < C) atomicAdd(&grad[J.w + i * C + j], acc[p][q]);
+            else if (J.b >= 0) atomicAdd(&grad[J.b + i], acc[p][q]);
+        }
 }
-
-// [x; a] and [h1; c] rows for the weight gradients
-__global__ void k_gnn_concat(int64_t n, const float* __restrict__ p, int fp, const float* __restrict__ q, int fq,
-                             float* __restrict__ out) {
-    const int f = fp + fq;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n * f; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t v = i / f;
-        const int j = (int)(i % f);
-        out[i] = j < fp ? p[v * fp + j] : q[v * fq + (j - fp)];
-    }
+// blockIdx.y: 0 = W2 and b2 (64 x 73, tiles of 4 x 5), 1 = W1 and b1 (64 x 9, 4 x 1),
+// 2 = P (8 x 64, 2 x 1), 3 = Z (4 x 64, 2 x 1)
+struct OuterJobs { OuterJob job[4]; };
+constexpr size_t outer_smem() { return sizeof(float) * OP_CHUNK * (H + H + MSG + 1); }
+__global__ void __launch_bounds__(OP_THREADS) k_gnn_outer(int64_t n, OuterJobs jobs, float* __restrict__ grad) {
+    extern __shared__ float osm[];
+    const OuterJob J = jobs.job[blockIdx.y];
+    if (blockIdx.y == 0) outer_job<4, 5>(n, J, grad, osm);
+    else if (blockIdx.y == 1) outer_job<4, 1>(n, J, grad, osm);
+    else outer_job<2, 1>(n, J, grad, osm);
 }
 
 __global__ void k_gnn_adam(int np, float* __restrict__ master, __nv_bfloat16* __restrict__ w16,
@@ -1092,8 +1158,10 @@ static void refresh_host_edge(gp_gnn* G, cudaStream_t s) {
     for (int j = 0; j < NEDGE; ++j) G->hedge[j] = __bfloat162float(h[j]);
 }
 
-// loss and gradients of one graph (gradients accumulated into G->grad)
-static float gnn_grad(Ctx& c, gp_gnn* G, const Level& L, int level, const uint8_t* label) {
+// gradients of one graph, accumulated into G->grad, its loss into the double after them
+static double* gnn_loss(gp_gnn* G) { return (double*)(G->grad + NPARAM + (NPARAM & 1)); }
+constexpr size_t kGradBytes = sizeof(float) * (NPARAM + (NPARAM & 1)) + sizeof(double);
+static void gnn_grad(Ctx& c, gp_gnn* G, const Level& L, int level, const uint8_t* label) {
     const DGraph& g = L.g;
     const int64_t n = g.n;
     auto mk = c.tmp->save();
@@ -1105,42 +1173,26 @@ static float gnn_grad(Ctx& c, gp_gnn* G, const Level& L, int level, const uint8_
     float* dc = c.tmp_alloc<float>(MSG * n);
     float* dm = c.tmp_alloc<float>(MSG * n);
     float* dpre1 = c.tmp_alloc<float>(H * n);
-    float* xa = c.tmp_alloc<float>(2 * F0 * n);
-    float* hc = c.tmp_alloc<float>((H + MSG) * n);
-    float* loss = c.tmp_alloc<float>(1);
-    memset_async(c, loss, 0, sizeof(float));
-    const int wg = grid_for(n * 32, 256, c.sm_count * 8), tg = grid_for(n, 128, c.sm_count * 8);
+    const GnnRows R = gnn_rows(L);
+    const int64_t units = std::max<int64_t>(R.nb[2] + R.nheavy, (R.nb[0] + 31) / 32 + (R.nb[1] + 7) / 8);
+    const int wg = grid_for(units, 1, c.sm_count * 8), tg = grid_for(n, 128, c.sm_count * 8);
     const float inv_e = g.m > 0 ? 1.f / (float)g.m : 0.f;
-    k_gnn_edge_bwd<<<wg, 256, 0, c.s>>>(g, G->w16, A.z, A.wdeg, A.sig, label, inv_e, dz, G->grad, loss);
+    k_gnn_edge_bwd<<<wg, 256, 0, c.s>>>(R, G->w16, A.z, A.wdeg, A.sig, label, inv_e, dz, G->grad, gnn_loss(G));
     GP_LAUNCHED(c);
     k_gnn_l2_bwd<<<tg, 128, 0, c.s>>>(n, G->w16, dz, A.h2, dpre2, dh1, dc);
     GP_LAUNCHED(c);
-    k_gnn_msg_bwd<<<wg, 256, 0, c.s>>>(g, dc, dm);
+    k_gnn_msg_bwd<<<wg, 256, 0, c.s>>>(R, dc, dm);
     GP_LAUNCHED(c);
     k_gnn_l1_bwd<<<tg, 128, 0, c.s>>>(n, G->w16, dh1, dm, A.h1, dpre1);
     GP_LAUNCHED(c);
-    const int cg = grid_for(n, OP_CHUNK, c.sm_count * 4);
-    k_gnn_concat<<<grid_for(n * 2 * F0, 256), 256, 0, c.s>>>(n, A.x, F0, A.a, F0, xa);
+    OuterJobs J;
+    J.job[0] = {dpre2, A.h1, A.c, H, H, MSG, O_W2, O_B2};    // dW2 = dpre2 [h1; c]^T, db2
+    J.job[1] = {dpre1, A.x, A.a, H, F0, F0, O_W1, O_B1};     // dW1 = dpre1 [x; a]^T, db1
+    J.job[2] = {dm, A.h1, nullptr, MSG, H, 0, O_P, -1};      // dP = dm h1^T
+    J.job[3] = {dz, A.h2, nullptr, ZD, H, 0, O_Z, -1};       // dZ = dz h2^T
+    k_gnn_outer<<<dim3((unsigned)grid_for(n, OP_CHUNK, c.sm_count * 2), 4), OP_THREADS, outer_smem(), c.s>>>(n, J, G->grad);
     GP_LAUNCHED(c);
-    k_gnn_concat<<<grid_for(n * (H + MSG), 256), 256, 0, c.s>>>(n, A.h1, H, A.c, MSG, hc);
-    GP_LAUNCHED(c);
-    auto outer = [&](const float* a, int ra, int R, const float* b, int rb, int C, int o) {
-        const size_t smem = sizeof(float) * OP_CHUNK * (R + C);
-        if (R * C > OP_THREADS * OP_PER_THREAD) throw GpError(GP_EINTERNAL, "outer product too large");
-        k_gnn_outer<<<cg, OP_THREADS, smem, c.s>>>(n, a, ra, R, b, rb, C, G->grad, o);
-        GP_LAUNCHED(c);
-    };
-    outer(dz, ZD, ZD, A.h2, H, H, O_Z);            // dZ = dz h2^T
-    outer(dpre2, H, H, hc, H + MSG, H + MSG, O_W2); // dW2 = dpre2 [h1; c]^T
-    outer(dpre2, H, H, nullptr, 0, 1, O_B2);        // db2
-    outer(dm, MSG, MSG, A.h1, H, H, O_P);           // dP = dm h1^T
-    outer(dpre1, H, H, xa, 2 * F0, 2 * F0, O_W1);   // dW1 = dpre1 [x; a]^T
-    outer(dpre1, H, H, nullptr, 0, 1, O_B1);        // db1
-    float h = 0.f;
-    GP_CUDA(cudaMemcpyAsync(&h, loss, sizeof(float), cudaMemcpyDeviceToHost, c.s));
-    c.sync();
     c.tmp->restore(mk);
-    return h;
 }
 
 // per-call context on the current device (own stream and arenas)
@@ -1164,7 +1216,7 @@ struct GnnCall {
 static Level level_of(Ctx& c, const DGraph& g) {
     Level L;
     L.g = g;
-    build_heavy(c, L);
+    build_heavy(c, L, false);
     return L;
 }
 
@@ -1203,12 +1255,12 @@ int gp_gnn_create(gp_gnn** out) {
         gp_gnn* G = new gp_gnn();
         GP_CUDA(cudaMalloc(&G->master, sizeof(float) * NPARAM));
         GP_CUDA(cudaMalloc(&G->w16, sizeof(__nv_bfloat16) * NPARAM));
-        GP_CUDA(cudaMalloc(&G->grad, sizeof(float) * NPARAM));
+        GP_CUDA(cudaMalloc(&G->grad, kGradBytes));
         GP_CUDA(cudaMalloc(&G->adam_m, sizeof(float) * NPARAM));
         GP_CUDA(cudaMalloc(&G->adam_v, sizeof(float) * NPARAM));
         GP_CUDA(cudaMemset(G->master, 0, sizeof(float) * NPARAM));
         GP_CUDA(cudaMemset(G->w16, 0, sizeof(__nv_bfloat16) * NPARAM));
-        GP_CUDA(cudaMemset(G->grad, 0, sizeof(float) * NPARAM));
+        GP_CUDA(cudaMemset(G->grad, 0, kGradBytes));
         GP_CUDA(cudaMemset(G->adam_m, 0, sizeof(float) * NPARAM));
         GP_CUDA(cudaMemset(G->adam_v, 0, sizeof(float) * NPARAM));
         *out = G;
@@ -1294,10 +1346,15 @@ int gp_gnn_grad_device(gp_gnn* G, int64_t n, const int64_t* d_rowptr, const int3
         GP_CUDA(cudaMemcpyAsync(call.pinned, d_rowptr + n, sizeof(int64_t), cudaMemcpyDeviceToHost, call.c.s));
         call.c.sync();
         const DGraph g = mkgraph(n, call.pinned[0], d_rowptr, d_colidx, d_vwgt, d_ewgt);
-        GP_CUDA(cudaMemsetAsync(G->grad, 0, sizeof(float) * NPARAM, call.c.s));
-        const float l = gnn_grad(call.c, G, level_of(call.c, g), level, d_label);
-        if (loss_out) *loss_out = l;
-        if (grad_out) GP_CUDA(cudaMemcpy(grad_out, G->grad, sizeof(float) * NPARAM, cudaMemcpyDeviceToHost));
+        GP_CUDA(cudaMemsetAsync(G->grad, 0, kGradBytes, call.c.s));
+        gnn_grad(call.c, G, level_of(call.c, g), level, d_label);
+        std::vector<char> h(kGradBytes);   // gradients and loss in one copy
+        GP_CUDA(cudaMemcpyAsync(h.data(), G->grad, kGradBytes, cudaMemcpyDeviceToHost, call.c.s));
+        call.c.sync();
+        double l;
+        memcpy(&l, h.data() + kGradBytes - sizeof(double), sizeof l);
+        if (loss_out) *loss_out = (float)l;
+        if (grad_out) memcpy(grad_out, h.data(), sizeof(float) * NPARAM);
     });
 }
 
@@ -1310,8 +1367,7 @@ int gp_gnn_train_step_device(gp_gnn* G, int32_t ngraphs, const int64_t* ns, cons
         if (!G || ngraphs <= 0 || !ns || !d_rowptrs || !d_colidxs || !d_labels)
             throw GpError(GP_EINVAL, "bad arguments");
         GnnCall call(G, (cudaStream_t)stream);
-        GP_CUDA(cudaMemsetAsync(G->grad, 0, sizeof(float) * NPARAM, call.c.s));
-        float tot = 0.f;
+        GP_CUDA(cudaMemsetAsync(G->grad, 0, kGradBytes, call.c.s));
         for (int32_t i = 0; i < ngraphs; ++i) {
             if (ns[i] <= 0) continue;
             GP_CUDA(cudaMemcpyAsync(call.pinned, d_rowptrs[i] + ns[i], sizeof(int64_t), cudaMemcpyDeviceToHost, call.c.s));
@@ -1319,7 +1375,7 @@ int gp_gnn_train_step_device(gp_gnn* G, int32_t ngraphs, const int64_t* ns, cons
             const DGraph g = mkgraph(ns[i], call.pinned[0], d_rowptrs[i], d_colidxs[i], d_vwgts ? d_vwgts[i] : nullptr,
                                      d_ewgts ? d_ewgts[i] : nullptr);
             auto km = call.c.keep->save();
-            tot += gnn_grad(call.c, G, level_of(call.c, g), levels ? levels[i] : 0, d_labels[i]);
+            gnn_grad(call.c, G, level_of(call.c, g), levels ? levels[i] : 0, d_labels[i]);
             call.c.keep->restore(km);
         }
         G->step += 1;
@@ -1328,8 +1384,10 @@ int gp_gnn_train_step_device(gp_gnn* G, int32_t ngraphs, const int64_t* ns, cons
         k_gnn_adam<<<grid_for(NPARAM, 256), 256, 0, call.c.s>>>(NPARAM, G->master, G->w16, G->grad, G->adam_m,
                                                                 G->adam_v, lr, b1, b2, 1e-8f, c1, c2);
         GP_LAUNCHED(call.c);
+        double tot = 0;   // read with the step's other results
+        GP_CUDA(cudaMemcpyAsync(&tot, gnn_loss(G), sizeof tot, cudaMemcpyDeviceToHost, call.c.s));
         refresh_host_edge(G, call.c.s);
-        if (loss_out) *loss_out = tot / (float)ngraphs;
+        if (loss_out) *loss_out = (float)(tot / (double)ngraphs);
     });
 }
 

@@ -210,7 +210,8 @@ void gnn_move_priorities(Ctx& c, const gp_gnn* G, const DGraph& g, int level, co
 
 // gp_coarsen.cu
 // the row buckets of a level (a coarse level of contract_level has them)
-void build_heavy(Ctx& c, Level& L);
+// (units = false: without the cost prefix of the connectivity pass's units)
+void build_heavy(Ctx& c, Level& L, bool units = true);
 // prio: per-entry matching priority replacing the edge weight (nullptr: weights)
 int64_t match_level(Ctx& c, const Level& L, int level, const Params& P, int32_t* match, int* rounds_out,
                     const int32_t* prio = nullptr);
