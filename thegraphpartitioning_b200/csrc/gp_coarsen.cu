@@ -1093,115 +1093,32 @@ __global__ void k_long_rows(int64_t nc, const int64_t* __restrict__ cdeg, int32_
     }
 }
 
-// tiers C and C2: one CTA per row, table in shared memory, two phases.
+// tiers C1, C and C2: one CTA per row, table in shared memory, two phases.
 // Phase 1 reads the walk once (straight from the fine CSR) and inserts every
 // entry into a 64-bit slot (key + 1) << 32 | (deg - j), zero meaning empty:
 // the claiming compare-and-swap stores the first position seen, later copies
 // raise it by atomicMax (the largest deg - j is the first occurrence);
 // weights add up in wsum, and position j keeps its slot in hj[j].  Phase 2:
-// warps ballot the first-occurrence flags (slot value == deg - j) of 32
-// consecutive positions into one word each, one block scan over the word
-// popcounts gives each word's base rank, and a second sweep writes the first
-// occurrences at base + rank within the word, then empties their slots (each
-// used slot has exactly one first occurrence), so the table is clear for the
-// CTA's next row.  words: 2 * ceil(deg/32) ints (bits, then prefix).
+// every warp takes a contiguous range of 32-position words, ballots their
+// first-occurrence flags (slot value == deg - j; lane i keeps word i's), and
+// scans their counts by shuffles; the warps' totals meet in shared memory, and
+// the warps write the first occurrences at their ranks, emptying their slots (each
+// used slot has exactly one), so the table is clear for the CTA's next row.
+// What bounds a row of a few thousand entries is its chain of latencies: three
+// barriers, and the loads list -> members -> row pointers -> ids -> cmap, of which
+// the first three are taken for the next row while this one is worked on.
+// (Seven barriers, bitmap and ranks in shared memory and every row's chain in the
+// open: C2 / C / C1 on R-MAT 24 37.9 / 18.5 / 17.2 ms in all; now 35.2 / 16.8 / 15.2.)
 constexpr uint16_t NO_SLOT = 0xFFFF;
-template <int T>
-__device__ void cta_dedup(const DGraph& g, const int32_t* __restrict__ cmap, const Walk& W, int64_t o, int64_t deg,
-                          int32_t self, unsigned long long* slot, int32_t* wsum, uint16_t* hj, int lg,
-                          int32_t* words, int32_t* __restrict__ tci, int32_t* __restrict__ tew, int32_t* cnt_out,
-                          int32_t* sh, int32_t* err) {
-    const uint32_t S = 1u << lg, mask = S - 1u;
-    for (int64_t base = 0; base < deg; base += 4 * T) {
-        int32_t cu[4], wt[4];
-        unsigned long long val[4], old[4];
-        uint32_t h[4];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const int64_t j = base + c * T + threadIdx.x;
-            cu[c] = self; wt[c] = 0;
-            if (j < deg) walk_load(g, cmap, W, j, cu[c], wt[c]);
-            val[c] = ((unsigned long long)((uint32_t)cu[c] + 1u) << 32) | (uint32_t)(deg - j);
-        }
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            h[c] = slot_hash(cu[c], lg);
-            old[c] = cu[c] != self ? atomicCAS(&slot[h[c]], 0ull, val[c]) : 0ull;
-        }
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const int64_t j = base + c * T + threadIdx.x;
-            if (j >= deg) continue;
-            if (cu[c] == self) { hj[j] = NO_SLOT; continue; }
-            const uint32_t tag = (uint32_t)cu[c] + 1u;
-            uint32_t probe = 1;
-            while (old[c] != 0ull && (uint32_t)(old[c] >> 32) != tag && probe < S) {
-                h[c] = (h[c] + 1) & mask;
-                old[c] = atomicCAS(&slot[h[c]], 0ull, val[c]);
-                ++probe;
-            }
-            if (old[c] != 0ull && (uint32_t)(old[c] >> 32) != tag) { atomicExch(err, 1); hj[j] = NO_SLOT; continue; }
-            if (old[c] != 0ull && old[c] < val[c]) atomicMax(&slot[h[c]], val[c]);
-            atomicAdd(&wsum[h[c]], wt[c]);
-            hj[j] = (uint16_t)h[c];
-        }
-    }
-    __syncthreads();
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarp = T / 32;
-    const int64_t nwords = (deg + 31) / 32;
-    int32_t* bits = words;
-    int32_t* wpre = words + nwords;
-    for (int64_t wi = wid; wi < nwords; wi += nwarp) {
-        const int64_t j = wi * 32 + lane;
-        bool first = false;
-        if (j < deg) {
-            const uint16_t hh = hj[j];
-            first = hh != NO_SLOT && (uint32_t)slot[hh] == (uint32_t)(deg - j);
-        }
-        const uint32_t word = __ballot_sync(0xffffffffu, first);
-        if (lane == 0) bits[wi] = (int32_t)word;
-    }
-    __syncthreads();
-    // exclusive scan of word popcounts: contiguous word ranges per thread
-    const int64_t per = (nwords + T - 1) / T;
-    const int64_t w0 = (int64_t)threadIdx.x * per, w1 = w0 + per < nwords ? w0 + per : nwords;
-    int32_t mine = 0;
-    for (int64_t wi = w0; wi < w1; ++wi) mine += __popc((uint32_t)bits[wi]);
-    int32_t tot;
-    int32_t run = block_scan_excl(mine, sh, tot);
-    for (int64_t wi = w0; wi < w1; ++wi) { wpre[wi] = run; run += __popc((uint32_t)bits[wi]); }
-    __syncthreads();
-    const uint32_t lt = (1u << lane) - 1u;
-    for (int64_t wi = wid; wi < nwords; wi += nwarp) {
-        const uint32_t word = (uint32_t)bits[wi];
-        if (!((word >> lane) & 1u)) continue;
-        const uint16_t hh = hj[wi * 32 + lane];
-        const int32_t r = wpre[wi] + __popc(word & lt);
-        if (!GP_IN(r, deg) || !GP_IN(hh, S)) continue;
-        tci[o + r] = (int32_t)((uint32_t)(slot[hh] >> 32) - 1u);
-        tew[o + r] = wsum[hh];
-    }
-    __syncthreads();
-    for (int64_t wi = wid; wi < nwords; wi += nwarp) {
-        const uint32_t word = (uint32_t)bits[wi];
-        if (!((word >> lane) & 1u)) continue;
-        const uint16_t hh = hj[wi * 32 + lane];
-        slot[hh] = 0ull;
-        wsum[hh] = 0;
-    }
-    if (threadIdx.x == 0) *cnt_out = tot;
-    __syncthreads();
-}
 
 // shared memory of an on-chip tier: SLOTS 64-bit slots and int32 weight sums,
-// a slot id per walk position, two words per 32 entries of the longest row
+// a slot id per walk position
 template <int SLOTS, int MAXROW>
 constexpr size_t cta_dedup_smem() {
-    return (sizeof(unsigned long long) + sizeof(int32_t)) * SLOTS + sizeof(uint16_t) * MAXROW +
-           sizeof(int32_t) * 2 * ((MAXROW + 31) / 32);
+    return (sizeof(unsigned long long) + sizeof(int32_t)) * SLOTS + sizeof(uint16_t) * MAXROW;
 }
 
-// tiers C and C2: table of at least twice the row length, at most SLOTS
+// table of at least twice the row length, at most SLOTS
 template <int T, int SLOTS, int MAXROW>
 __global__ void __launch_bounds__(T) k_dedup_cta_smem(DGraph g, const int32_t* __restrict__ cmap,
                                                       const int32_t* __restrict__ mem, const int32_t* __restrict__ list,
@@ -1210,22 +1127,109 @@ __global__ void __launch_bounds__(T) k_dedup_cta_smem(DGraph g, const int32_t* _
                                                       int32_t* __restrict__ tew, int32_t* __restrict__ cnt,
                                                       int32_t* __restrict__ err) {
     static_assert(SLOTS <= 65535, "slot ids are 16-bit");
+    constexpr int NW = T / 32;
+    static_assert((MAXROW + 32 * NW - 1) / (32 * NW) <= 32, "a warp's words fit in its lanes");
     extern __shared__ __align__(16) unsigned char stab_raw[];
     unsigned long long* slot = (unsigned long long*)stab_raw;          // SLOTS
     int32_t* wsum = (int32_t*)(slot + SLOTS);                          // SLOTS
     uint16_t* hj = (uint16_t*)(wsum + SLOTS);                          // MAXROW
-    int32_t* words = (int32_t*)(hj + ((MAXROW + 1) & ~1));             // 2 * MAXROW / 32
-    __shared__ int32_t sh[33];
+    __shared__ int32_t s_tot[NW];
     for (int i = threadIdx.x; i < SLOTS; i += T) { slot[i] = 0ull; wsum[i] = 0; }
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const uint32_t lt = (1u << lane) - 1u;
+    int64_t li = blockIdx.x;
+    if (li >= nlist) return;
+    int32_t self = list[li], deg = (int32_t)cdeg[self];
+    int64_t o = off[self];
+    Walk W = walk_of(g, mem, self);
     __syncthreads();
-    for (int64_t li = blockIdx.x; li < nlist; li += gridDim.x) {
-        const int64_t c = list[li];
-        const int64_t deg = cdeg[c];
-        int64_t S = 1;
+    for (;;) {
+        const int64_t ln = li + gridDim.x;
+        const int32_t cn = ln < nlist ? list[ln] : -1;   // the next row, its loads one phase ahead of their use
         int lg = 0;
-        while (S < 2 * deg && S < SLOTS) { S <<= 1; ++lg; }
-        cta_dedup<T>(g, cmap, walk_of(g, mem, c), off[c], deg, (int32_t)c, slot, wsum, hj, lg, words, tci, tew,
-                     &cnt[c], sh, err);
+        while ((1 << lg) < 2 * deg && (1 << lg) < SLOTS) ++lg;
+        const uint32_t S = 1u << lg, mask = S - 1u;
+        for (int32_t base = 0; base < deg; base += 4 * T) {
+            int32_t cu[4], wt[4];
+            unsigned long long val[4], old[4];
+            uint32_t h[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int32_t j = base + c * T + threadIdx.x;
+                cu[c] = self; wt[c] = 0;
+                if (j < deg) walk_load(g, cmap, W, j, cu[c], wt[c]);
+                val[c] = ((unsigned long long)((uint32_t)cu[c] + 1u) << 32) | (uint32_t)(deg - j);
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                h[c] = slot_hash(cu[c], lg);
+                old[c] = cu[c] != self ? atomicCAS(&slot[h[c]], 0ull, val[c]) : 0ull;
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int32_t j = base + c * T + threadIdx.x;
+                if (j >= deg) continue;
+                if (cu[c] == self) { hj[j] = NO_SLOT; continue; }
+                const uint32_t tag = (uint32_t)cu[c] + 1u;
+                uint32_t probe = 1;
+                while (old[c] != 0ull && (uint32_t)(old[c] >> 32) != tag && probe < S) {
+                    h[c] = (h[c] + 1) & mask;
+                    old[c] = atomicCAS(&slot[h[c]], 0ull, val[c]);
+                    ++probe;
+                }
+                if (old[c] != 0ull && (uint32_t)(old[c] >> 32) != tag) { atomicExch(err, 1); hj[j] = NO_SLOT; continue; }
+                if (old[c] != 0ull && old[c] < val[c]) atomicMax(&slot[h[c]], val[c]);
+                atomicAdd(&wsum[h[c]], wt[c]);
+                hj[j] = (uint16_t)h[c];
+            }
+        }
+        int32_t a = 0, b = -1, ndeg = 0;
+        int64_t no = 0;
+        if (cn >= 0) { a = mem[2 * (int64_t)cn]; b = mem[2 * (int64_t)cn + 1]; ndeg = (int32_t)cdeg[cn]; no = off[cn]; }
+        __syncthreads();
+        const int32_t nwords = (deg + 31) / 32, wpw = (nwords + NW - 1) / NW, wbeg = wid * wpw;
+        uint32_t mine = 0;   // lane i: first-occurrence flags of word wbeg + i
+        for (int32_t i = 0; i < wpw && wbeg + i < nwords; ++i) {
+            const int32_t j = (wbeg + i) * 32 + lane;
+            bool first = false;
+            if (j < deg) {
+                const uint16_t hh = hj[j];
+                first = hh != NO_SLOT && (uint32_t)slot[hh] == (uint32_t)(deg - j);
+            }
+            const uint32_t word = __ballot_sync(0xffffffffu, first);
+            if (lane == i) mine = word;
+        }
+        const int32_t pop = __popc(mine), inc = warp_incl_scan<int32_t>(pop);
+        if (lane == 31) s_tot[wid] = inc;
+        Walk nW;
+        nW.ea = 0; nW.da = 0; nW.eb = 0;
+        if (cn >= 0) {
+            nW.ea = g.rp[a];
+            nW.da = g.rp[a + 1] - nW.ea;
+            if (b >= 0) nW.eb = g.rp[b];
+        }
+        __syncthreads();
+        const int32_t wt = lane < NW ? s_tot[lane] : 0;
+        const int32_t before = (int32_t)__reduce_add_sync(0xffffffffu, (uint32_t)(lane < wid ? wt : 0));
+        if (wid == 0) {
+            const int32_t tot = (int32_t)__reduce_add_sync(0xffffffffu, (uint32_t)wt);
+            if (lane == 0) cnt[self] = tot;
+        }
+        const int32_t at = before + inc - pop;
+        for (int32_t i = 0; i < wpw && wbeg + i < nwords; ++i) {
+            const uint32_t word = __shfl_sync(0xffffffffu, mine, i);
+            const int32_t r = __shfl_sync(0xffffffffu, at, i) + __popc(word & lt);
+            if (!((word >> lane) & 1u)) continue;
+            const uint16_t hh = hj[(wbeg + i) * 32 + lane];
+            if (!GP_IN(r, deg) || !GP_IN(hh, S)) continue;
+            tci[o + r] = (int32_t)((uint32_t)(slot[hh] >> 32) - 1u);
+            tew[o + r] = wsum[hh];
+            slot[hh] = 0ull;   // nobody else looks at this slot any more
+            wsum[hh] = 0;
+        }
+        if (cn < 0) break;
+        __syncthreads();
+        li = ln; self = cn; deg = ndeg; o = no; W = nW;
     }
 }
 
