@@ -321,6 +321,19 @@ struct DGraph {
     const int32_t* vw = nullptr;   // nullptr = unit
 };
 
+// the next unit of block lb out of nlb for whichever of its warps asks (all 32
+// lanes): chunks of one unit per warp, dealt to the blocks in turn.  next: a
+// shared counter that starts at zero.  A warp that meets a long row holds up
+// nobody, where units assigned to warps kept a whole block's slots for its
+// slowest warp.
+__device__ __forceinline__ int64_t block_unit(uint32_t* next, int64_t lb, int64_t nlb) {
+    const uint32_t nw = blockDim.x >> 5;
+    uint32_t t = 0;
+    if ((threadIdx.x & 31) == 0) t = atomicAdd(next, 1u);
+    t = __shfl_sync(0xffffffffu, t, 0);
+    return ((int64_t)(t / nw) * nlb + lb) * nw + t % nw;
+}
+
 // ---------------------------------------------------------------- launch helpers
 inline int grid_for(int64_t items, int per_block, int cap = 148 * 16) {
     int64_t g = (items + per_block - 1) / per_block;

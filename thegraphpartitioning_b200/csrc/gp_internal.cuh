@@ -223,7 +223,7 @@ int initial_partition(Ctx& c, const Level& L, const Params& P, int32_t* part_out
 
 // gp_refine.cu
 int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int level, const Tracer& tr);
-int64_t conn_max_warps(const Ctx& c);   // most light warps a connectivity pass launches
+int64_t conn_max_ranges(const Ctx& c);   // most light warps a connectivity pass launches
 void project(Ctx& c, const Level& fine, const int32_t* part_coarse, int32_t* part_fine);
 void part_weights(Ctx& c, const DGraph& g, const int32_t* part, int32_t k, int64_t* pw);
 void cut_and_weights(Ctx& c, const DGraph& g, const int32_t* part, int32_t k, int64_t* d_cross2, int64_t* d_pw);

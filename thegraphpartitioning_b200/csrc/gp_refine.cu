@@ -93,7 +93,8 @@ struct ConnArgs {
     int64_t nitems;
     const int32_t* bucket[3];
     int64_t nbucket[3];
-    const int64_t* wfirst;      // first light unit of each light warp, and the end (nw + 1)
+    const int64_t* wfirst;      // first light unit of each range, and the end (nranges + 1)
+    int64_t nranges;
     int32_t* dest;
     int32_t* gain;
     const void* pc;             // the partition: PT[n], uint8 (k <= 256), uint16 (k <= 1024) or int32
@@ -576,6 +577,8 @@ __global__ void __launch_bounds__(RT, SHORT ? 4 : 5) k_conn(ConnArgs A) {
     uint64_t* s_k = sh.k;
     int32_t* s_q = sh.q;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    __shared__ uint32_t s_next;   // light blocks: ranges taken so far
+    if (threadIdx.x == 0) s_next = 0;
     for (int i = threadIdx.x; i < RW * k; i += RT) hist_all[i] = 0;
     int32_t light;
     bool full;
@@ -674,12 +677,15 @@ __global__ void __launch_bounds__(RT, SHORT ? 4 : 5) k_conn(ConnArgs A) {
     } else {
         int32_t* hist = hist_all + w * k;
         ConnRowS* rows = s_rows + w * 32;
-        const int64_t wid = ((int64_t)(blockIdx.x - A.nitems) * RT + threadIdx.x) >> 5;
-        // contiguous units of equal total cost (k_warp_bounds), taken 8 at a time
-        const int64_t u0 = A.wfirst[wid], u1 = A.wfirst[wid + 1];
         int64_t cdeg = 0;   // degree sum of this lane's candidates
-        for (int64_t ub = u0; ub < u1; ub += 8)
-            conn_group<PT, SHORT>(A, ub, (int)(u1 - ub < 8 ? u1 - ub : 8), mode, full, over, light, hist, rows, acc, cdeg);
+        for (;;) {
+            const int64_t r = block_unit(&s_next, blockIdx.x - A.nitems, gridDim.x - A.nitems);
+            if (r >= A.nranges) break;
+            const int64_t u0 = A.wfirst[r], u1 = A.wfirst[r + 1];
+            for (int64_t ub = u0; ub < u1; ub += 8)
+                conn_group<PT, SHORT>(A, ub, (int)(u1 - ub < 8 ? u1 - ub : 8), mode, full, over, light, hist, rows, acc,
+                                      cdeg);
+        }
         cdeg = warp_sum(cdeg);
         if (lane == 0 && cdeg) atomicAdd((unsigned long long*)&A.status[S_CDEG], (unsigned long long)cdeg);
     }
@@ -877,13 +883,48 @@ __device__ __forceinline__ void ab_warp(const ApplyArgs& A, int64_t v, int32_t* 
     if (lane == 0 && g2 >= 0) ab_commit<PT>(A, v, p, d, end - beg, delta, cnt);
 }
 
-template <class PT>
-__global__ void __launch_bounds__(RT, 4) k_lp_apply(ApplyArgs A) {
-    extern __shared__ int32_t delta[];   // part-weight changes (32-bit shared atomics, see rb_delta_begin)
-    __shared__ int64_t s_red[RW];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+// a block's part-weight changes (32-bit shared atomics, see rb_delta_begin) and
+// moves, added to the totals
+__device__ __forceinline__ void ab_begin(const ApplyArgs& A, int32_t* delta) {
     for (int q = threadIdx.x; q < A.k; q += RT) delta[q] = 0;
     __syncthreads();
+}
+__device__ __forceinline__ void ab_end(const ApplyArgs& A, const int32_t* delta, AbCount cnt) {
+    cnt.moves = warp_sum(cnt.moves);
+    cnt.deg = warp_sum(cnt.deg);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0 && cnt.moves) {
+        atomicAdd((unsigned long long*)&A.step[S_STEP_MOVES], (unsigned long long)cnt.moves);
+        atomicAdd((unsigned long long*)&A.step[S_MVDEG], (unsigned long long)cnt.deg);
+    }
+    for (int q = threadIdx.x; q < A.k; q += RT)
+        if (delta[q]) atomicAdd((unsigned long long*)&A.pw[q], (unsigned long long)(int64_t)delta[q]);
+}
+
+// the candidates of bucket 0 on large levels, one per lane (their registers
+// apart from k_lp_apply's, as k_conn_short)
+template <class PT>
+__global__ void __launch_bounds__(RT) k_lp_short(ApplyArgs A) {
+    extern __shared__ int32_t delta[];
+    ab_begin(A, delta);
+    AbCount cnt;
+    const int64_t n0 = A.status[S_NL0];
+    for (int64_t i0 = (int64_t)blockIdx.x * RT + (threadIdx.x & ~31); i0 < n0; i0 += (int64_t)gridDim.x * RT) {
+        const int64_t i = i0 + (threadIdx.x & 31);
+        ab_short<PT>(A, i < n0 ? A.clist[0][i] : -1, delta, cnt);
+    }
+    ab_end(A, delta, cnt);
+}
+
+// every other candidate row (split: bucket 0 is k_lp_short's)
+template <class PT>
+__global__ void __launch_bounds__(RT) k_lp_apply(ApplyArgs A, int split) {
+    extern __shared__ int32_t delta[];
+    __shared__ int64_t s_red[RW];
+    __shared__ uint32_t s_next;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (threadIdx.x == 0) s_next = 0;
+    ab_begin(A, delta);
     AbCount cnt;
     if ((int64_t)blockIdx.x < A.nitems) {
         const int32_t h = A.item_row[blockIdx.x];
@@ -915,35 +956,23 @@ __global__ void __launch_bounds__(RT, 4) k_lp_apply(ApplyArgs A) {
             }
         }
     } else {
-        const int64_t n0 = A.status[S_NL0], n1 = A.status[S_NL1], n2 = A.status[S_NL2];
-        const int64_t wid = ((int64_t)(blockIdx.x - A.nitems) * RT + threadIdx.x) >> 5;
-        const int64_t nw = ((int64_t)(gridDim.x - A.nitems) * RT) >> 5;
-        // short rows: one per lane when that still fills the launch's warps, else
-        // 16 lanes each (fewer rows one after another per warp)
-        const int rpw = n0 >= 32 * nw ? 32 : 2;
-        const int64_t U0 = (n0 + rpw - 1) / rpw;
-        for (int64_t u = wid; u < U0 + n1 + n2; u += nw) {
-            if (u < U0) {
-                const int64_t i = u * rpw + (rpw == 32 ? lane : lane >> 4);
-                const int64_t v = i < n0 ? A.clist[0][i] : -1;
-                if (rpw == 32) ab_short<PT>(A, v, delta, cnt);
-                else ab_tile<16, PT>(A, v, delta, cnt);
-            } else if (u < U0 + n1) {
-                ab_tile<kTile32, PT>(A, A.clist[1][u - U0], delta, cnt);
+        const int64_t n0 = split ? 0 : A.status[S_NL0], n1 = A.status[S_NL1], n2 = A.status[S_NL2];
+        // longest rows first
+        const int64_t U2 = n2, U21 = n2 + n1, U = U21 + (n0 + 1) / 2;
+        for (;;) {
+            const int64_t u = block_unit(&s_next, blockIdx.x - A.nitems, gridDim.x - A.nitems);
+            if (u >= U) break;
+            if (u >= U21) {
+                const int64_t i = (u - U21) * 2 + (lane >> 4);
+                ab_tile<16, PT>(A, i < n0 ? A.clist[0][i] : -1, delta, cnt);
+            } else if (u >= U2) {
+                ab_tile<kTile32, PT>(A, A.clist[1][u - U2], delta, cnt);
             } else {
-                ab_warp<PT>(A, A.clist[2][u - U0 - n1], delta, cnt);
+                ab_warp<PT>(A, A.clist[2][u], delta, cnt);
             }
         }
     }
-    cnt.moves = warp_sum(cnt.moves);
-    cnt.deg = warp_sum(cnt.deg);
-    __syncthreads();
-    if (lane == 0 && cnt.moves) {
-        atomicAdd((unsigned long long*)&A.step[S_STEP_MOVES], (unsigned long long)cnt.moves);
-        atomicAdd((unsigned long long*)&A.step[S_MVDEG], (unsigned long long)cnt.deg);
-    }
-    for (int q = threadIdx.x; q < A.k; q += RT)
-        if (delta[q]) atomicAdd((unsigned long long*)&A.pw[q], (unsigned long long)(int64_t)delta[q]);
+    ab_end(A, delta, cnt);
 }
 
 // ------------------------------------------------------------------ rebalance
@@ -1810,6 +1839,7 @@ __device__ void cta_refine_level(const CtaRefineArgs& R, unsigned char* rsm) {
         CA.item_beg = nullptr; CA.item_end = nullptr; CA.row_items = nullptr; CA.nitems = 0;
         for (int b = 0; b < 3; ++b) { CA.bucket[b] = R.bucket[b]; CA.nbucket[b] = R.nbucket[b]; CA.clist[b] = nullptr; }
         CA.wfirst = nullptr;
+        CA.nranges = 0;
         CA.dest = R.dest; CA.gain = R.gain; CA.status = R.status;
         CA.lock_next = nullptr; CA.prev = nullptr; CA.track_deg = -1; CA.host = nullptr; CA.nblocks = 0;
         CA.rb_all = R.tr_arrays ? 1 : 0;
@@ -2150,16 +2180,24 @@ static void trace_iter(Ctx& c, const RefineBufs& B, const int64_t* step_d, int64
 }
 
 constexpr int64_t kConnWarpCost = 8 * (8 + 28);
+// ranges of a block: one per warp until every SM has its resident blocks, then
+// up to kConnPer (24 to 200 are the same within 1%).  With one range per warp on
+// every level R-MAT 20 spent 53% of its warps' time at the end of their blocks,
+// behind the warp with a row of thousands of entries: its 73 passes took 11.1 ms
+// in all against 8.5, its move steps 1.85 against 1.24.
+constexpr int64_t kConnPer = 48;
+constexpr int64_t kConnFill = 5;     // resident blocks per SM
 // bucket-0 rows from which they take their own launch: below, a second launch
 // (about 3 us a pass) costs more than the registers
 constexpr int64_t kConnSplit = 32768;
+constexpr int64_t kConnSplitM = 1 << 21;   // entries (a pass of 30 us and more)
 constexpr int64_t kTrackShare = 32;
 constexpr int64_t kTrackMin = 1 << 22;   // entries from which the cut's change is tracked
-int64_t conn_max_warps(const Ctx& c) { return (int64_t)c.sm_count * c.ctas_per_sm * RW; }
+int64_t conn_max_ranges(const Ctx& c) { return (int64_t)c.sm_count * c.ctas_per_sm * RW; }
 
-// light warp t of a connectivity pass over nw warps takes the units
-// [first unit with cost prefix >= T * t / nw, the same for t + 1), T the total
-// cost: contiguous ranges of equal cost, the same for every pass of a level
+// range t of the nw of a connectivity pass holds the units [first unit with cost
+// prefix >= T * t / nw, the same for t + 1), T the total cost: contiguous ranges
+// of equal cost, the same for every pass of a level
 __global__ void k_warp_bounds(const int64_t* __restrict__ cost, int64_t nunits, int64_t nw,
                               int64_t* __restrict__ out) {
     const int64_t T = cost[nunits];
@@ -2191,26 +2229,26 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
     const int kpad = (k + 15) & ~15;
     const size_t conn_smem = kpad + sizeof(int32_t) * RW * k;
     // at most 1024 + 32 * GP_MAX_K bytes: below the 48 KB default, no attribute needed
-    // bucket-0 rows: their own launch on large levels
-    const bool split = L.nbucket[0] >= kConnSplit;
+    // bucket-0 rows: their own launches when they are many, and on levels whose
+    // longer rows are the work (k_conn without them runs at 48 registers)
+    const bool split = L.nbucket[0] >= kConnSplit || g.m >= kConnSplitM;
     const bool long_rows = !split || L.nitems + L.nbucket[1] + L.nbucket[2] > 0;
     const int64_t nunits = split ? L.nbucket[2] + L.nbucket[1] : L.nunits;
     const int64_t short_cost = split ? 0 : 2 * L.nbucket[0];
-    // a light warp's range costs as much as a group of 8 units of short rows,
-    // so that its lanes have rows to work on; on levels too small for 16 such
-    // warps per SM latency counts and units are spread thinner
-    const int64_t light_warps = std::min<int64_t>(
-        nunits, std::max<int64_t>((g.m + 32 * (L.nbucket[2] + L.nbucket[1]) + short_cost) / kConnWarpCost,
-                                  (int64_t)c.sm_count * 16));
-    const int light_blocks = (int)std::min<int64_t>(grid_for(light_warps, RW, c.sm_count * c.ctas_per_sm),
-                                                    (B.wfirst_cap - 1) / RW);
+    // a range costs as much as a group of 8 units of short rows, so that a warp's
+    // lanes have rows to work on; on levels too small for 16 such ranges per SM
+    // latency counts and units are spread thinner
+    const int64_t want = std::max<int64_t>(
+        (g.m + 32 * (L.nbucket[2] + L.nbucket[1]) + short_cost) / kConnWarpCost, (int64_t)c.sm_count * 16);
+    const int64_t nranges = std::max<int64_t>(std::min(std::min(nunits, want), B.wfirst_cap - 1), 1);
+    const int light_blocks = grid_for(
+        nranges, std::max<int64_t>(RW, std::min<int64_t>(kConnPer, nranges / (c.sm_count * kConnFill))),
+        c.sm_count * c.ctas_per_sm);
     const int grid = (int)L.nitems + light_blocks;
     const int short_grid = grid_for(L.nbucket[0], RT, c.sm_count * std::min(c.ctas_per_sm, 8));
-    // label propagation moves candidates of every bucket in one launch
-    const int lp_grid = split ? (int)L.nitems + std::max(light_blocks, grid_for(L.nbucket[0], 4 * RT, c.sm_count * 8)) : grid;
+    const int lp_grid = grid_for(L.nbucket[0], 4 * RT, c.sm_count * 8);
     if (long_rows) {
-        const int64_t nw = (int64_t)light_blocks * RW;
-        k_warp_bounds<<<grid_for(nw + 1, 256), 256, 0, c.s>>>(L.unit_cost, nunits, nw, B.wfirst);
+        k_warp_bounds<<<grid_for(nranges + 1, 256), 256, 0, c.s>>>(L.unit_cost, nunits, nranges, B.wfirst);
         GP_LAUNCHED(c);
     }
     int64_t best_cut = 0, best_mp = 0;
@@ -2247,8 +2285,9 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
         CA.nitems = L.nitems; CA.hhist = B.hhist; CA.hsum = B.hsum; CA.hdone = B.hdone;
         for (int b = 0; b < 3; ++b) { CA.bucket[b] = L.bucket[b]; CA.nbucket[b] = L.nbucket[b]; CA.clist[b] = B.clist[b]; }
         CA.wfirst = B.wfirst;
+        CA.nranges = nranges;
         CA.dest = B.dest; CA.gain = B.gain; CA.status = status;
-        CA.prev = step_d; CA.track_deg = track_deg; CA.rb_all = tr.on() ? 1 : 0; CA.host = c.h_pinned; CA.nblocks = (long_rows ? grid : 0) + (split ? short_grid : 0);
+        CA.prev = step_d; CA.track_deg = track_deg; CA.rb_all = tr.on() ? 1 : 0; CA.host = c.h_pinned; CA.nblocks = (long_rows ? grid : 0) + (split && L.nbucket[0] > 0 ? short_grid : 0);
         CA.pc = B.pc; CA.pc_next = B.pc_next; CA.lock_next = B.lock_next;   // the LP step's starting copy
         CA.pdg = B.pdg; CA.lp_dg = lp_dg;
         if (long_rows) {
@@ -2257,7 +2296,7 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
             kc<<<grid, RT, conn_smem, c.s>>>(CA);
             GP_LAUNCHED(c);
         }
-        if (split) {
+        if (split && L.nbucket[0] > 0) {
             auto ks = B.pcb == 1 ? k_conn_short<uint8_t> : k_conn_short<uint16_t>;
             ks<<<short_grid, RT, kpad, c.s>>>(CA);
             GP_LAUNCHED(c);
@@ -2338,9 +2377,15 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
                     tr.emit(ev);
                 }
             }
-            if (B.pcb == 1) k_lp_apply<uint8_t><<<lp_grid, RT, sizeof(int32_t) * k, c.s>>>(AA);
-            else k_lp_apply<uint16_t><<<lp_grid, RT, sizeof(int32_t) * k, c.s>>>(AA);
-            GP_LAUNCHED(c);
+            const size_t ksm = sizeof(int32_t) * k;
+            if (long_rows) {
+                (B.pcb == 1 ? k_lp_apply<uint8_t> : k_lp_apply<uint16_t>)<<<grid, RT, ksm, c.s>>>(AA, split ? 1 : 0);
+                GP_LAUNCHED(c);
+            }
+            if (split && L.nbucket[0] > 0) {
+                (B.pcb == 1 ? k_lp_short<uint8_t> : k_lp_short<uint16_t>)<<<lp_grid, RT, ksm, c.s>>>(AA);
+                GP_LAUNCHED(c);
+            }
             // copy pass + afterburner: candidate rows with gathered part (pcb bytes), dest and gain per entry
             c.bytes += (9 + B.pcb) * n + 16 * nlist + cdeg * (4 + (g.ew ? 4 : 0) + 8 + B.pcb);
             std::swap(B.lock, B.lock_next);
