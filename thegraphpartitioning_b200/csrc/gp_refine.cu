@@ -77,6 +77,26 @@ __device__ __forceinline__ bool lp_candidate(int32_t g, int32_t own, int32_t den
 // [S_CDEG] the sum of their degrees.  Rebalance candidates are the vertices
 // with dest >= 0, [S_CDEG] their number; they are collected in vertex order
 // afterwards.
+
+// What decides whether a pass is the level's last (the host loop's rule, from
+// its state before the pass): such a pass sweeps nothing when the cut's change
+// is known.
+struct ConnStop {
+    int64_t cross2, best_cut, best_mp;   // cross weight before the step; best state so far
+    int may;        // 0: the level goes on in any case, or the step's change is not tracked
+    int patience;   // one more state without a significant improvement ends the level
+    int idle;       // a step without moves ends the level
+};
+// state (cut, heaviest part) against the best one: better, and by how much
+__device__ __host__ __forceinline__ bool state_better(int64_t cut, int64_t mp, int64_t best_cut, int64_t best_mp,
+                                                      int64_t Lmax, bool& signif) {
+    const bool cb = mp <= Lmax, bb = best_mp <= Lmax;
+    signif = false;
+    if (cb && !bb) { signif = true; return true; }
+    if (cb && bb) { signif = 1000 * cut < 999 * best_cut; return cut < best_cut; }
+    if (!cb && !bb) { signif = mp < best_mp; return mp < best_mp || (mp == best_mp && cut < best_cut); }
+    return false;
+}
 struct ConnArgs {
     DGraph g;
     int32_t k;
@@ -109,6 +129,7 @@ struct ConnArgs {
     const int64_t* prev;        // status block of the iteration before (nullptr: none)
     int64_t track_deg;          // its step's cross-weight change is known (k_track) when the moved rows
                                 // had at most this many entries (-1: never)
+    ConnStop stop;
     int rb_all;                 // rebalancing passes store proposals of every row (trace)
     int64_t* host;              // host-resident copy of the status block, written by the pass's last
     int nblocks;                // block out of nblocks (over all its launches)
@@ -486,10 +507,20 @@ __device__ __forceinline__ int conn_head(const ConnArgs& A, uint8_t* over, ConnH
     __syncthreads();
     const int64_t maxpw = sh.maxpw;
     light = sh.light;
-    const int mode = A.force_eval ? MODE_EVAL : (maxpw > Lmax ? MODE_RB : MODE_LP);
+    int mode = A.force_eval ? MODE_EVAL : (maxpw > Lmax ? MODE_RB : MODE_LP);
     // a rebalancing pass sweeps only the rows of overweight parts when k_track
-    // has the last step's change of the cut (the same test there)
-    full = mode != MODE_RB || !A.prev || A.prev[S_MVDEG] > A.track_deg;
+    // has the last step's change of the cut (the same test there), the level's
+    // last pass nothing
+    const bool known = A.prev && A.prev[S_MVDEG] <= A.track_deg;
+    full = mode != MODE_RB || !known;
+    if (known && A.stop.may) {
+        bool signif;
+        state_better((A.stop.cross2 + A.prev[S_DELTA]) / 2, maxpw, A.stop.best_cut, A.stop.best_mp, Lmax, signif);
+        if (A.force_eval || (!signif && A.stop.patience) || (A.stop.idle && A.prev[S_STEP_MOVES] == 0)) {
+            mode = MODE_EVAL;
+            full = false;
+        }
+    }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         A.status[S_MAXPW] = maxpw; A.status[S_MODE] = mode; A.status[S_LIGHT] = light;
     }
@@ -542,7 +573,7 @@ __global__ void __launch_bounds__(RT, 4) k_conn_short(ConnArgs A) {
     const int mode = conn_head(A, over, sh, light, full);
     const int lane = threadIdx.x & 31;
     int64_t acc = 0, cdeg = 0;
-    const int64_t n0 = A.nbucket[0];
+    const int64_t n0 = mode == MODE_EVAL && !full ? 0 : A.nbucket[0];
     for (int64_t i0 = (int64_t)blockIdx.x * RT + (threadIdx.x & ~31); i0 < n0; i0 += (int64_t)gridDim.x * RT) {
         const int64_t i = i0 + lane;
         const ConnRow r = conn_row<PT>(A, i < n0 ? A.bucket[0][i] : -1, mode, full, over);
@@ -585,7 +616,9 @@ __global__ void __launch_bounds__(RT, SHORT ? 4 : 5) k_conn(ConnArgs A) {
     const int mode = conn_head(A, over, sh, light, full);
     int64_t acc = 0;  // directed cross weight (this thread)
 
-    if ((int64_t)blockIdx.x < A.nitems) {
+    if (mode == MODE_EVAL && !full) {
+        // nothing to sweep
+    } else if ((int64_t)blockIdx.x < A.nitems) {
         // ---- one piece of a long row per CTA; pieces of the same row are
         // combined in global accumulators and the last CTA decides
         int32_t* hist = hist_all;
@@ -1282,14 +1315,17 @@ __global__ void k_rb_strong_apply(int64_t cnt, const uint64_t* __restrict__ keys
 // v changes by w ([new v != new u] - [old v != old u]); its mirror (u, v), the
 // same weight on a symmetric graph, is counted with it when u did not move.
 // Exact integers, so that the pass after it need not sweep the rows it looks
-// for no move in: on the 256^3 grid (k = 32) the rebalancing passes, two thirds
-// of all, sweep one part in 32 instead of every row: all its passes take 47 ->
-// 32 ms, k_track 2.5 ms.  Left out when the
-// next pass sweeps every row anyway: no overweight part, or moved rows of more
-// than track_deg entries.  A block compares the partitions over its range of
-// vertices, 4 bytes per lane, and queues the moved ones; its threads take the
-// short rows of the queue, its warps the longer ones (a shared ticket: their
-// lengths differ widely); blocks [0, nitems) take the pieces of the heavy rows.
+// for no move in, and a pass that would end the level sweeps nothing: on the
+// 256^3 grid (k = 32) the rebalancing passes, two thirds of all, sweep one part in
+// 32 instead of every row: all its passes take 47 -> 32 ms, k_track 2.8 ms; on
+// R-MAT 24 they take 119 -> 102 ms, k_track 13.  Left out when the next pass sweeps
+// every row anyway: no overweight part and a level that may go on, or moved rows
+// of more than track_deg entries.  Blocks [0, nitems) take the pieces of the heavy
+// rows, range_blocks the warp rows by the connectivity pass's ranges (block_unit:
+// moved rows' lengths differ widely; one range of vertices per block, short and
+// long rows alike, took 49 ms on R-MAT 24 instead of 13), the others compare the
+// partitions over a range of vertices each, 4 bytes per lane, and queue the moved
+// short rows, which then get a thread each.
 struct TrackArgs {
     DGraph g;
     int32_t k;
@@ -1299,8 +1335,13 @@ struct TrackArgs {
     const void* pc_old;         // before it
     int64_t* step;              // its status block
     int64_t track_deg;
-    int32_t heavy_deg;
+    void* pair;                 // PartPair[n], filled by k_track_pairs
+    const int32_t* bucket[3];
+    int64_t nbucket[3];
+    const int64_t* wfirst;      // the connectivity pass's ranges of longer rows
+    int64_t nranges, range_blocks;
     int32_t range;              // vertices per block, a multiple of 4 * RT up to kTrackRange
+    int always;                 // also when no part is overweight (the next pass may be the level's last)
     const int32_t* heavy;
     const int32_t* item_row;
     const int64_t* item_beg;
@@ -1308,36 +1349,108 @@ struct TrackArgs {
     int64_t nitems;
 };
 constexpr int kTrackRange = 8192;
+// Part before and after the step: two gathers, or one where the moved rows have
+// enough entries (a quarter of the vertices) to pay for k_track_pairs, which
+// puts both into one word per vertex (R-MAT 24: k_track 17.0 -> 13.1 ms in all;
+// on meshes, where few vertices move, the pass over the vertices would cost more
+// than the gathers: 256^3 grid 3.3 ms for 164 steps).
+template <class PT> struct PartPair;
+template <> struct PartPair<uint8_t> { using T = uint16_t; };
+template <> struct PartPair<uint16_t> { using T = uint32_t; };
+__device__ __forceinline__ bool track_packed(const TrackArgs& T) { return 4 * T.step[S_MVDEG] >= T.g.n; }
 template <class PT>
-__device__ __forceinline__ int32_t track_term(const TrackArgs& T, int64_t e, int32_t po, int32_t pn) {
-    const int32_t u = __ldcs(&T.g.ci[e]);
-    if (!GP_IN(u, T.g.n)) return 0;
-    const int32_t uo = __ldg((const PT*)T.pc_old + u), un = __ldg((const PT*)T.pc + u);
+__device__ __forceinline__ uint32_t track_pair(const TrackArgs& T, bool packed, int32_t u) {
+    if (packed) return (uint32_t)__ldg((const typename PartPair<PT>::T*)T.pair + u);
+    return (uint32_t)__ldg((const PT*)T.pc_old + u) | ((uint32_t)__ldg((const PT*)T.pc + u) << (8 * sizeof(PT)));
+}
+__device__ __forceinline__ bool track_runs(const TrackArgs& T) {
+    if (T.step[S_STEP_MOVES] == 0 || T.step[S_MVDEG] > T.track_deg) return false;   // uniform
+    int over = 0;
+    for (int q = threadIdx.x; q < T.k; q += RT) over |= T.pw[q] > T.Lmax ? 1 : 0;
+    return __syncthreads_or(over) || T.always;
+}
+template <class PT>
+__global__ void __launch_bounds__(RT) k_track_pairs(TrackArgs T) {
+    if (!track_packed(T) || !track_runs(T)) return;
+    using QT = typename PartPair<PT>::T;
+    QT* pair = (QT*)T.pair;
+    for (int64_t v = (int64_t)blockIdx.x * RT + threadIdx.x; v < T.g.n; v += (int64_t)gridDim.x * RT)
+        pair[v] = (QT)(((const PT*)T.pc_old)[v] | ((QT)((const PT*)T.pc)[v] << (8 * sizeof(PT))));
+}
+template <class PT>
+__device__ __forceinline__ int32_t track_change(uint32_t x, int32_t po, int32_t pn, int32_t w) {
+    const int32_t uo = (int32_t)(x & (PT)~(PT)0), un = (int32_t)(x >> (8 * sizeof(PT)));
     const int32_t c = (pn != un ? 1 : 0) - (po != uo ? 1 : 0);
-    const int32_t w = T.g.ew ? __ldcs(&T.g.ew[e]) : 1;
     return uo == un ? 2 * c * w : c * w;
+}
+// this thread's part (t of nt) of entries [beg, end), four consecutive ones at a time
+template <class PT>
+__device__ __forceinline__ int64_t track_sum(const TrackArgs& T, bool packed, int64_t beg, int64_t end, int t, int nt,
+                                             int32_t po, int32_t pn) {
+    const bool v4 = aligned16(T.g.ci) && aligned16(T.g.ew);
+    int64_t sum = 0;
+    for (int64_t base = beg & ~(int64_t)3; base < end; base += 4 * (int64_t)nt) {
+        int32_t u[4], w[4];
+        uint32_t x[4];
+        const int64_t e4 = base + 4 * t;
+        ld4_row(T.g.ci, e4, beg, end, v4, -1, u);
+        if (T.g.ew) ld4_row(T.g.ew, e4, beg, end, v4, 0, w);
+        else {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) w[c] = 1;
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) x[c] = u[c] >= 0 && GP_IN(u[c], T.g.n) ? track_pair<PT>(T, packed, u[c]) : 0u;
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            if (u[c] >= 0 && GP_IN(u[c], T.g.n)) sum += track_change<PT>(x[c], po, pn, w[c]);
+    }
+    return sum;
 }
 template <class PT>
 __global__ void __launch_bounds__(RT) k_track(TrackArgs T) {
     __shared__ int32_t s_queue[kTrackRange];
-    __shared__ int32_t s_cnt, s_ticket;
+    __shared__ int32_t s_cnt;
+    __shared__ uint32_t s_next;
     __shared__ int64_t s_red[RW];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (threadIdx.x == 0) { s_cnt = 0; s_ticket = 0; }
-    int over = 0;
-    for (int q = threadIdx.x; q < T.k; q += RT) over |= T.pw[q] > T.Lmax ? 1 : 0;
-    if (!__syncthreads_or(over)) return;
-    if (T.step[S_STEP_MOVES] == 0 || T.step[S_MVDEG] > T.track_deg) return;
+    if (threadIdx.x == 0) { s_cnt = 0; s_next = 0; }
+    if (!track_runs(T)) return;
+    const bool packed = track_packed(T);
+    constexpr int PB = 8 * sizeof(PT);
     int64_t acc = 0;
     if ((int64_t)blockIdx.x < T.nitems) {
-        const int32_t v = T.heavy[T.item_row[blockIdx.x]];
-        const int32_t po = ((const PT*)T.pc_old)[v], pn = ((const PT*)T.pc)[v];
-        if (po != pn)
-            for (int64_t e = T.item_beg[blockIdx.x] + threadIdx.x; e < T.item_end[blockIdx.x]; e += RT)
-                acc += track_term<PT>(T, e, po, pn);
+        const uint32_t x = track_pair<PT>(T, packed, T.heavy[T.item_row[blockIdx.x]]);
+        const int32_t po = (int32_t)(x & (PT)~(PT)0), pn = (int32_t)(x >> PB);
+        if (po != pn) acc = track_sum<PT>(T, packed, T.item_beg[blockIdx.x], T.item_end[blockIdx.x], threadIdx.x, RT, po, pn);
+    } else if ((int64_t)blockIdx.x < T.nitems + T.range_blocks) {
+        const int64_t U2 = T.nbucket[2], U21 = U2 + T.nbucket[1];
+        for (;;) {
+            const int64_t r = block_unit(&s_next, blockIdx.x - T.nitems, T.range_blocks);
+            if (r >= T.nranges) break;
+            const int64_t u0 = T.wfirst[r], u1 = T.wfirst[r + 1] < U21 ? T.wfirst[r + 1] : U21;
+            for (int64_t ub = u0; ub < u1; ub += 32) {
+                const int64_t u = ub + lane;
+                int32_t po = 0, pn = 0;
+                int64_t beg = 0, end = 0;
+                if (u < u1) {
+                    const int32_t v = u < U2 ? T.bucket[2][u] : T.bucket[1][u - U2];
+                    const uint32_t x = track_pair<PT>(T, packed, v);
+                    po = (int32_t)(x & (PT)~(PT)0); pn = (int32_t)(x >> PB);
+                    if (po != pn) { beg = T.g.rp[v]; end = T.g.rp[v + 1]; }
+                }
+                uint32_t todo = __ballot_sync(0xffffffffu, po != pn);
+                while (todo) {
+                    const int j = __ffs(todo) - 1;
+                    todo &= todo - 1;
+                    const int64_t b = __shfl_sync(0xffffffffu, beg, j), e = __shfl_sync(0xffffffffu, end, j);
+                    acc += track_sum<PT>(T, packed, b, e, lane, 32, __shfl_sync(0xffffffffu, po, j), __shfl_sync(0xffffffffu, pn, j));
+                }
+            }
+        }
     } else {
         constexpr int per = 4 / sizeof(PT);   // ids per 4-byte word
-        const int64_t v0 = (int64_t)(blockIdx.x - T.nitems) * T.range;
+        const int64_t v0 = ((int64_t)blockIdx.x - T.nitems - T.range_blocks) * T.range;
         for (int32_t i = threadIdx.x * per; i < T.range; i += RT * per) {
             const int64_t v = v0 + i;
             uint32_t a = 0, b = 0;
@@ -1369,20 +1482,13 @@ __global__ void __launch_bounds__(RT) k_track(TrackArgs T) {
             const int32_t v = s_queue[i];
             const int64_t beg = T.g.rp[v], end = T.g.rp[v + 1];
             if (end - beg > kShortDeg) continue;
-            const int32_t po = ((const PT*)T.pc_old)[v], pn = ((const PT*)T.pc)[v];
-            for (int64_t e = beg; e < end; ++e) acc += track_term<PT>(T, e, po, pn);
-        }
-        for (;;) {
-            int32_t i = 0;
-            if (lane == 0) i = atomicAdd(&s_ticket, 1);
-            i = __shfl_sync(0xffffffffu, i, 0);
-            if (i >= cnt) break;
-            const int32_t v = s_queue[i];
-            const int64_t beg = T.g.rp[v], end = T.g.rp[v + 1];
-            if (end - beg <= kShortDeg || end - beg > T.heavy_deg) continue;
-            const int32_t po = ((const PT*)T.pc_old)[v], pn = ((const PT*)T.pc)[v];
-#pragma unroll 4
-            for (int64_t e = beg + lane; e < end; e += 32) acc += track_term<PT>(T, e, po, pn);
+            const uint32_t x = track_pair<PT>(T, packed, v);
+            const int32_t po = (int32_t)(x & (PT)~(PT)0), pn = (int32_t)(x >> PB);
+            for (int64_t e = beg; e < end; ++e) {
+                const int32_t u = __ldcs(&T.g.ci[e]);
+                if (GP_IN(u, T.g.n))
+                    acc += track_change<PT>(track_pair<PT>(T, packed, u), po, pn, T.g.ew ? __ldcs(&T.g.ew[e]) : 1);
+            }
         }
     }
     acc = warp_sum(acc);
@@ -2180,20 +2286,29 @@ static void trace_iter(Ctx& c, const RefineBufs& B, const int64_t* step_d, int64
 }
 
 constexpr int64_t kConnWarpCost = 8 * (8 + 28);
-// ranges of a block: one per warp until every SM has its resident blocks, then
-// up to kConnPer (24 to 200 are the same within 1%).  With one range per warp on
-// every level R-MAT 20 spent 53% of its warps' time at the end of their blocks,
-// behind the warp with a row of thousands of entries: its 73 passes took 11.1 ms
-// in all against 8.5, its move steps 1.85 against 1.24.
-constexpr int64_t kConnPer = 48;
-constexpr int64_t kConnFill = 5;     // resident blocks per SM
+// light blocks of a pass: one range per warp up to two resident waves, then
+// ranges of kConnRangeCost that a block's warps share, and more blocks only where
+// theirs would cost more than kConnBlockCost.  With one range per warp on every
+// level R-MAT 20 spent 53% of its warps' time at the end of their blocks, behind
+// the warp with a row of thousands of entries: its 73 passes took 11.1 ms in all
+// against 8.5 (20,000 per block; 10,000: 9.2; 40,000: 8.7), its move steps 1.85
+// against 1.24.  R-MAT 24's take 114 ms with 700,000 per block, 101 with 340,000,
+// 96 with 170,000, 94 with 85,000.
+constexpr int64_t kConnWave = 10;            // blocks per SM, 5 resident
+constexpr int64_t kConnRangeCost = 768;
+constexpr int64_t kConnBlockCost = 98304;
 // bucket-0 rows from which they take their own launch: below, a second launch
 // (about 3 us a pass) costs more than the registers
 constexpr int64_t kConnSplit = 32768;
 constexpr int64_t kConnSplitM = 1 << 21;   // entries (a pass of 30 us and more)
-constexpr int64_t kTrackShare = 32;
+// moved rows' share of the entries up to which the cut's change is tracked: before
+// a pass that looks for moves in the overweight parts (an eighth to a half of the
+// rows) and before one that may be the level's last (R-MAT 24, passes and k_track:
+// 1/16 and 1/4 117 ms, 1/8 and 1/3 115, 1/4 and 1/2 116; 1/32 and never 120)
+constexpr int64_t kTrackShare = 8;
+constexpr int64_t kTrackLast = 3;
 constexpr int64_t kTrackMin = 1 << 22;   // entries from which the cut's change is tracked
-int64_t conn_max_ranges(const Ctx& c) { return (int64_t)c.sm_count * c.ctas_per_sm * RW; }
+int64_t conn_max_ranges(const Ctx& c) { return (int64_t)c.sm_count * c.ctas_per_sm * RW * 4; }
 
 // range t of the nw of a connectivity pass holds the units [first unit with cost
 // prefix >= T * t / nw, the same for t + 1), T the total cost: contiguous ranges
@@ -2238,12 +2353,13 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
     // a range costs as much as a group of 8 units of short rows, so that a warp's
     // lanes have rows to work on; on levels too small for 16 such ranges per SM
     // latency counts and units are spread thinner
-    const int64_t want = std::max<int64_t>(
-        (g.m + 32 * (L.nbucket[2] + L.nbucket[1]) + short_cost) / kConnWarpCost, (int64_t)c.sm_count * 16);
+    const int64_t cost = g.m + 32 * (L.nbucket[2] + L.nbucket[1]) + short_cost;
+    const int64_t wave = (int64_t)c.sm_count * kConnWave;
+    const int64_t want = std::max<int64_t>(std::max(std::min(cost / kConnWarpCost, wave * RW), cost / kConnRangeCost),
+                                           (int64_t)c.sm_count * 16);
     const int64_t nranges = std::max<int64_t>(std::min(std::min(nunits, want), B.wfirst_cap - 1), 1);
-    const int light_blocks = grid_for(
-        nranges, std::max<int64_t>(RW, std::min<int64_t>(kConnPer, nranges / (c.sm_count * kConnFill))),
-        c.sm_count * c.ctas_per_sm);
+    const int light_blocks = (int)std::min<int64_t>(grid_for(nranges, RW, c.sm_count * c.ctas_per_sm),
+                                                    std::max(wave, cost / kConnBlockCost));
     const int grid = (int)L.nitems + light_blocks;
     const int short_grid = grid_for(L.nbucket[0], RT, c.sm_count * std::min(c.ctas_per_sm, 8));
     const int lp_grid = grid_for(L.nbucket[0], 4 * RT, c.sm_count * 8);
@@ -2258,10 +2374,12 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
     int64_t* step_d = nullptr;   // status block of the last step
     int64_t cross2 = 0;          // directed cross weight of the current state
     // the cut's change over a step is taken from the moved rows when they hold
-    // few of the entries (two gathers each, unbalanced; a pass over every row one
-    // gather each), on levels whose passes cost more than k_track's launch; an
-    // input that is not symmetric has no mirror entries
-    const int64_t track_deg = P.symmetric && g.m >= kTrackMin ? g.m / kTrackShare : -1;
+    // few of the entries, on levels whose passes cost more than k_track's launches;
+    // an input that is not symmetric has no mirror entries
+    const bool track = P.symmetric && g.m >= kTrackMin;
+    int64_t track_deg = -1;         // of the step before this pass
+    ConnStop stop;
+    memset(&stop, 0, sizeof stop);
     int32_t track_range = 4 * RT;   // about 8 blocks per SM
     while (track_range < kTrackRange && n > (int64_t)track_range * c.sm_count * 8) track_range *= 2;
     const bool move_head = B.mp && P.gnn && gnn_has_move_head(P.gnn);
@@ -2287,7 +2405,7 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
         CA.wfirst = B.wfirst;
         CA.nranges = nranges;
         CA.dest = B.dest; CA.gain = B.gain; CA.status = status;
-        CA.prev = step_d; CA.track_deg = track_deg; CA.rb_all = tr.on() ? 1 : 0; CA.host = c.h_pinned; CA.nblocks = (long_rows ? grid : 0) + (split && L.nbucket[0] > 0 ? short_grid : 0);
+        CA.prev = step_d; CA.track_deg = track_deg; CA.stop = stop; CA.rb_all = tr.on() ? 1 : 0; CA.host = c.h_pinned; CA.nblocks = (long_rows ? grid : 0) + (split && L.nbucket[0] > 0 ? short_grid : 0);
         CA.pc = B.pc; CA.pc_next = B.pc_next; CA.lock_next = B.lock_next;   // the LP step's starting copy
         CA.pdg = B.pdg; CA.lp_dg = lp_dg;
         if (long_rows) {
@@ -2325,11 +2443,8 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
             GP_CUDA(cudaMemcpyAsync(B.best_pw, B.pw, sizeof(int64_t) * k, cudaMemcpyDeviceToDevice, c.s));
         } else {
             const int64_t nmoves = c.h_pinned[H_MOVES];
-            const bool cb = cur_mp <= Lmax, bb = best_mp <= Lmax;
-            bool better = false, signif = false;
-            if (cb && !bb) { better = true; signif = true; }
-            else if (cb && bb) { better = cur_cut < best_cut; signif = 1000 * cur_cut < 999 * best_cut; }
-            else if (!cb && !bb) { better = cur_mp < best_mp || (cur_mp == best_mp && cur_cut < best_cut); signif = cur_mp < best_mp; }
+            bool signif;
+            const bool better = state_better(cur_cut, cur_mp, best_cut, best_mp, Lmax, signif);
             if (better) {
                 best_cut = cur_cut; best_mp = cur_mp;
                 GP_CUDA(cudaMemcpyAsync(B.best, B.pc, (size_t)B.pcb * n, cudaMemcpyDeviceToDevice, c.s));
@@ -2346,6 +2461,7 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
             if (stall >= P.o.refine_patience || lp_idle || rb_stuck) break;
         }
         if (final_eval) break;
+        if (dev_mode == MODE_EVAL) throw GpError(GP_EINTERNAL, "refinement pass ended a level that goes on");
         int mode;
         if (dev_mode == MODE_RB) { mode = (rb_streak >= P.o.strong_after) ? 2 : 1; ++rb_streak; }
         else { mode = 0; rb_streak = 0; }
@@ -2469,13 +2585,27 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
             }
             c.tmp->restore(mk);
         }
-        if (track_deg >= 0) {
+        if (track) {
+            // the next pass is the level's last when it does not improve on the best
+            // state (or in any case): all it would compute is the cut
+            stop.may = stall + 1 >= P.o.refine_patience || it + 1 == P.o.refine_max_iters ? 1 : 0;
+            stop.cross2 = cross2; stop.best_cut = best_cut; stop.best_mp = best_mp;
+            stop.patience = stall + 1 >= P.o.refine_patience ? 1 : 0;
+            stop.idle = mode == 2 || (mode == 0 && prev_moves == 0) ? 1 : 0;
+            track_deg = stop.may ? g.m / kTrackLast : g.m / kTrackShare;
             TrackArgs T;
             T.g = g; T.k = k; T.Lmax = Lmax; T.pw = B.pw; T.pc = B.pc; T.pc_old = B.pc_next; T.step = step_d;
-            T.track_deg = track_deg; T.heavy_deg = L.heavy_deg; T.heavy = L.heavy; T.item_row = L.item_row;
+            T.track_deg = track_deg; T.pair = B.ckeys2; T.heavy = L.heavy; T.item_row = L.item_row;
             T.item_beg = L.item_beg; T.item_end = L.item_end; T.nitems = L.nitems;
             T.range = track_range;
-            const int tg = (int)(L.nitems + (n + track_range - 1) / track_range);
+            T.always = stop.may;
+            for (int b = 0; b < 3; ++b) { T.bucket[b] = L.bucket[b]; T.nbucket[b] = L.nbucket[b]; }
+            T.wfirst = B.wfirst;
+            T.nranges = long_rows && L.nbucket[1] + L.nbucket[2] > 0 ? nranges : 0;
+            T.range_blocks = T.nranges > 0 ? light_blocks : 0;
+            const int tg = (int)(L.nitems + T.range_blocks + (n + track_range - 1) / track_range);
+            (B.pcb == 1 ? k_track_pairs<uint8_t> : k_track_pairs<uint16_t>)<<<grid_for(n, 4 * RT), RT, 0, c.s>>>(T);
+            GP_LAUNCHED(c);
             (B.pcb == 1 ? k_track<uint8_t> : k_track<uint16_t>)<<<tg, RT, 0, c.s>>>(T);
             GP_LAUNCHED(c);
         }
