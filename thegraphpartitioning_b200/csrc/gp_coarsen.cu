@@ -1093,99 +1093,177 @@ __global__ void k_long_rows(int64_t nc, const int64_t* __restrict__ cdeg, int32_
     }
 }
 
+// A slot of the one-block tiers' tables: a key and its first walk position.
+// PB > 0: 32 bits, key << PB | position (position < 2^PB, key < 2^(32 - PB) - 1),
+// all ones meaning empty: native compare-and-swap and minimum, 8 bytes a slot
+// with the weight.  PB = 0: 64 bits, (key + 1) << 32 | (deg - position), zero
+// meaning empty, the first position being the maximum.
+template <int PB>
+struct Slot {
+    using T = uint32_t;
+    static constexpr T EMPTY = 0xFFFFFFFFu;
+    static __device__ __forceinline__ T make(int32_t key, int32_t j, int32_t) { return ((uint32_t)key << PB) | (uint32_t)j; }
+    static __device__ __forceinline__ bool same(T a, T b) { return ((a ^ b) >> PB) == 0u; }
+    static __device__ __forceinline__ T cas(T* s, T v) { return atomicCAS(s, EMPTY, v); }
+    static __device__ __forceinline__ void first(T* s, T old, T v) { if (v < old) atomicMin(s, v); }
+    static __device__ __forceinline__ int32_t pos(T v, int32_t) { return (int32_t)(v & ((1u << PB) - 1u)); }
+    static __device__ __forceinline__ int32_t key(T v) { return (int32_t)(v >> PB); }
+};
+template <>
+struct Slot<0> {
+    using T = unsigned long long;
+    static constexpr T EMPTY = 0ull;
+    static __device__ __forceinline__ T make(int32_t key, int32_t j, int32_t deg) {
+        return ((unsigned long long)((uint32_t)key + 1u) << 32) | (uint32_t)(deg - j);
+    }
+    static __device__ __forceinline__ bool same(T a, T b) { return (uint32_t)((a ^ b) >> 32) == 0u; }
+    static __device__ __forceinline__ T cas(T* s, T v) { return atomicCAS(s, EMPTY, v); }
+    static __device__ __forceinline__ void first(T* s, T old, T v) { if (v > old) atomicMax(s, v); }
+    static __device__ __forceinline__ int32_t pos(T v, int32_t deg) { return deg - (int32_t)(uint32_t)v; }
+    static __device__ __forceinline__ int32_t key(T v) { return (int32_t)((uint32_t)(v >> 32) - 1u); }
+};
+// Inserts up to four entries of this thread (cu == self: none) into a table of
+// 2^lg slots and adds their weights; h: their slots.  The probes of the four go
+// on together, so that their shared-memory round trips overlap, in odd steps of
+// the key's own (full cycles; unit steps pile up in tables three quarters full).
+// R-MAT 24, rows of 4097-12288 / 2049-4096 / 513-2048 / 12289-65536 entries, in all:
+// 31.1 / 15.3 / 13.8 / 46.0 ms one entry after the other, 22.7 / 13.1 / 12.8 / 41.2
+// together, 20.9 / 12.5 / 12.0 / 39.6 with the steps.
+template <int PB>
+__device__ __forceinline__ void slots_insert(typename Slot<PB>::T* slot, int32_t* wsum, int lg, int32_t self,
+                                             const int32_t (&cu)[4], const int32_t (&wt)[4],
+                                             const typename Slot<PB>::T (&val)[4], uint32_t (&h)[4], int32_t* err) {
+    using S = Slot<PB>;
+    const uint32_t mask = (1u << lg) - 1u;
+    typename S::T old[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        h[c] = slot_hash(cu[c], lg);
+        old[c] = cu[c] != self ? S::cas(&slot[h[c]], val[c]) : S::EMPTY;
+    }
+    for (uint32_t probe = 1; probe <= mask; ++probe) {
+        bool any = false;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (old[c] != S::EMPTY && !S::same(old[c], val[c])) {
+                any = true;
+                h[c] = (h[c] + (((uint32_t)cu[c] * 0x85EBCA77u) >> 24 | 1u)) & mask;
+                old[c] = S::cas(&slot[h[c]], val[c]);
+            }
+        }
+        if (!any) break;
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        if (cu[c] == self) continue;
+        if (old[c] != S::EMPTY && !S::same(old[c], val[c])) { atomicExch(err, 1); continue; }
+        if (old[c] != S::EMPTY) S::first(&slot[h[c]], old[c], val[c]);
+        atomicAdd(&wsum[h[c]], wt[c]);
+    }
+}
+
 // tiers C1, C and C2: one CTA per row, table in shared memory, two phases.
 // Phase 1 reads the walk once (straight from the fine CSR) and inserts every
-// entry into a 64-bit slot (key + 1) << 32 | (deg - j), zero meaning empty:
-// the claiming compare-and-swap stores the first position seen, later copies
-// raise it by atomicMax (the largest deg - j is the first occurrence);
-// weights add up in wsum, and position j keeps its slot in hj[j].  Phase 2:
-// every warp takes a contiguous range of 32-position words, ballots their
-// first-occurrence flags (slot value == deg - j; lane i keeps word i's), and
-// scans their counts by shuffles; the warps' totals meet in shared memory, and
-// the warps write the first occurrences at their ranks, emptying their slots (each
-// used slot has exactly one), so the table is clear for the CTA's next row.
+// entry (Slot): the claiming compare-and-swap stores the first position seen, an
+// earlier one replaces it; weights add up in wsum, and position j keeps its slot
+// in hj[j].  Phase 2: every warp takes a contiguous range of 32-position words,
+// ballots their first-occurrence flags (lane i keeps word i's), and scans their
+// counts by shuffles; the warps' totals meet in shared memory, and the warps
+// write the first occurrences at their ranks, emptying their slots (each used
+// slot has exactly one), so the table is clear for the CTA's next row.
 // What bounds a row of a few thousand entries is its chain of latencies: three
-// barriers, and the loads list -> members -> row pointers -> ids -> cmap, of which
-// the first three are taken for the next row while this one is worked on.
-// (Seven barriers, bitmap and ranks in shared memory and every row's chain in the
-// open: C2 / C / C1 on R-MAT 24 37.9 / 18.5 / 17.2 ms in all; now 35.2 / 16.8 / 15.2.)
+// barriers, and the loads list -> members -> row pointers -> ids -> cmap.  The
+// headers are taken two rows ahead, the ids and weights one sweep ahead (the
+// first sweep of the next row before this row's barriers).
+// C2 / C / C1 on R-MAT 24, in all: 37.9 / 18.5 / 17.2 ms with seven barriers,
+// bitmap and ranks in shared memory and every chain in the open, 35.2 / 16.8 /
+// 15.2 with headers one row ahead, 20.9 / 12.5 / 12.0 with ids ahead, 32-bit slots
+// and the probes of a thread's four entries together.
 constexpr uint16_t NO_SLOT = 0xFFFF;
+constexpr int TC1_PB = 11, TC_PB = 12, TC2_PB = 14, TC3_PB = 16;   // position bits of each tier's 32-bit slots
+template <int PB>
+static bool slot_fits(int64_t nc) { return nc < ((int64_t)1 << (32 - PB)); }
 
-// shared memory of an on-chip tier: SLOTS 64-bit slots and int32 weight sums,
-// a slot id per walk position
-template <int SLOTS, int MAXROW>
+// shared memory of an on-chip tier: SLOTS slots and int32 weight sums, a slot id
+// per walk position
+template <int SLOTS, int MAXROW, int PB>
 constexpr size_t cta_dedup_smem() {
-    return (sizeof(unsigned long long) + sizeof(int32_t)) * SLOTS + sizeof(uint16_t) * MAXROW;
+    return (sizeof(typename Slot<PB>::T) + sizeof(int32_t)) * SLOTS + sizeof(uint16_t) * MAXROW;
 }
 
 // table of at least twice the row length, at most SLOTS
-template <int T, int SLOTS, int MAXROW>
-__global__ void __launch_bounds__(T) k_dedup_cta_smem(DGraph g, const int32_t* __restrict__ cmap,
-                                                      const int32_t* __restrict__ mem, const int32_t* __restrict__ list,
-                                                      int64_t nlist, const int64_t* __restrict__ off,
-                                                      const int64_t* __restrict__ cdeg, int32_t* __restrict__ tci,
-                                                      int32_t* __restrict__ tew, int32_t* __restrict__ cnt,
-                                                      int32_t* __restrict__ err) {
+template <int T, int SLOTS, int MAXROW, int PB>
+__global__ void __launch_bounds__(T, 1024 / T)
+    k_dedup_cta_smem(DGraph g, const int32_t* __restrict__ cmap, const int32_t* __restrict__ mem,
+                     const int32_t* __restrict__ list, int64_t nlist, const int64_t* __restrict__ off,
+                     const int64_t* __restrict__ cdeg, int32_t* __restrict__ tci, int32_t* __restrict__ tew,
+                     int32_t* __restrict__ cnt, int32_t* __restrict__ err) {
     static_assert(SLOTS <= 65535, "slot ids are 16-bit");
+    static_assert(PB == 0 || (1 << PB) >= MAXROW, "positions fit");
     constexpr int NW = T / 32;
     static_assert((MAXROW + 32 * NW - 1) / (32 * NW) <= 32, "a warp's words fit in its lanes");
+    using S = Slot<PB>;
+    using ST = typename S::T;
     extern __shared__ __align__(16) unsigned char stab_raw[];
-    unsigned long long* slot = (unsigned long long*)stab_raw;          // SLOTS
+    ST* slot = (ST*)stab_raw;                                          // SLOTS
     int32_t* wsum = (int32_t*)(slot + SLOTS);                          // SLOTS
     uint16_t* hj = (uint16_t*)(wsum + SLOTS);                          // MAXROW
     __shared__ int32_t s_tot[NW];
-    for (int i = threadIdx.x; i < SLOTS; i += T) { slot[i] = 0ull; wsum[i] = 0; }
+    for (int i = threadIdx.x; i < SLOTS; i += T) { slot[i] = S::EMPTY; wsum[i] = 0; }
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t lt = (1u << lane) - 1u;
     int64_t li = blockIdx.x;
     if (li >= nlist) return;
     int32_t self = list[li], deg = (int32_t)cdeg[self];
-    int64_t o = off[self];
     Walk W = walk_of(g, mem, self);
+    int32_t u[4], wt[4];   // ids and weights of the sweep to come
+    auto ahead = [&](const Walk& X, int32_t base, int32_t d) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int32_t j = base + c * T + threadIdx.x;
+            u[c] = -1; wt[c] = 0;
+            if (j < d) {
+                const int64_t e = X.entry(j);
+                u[c] = __ldcs(&g.ci[e]);
+                wt[c] = g.ew ? __ldcs(&g.ew[e]) : 1;
+            }
+        }
+    };
+    ahead(W, 0, deg);
+    int64_t ln = li + gridDim.x;
+    int32_t cn = ln < nlist ? list[ln] : -1;   // the next row: its header complete,
+    int32_t ndeg = 0;
+    Walk nW{0, 0, 0};
+    if (cn >= 0) { ndeg = (int32_t)cdeg[cn]; nW = walk_of(g, mem, cn); }
     __syncthreads();
     for (;;) {
-        const int64_t ln = li + gridDim.x;
-        const int32_t cn = ln < nlist ? list[ln] : -1;   // the next row, its loads one phase ahead of their use
+        const int64_t l2 = ln + gridDim.x;
+        const int32_t c2 = l2 < nlist ? list[l2] : -1;   // the one after it, its loads one phase ahead of their use
+        const int64_t o = off[self];
         int lg = 0;
         while ((1 << lg) < 2 * deg && (1 << lg) < SLOTS) ++lg;
-        const uint32_t S = 1u << lg, mask = S - 1u;
         for (int32_t base = 0; base < deg; base += 4 * T) {
-            int32_t cu[4], wt[4];
-            unsigned long long val[4], old[4];
+            int32_t cu[4], cw[4];
+            ST val[4];
             uint32_t h[4];
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                const int32_t j = base + c * T + threadIdx.x;
-                cu[c] = self; wt[c] = 0;
-                if (j < deg) walk_load(g, cmap, W, j, cu[c], wt[c]);
-                val[c] = ((unsigned long long)((uint32_t)cu[c] + 1u) << 32) | (uint32_t)(deg - j);
+                cu[c] = u[c] < 0 ? self : (GP_IN(u[c], g.n) ? cmap[u[c]] : 0);
+                cw[c] = wt[c];
             }
+            if (base + 4 * T < deg) ahead(W, base + 4 * T, deg);
+            else if (cn >= 0) ahead(nW, 0, ndeg);
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                h[c] = slot_hash(cu[c], lg);
-                old[c] = cu[c] != self ? atomicCAS(&slot[h[c]], 0ull, val[c]) : 0ull;
-            }
+            for (int c = 0; c < 4; ++c) val[c] = S::make(cu[c], base + c * T + (int32_t)threadIdx.x, deg);
+            slots_insert<PB>(slot, wsum, lg, self, cu, cw, val, h, err);
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 const int32_t j = base + c * T + threadIdx.x;
-                if (j >= deg) continue;
-                if (cu[c] == self) { hj[j] = NO_SLOT; continue; }
-                const uint32_t tag = (uint32_t)cu[c] + 1u;
-                uint32_t probe = 1;
-                while (old[c] != 0ull && (uint32_t)(old[c] >> 32) != tag && probe < S) {
-                    h[c] = (h[c] + 1) & mask;
-                    old[c] = atomicCAS(&slot[h[c]], 0ull, val[c]);
-                    ++probe;
-                }
-                if (old[c] != 0ull && (uint32_t)(old[c] >> 32) != tag) { atomicExch(err, 1); hj[j] = NO_SLOT; continue; }
-                if (old[c] != 0ull && old[c] < val[c]) atomicMax(&slot[h[c]], val[c]);
-                atomicAdd(&wsum[h[c]], wt[c]);
-                hj[j] = (uint16_t)h[c];
+                if (j < deg) hj[j] = cu[c] == self ? NO_SLOT : (uint16_t)h[c];
             }
         }
-        int32_t a = 0, b = -1, ndeg = 0;
-        int64_t no = 0;
-        if (cn >= 0) { a = mem[2 * (int64_t)cn]; b = mem[2 * (int64_t)cn + 1]; ndeg = (int32_t)cdeg[cn]; no = off[cn]; }
+        int32_t a = 0, b = -1, d2 = 0;
+        if (c2 >= 0) { a = mem[2 * (int64_t)c2]; b = mem[2 * (int64_t)c2 + 1]; d2 = (int32_t)cdeg[c2]; }
         __syncthreads();
         const int32_t nwords = (deg + 31) / 32, wpw = (nwords + NW - 1) / NW, wbeg = wid * wpw;
         uint32_t mine = 0;   // lane i: first-occurrence flags of word wbeg + i
@@ -1194,25 +1272,24 @@ __global__ void __launch_bounds__(T) k_dedup_cta_smem(DGraph g, const int32_t* _
             bool first = false;
             if (j < deg) {
                 const uint16_t hh = hj[j];
-                first = hh != NO_SLOT && (uint32_t)slot[hh] == (uint32_t)(deg - j);
+                first = hh != NO_SLOT && S::pos(slot[hh], deg) == j;
             }
             const uint32_t word = __ballot_sync(0xffffffffu, first);
             if (lane == i) mine = word;
         }
         const int32_t pop = __popc(mine), inc = warp_incl_scan<int32_t>(pop);
         if (lane == 31) s_tot[wid] = inc;
-        Walk nW;
-        nW.ea = 0; nW.da = 0; nW.eb = 0;
-        if (cn >= 0) {
-            nW.ea = g.rp[a];
-            nW.da = g.rp[a + 1] - nW.ea;
-            if (b >= 0) nW.eb = g.rp[b];
+        Walk W2{0, 0, 0};
+        if (c2 >= 0) {
+            W2.ea = g.rp[a];
+            W2.da = g.rp[a + 1] - W2.ea;
+            if (b >= 0) W2.eb = g.rp[b];
         }
         __syncthreads();
-        const int32_t wt = lane < NW ? s_tot[lane] : 0;
-        const int32_t before = (int32_t)__reduce_add_sync(0xffffffffu, (uint32_t)(lane < wid ? wt : 0));
+        const int32_t wtot = lane < NW ? s_tot[lane] : 0;
+        const int32_t before = (int32_t)__reduce_add_sync(0xffffffffu, (uint32_t)(lane < wid ? wtot : 0));
         if (wid == 0) {
-            const int32_t tot = (int32_t)__reduce_add_sync(0xffffffffu, (uint32_t)wt);
+            const int32_t tot = (int32_t)__reduce_add_sync(0xffffffffu, (uint32_t)wtot);
             if (lane == 0) cnt[self] = tot;
         }
         const int32_t at = before + inc - pop;
@@ -1221,15 +1298,15 @@ __global__ void __launch_bounds__(T) k_dedup_cta_smem(DGraph g, const int32_t* _
             const int32_t r = __shfl_sync(0xffffffffu, at, i) + __popc(word & lt);
             if (!((word >> lane) & 1u)) continue;
             const uint16_t hh = hj[(wbeg + i) * 32 + lane];
-            if (!GP_IN(r, deg) || !GP_IN(hh, S)) continue;
-            tci[o + r] = (int32_t)((uint32_t)(slot[hh] >> 32) - 1u);
+            if (!GP_IN(r, deg) || !GP_IN(hh, SLOTS)) continue;
+            tci[o + r] = S::key(slot[hh]);
             tew[o + r] = wsum[hh];
-            slot[hh] = 0ull;   // nobody else looks at this slot any more
+            slot[hh] = S::EMPTY;   // nobody else looks at this slot any more
             wsum[hh] = 0;
         }
         if (cn < 0) break;
         __syncthreads();
-        li = ln; self = cn; deg = ndeg; o = no; W = nW;
+        ln = l2; self = cn; deg = ndeg; W = nW; cn = c2; ndeg = d2; nW = W2;
     }
 }
 
@@ -1258,22 +1335,25 @@ static int32_t* longest_first(Ctx& c, const int32_t* list, int64_t nlist, const 
 // tier C3: one 1024-thread CTA per row of TC2_ROW < d <= TC3_ROW walk entries.
 // Pass 0 gathers the walk through cmap once and leaves the mapped ids and
 // weights in the row's range of the scratch arrays (key_at, w_at); passes
-// 1..P-1 read them from there (P = the power of two with d / P <= TC3_KEYS).
+// 1..P-1 read them from there (P = the power of two with min(d, nc) / P <=
+// TC3_KEYS: there are at most nc keys).
 // Pass p inserts only the keys whose pass hash is p into the 16384-slot table
-// (the same 64-bit slots as tier C: (key + 1) << 32 | (d - j), first position
-// kept by atomicMax, weights summed), then every used slot marks its first
+// (Slot, weights summed), then every used slot marks its first
 // position in a bitmap of the walk, leaves its weight sum at that position of
 // w_at (later passes never read the weights of another pass's keys), and is
 // cleared.  After the passes one block scan ranks
 // the marked positions and the keys are written in first-occurrence order, as
-// every other tier writes them.
+// every other tier writes them.  Each sweep's ids are loaded a sweep ahead (39.6
+// -> 38.7 ms on R-MAT 24; 46.8 with the entries' probes one after the other).
+template <int PB>
 constexpr size_t tc3_smem() {
-    return (sizeof(unsigned long long) + sizeof(int32_t)) * TC2_SLOTS + sizeof(uint32_t) * 2 * (TC3_ROW / 32);
+    return (sizeof(typename Slot<PB>::T) + sizeof(int32_t)) * TC2_SLOTS + sizeof(uint32_t) * 2 * (TC3_ROW / 32);
 }
 __device__ __forceinline__ uint32_t pass_of(int32_t key, int lgp) {
     return lgp ? ((uint32_t)key * 0x85EBCA77u) >> (32 - lgp) : 0u;
 }
-__global__ void __launch_bounds__(TC2_T) k_dedup_multipass(DGraph g, const int32_t* __restrict__ cmap,
+template <int PB>
+__global__ void __launch_bounds__(TC2_T) k_dedup_multipass(DGraph g, int64_t nc, const int32_t* __restrict__ cmap,
                                                            const int32_t* __restrict__ mem,
                                                            const int32_t* __restrict__ list, int64_t nlist,
                                                            const int64_t* __restrict__ off,
@@ -1284,12 +1364,14 @@ __global__ void __launch_bounds__(TC2_T) k_dedup_multipass(DGraph g, const int32
     constexpr int T = TC2_T, S = TC2_SLOTS, LG = 14;
     static_assert((1 << LG) == S, "table size");
     extern __shared__ __align__(16) unsigned char mp_raw[];
-    unsigned long long* slot = (unsigned long long*)mp_raw;            // S
+    using SL = Slot<PB>;
+    using ST = typename SL::T;
+    ST* slot = (ST*)mp_raw;                                            // S
     int32_t* wsum = (int32_t*)(slot + S);                              // S
     uint32_t* bits = (uint32_t*)(wsum + S);                            // TC3_ROW / 32
     int32_t* wpre = (int32_t*)(bits + TC3_ROW / 32);                   // TC3_ROW / 32
     __shared__ int32_t sh[33];
-    for (int i = threadIdx.x; i < S; i += T) { slot[i] = 0ull; wsum[i] = 0; }
+    for (int i = threadIdx.x; i < S; i += T) { slot[i] = SL::EMPTY; wsum[i] = 0; }
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarp = T / 32;
     for (int64_t li = blockIdx.x; li < nlist; li += gridDim.x) {
         const int64_t c = list[li];
@@ -1298,20 +1380,34 @@ __global__ void __launch_bounds__(TC2_T) k_dedup_multipass(DGraph g, const int32
         const Walk W = walk_of(g, mem, c);
         const int64_t nwords = (deg + 31) / 32;
         int lgp = 0;
-        while ((deg >> lgp) > TC3_KEYS) ++lgp;
+        const int64_t most = deg < nc ? deg : nc;
+        while ((most >> lgp) > TC3_KEYS) ++lgp;
         for (int64_t i = threadIdx.x; i < nwords; i += T) bits[i] = 0u;
         __syncthreads();
+        int32_t u[4], uw[4];   // the sweep to come: ids and weights (pass 0) or mapped ids
+        auto ahead = [&](uint32_t pass, int64_t base) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int64_t j = base + q * T + threadIdx.x;
+                u[q] = pass ? self : -1; uw[q] = 0;
+                if (j >= deg) continue;
+                if (pass) { u[q] = __ldcg(&key_at[o + j]); continue; }   // this thread's own store
+                const int64_t e = W.entry(j);
+                u[q] = __ldcs(&g.ci[e]);
+                uw[q] = g.ew ? __ldcs(&g.ew[e]) : 1;
+            }
+        };
+        ahead(0, 0);
         for (uint32_t pass = 0; pass < (1u << lgp); ++pass) {
             for (int64_t base = 0; base < deg; base += 4 * T) {
                 int32_t cu[4], wt[4];
                 if (pass == 0) {
-                    // all four gathers in flight before the stores
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
-                        const int64_t j = base + q * T + threadIdx.x;
-                        cu[q] = self; wt[q] = 0;
-                        if (j < deg) walk_load(g, cmap, W, j, cu[q], wt[q]);
+                        cu[q] = u[q] < 0 ? self : (GP_IN(u[q], g.n) ? cmap[u[q]] : 0);
+                        wt[q] = uw[q];
                     }
+                    if (base + 4 * T < deg) ahead(0, base + 4 * T);
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         const int64_t j = base + q * T + threadIdx.x;
@@ -1322,45 +1418,30 @@ __global__ void __launch_bounds__(TC2_T) k_dedup_multipass(DGraph g, const int32
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         const int64_t j = base + q * T + threadIdx.x;
-                        cu[q] = j < deg ? __ldcg(&key_at[o + j]) : self;
-                    }
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const int64_t j = base + q * T + threadIdx.x;
-                        if (cu[q] != self && pass_of(cu[q], lgp) != pass) cu[q] = self;
+                        cu[q] = u[q] != self && pass_of(u[q], lgp) == pass ? u[q] : self;
                         wt[q] = cu[q] != self ? __ldcg(&w_at[o + j]) : 0;
                     }
+                    if (base + 4 * T < deg) ahead(pass, base + 4 * T);
                 }
+                if (base + 4 * T >= deg && pass + 1 < (1u << lgp)) ahead(pass + 1, 0);
+                ST val[4];
+                uint32_t h[4];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    if (cu[q] == self) continue;
-                    const int64_t j = base + q * T + threadIdx.x;
-                    const unsigned long long val = ((unsigned long long)((uint32_t)cu[q] + 1u) << 32) | (uint32_t)(deg - j);
-                    const uint32_t tag = (uint32_t)cu[q] + 1u;
-                    uint32_t h = slot_hash(cu[q], LG);
-                    unsigned long long old = atomicCAS(&slot[h], 0ull, val);
-                    uint32_t probe = 1;
-                    while (old != 0ull && (uint32_t)(old >> 32) != tag && probe < (uint32_t)S) {
-                        h = (h + 1) & (S - 1);
-                        old = atomicCAS(&slot[h], 0ull, val);
-                        ++probe;
-                    }
-                    if (old != 0ull && (uint32_t)(old >> 32) != tag) { atomicExch(err, 1); continue; }
-                    if (old != 0ull && old < val) atomicMax(&slot[h], val);
-                    atomicAdd(&wsum[h], wt[q]);
-                }
+                for (int q = 0; q < 4; ++q)
+                    val[q] = SL::make(cu[q], (int32_t)base + q * T + (int32_t)threadIdx.x, (int32_t)deg);
+                slots_insert<PB>(slot, wsum, LG, self, cu, wt, val, h, err);
             }
             __syncthreads();
             // the pass's keys: mark first positions, park key and weight there, clear
             for (int i = threadIdx.x; i < S; i += T) {
-                const unsigned long long v = slot[i];
-                if (!v) continue;
-                const int64_t j = deg - (int64_t)(uint32_t)v;
+                const ST v = slot[i];
+                if (v == SL::EMPTY) continue;
+                const int64_t j = SL::pos(v, (int32_t)deg);
                 if (GP_IN(j, deg)) {
                     atomicOr(&bits[j >> 5], 1u << (j & 31));
                     w_at[o + j] = wsum[i];
                 }
-                slot[i] = 0ull;
+                slot[i] = SL::EMPTY;
                 wsum[i] = 0;
             }
             __syncthreads();
@@ -1670,35 +1751,34 @@ void contract_level(Ctx& c, Level& fine, Level& coarse, const int32_t* match, in
         c.sync();
         nC = c.h_pinned[0]; nD = c.h_pinned[1]; nC2 = c.h_pinned[3]; nC3 = c.h_pinned[4]; nC1 = c.h_pinned[5];
     }
-    if (nC1 > 0) {
-        k_dedup_cta_smem<TC1_T, TC1_SLOTS, TC1_ROW>
-            <<<(unsigned)std::min<int64_t>(nC1, (int64_t)c.sm_count * c.ctas_per_sm), TC1_T,
-               cta_dedup_smem<TC1_SLOTS, TC1_ROW>(), c.s>>>(g, fine.cmap, mem, listC1, nC1, off, cdeg, tci, tew, rowcnt,
-                                                            err);
-        GP_LAUNCHED(c);
-    }
-    if (nC > 0) {
-        // one CTA per row: the block scheduler balances rows of unequal length
-        k_dedup_cta_smem<TC_T, TC_SLOTS, TC_ROW>
-            <<<(unsigned)std::min<int64_t>(nC, (int64_t)c.sm_count * c.ctas_per_sm), TC_T,
-               cta_dedup_smem<TC_SLOTS, TC_ROW>(), c.s>>>(g, fine.cmap, mem, listC, nC, off, cdeg, tci, tew, rowcnt,
-                                                          err);
-        GP_LAUNCHED(c);
-    }
+    // one CTA per row: the block scheduler balances rows of unequal length
     if (nC2 > c.sm_count) listC2 = longest_first(c, listC2, nC2, cdeg, TC2_ROW);
     if (nC3 > c.sm_count) listC3 = longest_first(c, listC3, nC3, cdeg, TC3_ROW);
-    if (nC2 > 0) {
-        k_dedup_cta_smem<TC2_T, TC2_SLOTS, TC2_ROW>
-            <<<(unsigned)std::min<int64_t>(nC2, (int64_t)c.sm_count * c.ctas_per_sm), TC2_T,
-               cta_dedup_smem<TC2_SLOTS, TC2_ROW>(), c.s>>>(g, fine.cmap, mem, listC2, nC2, off, cdeg, tci, tew, rowcnt,
-                                                            err);
+    auto cta_tier = [&](auto kernel, const int32_t* list, int64_t nl, int T, size_t smem) {
+        kernel<<<(unsigned)std::min<int64_t>(nl, (int64_t)c.sm_count * c.ctas_per_sm), T, smem, c.s>>>(
+            g, fine.cmap, mem, list, nl, off, cdeg, tci, tew, rowcnt, err);
         GP_LAUNCHED(c);
+    };
+    if (nC1 > 0) {
+        if (slot_fits<TC1_PB>(nc)) cta_tier(k_dedup_cta_smem<TC1_T, TC1_SLOTS, TC1_ROW, TC1_PB>, listC1, nC1, TC1_T, cta_dedup_smem<TC1_SLOTS, TC1_ROW, TC1_PB>());
+        else cta_tier(k_dedup_cta_smem<TC1_T, TC1_SLOTS, TC1_ROW, 0>, listC1, nC1, TC1_T, cta_dedup_smem<TC1_SLOTS, TC1_ROW, 0>());
+    }
+    if (nC > 0) {
+        if (slot_fits<TC_PB>(nc)) cta_tier(k_dedup_cta_smem<TC_T, TC_SLOTS, TC_ROW, TC_PB>, listC, nC, TC_T, cta_dedup_smem<TC_SLOTS, TC_ROW, TC_PB>());
+        else cta_tier(k_dedup_cta_smem<TC_T, TC_SLOTS, TC_ROW, 0>, listC, nC, TC_T, cta_dedup_smem<TC_SLOTS, TC_ROW, 0>());
+    }
+    if (nC2 > 0) {
+        if (slot_fits<TC2_PB>(nc)) cta_tier(k_dedup_cta_smem<TC2_T, TC2_SLOTS, TC2_ROW, TC2_PB>, listC2, nC2, TC2_T, cta_dedup_smem<TC2_SLOTS, TC2_ROW, TC2_PB>());
+        else cta_tier(k_dedup_cta_smem<TC2_T, TC2_SLOTS, TC2_ROW, 0>, listC2, nC2, TC2_T, cta_dedup_smem<TC2_SLOTS, TC2_ROW, 0>());
     }
     if (nC3 > 0) {
         // key and weight of each first occurrence are parked at its walk position
         // in mapped / mw (free at these rows: only tier-D rows use them otherwise)
-        k_dedup_multipass<<<(unsigned)std::min<int64_t>(nC3, (int64_t)c.sm_count * c.ctas_per_sm), TC2_T, tc3_smem(),
-                            c.s>>>(g, fine.cmap, mem, listC3, nC3, off, cdeg, mapped, mw, tci, tew, rowcnt, err);
+        const bool fits = slot_fits<TC3_PB>(nc);
+        (fits ? k_dedup_multipass<TC3_PB> : k_dedup_multipass<0>)<<<
+            (unsigned)std::min<int64_t>(nC3, (int64_t)c.sm_count * c.ctas_per_sm), TC2_T,
+            fits ? tc3_smem<TC3_PB>() : tc3_smem<0>(), c.s>>>(g, nc, fine.cmap, mem, listC3, nC3, off, cdeg, mapped, mw,
+                                                              tci, tew, rowcnt, err);
         GP_LAUNCHED(c);
     }
     if (nD > 0) {
@@ -1802,13 +1882,17 @@ void coarsen_smem_caps() {
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smA2));
     GP_CUDA(cudaFuncSetAttribute(k_dedup_warp<TB_ROW, TB_SLOTS, TB_WARPS, int16_t>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smB));
-    GP_CUDA(cudaFuncSetAttribute(k_dedup_cta_smem<TC1_T, TC1_SLOTS, TC1_ROW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)cta_dedup_smem<TC1_SLOTS, TC1_ROW>()));
-    GP_CUDA(cudaFuncSetAttribute(k_dedup_cta_smem<TC_T, TC_SLOTS, TC_ROW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)cta_dedup_smem<TC_SLOTS, TC_ROW>()));
-    GP_CUDA(cudaFuncSetAttribute(k_dedup_cta_smem<TC2_T, TC2_SLOTS, TC2_ROW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)cta_dedup_smem<TC2_SLOTS, TC2_ROW>()));
-    GP_CUDA(cudaFuncSetAttribute(k_dedup_multipass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc3_smem()));
+    auto big_smem = [](auto kernel, size_t bytes) {
+        GP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    };
+    big_smem(k_dedup_cta_smem<TC1_T, TC1_SLOTS, TC1_ROW, TC1_PB>, cta_dedup_smem<TC1_SLOTS, TC1_ROW, TC1_PB>());
+    big_smem(k_dedup_cta_smem<TC1_T, TC1_SLOTS, TC1_ROW, 0>, cta_dedup_smem<TC1_SLOTS, TC1_ROW, 0>());
+    big_smem(k_dedup_cta_smem<TC_T, TC_SLOTS, TC_ROW, TC_PB>, cta_dedup_smem<TC_SLOTS, TC_ROW, TC_PB>());
+    big_smem(k_dedup_cta_smem<TC_T, TC_SLOTS, TC_ROW, 0>, cta_dedup_smem<TC_SLOTS, TC_ROW, 0>());
+    big_smem(k_dedup_cta_smem<TC2_T, TC2_SLOTS, TC2_ROW, TC2_PB>, cta_dedup_smem<TC2_SLOTS, TC2_ROW, TC2_PB>());
+    big_smem(k_dedup_cta_smem<TC2_T, TC2_SLOTS, TC2_ROW, 0>, cta_dedup_smem<TC2_SLOTS, TC2_ROW, 0>());
+    big_smem(k_dedup_multipass<TC3_PB>, tc3_smem<TC3_PB>());
+    big_smem(k_dedup_multipass<0>, tc3_smem<0>());
 }
 
 }  // namespace gp
