@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(IP_T) k_initpart(DGraph g, int32_t k, uint64_t
         for (int i = 0; i < IP_T / 32; ++i) s += red[i];
         int64_t mp = 0;
         for (int q = 0; q < k; ++q) mp = S.WL[q] > mp ? S.WL[q] : mp;
-        tcut[t] = s / 2;
+        tcut[t] = s;
         tmaxpw[t] = mp;
     }
 }
@@ -275,7 +275,10 @@ __global__ void __launch_bounds__(IP_T) k_initpart(DGraph g, int32_t k, uint64_t
 // vertex and whose split key takes a binary search over (distance, id):
 // 823 vertices k = 8 893 -> 143 us, random geometric 8,864 vertices k = 300
 // 44.0 -> 1.5 ms, Chung-Lu 1,789 vertices k = 64 5.4 -> 1.7 ms, R-MAT (dense)
-// 1,999 vertices k = 64 11.2 -> 3.5 ms.
+// 1,999 vertices k = 64 11.2 -> 3.5 ms; the last two 0.91 and 1.38 ms with the cuts
+// in k_trial_cuts and NB = 4 entries of a lane in flight.  NB = 4 from a mean
+// degree of 32 on rows in L2; on the random geometric graph (degree 12) it takes
+// 1.8 ms.
 constexpr int32_t IPC_FAR = 0xFFFF;    // unreached / no crossing distance below it
 constexpr int IPC_BINS = 16;
 
@@ -325,7 +328,7 @@ __device__ __forceinline__ int32_t ipc_slot(int32_t* counter) {
 // BFS inside every splitting label from the sources queued at [0, tail) with
 // distance 0.  CROSS: track the crossing distances and stop once every
 // splitting label has one.  nv: vertices of splitting labels.
-template <bool CSR_SM, bool CROSS>
+template <bool CSR_SM, bool CROSS, int NB>
 __device__ void ipc_bfs(const DGraph& g, const IpcRows<CSR_SM>& R, uint32_t* state, uint16_t* queue, uint16_t* list,
                         const IpcLabels& S, IpcShared& sh, int32_t k, int32_t nv, int tile, int64_t davg) {
     const int32_t n = (int32_t)g.n;
@@ -358,13 +361,13 @@ __device__ void ipc_bfs(const DGraph& g, const IpcRows<CSR_SM>& R, uint32_t* sta
                 const uint32_t want = (state[v] & 0xFFFF0000u) | (uint32_t)r;
                 const int64_t end = R.beg(v + 1);
                 bool hit = false;
-                for (int64_t e0 = R.beg(v); e0 < end && !hit; e0 += 32) {
-                    const int64_t e = e0 + lane;
+                for (int64_t e0 = R.beg(v); e0 < end && !hit; e0 += 32 * NB) {
+                    int32_t u[NB];
+#pragma unroll
+                    for (int b = 0; b < NB; ++b) { const int64_t e = e0 + 32 * b + lane; u[b] = e < end ? R.id(e) : -1; }
                     bool f = false;
-                    if (e < end) {
-                        const int32_t u = R.id(e);
-                        f = GP_IN(u, n) && state[u] == want;
-                    }
+#pragma unroll
+                    for (int b = 0; b < NB; ++b) f = f || (u[b] >= 0 && GP_IN(u[b], n) && state[u[b]] == want);
                     hit = __any_sync(0xffffffffu, f);
                 }
                 if (hit && lane == 0) {
@@ -383,10 +386,15 @@ __device__ void ipc_bfs(const DGraph& g, const IpcRows<CSR_SM>& R, uint32_t* sta
                 }
                 const uint32_t open = lab | (uint32_t)IPC_FAR;
                 const int64_t end = R.beg(v + 1);
-                for (int64_t e = R.beg(v) + tl; e < end; e += tile) {
-                    const int32_t u = R.id(e);
-                    if (GP_IN(u, n) && state[u] == open && atomicCAS(&state[u], open, lab | (uint32_t)(r + 1)) == open)
-                        queue[ipc_slot(&sh.tail)] = (uint16_t)u;
+                for (int64_t e0 = R.beg(v) + tl; e0 < end; e0 += (int64_t)NB * tile) {
+                    int32_t u[NB];
+#pragma unroll
+                    for (int b = 0; b < NB; ++b) { const int64_t e = e0 + b * tile; u[b] = e < end ? R.id(e) : -1; }
+#pragma unroll
+                    for (int b = 0; b < NB; ++b)
+                        if (u[b] >= 0 && GP_IN(u[b], n) && state[u[b]] == open &&
+                            atomicCAS(&state[u[b]], open, lab | (uint32_t)(r + 1)) == open)
+                            queue[ipc_slot(&sh.tail)] = (uint16_t)u[b];
                 }
             }
         }
@@ -409,10 +417,10 @@ __device__ void ipc_bfs(const DGraph& g, const IpcRows<CSR_SM>& R, uint32_t* sta
 }
 
 // one trial per CTA; shared memory: ipc_smem(n, m, k, CSR_SM, lists on chip)
-template <bool CSR_SM>
+template <bool CSR_SM, int NB>
 __global__ void __launch_bounds__(IP_T) k_initpart_chip(DGraph g, int32_t k, uint64_t seed, int32_t* __restrict__ labels,
                                                         uint16_t* __restrict__ lists, int64_t* __restrict__ tcut,
-                                                        int64_t* __restrict__ tmaxpw, int tile) {
+                                                        int64_t* __restrict__ tmaxpw, int tile, int cut) {
     extern __shared__ __align__(16) unsigned char ipc_raw[];
     __shared__ IpcShared sh;
     const int32_t n = (int32_t)g.n;
@@ -509,7 +517,7 @@ __global__ void __launch_bounds__(IP_T) k_initpart_chip(DGraph g, int32_t k, uin
                 queue[atomicAdd(&sh.tail, 1)] = (uint16_t)v;
             }
         __syncthreads();
-        ipc_bfs<CSR_SM, false>(g, R, state, queue, list, S, sh, k, nv, tile, davg);
+        ipc_bfs<CSR_SM, false, NB>(g, R, state, queue, list, S, sh, k, nv, tile, davg);
         // pseudo-peripheral vertex: largest distance, smallest id
         const int32_t reached = sh.tail;
         for (int32_t i0 = threadIdx.x & ~31; i0 < reached; i0 += blockDim.x) {
@@ -532,7 +540,7 @@ __global__ void __launch_bounds__(IP_T) k_initpart_chip(DGraph g, int32_t k, uin
                 atomicAdd(&sh.nact, 1);
             }
         __syncthreads();
-        ipc_bfs<CSR_SM, true>(g, R, state, queue, list, S, sh, k, nv, tile, davg);
+        ipc_bfs<CSR_SM, true, NB>(g, R, state, queue, list, S, sh, k, nv, tile, davg);
         for (int32_t q = threadIdx.x; q < k; q += blockDim.x)
             if (S.cnt_d[q] > 1 && S.crit[q] < 0) S.crit[q] = IPC_FAR;   // its component ended below the target
         __syncthreads();
@@ -597,10 +605,10 @@ __global__ void __launch_bounds__(IP_T) k_initpart_chip(DGraph g, int32_t k, uin
         }
         __syncthreads();
     }
-    // the trial's cut and heaviest part
+    // the trial's cut (cut: 0: k_trial_cuts adds it up) and heaviest part
     int64_t cross = 0;
     const int tl = threadIdx.x & (tile - 1);
-    for (int32_t v = threadIdx.x / tile; v < n; v += blockDim.x / tile) {
+    for (int32_t v = cut ? threadIdx.x / tile : n; v < n; v += blockDim.x / tile) {
         const uint32_t pv = state[v] >> 16;
         const int64_t end = R.beg(v + 1);
         for (int64_t e = R.beg(v) + tl; e < end; e += tile) {
@@ -619,14 +627,83 @@ __global__ void __launch_bounds__(IP_T) k_initpart_chip(DGraph g, int32_t k, uin
     if (threadIdx.x == 0) {
         int64_t s = 0;
         for (int i = 0; i < nwarp; ++i) { s += sh.red[i]; mp = s_mp[i] > mp ? s_mp[i] : mp; }
-        tcut[t] = s / 2;
+        tcut[t] = s;
         tmaxpw[t] = mp;
     }
     for (int32_t v = threadIdx.x; v < n; v += blockDim.x) labels[(int64_t)t * n + v] = (int32_t)(state[v] >> 16);
 }
 
+// Directed cross weights of 16 trials (blockIdx.y) over the rows of blockIdx.x's
+// warps: the trials' labels lie in shared memory 16 to a vertex (LT: uint8 for k
+// <= 256, else uint16), so an entry and its weight are read once for all of them
+// and its neighbour's labels are one or two 16-byte loads.  Inside the trial's own
+// block the sweep read every entry per trial, one in flight per lane, on 64 of 148
+// SMs: about 0.9 of the 3.5 ms of 64 trials on R-MAT's coarsest graph (1,999
+// vertices, 2.7 M entries), here 87 us.
+constexpr int TC_G = 16;
+template <class LT>
+__global__ void __launch_bounds__(512) k_trial_cuts(DGraph g, int32_t T, const int32_t* __restrict__ labels,
+                                                    unsigned long long* __restrict__ tcut) {
+    extern __shared__ __align__(16) unsigned char tc_raw[];
+    constexpr int NV = TC_G * sizeof(LT) / 16;   // 16-byte words per vertex
+    constexpr int PW = 4 / sizeof(LT);           // labels per 32-bit word
+    __shared__ uint32_t s_sum[TC_G];
+    LT* lab = (LT*)tc_raw;
+    const int32_t n = (int32_t)g.n, t0 = blockIdx.y * TC_G;
+    if (threadIdx.x < TC_G) s_sum[threadIdx.x] = 0;
+    for (int t = 0; t < TC_G; ++t)
+        for (int32_t v = threadIdx.x; v < n; v += blockDim.x)
+            lab[(int64_t)v * TC_G + t] = t0 + t < T ? (LT)labels[(int64_t)(t0 + t) * n + v] : (LT)0;
+    __syncthreads();
+    const uint4* lv = (const uint4*)lab;
+    const int lane = threadIdx.x & 31;
+    uint32_t acc[TC_G];   // the weights of all entries add up to less than 2^32
+#pragma unroll
+    for (int t = 0; t < TC_G; ++t) acc[t] = 0;
+    const int32_t nw = (int32_t)(gridDim.x * blockDim.x) >> 5;
+    for (int32_t v = (int32_t)(blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < n; v += nw) {
+        uint4 mine[NV];
+#pragma unroll
+        for (int i = 0; i < NV; ++i) mine[i] = lv[(int64_t)v * NV + i];
+        const int64_t end = g.rp[v + 1];
+        for (int64_t e0 = g.rp[v] + lane; e0 < end; e0 += 128) {
+            int32_t u[4];
+            uint32_t w[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int64_t e = e0 + 32 * c;
+                u[c] = e < end ? __ldg(&g.ci[e]) : -1;
+                w[c] = e < end ? (g.ew ? (uint32_t)__ldg(&g.ew[e]) : 1u) : 0u;
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                if (u[c] < 0 || !GP_IN(u[c], n)) continue;
+#pragma unroll
+                for (int i = 0; i < NV; ++i) {
+                    const uint4 o = lv[(int64_t)u[c] * NV + i];
+                    const uint32_t x[4] = {o.x ^ mine[i].x, o.y ^ mine[i].y, o.z ^ mine[i].z, o.w ^ mine[i].w};
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+#pragma unroll
+                        for (int b = 0; b < PW; ++b)
+                            acc[(i * 4 + q) * PW + b] += ((x[q] >> (8 * sizeof(LT) * b)) & (LT)~(LT)0) ? w[c] : 0u;
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < TC_G; ++t) {
+        const uint32_t x = __reduce_add_sync(0xffffffffu, acc[t]);
+        if (lane == 0 && x) atomicAdd(&s_sum[t], x);
+    }
+    __syncthreads();
+    if (threadIdx.x < TC_G && t0 + (int)threadIdx.x < T && s_sum[threadIdx.x])
+        atomicAdd(&tcut[t0 + threadIdx.x], (unsigned long long)s_sum[threadIdx.x]);
+}
+
 // the kept trial: balanced before not, then (not balanced) the smaller heaviest
-// part, then the lower cut, then the lower trial; one warp
+// part, then the lower cut, then the lower trial; one warp.  tcut: directed cross
+// weights
 __global__ void k_pick_trial(int T, const int64_t* __restrict__ tcut, const int64_t* __restrict__ tmaxpw, int64_t Lmax,
                              int64_t* __restrict__ best) {
     const int lane = threadIdx.x & 31;
@@ -635,7 +712,7 @@ __global__ void k_pick_trial(int T, const int64_t* __restrict__ tcut, const int6
     auto take = [&](int64_t a2, int64_t b2, int t2) {
         if (a2 < a || (a2 == a && (b2 < b || (b2 == b && t2 < bt)))) { a = a2; b = b2; bt = t2; }
     };
-    for (int t = lane; t < T; t += 32) take(tmaxpw[t] > Lmax ? tmaxpw[t] : Lmax, tcut[t], t);
+    for (int t = lane; t < T; t += 32) take(tmaxpw[t] > Lmax ? tmaxpw[t] : Lmax, tcut[t] / 2, t);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const int64_t a2 = __shfl_xor_sync(0xffffffffu, a, o), b2 = __shfl_xor_sync(0xffffffffu, b, o);
@@ -652,6 +729,10 @@ static int bits_for64(int64_t x) {
 }
 
 size_t initpart_smem_max();
+
+// entries from which the trials' cuts are added up by k_trial_cuts (a launch of
+// 5 us and more; one trial's own sweep is about 0.3 us per 1000 entries)
+constexpr int64_t kTrialCuts = 65536;
 
 int initial_partition(Ctx& c, const Level& L, const Params& P, int32_t* part_out) {
     const int64_t n = L.g.n, m = L.g.m;
@@ -675,11 +756,19 @@ int initial_partition(Ctx& c, const Level& L, const Params& P, int32_t* part_out
         const int tile = davg <= 8 ? 8 : (davg <= 16 ? 16 : 32);
         const int threads = (n <= 4096 && m <= 65536) ? IP_T / 2 : IP_T;
         const size_t smem = chip + (lists_on ? lists : 0) + (csr_on ? csr : 0);
-        if (csr_on)
-            k_initpart_chip<true><<<T, threads, smem, c.s>>>(L.g, P.k, P.seed, labels, glists, tcut, tmaxpw, tile);
-        else
-            k_initpart_chip<false><<<T, threads, smem, c.s>>>(L.g, P.k, P.seed, labels, glists, tcut, tmaxpw, tile);
+        // cuts of all trials together: rows in L2, labels of 16 trials on chip
+        const size_t lab = (size_t)n * TC_G * (P.k <= 256 ? 1 : 2);
+        const bool cuts = !csr_on && m >= kTrialCuts && lab <= cap;
+        auto kernel = csr_on ? k_initpart_chip<true, 1> : (davg >= 32 ? k_initpart_chip<false, 4> : k_initpart_chip<false, 1>);
+        kernel<<<T, threads, smem, c.s>>>(L.g, P.k, P.seed, labels, glists, tcut, tmaxpw, tile, cuts ? 0 : 1);
         GP_LAUNCHED(c);
+        if (cuts) {
+            const dim3 grid((unsigned)std::max<int64_t>(1, std::min<int64_t>(c.sm_count * TC_G / T + 1, (n + 15) / 16)),
+                            (unsigned)((T + TC_G - 1) / TC_G));
+            (P.k <= 256 ? k_trial_cuts<uint8_t> : k_trial_cuts<uint16_t>)<<<grid, 512, lab, c.s>>>(
+                L.g, T, labels, (unsigned long long*)tcut);
+            GP_LAUNCHED(c);
+        }
     } else {
         int32_t* dists = c.tmp_alloc<int32_t>((int64_t)T * n);
         const size_t base = (size_t)P.k * (9 * sizeof(int64_t) + 3 * sizeof(int32_t));
@@ -711,8 +800,11 @@ void initpart_smem_caps() {
     // static shared memory of the kernel (flags, reductions) stays outside the cap
     const size_t cap = std::max(need, (size_t)optin > 4096 ? (size_t)optin - 4096 : need);
     GP_CUDA(cudaFuncSetAttribute(k_initpart, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
-    GP_CUDA(cudaFuncSetAttribute(k_initpart_chip<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
-    GP_CUDA(cudaFuncSetAttribute(k_initpart_chip<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
+    GP_CUDA(cudaFuncSetAttribute(k_trial_cuts<uint8_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
+    GP_CUDA(cudaFuncSetAttribute(k_trial_cuts<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
+    GP_CUDA(cudaFuncSetAttribute(k_initpart_chip<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
+    GP_CUDA(cudaFuncSetAttribute(k_initpart_chip<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
+    GP_CUDA(cudaFuncSetAttribute(k_initpart_chip<false, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
     g_ip_smem_max = cap;
 }
 
