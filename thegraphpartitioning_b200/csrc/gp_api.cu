@@ -108,52 +108,33 @@ __device__ __forceinline__ void check_entry(int64_t n, int64_t e, int64_t v, int
         finger += (uint32_t)v < (uint32_t)u ? h : 0ull - h;
     }
 }
-// entries of a row-pointer-checked CSR, entry-sliced (csr_row_of /
-// csr_window_lane), eight groups of 32 entries loaded together
-__global__ void k_check_rows(int64_t n, int64_t m, int64_t slice, const int64_t* __restrict__ rp,
+// entries of a row-pointer-checked CSR, entry-sliced (csr_sweep), up to eight
+// groups of 32 entries loaded together
+constexpr int kCheckG = 6;
+__global__ void __launch_bounds__(256, 4) k_check_rows(int64_t n, int64_t m, int64_t slice, const int64_t* __restrict__ rp,
                              const int32_t* __restrict__ ci,
                              const int32_t* __restrict__ ew, int check, unsigned long long* err, int64_t* sums) {
     const int lane = threadIdx.x & 31;
-    const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const int64_t nslice = (m + slice - 1) / slice;
     int64_t local = 0;
     uint64_t finger = 0;
-    for (int64_t sl = wid; sl < nslice; sl += nw) {
-        const int64_t o0 = sl * slice, o1 = o0 + slice < m ? o0 + slice : m;
-        int64_t cb = csr_row_of(rp, n, o0), s = 0, wend = 0;
-        auto window = [&]() {
-            s = cb + lane < n ? rp[cb + lane] : m;
-            wend = rp[cb + 32 < n ? cb + 32 : n];
-        };
-        window();
-        int64_t o = o0;
-        while (o < o1) {
-            const int64_t lim = o1 < wend ? o1 : wend;
-            if (o + 256 <= lim) {
-                int32_t u[8], w[8];
-                int64_t v[8];
+    csr_sweep<kCheckG, int>(rp, n, m, slice, [](int64_t, int64_t) { return 0; },
+                   [&](auto full, int64_t o, int64_t lim, int64_t o0, int64_t cb, int32_t s, int) {
+        int32_t u[kCheckG], w[kCheckG], v[kCheckG];
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const int64_t oi = o + 32 * q + lane;
-                    v[q] = cb + csr_window_lane(s, oi);
-                    u[q] = check >= 1 ? __ldcs(&ci[oi]) : 0;
-                    w[q] = ew ? __ldcs(&ew[oi]) : 1;
-                }
-#pragma unroll
-                for (int q = 0; q < 8; ++q) check_entry(n, o + 32 * q + lane, v[q], u[q], w[q], check, err, local, finger);
-                o += 256;
-            } else if (o < lim) {
-                const int64_t oi = o + lane;
-                const int64_t v = cb + csr_window_lane(s, oi);
-                if (oi < lim) check_entry(n, oi, v, check >= 1 ? ci[oi] : 0, ew ? ew[oi] : 1, check, err, local, finger);
-                o = o + 32 < lim ? o + 32 : lim;
-            } else {
-                cb += 32;   // o >= wend: o lies in a later row
-                window();
-            }
+        for (int q = 0; q < kCheckG; ++q) {
+            if (!full && o + 32 * q >= lim) break;
+            const int64_t oi = o + 32 * q + lane;
+            v[q] = (int32_t)(cb + csr_lane(s, (int32_t)(oi - o0)));
+            u[q] = (full || oi < lim) && check >= 1 ? __ldcs(&ci[oi]) : 0;
+            w[q] = (full || oi < lim) && ew ? __ldcs(&ew[oi]) : 1;
         }
-    }
+#pragma unroll
+        for (int q = 0; q < kCheckG; ++q) {
+            if (!full && o + 32 * q >= lim) break;
+            const int64_t oi = o + 32 * q + lane;
+            if (full || oi < lim) check_entry(n, oi, v[q], u[q], w[q], check, err, local, finger);
+        }
+    });
     for (int o = 16; o > 0; o >>= 1) {
         local += __shfl_xor_sync(0xffffffffu, local, o);
         finger += __shfl_xor_sync(0xffffffffu, finger, o);

@@ -1619,63 +1619,31 @@ __global__ void k_td_rows(const int32_t* __restrict__ list, int64_t n, const int
 
 // warp per coarse row: temporary (walk-bound offsets) -> final CSR
 // Packs every row's deduplicated entries (crp[c + 1] - crp[c] of them at
-// walk offset off[c] of tci / tew) into the coarse CSR.  The output is cut
-// into slices of `slice` entries (csr_slice), one warp each: the warp finds the row
-// holding its first entry by binary search over crp, then keeps a window of
-// 32 consecutive rows (start and source offset, one row per lane); the row of
-// an output position is the last window row starting at or before it (five
-// shuffle steps).  Eight groups of 32 entries are loaded before any is stored.
-__device__ __forceinline__ int64_t cp_source(int64_t oi, int64_t s, int64_t src) {
-    const int l = csr_window_lane(s, oi);
-    return __shfl_sync(0xffffffffu, src, l) + (oi - __shfl_sync(0xffffffffu, s, l));
-}
+// walk offset off[c] of tci / tew) into the coarse CSR, entry-sliced (csr_sweep);
+// up to eight groups of 32 entries are loaded before any is stored.
 __global__ void __launch_bounds__(256) k_contract_copy(int64_t nc, int64_t cm, int64_t slice,
                                                        const int64_t* __restrict__ off,
                                                        const int64_t* __restrict__ crp, const int32_t* __restrict__ tci,
                                                        const int32_t* __restrict__ tew, int32_t* __restrict__ ci,
                                                        int32_t* __restrict__ ew) {
     const int lane = threadIdx.x & 31;
-    const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const int64_t nslice = (cm + slice - 1) / slice;
-    for (int64_t sl = wid; sl < nslice; sl += nw) {
-        const int64_t o0 = sl * slice, o1 = o0 + slice < cm ? o0 + slice : cm;
-        int64_t cb = csr_row_of(crp, nc, o0), s = 0, src = 0, wend = 0;
-        auto window = [&]() {   // rows cb .. cb + 31; wend = first output entry past them
-            const int64_t r = cb + lane;
-            s = r < nc ? crp[r] : cm;
-            src = r < nc ? off[r] : 0;
-            wend = crp[cb + 32 < nc ? cb + 32 : nc];
-        };
-        window();
-        int64_t o = o0;
-        while (o < o1) {
-            const int64_t lim = o1 < wend ? o1 : wend;
-            if (o + 256 <= lim) {
-                int32_t a[8], b[8];
+    // payload: source of output entry 0 as seen from the row
+    csr_sweep<8, int64_t>(crp, nc, cm, slice, [&](int64_t r, int64_t start) { return r < nc ? off[r] - start : 0; },
+                       [&](auto full, int64_t o, int64_t lim, int64_t o0, int64_t, int32_t s, int64_t src) {
+        int32_t a[8], b[8];
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const int64_t p = cp_source(o + 32 * q + lane, s, src);
-                    a[q] = __ldcs(&tci[p]);
-                    b[q] = __ldcs(&tew[p]);
-                }
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    ci[o + 32 * q + lane] = a[q];
-                    ew[o + 32 * q + lane] = b[q];
-                }
-                o += 256;
-            } else if (o < lim) {
-                const int64_t oi = o + lane;
-                const int64_t p = cp_source(oi, s, src);
-                if (oi < lim) { ci[oi] = tci[p]; ew[oi] = tew[p]; }
-                o = o + 32 < lim ? o + 32 : lim;
-            } else {
-                cb += 32;   // o >= wend: o lies in a later row
-                window();
-            }
+        for (int q = 0; q < 8; ++q) {
+            if (!full && o + 32 * q >= lim) break;
+            const int64_t oi = o + 32 * q + lane;
+            const int64_t p = __shfl_sync(0xffffffffu, src, csr_lane(s, (int32_t)(oi - o0))) + oi;
+            if (full || oi < lim) { a[q] = __ldcs(&tci[p]); b[q] = __ldcs(&tew[p]); }
         }
-    }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int64_t oi = o + 32 * q + lane;
+            if (full || oi < lim) { ci[oi] = a[q]; ew[oi] = b[q]; }
+        }
+    });
 }
 
 void contract_level(Ctx& c, Level& fine, Level& coarse, const int32_t* match, int64_t pairs) {

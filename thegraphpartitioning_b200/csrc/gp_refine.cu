@@ -1527,60 +1527,37 @@ __global__ void k_part_weights(int64_t n, const int32_t* __restrict__ part, cons
     }
 }
 
-// warp per row: directed cross weight (d_cross2 accumulates 2*cut)
-// directed cross weight, entry-sliced (csr_row_of / csr_window_lane): each
-// lane of a window also holds its row's part; eight groups of 32 entries have
-// their column ids loaded, then their neighbours' parts gathered, together
-__global__ void __launch_bounds__(RT) k_cut(DGraph g, int64_t slice, const int32_t* __restrict__ part,
+// directed cross weight, entry-sliced (csr_sweep): each lane of a window also
+// holds its row's part; up to eight groups of 32 entries have their column ids
+// loaded, then their neighbours' parts gathered, together.  PT: part ids of 1
+// byte where a compacted copy pays (kCutCompact), else the caller's int32
+constexpr int kCutG = 4;
+template <class PT>
+__global__ void __launch_bounds__(RT, 6) k_cut(DGraph g, int64_t slice, const PT* __restrict__ part,
                                             int64_t* __restrict__ cross2) {
     __shared__ int64_t s_red[RW];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int64_t wid = ((int64_t)blockIdx.x * RT + threadIdx.x) >> 5;
-    const int64_t nw = ((int64_t)gridDim.x * RT) >> 5;
-    const int64_t n = g.n, m = g.m, nslice = (m + slice - 1) / slice;
+    const int64_t n = g.n;
     int64_t acc = 0;
-    for (int64_t sl = wid; sl < nslice; sl += nw) {
-        const int64_t o0 = sl * slice, o1 = o0 + slice < m ? o0 + slice : m;
-        int64_t cb = csr_row_of(g.rp, n, o0), s = 0, wend = 0;
-        int32_t pv = 0;
-        auto window = [&]() {
-            const int64_t r = cb + lane;
-            s = r < n ? g.rp[r] : m;
-            pv = r < n ? part[r] : 0;
-            wend = g.rp[cb + 32 < n ? cb + 32 : n];
-        };
-        window();
-        int64_t o = o0;
-        while (o < o1) {
-            const int64_t lim = o1 < wend ? o1 : wend;
-            if (o + 256 <= lim) {
-                int32_t u[8], pr[8], wt[8];
+    csr_sweep<kCutG, int32_t>(g.rp, n, g.m, slice, [&](int64_t r, int64_t) { return r < n ? (int32_t)part[r] : 0; },
+                       [&](auto full, int64_t o, int64_t lim, int64_t o0, int64_t, int32_t s, int32_t pv) {
+        int32_t u[kCutG], pr[kCutG], wt[kCutG];
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const int64_t oi = o + 32 * q + lane;
-                    pr[q] = __shfl_sync(0xffffffffu, pv, csr_window_lane(s, oi));
-                    u[q] = __ldcs(&g.ci[oi]);
-                    wt[q] = g.ew ? __ldcs(&g.ew[oi]) : 1;
-                }
-#pragma unroll
-                for (int q = 0; q < 8; ++q) u[q] = GP_IN(u[q], n) ? part[u[q]] : pr[q];
-#pragma unroll
-                for (int q = 0; q < 8; ++q) acc += u[q] != pr[q] ? wt[q] : 0;
-                o += 256;
-            } else if (o < lim) {
-                const int64_t oi = o + lane;
-                const int32_t p = __shfl_sync(0xffffffffu, pv, csr_window_lane(s, oi));
-                if (oi < lim) {
-                    const int32_t u = __ldcs(&g.ci[oi]);
-                    if (GP_IN(u, n) && part[u] != p) acc += g.ew ? __ldcs(&g.ew[oi]) : 1;
-                }
-                o = o + 32 < lim ? o + 32 : lim;
-            } else {
-                cb += 32;   // o >= wend: o lies in a later row
-                window();
+        for (int q = 0; q < kCutG; ++q) {
+            u[q] = -1; pr[q] = 0; wt[q] = 0;
+            if (!full && o + 32 * q >= lim) continue;
+            const int64_t oi = o + 32 * q + lane;
+            pr[q] = __shfl_sync(0xffffffffu, pv, csr_lane(s, (int32_t)(oi - o0)));
+            if (full || oi < lim) {
+                u[q] = __ldcs(&g.ci[oi]);
+                wt[q] = g.ew ? __ldcs(&g.ew[oi]) : 1;
             }
         }
-    }
+#pragma unroll
+        for (int q = 0; q < kCutG; ++q) u[q] = u[q] >= 0 && GP_IN(u[q], n) ? (int32_t)__ldg(&part[u[q]]) : pr[q];
+#pragma unroll
+        for (int q = 0; q < kCutG; ++q) acc += u[q] != pr[q] ? wt[q] : 0;
+    });
     acc = warp_sum(acc);
     if (lane == 0) s_red[w] = acc;
     __syncthreads();
@@ -1604,12 +1581,33 @@ void part_weights(Ctx& c, const DGraph& g, const int32_t* part, int32_t k, int64
     c.bytes += 4 * g.n + (g.vw ? 4 * g.n : 0);
 }
 
+// entries from which the cut gathers from a copy of the parts in bytes, on graphs
+// of a mean degree of 8 and more (the copy costs 5 bytes a vertex): R-MAT 22, 4.2 M
+// vertices, 128 M entries, 592 us from int32, 568 from bytes, the copy included
+constexpr int64_t kCutCompact = 1 << 20;
+__global__ void k_compact_part(int64_t n, const int32_t* __restrict__ part, void* pc, int pcb);
 void cut_and_weights(Ctx& c, const DGraph& g, const int32_t* part, int32_t k, int64_t* d_cross2, int64_t* d_pw) {
     memset_async(c, d_cross2, 0, sizeof(int64_t));
     const int64_t slice = csr_slice(g.m, c.sm_count);
-    k_cut<<<grid_for((g.m + slice - 1) / slice * 32, RT, c.sm_count * c.ctas_per_sm), RT, 0, c.s>>>(g, slice, part,
-                                                                                                   d_cross2);
+    const int grid = grid_for((g.m + slice - 1) / slice * 32, RT, c.sm_count * c.ctas_per_sm);
+    uint8_t* pc = nullptr;
+    auto mk = c.tmp->save();
+    if (k <= 256 && g.m >= kCutCompact && g.m >= 8 * g.n) {
+        try {
+            pc = c.tmp_alloc<uint8_t>(g.n);
+        } catch (const GpError&) {   // no memory for it: the caller's array serves
+            cudaGetLastError();
+        }
+    }
+    if (pc) {
+        k_compact_part<<<grid_for(g.n, 256), 256, 0, c.s>>>(g.n, part, pc, 1);
+        GP_LAUNCHED(c);
+        k_cut<uint8_t><<<grid, RT, 0, c.s>>>(g, slice, pc, d_cross2);
+    } else {
+        k_cut<int32_t><<<grid, RT, 0, c.s>>>(g, slice, part, d_cross2);
+    }
     GP_LAUNCHED(c);
+    c.tmp->restore(mk);
     c.bytes += 8 * (g.n + 1) + 8 * g.m + (g.ew ? 4 * g.m : 0) + 4 * g.n;
     if (d_pw) part_weights(c, g, part, k, d_pw);
 }
