@@ -715,14 +715,16 @@ __global__ void __launch_bounds__(256) k_gnn_edge_bwd(GnnRows R, const __nv_bflo
                                float* __restrict__ grad, double* __restrict__ loss) {
     __shared__ float sA[ZD];
     __shared__ float sc[4];
-    __shared__ float sg[ZD + 5];
+    __shared__ float sg[ZD + 4];
+    __shared__ double s_ls[8];   // 256 threads
     if (threadIdx.x < ZD) sA[threadIdx.x] = wload(w, O_A + threadIdx.x);
     if (threadIdx.x < 4) sc[threadIdx.x] = wload(w, O_BETA + threadIdx.x);
-    if (threadIdx.x < ZD + 5) sg[threadIdx.x] = 0.f;
+    if (threadIdx.x < ZD + 4) sg[threadIdx.x] = 0.f;
     __syncthreads();
     const DGraph& g = R.g;
     const int lane = threadIdx.x & 31;
-    float gA[ZD] = {0.f, 0.f, 0.f, 0.f}, gb = 0.f, gg = 0.f, gd = 0.f, ge = 0.f, ls = 0.f;
+    float gA[ZD] = {0.f, 0.f, 0.f, 0.f}, gb = 0.f, gg = 0.f, gd = 0.f, ge = 0.f;
+    double ls = 0.;   // the loss's terms add up in 64 bits
     float zv[ZD], wdv = 0.f;
     auto pre = [&](int64_t v) {
         const float4 q = reinterpret_cast<const float4*>(z)[v];
@@ -737,7 +739,7 @@ __global__ void __launch_bounds__(256) k_gnn_edge_bwd(GnnRows R, const __nv_bflo
         const float y = label[e] ? 1.f : 0.f;
         const float s = 1.f / (1.f + expf(-t));
         // BCE with logits, stable form
-        ls += (fmaxf(t, 0.f) - t * y + log1pf(expf(-fabsf(t)))) * inv_e;
+        ls += (double)(fmaxf(t, 0.f) - t * y + log1pf(expf(-fabsf(t))));
         const float dt = (s - y) * inv_e;
         const float4 q = reinterpret_cast<const float4*>(z)[u];
         const float zu[ZD] = {q.x, q.y, q.z, q.w};
@@ -755,17 +757,25 @@ __global__ void __launch_bounds__(256) k_gnn_edge_bwd(GnnRows R, const __nv_bflo
         reinterpret_cast<float4*>(dz)[v] = make_float4(dzv[0], dzv[1], dzv[2], dzv[3]);
     };
     rows_bwd<ZD>(R, pre, body, fin);
-    float part[ZD + 5] = {gA[0], gA[1], gA[2], gA[3], gb, gg, gd, ls, ge};
-    warp_reduce_vec<ZD + 5>(part);
-    if (lane == 0)
-        for (int j = 0; j < ZD + 5; ++j) atomicAdd(&sg[j], part[j]);
+    float part[ZD + 4] = {gA[0], gA[1], gA[2], gA[3], gb, gg, gd, ge};
+    warp_reduce_vec<ZD + 4>(part);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ls += __shfl_xor_sync(0xffffffffu, ls, o);
+    if (lane == 0) {
+        for (int j = 0; j < ZD + 4; ++j) atomicAdd(&sg[j], part[j]);
+        s_ls[threadIdx.x >> 5] = ls;
+    }
     __syncthreads();
     if (threadIdx.x < ZD) atomicAdd(&grad[O_A + threadIdx.x], sg[threadIdx.x]);
     if (threadIdx.x == ZD) atomicAdd(&grad[O_BETA], sg[ZD]);
     if (threadIdx.x == ZD + 1) atomicAdd(&grad[O_GAMMA], sg[ZD + 1]);
     if (threadIdx.x == ZD + 2) atomicAdd(&grad[O_DELTA], sg[ZD + 2]);
-    if (threadIdx.x == ZD + 3) atomicAdd(loss, (double)sg[ZD + 3]);   // the blocks' sums in 64 bits
-    if (threadIdx.x == ZD + 4) atomicAdd(&grad[O_ETA], sg[ZD + 4]);
+    if (threadIdx.x == ZD + 3) atomicAdd(&grad[O_ETA], sg[ZD + 3]);
+    if (threadIdx.x == ZD + 4) {
+        double x = 0.;
+        for (int i = 0; i < 8; ++i) x += s_ls[i];
+        if (x != 0.) atomicAdd(loss, x / (double)g.m);
+    }
 }
 
 // dpre2 = (Z^T dz) * [h2 > 0]; dh1 (direct part) and dc from W2^T dpre2; thread per vertex
