@@ -1318,7 +1318,7 @@ __global__ void k_rb_strong_apply(int64_t cnt, const uint64_t* __restrict__ keys
 // for no move in, and a pass that would end the level sweeps nothing: on the
 // 256^3 grid (k = 32) the rebalancing passes, two thirds of all, sweep one part in
 // 32 instead of every row: all its passes take 47 -> 32 ms, k_track 2.8 ms; on
-// R-MAT 24 they take 119 -> 102 ms, k_track 13.  Left out when the next pass sweeps
+// R-MAT 24 they take 116 -> 101 ms, k_track 13.  Left out when the next pass sweeps
 // every row anyway: no overweight part and a level that may go on, or moved rows
 // of more than track_deg entries.  Blocks [0, nitems) take the pieces of the heavy
 // rows, range_blocks the warp rows by the connectivity pass's ranges (block_unit:
@@ -1335,7 +1335,6 @@ struct TrackArgs {
     const void* pc_old;         // before it
     int64_t* step;              // its status block
     int64_t track_deg;
-    void* pair;                 // PartPair[n], filled by k_track_pairs
     const int32_t* bucket[3];
     int64_t nbucket[3];
     const int64_t* wfirst;      // the connectivity pass's ranges of longer rows
@@ -1349,18 +1348,10 @@ struct TrackArgs {
     int64_t nitems;
 };
 constexpr int kTrackRange = 8192;
-// Part before and after the step: two gathers, or one where the moved rows have
-// enough entries (a quarter of the vertices) to pay for k_track_pairs, which
-// puts both into one word per vertex (R-MAT 24: k_track 17.0 -> 13.1 ms in all;
-// on meshes, where few vertices move, the pass over the vertices would cost more
-// than the gathers: 256^3 grid 3.3 ms for 164 steps).
-template <class PT> struct PartPair;
-template <> struct PartPair<uint8_t> { using T = uint16_t; };
-template <> struct PartPair<uint16_t> { using T = uint32_t; };
-__device__ __forceinline__ bool track_packed(const TrackArgs& T) { return 4 * T.step[S_MVDEG] >= T.g.n; }
+// part of u before and after the step (both in one word per vertex, filled by a
+// kernel of its own, measured the same on R-MAT 24: 13.2 + 0.4 ms against 12.7)
 template <class PT>
-__device__ __forceinline__ uint32_t track_pair(const TrackArgs& T, bool packed, int32_t u) {
-    if (packed) return (uint32_t)__ldg((const typename PartPair<PT>::T*)T.pair + u);
+__device__ __forceinline__ uint32_t track_pair(const TrackArgs& T, int32_t u) {
     return (uint32_t)__ldg((const PT*)T.pc_old + u) | ((uint32_t)__ldg((const PT*)T.pc + u) << (8 * sizeof(PT)));
 }
 __device__ __forceinline__ bool track_runs(const TrackArgs& T) {
@@ -1370,14 +1361,6 @@ __device__ __forceinline__ bool track_runs(const TrackArgs& T) {
     return __syncthreads_or(over) || T.always;
 }
 template <class PT>
-__global__ void __launch_bounds__(RT) k_track_pairs(TrackArgs T) {
-    if (!track_packed(T) || !track_runs(T)) return;
-    using QT = typename PartPair<PT>::T;
-    QT* pair = (QT*)T.pair;
-    for (int64_t v = (int64_t)blockIdx.x * RT + threadIdx.x; v < T.g.n; v += (int64_t)gridDim.x * RT)
-        pair[v] = (QT)(((const PT*)T.pc_old)[v] | ((QT)((const PT*)T.pc)[v] << (8 * sizeof(PT))));
-}
-template <class PT>
 __device__ __forceinline__ int32_t track_change(uint32_t x, int32_t po, int32_t pn, int32_t w) {
     const int32_t uo = (int32_t)(x & (PT)~(PT)0), un = (int32_t)(x >> (8 * sizeof(PT)));
     const int32_t c = (pn != un ? 1 : 0) - (po != uo ? 1 : 0);
@@ -1385,7 +1368,7 @@ __device__ __forceinline__ int32_t track_change(uint32_t x, int32_t po, int32_t 
 }
 // this thread's part (t of nt) of entries [beg, end), four consecutive ones at a time
 template <class PT>
-__device__ __forceinline__ int64_t track_sum(const TrackArgs& T, bool packed, int64_t beg, int64_t end, int t, int nt,
+__device__ __forceinline__ int64_t track_sum(const TrackArgs& T, int64_t beg, int64_t end, int t, int nt,
                                              int32_t po, int32_t pn) {
     const bool v4 = aligned16(T.g.ci) && aligned16(T.g.ew);
     int64_t sum = 0;
@@ -1400,7 +1383,7 @@ __device__ __forceinline__ int64_t track_sum(const TrackArgs& T, bool packed, in
             for (int c = 0; c < 4; ++c) w[c] = 1;
         }
 #pragma unroll
-        for (int c = 0; c < 4; ++c) x[c] = u[c] >= 0 && GP_IN(u[c], T.g.n) ? track_pair<PT>(T, packed, u[c]) : 0u;
+        for (int c = 0; c < 4; ++c) x[c] = u[c] >= 0 && GP_IN(u[c], T.g.n) ? track_pair<PT>(T, u[c]) : 0u;
 #pragma unroll
         for (int c = 0; c < 4; ++c)
             if (u[c] >= 0 && GP_IN(u[c], T.g.n)) sum += track_change<PT>(x[c], po, pn, w[c]);
@@ -1416,13 +1399,12 @@ __global__ void __launch_bounds__(RT) k_track(TrackArgs T) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (threadIdx.x == 0) { s_cnt = 0; s_next = 0; }
     if (!track_runs(T)) return;
-    const bool packed = track_packed(T);
     constexpr int PB = 8 * sizeof(PT);
     int64_t acc = 0;
     if ((int64_t)blockIdx.x < T.nitems) {
-        const uint32_t x = track_pair<PT>(T, packed, T.heavy[T.item_row[blockIdx.x]]);
+        const uint32_t x = track_pair<PT>(T, T.heavy[T.item_row[blockIdx.x]]);
         const int32_t po = (int32_t)(x & (PT)~(PT)0), pn = (int32_t)(x >> PB);
-        if (po != pn) acc = track_sum<PT>(T, packed, T.item_beg[blockIdx.x], T.item_end[blockIdx.x], threadIdx.x, RT, po, pn);
+        if (po != pn) acc = track_sum<PT>(T, T.item_beg[blockIdx.x], T.item_end[blockIdx.x], threadIdx.x, RT, po, pn);
     } else if ((int64_t)blockIdx.x < T.nitems + T.range_blocks) {
         const int64_t U2 = T.nbucket[2], U21 = U2 + T.nbucket[1];
         for (;;) {
@@ -1435,7 +1417,7 @@ __global__ void __launch_bounds__(RT) k_track(TrackArgs T) {
                 int64_t beg = 0, end = 0;
                 if (u < u1) {
                     const int32_t v = u < U2 ? T.bucket[2][u] : T.bucket[1][u - U2];
-                    const uint32_t x = track_pair<PT>(T, packed, v);
+                    const uint32_t x = track_pair<PT>(T, v);
                     po = (int32_t)(x & (PT)~(PT)0); pn = (int32_t)(x >> PB);
                     if (po != pn) { beg = T.g.rp[v]; end = T.g.rp[v + 1]; }
                 }
@@ -1444,7 +1426,7 @@ __global__ void __launch_bounds__(RT) k_track(TrackArgs T) {
                     const int j = __ffs(todo) - 1;
                     todo &= todo - 1;
                     const int64_t b = __shfl_sync(0xffffffffu, beg, j), e = __shfl_sync(0xffffffffu, end, j);
-                    acc += track_sum<PT>(T, packed, b, e, lane, 32, __shfl_sync(0xffffffffu, po, j), __shfl_sync(0xffffffffu, pn, j));
+                    acc += track_sum<PT>(T, b, e, lane, 32, __shfl_sync(0xffffffffu, po, j), __shfl_sync(0xffffffffu, pn, j));
                 }
             }
         }
@@ -1482,12 +1464,12 @@ __global__ void __launch_bounds__(RT) k_track(TrackArgs T) {
             const int32_t v = s_queue[i];
             const int64_t beg = T.g.rp[v], end = T.g.rp[v + 1];
             if (end - beg > kShortDeg) continue;
-            const uint32_t x = track_pair<PT>(T, packed, v);
+            const uint32_t x = track_pair<PT>(T, v);
             const int32_t po = (int32_t)(x & (PT)~(PT)0), pn = (int32_t)(x >> PB);
             for (int64_t e = beg; e < end; ++e) {
                 const int32_t u = __ldcs(&T.g.ci[e]);
                 if (GP_IN(u, T.g.n))
-                    acc += track_change<PT>(track_pair<PT>(T, packed, u), po, pn, T.g.ew ? __ldcs(&T.g.ew[e]) : 1);
+                    acc += track_change<PT>(track_pair<PT>(T, u), po, pn, T.g.ew ? __ldcs(&T.g.ew[e]) : 1);
             }
         }
     }
@@ -2295,8 +2277,8 @@ constexpr int64_t kConnWarpCost = 8 * (8 + 28);
 // theirs would cost more than kConnBlockCost.  With one range per warp on every
 // level R-MAT 20 spent 53% of its warps' time at the end of their blocks, behind
 // the warp with a row of thousands of entries: its 73 passes took 11.1 ms in all
-// against 8.5 (20,000 per block; 10,000: 9.2; 40,000: 8.7), its move steps 1.85
-// against 1.24.  R-MAT 24's take 114 ms with 700,000 per block, 101 with 340,000,
+// against 8.5, its move steps 1.85 against 1.24 (passes, the last of each level
+// skipped: 6.75 ms with 20,000 per block, 7.33 with 10,000, 6.91 with 42,000).  R-MAT 24's take 114 ms with 700,000 per block, 101 with 340,000,
 // 96 with 170,000, 94 with 85,000.
 constexpr int64_t kConnWave = 10;            // blocks per SM, 5 resident
 constexpr int64_t kConnRangeCost = 768;
@@ -2308,7 +2290,7 @@ constexpr int64_t kConnSplitM = 1 << 21;   // entries (a pass of 30 us and more)
 // moved rows' share of the entries up to which the cut's change is tracked: before
 // a pass that looks for moves in the overweight parts (an eighth to a half of the
 // rows) and before one that may be the level's last (R-MAT 24, passes and k_track:
-// 1/16 and 1/4 117 ms, 1/8 and 1/3 115, 1/4 and 1/2 116; 1/32 and never 120)
+// 1/16 and 1/4 117 ms, 1/8 and 1/3 115, 1/4 and 1/2 116)
 constexpr int64_t kTrackShare = 8;
 constexpr int64_t kTrackLast = 3;
 constexpr int64_t kTrackMin = 1 << 22;   // entries from which the cut's change is tracked
@@ -2602,7 +2584,7 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
             track_deg = stop.may ? g.m / kTrackLast : g.m / kTrackShare;
             TrackArgs T;
             T.g = g; T.k = k; T.Lmax = Lmax; T.pw = B.pw; T.pc = B.pc; T.pc_old = B.pc_next; T.step = step_d;
-            T.track_deg = track_deg; T.pair = B.ckeys2; T.heavy = L.heavy; T.item_row = L.item_row;
+            T.track_deg = track_deg; T.heavy = L.heavy; T.item_row = L.item_row;
             T.item_beg = L.item_beg; T.item_end = L.item_end; T.nitems = L.nitems;
             T.range = track_range;
             T.always = stop.may;
@@ -2611,8 +2593,6 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
             T.nranges = long_rows && L.nbucket[1] + L.nbucket[2] > 0 ? nranges : 0;
             T.range_blocks = T.nranges > 0 ? light_blocks : 0;
             const int tg = (int)(L.nitems + T.range_blocks + (n + track_range - 1) / track_range);
-            (B.pcb == 1 ? k_track_pairs<uint8_t> : k_track_pairs<uint16_t>)<<<grid_for(n, 4 * RT), RT, 0, c.s>>>(T);
-            GP_LAUNCHED(c);
             (B.pcb == 1 ? k_track<uint8_t> : k_track<uint16_t>)<<<tg, RT, 0, c.s>>>(T);
             GP_LAUNCHED(c);
         }
