@@ -12,6 +12,7 @@
 
 #include <mutex>
 #include <memory>
+#include <random>
 #include <cstring>
 
 namespace gp {
@@ -88,35 +89,48 @@ __global__ void k_check_rowptr(int64_t n, int64_t m, const int64_t* __restrict__
 
 // one entry: weight >= 1, column id in range, no self loop (the smallest
 // (code, index) reported wins, whatever the order of the checks)
-// and the symmetry fingerprint: the sum over entries of w times a 64-bit hash of
-// the unordered pair, positive for v < u and negative for v > u (mod 2^64).
-// Zero for every symmetric graph; an asymmetric one has weights whose signed
-// sums per pair are not all zero, and a random hash of the pairs then cancels
-// with probability about 2^-64.
+// and the symmetry fingerprint: two sums over the entries, of w times the low and
+// of w times the high half of a 64-bit hash of the unordered pair, positive for
+// v < u and negative for v > u.  The weights add up to less than 2^31 (else the
+// input is refused), so both sums are exact integers.  They are zero for every
+// symmetric graph.  In an asymmetric one some pair's signed weights add up to
+// d != 0; whatever the other pairs add, at most one value of that pair's half hash
+// cancels the sum, in each half: 2^-64 for hashes drawn at random.  They are a
+// bijective mix (degski's, two multiplications) of the pair and a key drawn anew for
+// each call, so no input can be built to cancel (a fixed hash allows that, and with
+// sums mod 2^64 a weight divisible by 2^t leaves only 64 - t bits).
 __device__ __forceinline__ void check_entry(int64_t n, int64_t e, int64_t v, int32_t u, int32_t w, int check,
-                                            unsigned long long* err, int64_t& local, uint64_t& finger) {
+                                            uint64_t key, unsigned long long* err, int64_t& local, int64_t& lo,
+                                            int64_t& hi) {
     if (w < 1) report(err, V_EWGT, e);
     local += w;
     if (check >= 1) {
         if (u < 0 || u >= n) report(err, V_COLIDX, e);
         else if (u == v) report(err, V_SELF, v);
-        const uint32_t a = (uint32_t)v < (uint32_t)u ? (uint32_t)v : (uint32_t)u;
-        const uint32_t b = (uint32_t)v < (uint32_t)u ? (uint32_t)u : (uint32_t)v;
-        uint32_t x = a * 0x9E3779B1u + b * 0x85EBCA77u, y = a * 0xC2B2AE3Du + b * 0x27D4EB2Fu;
-        x ^= x >> 15; y ^= y >> 13;
-        const uint64_t h = ((uint64_t)(x * 0x85EBCA6Bu ^ y) * (y | 1u) + x) * (uint64_t)(uint32_t)w;
-        finger += (uint32_t)v < (uint32_t)u ? h : 0ull - h;
+        const bool up = (uint32_t)v < (uint32_t)u;
+        const uint32_t a = up ? (uint32_t)v : (uint32_t)u, b = up ? (uint32_t)u : (uint32_t)v;
+        uint64_t h = (((uint64_t)a << 32) | b) ^ key;
+        h ^= h >> 32; h *= 0xD6E8FEB86659FD93ull;
+        h ^= h >> 32; h *= 0xD6E8FEB86659FD93ull;
+        h ^= h >> 32;
+        const int32_t sw = up ? w : -w;
+        lo += (int64_t)sw * (int64_t)(uint32_t)h;
+        hi += (int64_t)sw * (int64_t)(uint32_t)(h >> 32);
     }
 }
-// entries of a row-pointer-checked CSR, entry-sliced (csr_sweep), up to eight
-// groups of 32 entries loaded together
+// entries of a row-pointer-checked CSR, entry-sliced (csr_sweep), up to kCheckG
+// groups of 32 entries loaded together.  What bounds it is instructions: row search,
+// hash and sums of every entry.  Three blocks per SM, so that nothing spills (four:
+// 2 to 4 % slower).  1.71 ms for R-MAT 24, 0.53 for the 256^3 grid; Mix13 in place of
+// the shorter mix 1.88 and 0.58, the input check without a fingerprint 1.50 and 0.84
+// (before csr_sweep)
 constexpr int kCheckG = 6;
-__global__ void __launch_bounds__(256, 4) k_check_rows(int64_t n, int64_t m, int64_t slice, const int64_t* __restrict__ rp,
+__global__ void __launch_bounds__(256, 3) k_check_rows(int64_t n, int64_t m, int64_t slice, const int64_t* __restrict__ rp,
                              const int32_t* __restrict__ ci,
-                             const int32_t* __restrict__ ew, int check, unsigned long long* err, int64_t* sums) {
+                             const int32_t* __restrict__ ew, int check, uint64_t key, unsigned long long* err,
+                             int64_t* sums) {
     const int lane = threadIdx.x & 31;
-    int64_t local = 0;
-    uint64_t finger = 0;
+    int64_t local = 0, lo = 0, hi = 0;
     csr_sweep<kCheckG, int>(rp, n, m, slice, [](int64_t, int64_t) { return 0; },
                    [&](auto full, int64_t o, int64_t lim, int64_t o0, int64_t cb, int32_t s, int) {
         int32_t u[kCheckG], w[kCheckG], v[kCheckG];
@@ -132,16 +146,18 @@ __global__ void __launch_bounds__(256, 4) k_check_rows(int64_t n, int64_t m, int
         for (int q = 0; q < kCheckG; ++q) {
             if (!full && o + 32 * q >= lim) break;
             const int64_t oi = o + 32 * q + lane;
-            if (full || oi < lim) check_entry(n, oi, v[q], u[q], w[q], check, err, local, finger);
+            if (full || oi < lim) check_entry(n, oi, v[q], u[q], w[q], check, key, err, local, lo, hi);
         }
     });
     for (int o = 16; o > 0; o >>= 1) {
         local += __shfl_xor_sync(0xffffffffu, local, o);
-        finger += __shfl_xor_sync(0xffffffffu, finger, o);
+        lo += __shfl_xor_sync(0xffffffffu, lo, o);
+        hi += __shfl_xor_sync(0xffffffffu, hi, o);
     }
     if (lane == 0) {
         atomicAdd((unsigned long long*)&sums[1], (unsigned long long)local);
-        atomicAdd((unsigned long long*)&sums[2], (unsigned long long)finger);
+        atomicAdd((unsigned long long*)&sums[2], (unsigned long long)lo);
+        atomicAdd((unsigned long long*)&sums[3], (unsigned long long)hi);
     }
 }
 
@@ -202,9 +218,9 @@ static int bits_for(int64_t x) {
 static int64_t validate(Ctx& c, const DGraph& g, int check, bool& symmetric) {
     auto mk = c.tmp->save();
     unsigned long long* err = (unsigned long long*)c.tmp_alloc<int64_t>(4);
-    int64_t* sums = c.tmp_alloc<int64_t>(3);
+    int64_t* sums = c.tmp_alloc<int64_t>(4);
     GP_CUDA(cudaMemsetAsync(err, 0xff, 8, c.s));
-    memset_async(c, sums, 0, 24);
+    memset_async(c, sums, 0, 32);
     k_check_rowptr<<<grid_for(g.n, 256), 256, 0, c.s>>>(g.n, g.m, g.rp, g.vw, err, sums);
     GP_LAUNCHED(c);
     GP_CUDA(cudaMemcpyAsync(c.h_pinned, err, 8, cudaMemcpyDeviceToHost, c.s));
@@ -212,17 +228,19 @@ static int64_t validate(Ctx& c, const DGraph& g, int check, bool& symmetric) {
     uint64_t e0 = (uint64_t)c.h_pinned[0];
     if (e0 != ~0ull) throw GpError(GP_EINVAL, verr((int)(e0 >> 48), (int64_t)(e0 & ((1ull << 48) - 1))));
     const int64_t slice = csr_slice(g.m, c.sm_count);
+    std::random_device draw;
+    const uint64_t key = ((uint64_t)draw() << 32) | draw();
     k_check_rows<<<grid_for((g.m + slice - 1) / slice * 32, 256, c.sm_count * 8), 256, 0, c.s>>>(
-        g.n, g.m, slice, g.rp, g.ci, g.ew, check, err, sums);
+        g.n, g.m, slice, g.rp, g.ci, g.ew, check, key, err, sums);
     GP_LAUNCHED(c);
     c.bytes += 8 * (g.n + 1) + (g.vw ? 4 * g.n : 0) + (check >= 1 ? 4 * g.m : 0) + (g.ew ? 4 * g.m : 0);
     GP_CUDA(cudaMemcpyAsync(c.h_pinned, err, 8, cudaMemcpyDeviceToHost, c.s));
-    GP_CUDA(cudaMemcpyAsync(c.h_pinned + 1, sums, 24, cudaMemcpyDeviceToHost, c.s));
+    GP_CUDA(cudaMemcpyAsync(c.h_pinned + 1, sums, 32, cudaMemcpyDeviceToHost, c.s));
     c.sync();
     e0 = (uint64_t)c.h_pinned[0];
     if (e0 != ~0ull) throw GpError(GP_EINVAL, verr((int)(e0 >> 48), (int64_t)(e0 & ((1ull << 48) - 1))));
     const int64_t W = c.h_pinned[1], EW = c.h_pinned[2];
-    symmetric = check >= 1 && c.h_pinned[3] == 0;
+    symmetric = check >= 1 && c.h_pinned[3] == 0 && c.h_pinned[4] == 0;
     if (W > INT32_MAX) throw GpError(GP_EINVAL, "sum of vertex weights exceeds int32");
     if (EW > INT32_MAX) throw GpError(GP_EINVAL, "sum of edge weights exceeds int32");
     if (check >= 2 && g.m > 0) {

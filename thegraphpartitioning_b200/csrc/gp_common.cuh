@@ -172,7 +172,7 @@ __device__ __forceinline__ int csr_window_lane(int64_t s, int64_t oi) {
 // oi being that of lane csr_lane(s, oi - o0).  On rows of a few entries a window
 // ends before 256: one group of 32 entries at a time, each behind its window's
 // loads, took 1042 us for the cut of a 256^3 grid, 925 for its input check and
-// 928 for the copy of its first contraction; now 406, 521 and 450.
+// 928 for the copy of its first contraction; now 406, 534 and 450.
 __device__ __forceinline__ int csr_lane(int32_t s, int32_t oi) {
     int l = 0;
 #pragma unroll
