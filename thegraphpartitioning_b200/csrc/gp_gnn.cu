@@ -559,35 +559,39 @@ __global__ void __launch_bounds__(L2_T, 4) k_gnn_l2(int64_t n, const __nv_bfloat
 // signature bit of vertex x (0..127)
 __host__ __device__ __forceinline__ uint32_t nb_bit(int32_t x) { return fmix32((uint32_t)x * 0x9E3779B1u) >> 25; }
 
-// 128-bit neighbour signature of every vertex: 32 vertices per warp, rows of at
-// most 32 entries by their lane, longer ones by the warp one after another
+// 128-bit neighbour signature of every vertex: rows of at most 32 entries by a lane
+// each, 32 consecutive vertices per warp; longer ones by a warp each, which takes them
+// from the buckets' lists (met among a warp's 32 vertices and swept one after another,
+// the hubs of a Chung-Lu graph of 262,111 vertices, numbered side by side, took
+// 156 us instead of 9; a warp for every row 26)
 __device__ __forceinline__ void sig_add(int32_t u, uint32_t (&w)[4]) {
     const uint32_t b = nb_bit(u), m = 1u << (b & 31), q = b >> 5;
     w[0] |= q == 0 ? m : 0u; w[1] |= q == 1 ? m : 0u; w[2] |= q == 2 ? m : 0u; w[3] |= q == 3 ? m : 0u;
 }
-__global__ void k_gnn_sig(DGraph g, uint4* __restrict__ sig) {
+__global__ void k_gnn_sig(GnnRows R, uint4* __restrict__ sig) {
+    const DGraph& g = R.g;
     const int lane = threadIdx.x & 31;
     const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t v0 = wid * 32; v0 < g.n; v0 += nw * 32) {
-        const int64_t v = v0 + lane;
-        const int64_t beg = v < g.n ? g.rp[v] : 0, end = v < g.n ? g.rp[v + 1] : 0;
-        const bool is_long = end - beg > 32;
-        if (v < g.n && !is_long) {
-            uint32_t w[4] = {0, 0, 0, 0};
-#pragma unroll 4
-            for (int64_t e = beg; e < end; ++e) sig_add(__ldg(&g.ci[e]), w);
-            sig[v] = make_uint4(w[0], w[1], w[2], w[3]);
-        }
-        for (uint32_t todo = __ballot_sync(0xffffffffu, is_long); todo; todo &= todo - 1) {
-            const int src = __ffs(todo) - 1;
-            const int64_t b2 = __shfl_sync(0xffffffffu, beg, src), e2 = __shfl_sync(0xffffffffu, end, src);
-            uint32_t w[4] = {0, 0, 0, 0};
+    const int64_t nlong = R.nheavy + R.nb[2], units = nlong + (g.n + 31) / 32;
+    for (int64_t i = wid; i < units; i += nw) {
+        uint32_t w[4] = {0, 0, 0, 0};
+        if (i < nlong) {
+            const int64_t v = i < R.nheavy ? R.heavy[i] : R.b[2][i - R.nheavy];   // the longest first
+            const int64_t end = g.rp[v + 1];
 #pragma unroll 16
-            for (int64_t e = b2 + lane; e < e2; e += 32) sig_add(__ldcs(&g.ci[e]), w);
+            for (int64_t e = g.rp[v] + lane; e < end; e += 32) sig_add(__ldcs(&g.ci[e]), w);
 #pragma unroll
             for (int q = 0; q < 4; ++q) w[q] = __reduce_or_sync(0xffffffffu, w[q]);
-            if (lane == 0) sig[v0 + src] = make_uint4(w[0], w[1], w[2], w[3]);
+            if (lane == 0) sig[v] = make_uint4(w[0], w[1], w[2], w[3]);
+        } else {
+            const int64_t v = (i - nlong) * 32 + lane;
+            const int64_t beg = v < g.n ? g.rp[v] : 0, end = v < g.n ? g.rp[v + 1] : 0;
+            if (v < g.n && end - beg <= kTile32) {
+#pragma unroll 4
+                for (int64_t e = beg; e < end; ++e) sig_add(__ldg(&g.ci[e]), w);
+                sig[v] = make_uint4(w[0], w[1], w[2], w[3]);
+            }
         }
     }
 }
@@ -982,7 +986,7 @@ static void gnn_forward(Ctx& c, const gp_gnn* G, const Level& L, int level, bool
     k_gnn_vfeat<<<vg, 256, 0, c.s>>>(n, g.rp, g.vw, (float)level, g.ew ? 0 : 1, (float4*)A.x, A.wdeg);
     GP_LAUNCHED(c);
     A.sig = (uint4*)c.tmp->alloc(sizeof(uint4) * (size_t)std::max<int64_t>(n, 1));
-    k_gnn_sig<<<grid_for(n, 256, c.sm_count * 32), 256, 0, c.s>>>(g, A.sig);
+    k_gnn_sig<<<grid_for((L.nheavy + L.nbucket[2]) * 32 + n, 256, c.sm_count * 32), 256, 0, c.s>>>(R, A.sig);
     GP_LAUNCHED(c);
     rowsum(ValRow4{g.ci, (const float4*)A.x}, FinMean<F0>{g.rp, A.a}, std::integral_constant<int, F0>());
     const bool wide = n >= kGnnWide;
