@@ -101,7 +101,10 @@ __device__ void ip_bfs(const DGraph& g, const int32_t* lab, int32_t* dist, const
 
 // Trials of graphs too large for k_initpart_chip (coarsening that stalled
 // above 65,534 vertices, or no room for its shared-memory state): labels and
-// distances in the trial's slices of the global arrays
+// distances in the trial's slices of the global arrays.  What bounds it is the
+// latency of its sweeps over all vertices, so two blocks per SM (32 registers) pay
+// when there are more trials than SMs: 256 trials of a Chung-Lu graph of 30,700
+// vertices, k = 1000, 284 ms against 441 with one block of 58 registers.
 __global__ void __launch_bounds__(IP_T) k_initpart(DGraph g, int32_t k, uint64_t seed, int32_t* __restrict__ labels,
                                                     int32_t* __restrict__ dists, int64_t* __restrict__ tcut,
                                                     int64_t* __restrict__ tmaxpw, int key_iters) {
@@ -122,6 +125,11 @@ __global__ void __launch_bounds__(IP_T) k_initpart(DGraph g, int32_t k, uint64_t
     }
     int32_t* lab = labels + (int64_t)t * n;
     int32_t* dist = dists + (int64_t)t * n;
+    // two opaque pointers: the compiler otherwise keeps addresses derived from both
+    // arrays per loop and spills 100 bytes at 32 registers (the trial above, 64 times:
+    // 250 ms instead of 233; random geometric, 68,672 vertices, k = 8: 1375
+    // instead of 1250)
+    asm volatile("" : "+l"(lab), "+l"(dist));
     const uint64_t ts = trial_salt(seed, t);
     for (int64_t v = threadIdx.x; v < n; v += blockDim.x) lab[v] = 0;
     for (int q = threadIdx.x; q < k; q += blockDim.x) S.cnt[q] = (q == 0) ? k : 0;
