@@ -2408,10 +2408,12 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
         if (c.profile) GP_CUDA(cudaEventRecord(c.ev_b, c.s));
         // rowptr, colidx, weights, gathered part[u] (pcb bytes); part[v], lock[v] read; proposal and gain written
         c.sync();   // the pass wrote its status block to c.h_pinned
-        // a pass that did not sweep every row: its rows' share is not known here, only
-        // the lists, parts and locks it read are counted
-        const int64_t conn_bytes = c.h_pinned[H_FULL] ? L.scan_bytes() - (4 - B.pcb) * g.m + B.pcb * n + n + 8 * n
-                                                      : (4 + B.pcb + 1) * n;
+        // a rebalancing pass that sweeps the rows of overweight parts only: their share
+        // is not known here, the lists and parts of all rows are counted; a pass that
+        // ends the level reads nothing
+        const bool swept = c.h_pinned[H_FULL] != 0;
+        const int64_t conn_bytes = swept ? L.scan_bytes() - (4 - B.pcb) * g.m + B.pcb * n + n + 8 * n
+                                         : (c.h_pinned[S_MODE] == MODE_EVAL ? 0 : (4 + B.pcb) * n);
         c.bytes += conn_bytes;
         if (c.profile) {
             float t = 0;
