@@ -2294,7 +2294,30 @@ constexpr int64_t kConnSplitM = 1 << 21;   // entries (a pass of 30 us and more)
 constexpr int64_t kTrackShare = 8;
 constexpr int64_t kTrackLast = 3;
 constexpr int64_t kTrackMin = 1 << 22;   // entries from which the cut's change is tracked
-int64_t conn_max_ranges(const Ctx& c) { return (int64_t)c.sm_count * c.ctas_per_sm * RW * 4; }
+// How a level's connectivity passes are cut: bucket-0 rows in their own launches
+// when they are many, and on levels whose longer rows are the work (k_conn without
+// them runs at 48 registers); the rest in contiguous ranges of light units.  A range
+// costs as much as a group of 8 units of short rows, so that a warp's lanes have
+// rows to work on; on levels too small for 16 such ranges per SM latency counts and
+// units are spread thinner
+struct ConnPlan {
+    bool split, long_rows;
+    int64_t nunits, cost, wave, nranges;
+};
+static ConnPlan conn_plan(const Ctx& c, const Level& L) {
+    ConnPlan p;
+    p.split = L.nbucket[0] >= kConnSplit || L.g.m >= kConnSplitM;
+    p.long_rows = !p.split || L.nitems + L.nbucket[1] + L.nbucket[2] > 0;
+    p.nunits = p.split ? L.nbucket[2] + L.nbucket[1] : L.nunits;
+    p.cost = L.g.m + 32 * (L.nbucket[2] + L.nbucket[1]) + (p.split ? 0 : 2 * L.nbucket[0]);
+    p.wave = (int64_t)c.sm_count * kConnWave;
+    const int64_t most = (int64_t)c.sm_count * c.ctas_per_sm * RW * 4;
+    const int64_t want = std::max<int64_t>(std::max(std::min(p.cost / kConnWarpCost, p.wave * RW), p.cost / kConnRangeCost),
+                                           (int64_t)c.sm_count * 16);
+    p.nranges = std::max<int64_t>(std::min(std::min(p.nunits, want), most), 1);
+    return p;
+}
+int64_t conn_ranges(const Ctx& c, const Level& L) { return conn_plan(c, L).nranges; }
 
 // range t of the nw of a connectivity pass holds the units [first unit with cost
 // prefix >= T * t / nw, the same for t + 1), T the total cost: contiguous ranges
@@ -2330,20 +2353,10 @@ int refine_level(Ctx& c, const Level& L, const Params& P, RefineBufs& B, int lev
     const int kpad = (k + 15) & ~15;
     const size_t conn_smem = kpad + sizeof(int32_t) * RW * k;
     // at most 1024 + 32 * GP_MAX_K bytes: below the 48 KB default, no attribute needed
-    // bucket-0 rows: their own launches when they are many, and on levels whose
-    // longer rows are the work (k_conn without them runs at 48 registers)
-    const bool split = L.nbucket[0] >= kConnSplit || g.m >= kConnSplitM;
-    const bool long_rows = !split || L.nitems + L.nbucket[1] + L.nbucket[2] > 0;
-    const int64_t nunits = split ? L.nbucket[2] + L.nbucket[1] : L.nunits;
-    const int64_t short_cost = split ? 0 : 2 * L.nbucket[0];
-    // a range costs as much as a group of 8 units of short rows, so that a warp's
-    // lanes have rows to work on; on levels too small for 16 such ranges per SM
-    // latency counts and units are spread thinner
-    const int64_t cost = g.m + 32 * (L.nbucket[2] + L.nbucket[1]) + short_cost;
-    const int64_t wave = (int64_t)c.sm_count * kConnWave;
-    const int64_t want = std::max<int64_t>(std::max(std::min(cost / kConnWarpCost, wave * RW), cost / kConnRangeCost),
-                                           (int64_t)c.sm_count * 16);
-    const int64_t nranges = std::max<int64_t>(std::min(std::min(nunits, want), B.wfirst_cap - 1), 1);
+    const ConnPlan cut = conn_plan(c, L);
+    const bool split = cut.split, long_rows = cut.long_rows;
+    const int64_t nunits = cut.nunits, cost = cut.cost, wave = cut.wave, nranges = cut.nranges;
+    if (nranges >= B.wfirst_cap) throw GpError(GP_EINTERNAL, "connectivity ranges exceed their array");
     const int light_blocks = (int)std::min<int64_t>(grid_for(nranges, RW, c.sm_count * c.ctas_per_sm),
                                                     std::max(wave, cost / kConnBlockCost));
     const int grid = (int)L.nitems + light_blocks;
