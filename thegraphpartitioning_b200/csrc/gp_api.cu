@@ -95,7 +95,7 @@ __global__ void k_check_rowptr(int64_t n, int64_t m, const int64_t* __restrict__
 // input is refused), so both sums are exact integers.  They are zero for every
 // symmetric graph.  In an asymmetric one some pair's signed weights add up to
 // d != 0; whatever the other pairs add, at most one value of that pair's half hash
-// cancels the sum, in each half: 2^-64 for hashes drawn at random.  They are a
+// cancels the sum in each half, 2^-64 for both with hashes drawn at random.  They are a
 // bijective mix (degski's, two multiplications) of the pair and a key drawn anew for
 // each call, so no input can be built to cancel (a fixed hash allows that, and with
 // sums mod 2^64 a weight divisible by 2^t leaves only 64 - t bits).

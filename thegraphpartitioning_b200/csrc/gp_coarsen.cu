@@ -6,9 +6,11 @@
 // around them (src/gpu_part.cu:1003-1152).
 //
 // Layout: CSR with int64 row pointers, int32 column ids and int32 weights;
-// a NULL weight array means unit weights (the input level only).  Rows longer
-// than kHeavyDeg are handled by one CTA each (blocks [0, nheavy) of a launch);
-// all other rows by one warp each (grid-stride over the remaining blocks).
+// a NULL weight array means unit weights (the input level only).  The matching
+// takes rows by degree bucket: rows longer than heavy_deg in pieces of a CTA each
+// (blocks [0, nitems) of a launch), rows of 17 entries and more a warp each, shorter
+// ones a thread each (16 lanes each where they are few).  The contraction takes
+// coarse rows by the length of their walk, in the tiers listed there.
 #define GP_TU_ID 2   // site ids of the bounds-checked build
 #include "gp_internal.cuh"
 
@@ -829,7 +831,7 @@ __global__ void k_cmap(DGraph g, const int32_t* __restrict__ match, const int64_
 // the rank of its first position, with the weights of all its positions
 // summed; c itself is dropped.
 //
-// Tiers A, B, C and C2 read the walk straight from the fine CSR, mapping each
+// Tiers S to C2 read the walk straight from the fine CSR, mapping each
 // column id through cmap as they go, and read it once.  Tier D reads its rows
 // three times, so k_fill_walk_d first writes those rows, mapped, into a walk
 // layout (row c at off[c]).  Every tier writes its unique entries at off[c]
@@ -839,12 +841,12 @@ __global__ void k_cmap(DGraph g, const int32_t* __restrict__ match, const int64_
 //   A2 d <= 256        one warp, 512-slot table
 //   B  d <= 512        one warp, 1024-slot table (11 KB per warp: 20 warps per SM)
 //   C1 d <= 2048       one CTA of 256 threads, two-phase (first position kept by
-//                      atomicMax of deg - j), 4096-slot table on chip (54 KB: four
-//                      CTAs per SM)
-//   C  d <= 4096       the same with 512 threads and an 8192-slot table (108 KB: two
-//                      CTAs per SM)
-//   C2 d <= 12288      the same with 1024 threads and a 16384-slot table (196 KB:
-//                      one CTA per SM; load factor at most 3/4)
+//                      an atomic minimum), 4096-slot table on chip (36 KB, 52 with
+//                      64-bit slots: four CTAs per SM)
+//   C  d <= 4096       the same with 512 threads and an 8192-slot table (72 KB, 104
+//                      with 64-bit slots: two CTAs per SM)
+//   C2 d <= 12288      the same with 1024 threads and a 16384-slot table (152 KB, 216
+//                      with 64-bit slots: one CTA per SM; load factor at most 3/4)
 //   C3 d <= 65536      one 1024-thread CTA, the C2 table in P = 2..8 passes: pass p
 //                      dedups the keys whose pass hash is p, first positions are
 //                      marked in a shared-memory bitmap of the whole walk

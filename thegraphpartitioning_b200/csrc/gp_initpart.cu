@@ -793,9 +793,9 @@ int initial_partition(Ctx& c, const Level& L, const Params& P, int32_t* part_out
     return bt;
 }
 
-// k_initpart may use the whole opt-in shared memory of a block (per-label
-// arrays, plus labels and distances when they fit); set once per device (the
-// cap is per kernel, shared by every thread of the process)
+// the trials' kernels may use the whole opt-in shared memory of a block (per-label
+// arrays; in k_initpart_chip also the vertices' state, lists and rows that fit); set
+// once per device (the cap is per kernel, shared by every thread of the process)
 static size_t g_ip_smem_max = 0;
 
 size_t initpart_smem_max() { return g_ip_smem_max; }

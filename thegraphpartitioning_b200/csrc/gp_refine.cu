@@ -74,9 +74,10 @@ __device__ __forceinline__ bool lp_candidate(int32_t g, int32_t own, int32_t den
 // status: [S_CROSS] += directed cross weight; [S_MAXPW], [S_MODE], [S_LIGHT]
 // written by CTA 0; LP candidates are appended to clist[bucket] (any order:
 // each is evaluated on its own), with [S_NL0..S_NL2] their counts and
-// [S_CDEG] the sum of their degrees.  Rebalance candidates are the vertices
-// with dest >= 0, [S_CDEG] their number; they are collected in vertex order
-// afterwards.
+// [S_CDEG] the sum of their degrees.  Rebalance candidates are the vertices of
+// overweight parts, [S_CDEG] their number; they are collected in vertex order
+// afterwards.  A rebalancing pass stores dest and gain of those only (of every
+// vertex when traced): the others' are left from the pass before.
 
 // What decides whether a pass is the level's last (the host loop's rule, from
 // its state before the pass): such a pass sweeps nothing when the cut's change
@@ -1317,8 +1318,8 @@ __global__ void k_rb_strong_apply(int64_t cnt, const uint64_t* __restrict__ keys
 // Exact integers, so that the pass after it need not sweep the rows it looks
 // for no move in, and a pass that would end the level sweeps nothing: on the
 // 256^3 grid (k = 32) the rebalancing passes, two thirds of all, sweep one part in
-// 32 instead of every row: all its passes take 47 -> 32 ms, k_track 2.8 ms; on
-// R-MAT 24 they take 116 -> 101 ms, k_track 13.  Left out when the next pass sweeps
+// 32 instead of every row: all its passes take 42 -> 30 ms, k_track 3.2 ms; on
+// R-MAT 24 they take 131 -> 102 ms, k_track 13.  Left out when the next pass sweeps
 // every row anyway: no overweight part and a level that may go on, or moved rows
 // of more than track_deg entries.  Blocks [0, nitems) take the pieces of the heavy
 // rows, range_blocks the warp rows by the connectivity pass's ranges (block_unit:
@@ -1510,7 +1511,7 @@ __global__ void k_part_weights(int64_t n, const int32_t* __restrict__ part, cons
 }
 
 // directed cross weight, entry-sliced (csr_sweep): each lane of a window also
-// holds its row's part; up to eight groups of 32 entries have their column ids
+// holds its row's part; up to kCutG groups of 32 entries have their column ids
 // loaded, then their neighbours' parts gathered, together.  PT: part ids of 1
 // byte where a compacted copy pays (kCutCompact), else the caller's int32
 constexpr int kCutG = 4;
@@ -1564,8 +1565,11 @@ void part_weights(Ctx& c, const DGraph& g, const int32_t* part, int32_t k, int64
 }
 
 // entries from which the cut gathers from a copy of the parts in bytes, on graphs
-// of a mean degree of 8 and more (the copy costs 5 bytes a vertex): R-MAT 22, 4.2 M
-// vertices, 128 M entries, 592 us from int32, 568 from bytes, the copy included
+// of a mean degree of 8 and more (the copy costs 5 bytes a vertex).  Whole calls
+// from int32 and from bytes, the copy included: R-MAT 18 / 19 / 20 / 21 / 22 (7.6 M to 128
+// M entries) 101 / 126 / 189 / 315 / 650 us and 93 / 118 / 180 / 304 / 626; Erdos-Renyi
+// graphs, whose parts are met evenly, of 2.6 / 10 / 60 M entries 81 / 127 / 378 and 81 / 130
+// / 386
 constexpr int64_t kCutCompact = 1 << 20;
 __global__ void k_compact_part(int64_t n, const int32_t* __restrict__ part, void* pc, int pcb);
 void cut_and_weights(Ctx& c, const DGraph& g, const int32_t* part, int32_t k, int64_t* d_cross2, int64_t* d_pw) {
@@ -1603,6 +1607,10 @@ void cut_and_weights(Ctx& c, const DGraph& g, const int32_t* part, int32_t k, in
 // multi-kernel path and the same integer results.  Rebalance candidates are
 // sorted by a bitonic network in shared memory on unique 64-bit keys
 // (source, loss bucket, id), then (destination, loss bucket, source, id).
+// The block's 64 registers per thread hold the short rows' thread-per-row form only
+// with spills (364 and 336 bytes); it still takes a random geometric graph of 8,000
+// vertices, k = 16, 3.7 -> 1.5 ms against a lane group per row, and 128 graphs of 1,000
+// vertices in one batch 3.1 -> 2.4.
 constexpr int CT = 1024, CW = CT / 32;
 constexpr int64_t kCtaMaxN = 16384;                 // candidates sorted in shared memory (8 B each)
 // A rebalance step of at most this many candidates is taken by one block
@@ -1843,9 +1851,10 @@ __device__ AbCount cta_rebalance(const RbCta& R, int mode, int64_t n, const int3
     return cnt;
 }
 
-// one rebalance step of the multi-kernel loop in one launch: candidates from
-// dest (n <= kCtaMaxN, locks cleared here) or from a compacted list; part
-// weights in and out of global memory; the step's moves added to *moves_out
+// one rebalance step of the multi-kernel loop in one launch: candidates are every
+// vertex of an overweight part (cand == nullptr, n <= kCtaMaxN; locks cleared and the
+// partition copied here) or a compacted list of them; part weights in and out of
+// global memory; the step's moves and their entries added to its status block
 __global__ void __launch_bounds__(CT, 1) k_rb_step_cta(RbCta R, int mode, int64_t n, const int32_t* cand,
                                                         int64_t ncand, int64_t* pw, int64_t* step) {
     extern __shared__ __align__(16) unsigned char rsm[];
@@ -2286,14 +2295,21 @@ constexpr int64_t kConnBlockCost = 98304;
 // bucket-0 rows from which they take their own launch: below, a second launch
 // (about 3 us a pass) costs more than the registers
 constexpr int64_t kConnSplit = 32768;
-constexpr int64_t kConnSplitM = 1 << 21;   // entries (a pass of 30 us and more)
+// or entries.  Refinement with 1 M / 2 M / 4 M entries: R-MAT 16 4.3 / 4.0 / 4.0 ms, R-MAT 17
+// 6.8 / 6.6 / 6.4, Erdos-Renyi of 2.6 M entries 8.9 / 8.9 / 9.1, R-MAT 20 15.7 / 15.7 / 15.6
+constexpr int64_t kConnSplitM = 1 << 21;
 // moved rows' share of the entries up to which the cut's change is tracked: before
 // a pass that looks for moves in the overweight parts (an eighth to a half of the
 // rows) and before one that may be the level's last (R-MAT 24, passes and k_track:
-// 1/16 and 1/4 117 ms, 1/8 and 1/3 115, 1/4 and 1/2 116)
+// 1/16 and 1/4 117 ms, 1/8 and 1/3 115, 1/4 and 1/2 116; the whole refinement of R-MAT 22
+// 40.4 / 40.4 / 41.0, of a 200^3 grid 43.1 with each)
 constexpr int64_t kTrackShare = 8;
 constexpr int64_t kTrackLast = 3;
-constexpr int64_t kTrackMin = 1 << 22;   // entries from which the cut's change is tracked
+// entries from which the cut's change is tracked.  Refinement with 2 M / 4 M / 8 M / never:
+// Erdos-Renyi of 2.5 M entries 14.8 / 14.3 / 14.2 / 14.3 ms, 100^3 grid (5.9 M) 21.7 / 21.7 /
+// 21.3 / 21.4, random geometric of 8 M 10.5 / 10.5 / 10.7 / 10.7, 200^3 grid (48 M) 43.2 /
+// 43.1 / 43.2 / 45.4, R-MAT 22 (128 M) 40.4 / 40.4 / 40.5 / 42.5
+constexpr int64_t kTrackMin = 1 << 22;
 // How a level's connectivity passes are cut: bucket-0 rows in their own launches
 // when they are many, and on levels whose longer rows are the work (k_conn without
 // them runs at 48 registers); the rest in contiguous ranges of light units.  A range
