@@ -1565,12 +1565,12 @@ void part_weights(Ctx& c, const DGraph& g, const int32_t* part, int32_t k, int64
 }
 
 // entries from which the cut gathers from a copy of the parts in bytes, on graphs
-// of a mean degree of 8 and more (the copy costs 5 bytes a vertex).  Whole calls
-// from int32 and from bytes, the copy included: R-MAT 18 / 19 / 20 / 21 / 22 (7.6 M to 128
-// M entries) 101 / 126 / 189 / 315 / 650 us and 93 / 118 / 180 / 304 / 626; Erdos-Renyi
-// graphs, whose parts are met evenly, of 2.6 / 10 / 60 M entries 81 / 127 / 378 and 81 / 130
-// / 386
-constexpr int64_t kCutCompact = 1 << 20;
+// of a mean degree of 8 and more (the copy costs 5 bytes a vertex and a launch).  Whole
+// calls from int32 and from bytes, the copy included: R-MAT 16 / 17 (1.8 and 3.7 M
+// entries) 68 / 78 us and 70 / 80, Erdos-Renyi of 2.6 M with weights 82 and 84; R-MAT 18 /
+// 19 / 20 / 21 / 22 (7.6 to 128 M) 101 / 126 / 189 / 315 / 650 and 93 / 118 / 180 / 304 / 626;
+// Erdos-Renyi, whose parts are met evenly, of 10 / 60 M 127 / 378 and 130 / 386
+constexpr int64_t kCutCompact = 1 << 22;
 __global__ void k_compact_part(int64_t n, const int32_t* __restrict__ part, void* pc, int pcb);
 void cut_and_weights(Ctx& c, const DGraph& g, const int32_t* part, int32_t k, int64_t* d_cross2, int64_t* d_pw) {
     memset_async(c, d_cross2, 0, sizeof(int64_t));
