@@ -766,7 +766,8 @@ int initial_partition(Ctx& c, const Level& L, const Params& P, int32_t* part_out
         const size_t smem = chip + (lists_on ? lists : 0) + (csr_on ? csr : 0);
         // cuts of all trials together: rows in L2, labels of 16 trials on chip
         const size_t lab = (size_t)n * TC_G * (P.k <= 256 ? 1 : 2);
-        const bool cuts = !csr_on && m >= kTrialCuts && lab <= cap;
+        // (16 trials per row of the grid, which has at most 65,535 rows)
+        const bool cuts = !csr_on && m >= kTrialCuts && lab <= cap && T <= 65535 * TC_G;
         auto kernel = csr_on ? k_initpart_chip<true, 1> : (davg >= 32 ? k_initpart_chip<false, 4> : k_initpart_chip<false, 1>);
         kernel<<<T, threads, smem, c.s>>>(L.g, P.k, P.seed, labels, glists, tcut, tmaxpw, tile, cuts ? 0 : 1);
         GP_LAUNCHED(c);
