@@ -59,3 +59,24 @@ def test_missing_mirror_matches_oracle(oracle_mod, gp, cuda):
     rp[row + 1:] -= 1
     ci = np.delete(ci, e)
     _run(oracle_mod, gp, cuda, rp, ci, np.ones(len(ci), np.int32), 6)
+
+
+@pytest.mark.parametrize("n,deg,k,w,opts", [(6000, 8, 8, None, {}), (6000, 8, 64, "w", {"heavy_deg": 100}), (2300, 7, 255, None, {}),
+                                            (900, 150, 4, None, {"coarsen_to": 900}), (25000, 9, 5, "w", {"check_input": -1}),
+                                            (5000, 30, 300, None, {"small_level_n": 16384})])
+def test_directed_graphs_match_oracle(oracle_mod, gp, cuda, n, deg, k, w, opts):
+    """Random directed graphs, almost no entry with its mirror, whose coarse graphs are
+    dense: the trials' searches go along the entries, never against them."""
+    rng = np.random.default_rng(n + k)
+    src = rng.integers(0, n, n * deg)
+    dst = (src + rng.integers(1, n, n * deg)) % n
+    src, dst = src[np.argsort(src, kind="stable")], dst
+    dst = np.where(src == dst, (dst + 1) % n, dst).astype(np.int32)
+    rp = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=n))]).astype(np.int64)
+    ew = rng.integers(1, 10, n * deg).astype(np.int32) if w else None
+    opts = dict(opts, init_trials=3)
+    d = lambda a: None if a is None else torch.from_numpy(a).to(cuda)
+    p_ref, s_ref, ev_ref = oracle_mod.partition(rp, dst, k, 0.03, 8, ewgt=ew, options=opts, trace=True)
+    p_gpu, s, ev_gpu = gp.partition(d(rp), d(dst), k, 0.03, 8, ewgt=d(ew), options=opts, trace=True)
+    compare_traces(ev_ref, ev_gpu)
+    assert np.array_equal(p_ref, p_gpu.cpu().numpy()) and s["cut"] == s_ref["cut"]

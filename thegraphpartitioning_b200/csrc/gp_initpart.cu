@@ -271,7 +271,8 @@ __global__ void __launch_bounds__(IP_T) k_initpart(DGraph g, int32_t k, uint64_t
 //    32 and more a level whose frontier F is large runs bottom-up instead
 //    (every unreached vertex scans its row until it meets the frontier): about
 //    n / F entries per unreached vertex against F whole rows, so bottom-up
-//    when unreached * n < F * F * degree;
+//    when unreached * n < F * F * degree.  Its rows are the frontier's mirrored,
+//    so only on inputs known to be symmetric;
 //  - the second BFS sums each label's frontier weight level by level, which
 //    gives the distance at which the label's target weight is crossed, and
 //    stops there; the crossing vertex among that distance's vertices (in id
@@ -428,7 +429,7 @@ __device__ void ipc_bfs(const DGraph& g, const IpcRows<CSR_SM>& R, uint32_t* sta
 template <bool CSR_SM, int NB>
 __global__ void __launch_bounds__(IP_T) k_initpart_chip(DGraph g, int32_t k, uint64_t seed, int32_t* __restrict__ labels,
                                                         uint16_t* __restrict__ lists, int64_t* __restrict__ tcut,
-                                                        int64_t* __restrict__ tmaxpw, int tile, int cut) {
+                                                        int64_t* __restrict__ tmaxpw, int tile, int cut, int symmetric) {
     extern __shared__ __align__(16) unsigned char ipc_raw[];
     __shared__ IpcShared sh;
     const int32_t n = (int32_t)g.n;
@@ -455,7 +456,7 @@ __global__ void __launch_bounds__(IP_T) k_initpart_chip(DGraph g, int32_t k, uin
     // queue and list: n ids each, on chip unless the caller brings them
     uint16_t* queue = lists ? lists + 2 * (int64_t)t * n : (uint16_t*)after;
     uint16_t* list = queue + n;
-    const int64_t davg = g.m / (n > 0 ? n : 1);
+    const int64_t davg = symmetric ? g.m / (n > 0 ? n : 1) : 0;   // 0: no level runs bottom-up
     const uint64_t ts = trial_salt(seed, t);
     int64_t wsum = 0;
     for (int32_t v = threadIdx.x; v < n; v += blockDim.x) { state[v] = 0; wsum += g.vw ? g.vw[v] : 1; }
@@ -769,7 +770,8 @@ int initial_partition(Ctx& c, const Level& L, const Params& P, int32_t* part_out
         // (16 trials per row of the grid, which has at most 65,535 rows)
         const bool cuts = !csr_on && m >= kTrialCuts && lab <= cap && T <= 65535 * TC_G;
         auto kernel = csr_on ? k_initpart_chip<true, 1> : (davg >= 32 ? k_initpart_chip<false, 4> : k_initpart_chip<false, 1>);
-        kernel<<<T, threads, smem, c.s>>>(L.g, P.k, P.seed, labels, glists, tcut, tmaxpw, tile, cuts ? 0 : 1);
+        kernel<<<T, threads, smem, c.s>>>(L.g, P.k, P.seed, labels, glists, tcut, tmaxpw, tile, cuts ? 0 : 1,
+                                            P.symmetric ? 1 : 0);
         GP_LAUNCHED(c);
         if (cuts) {
             const dim3 grid((unsigned)std::max<int64_t>(1, std::min<int64_t>(c.sm_count * TC_G / T + 1, (n + 15) / 16)),
