@@ -214,6 +214,24 @@ static int bits_for(int64_t x) {
     return b;
 }
 
+// k_check_rows with a new key: sums[1] += the weights, sums[2] and [3] the fingerprint
+static void check_rows(Ctx& c, const DGraph& g, int check, unsigned long long* err, int64_t* sums) {
+    const int64_t slice = csr_slice(g.m, c.sm_count);
+    std::random_device draw;
+    const uint64_t key = ((uint64_t)draw() << 32) | draw();
+    k_check_rows<<<grid_for((g.m + slice - 1) / slice * 32, 256, c.sm_count * 8), 256, 0, c.s>>>(
+        g.n, g.m, slice, g.rp, g.ci, g.ew, check, key, err, sums);
+    GP_LAUNCHED(c);
+}
+
+// the fingerprint of one level, whose weights add up to less than 2^31, left in
+// sums[2] and sums[3] (both zero: symmetric); sums: 5 words of scratch
+void symmetry_sums(Ctx& c, const DGraph& g, int64_t* sums) {
+    memset_async(c, sums, 0, 5 * sizeof(int64_t));
+    check_rows(c, g, 1, (unsigned long long*)(sums + 4), sums);
+    c.bytes += 8 * (g.n + 1) + 4 * g.m + (g.ew ? 4 * g.m : 0);
+}
+
 // returns total vertex weight; symmetric: the entries were checked and passed the fingerprint
 static int64_t validate(Ctx& c, const DGraph& g, int check, bool& symmetric) {
     auto mk = c.tmp->save();
@@ -227,12 +245,7 @@ static int64_t validate(Ctx& c, const DGraph& g, int check, bool& symmetric) {
     c.sync();
     uint64_t e0 = (uint64_t)c.h_pinned[0];
     if (e0 != ~0ull) throw GpError(GP_EINVAL, verr((int)(e0 >> 48), (int64_t)(e0 & ((1ull << 48) - 1))));
-    const int64_t slice = csr_slice(g.m, c.sm_count);
-    std::random_device draw;
-    const uint64_t key = ((uint64_t)draw() << 32) | draw();
-    k_check_rows<<<grid_for((g.m + slice - 1) / slice * 32, 256, c.sm_count * 8), 256, 0, c.s>>>(
-        g.n, g.m, slice, g.rp, g.ci, g.ew, check, key, err, sums);
-    GP_LAUNCHED(c);
+    check_rows(c, g, check, err, sums);
     c.bytes += 8 * (g.n + 1) + (g.vw ? 4 * g.n : 0) + (check >= 1 ? 4 * g.m : 0) + (g.ew ? 4 * g.m : 0);
     GP_CUDA(cudaMemcpyAsync(c.h_pinned, err, 8, cudaMemcpyDeviceToHost, c.s));
     GP_CUDA(cudaMemcpyAsync(c.h_pinned + 1, sums, 32, cudaMemcpyDeviceToHost, c.s));

@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(IP_T) k_initpart(DGraph g, int32_t k, uint64_t
 //    (every unreached vertex scans its row until it meets the frontier): about
 //    n / F entries per unreached vertex against F whole rows, so bottom-up
 //    when unreached * n < F * F * degree.  Its rows are the frontier's mirrored,
-//    so only on inputs known to be symmetric;
+//    so only on graphs that pass the symmetry fingerprint;
 //  - the second BFS sums each label's frontier weight level by level, which
 //    gives the distance at which the label's target weight is crossed, and
 //    stops there; the crossing vertex among that distance's vertices (in id
@@ -429,7 +429,8 @@ __device__ void ipc_bfs(const DGraph& g, const IpcRows<CSR_SM>& R, uint32_t* sta
 template <bool CSR_SM, int NB>
 __global__ void __launch_bounds__(IP_T) k_initpart_chip(DGraph g, int32_t k, uint64_t seed, int32_t* __restrict__ labels,
                                                         uint16_t* __restrict__ lists, int64_t* __restrict__ tcut,
-                                                        int64_t* __restrict__ tmaxpw, int tile, int cut, int symmetric) {
+                                                        int64_t* __restrict__ tmaxpw, int tile, int cut,
+                                                        const int64_t* __restrict__ asym) {
     extern __shared__ __align__(16) unsigned char ipc_raw[];
     __shared__ IpcShared sh;
     const int32_t n = (int32_t)g.n;
@@ -456,7 +457,8 @@ __global__ void __launch_bounds__(IP_T) k_initpart_chip(DGraph g, int32_t k, uin
     // queue and list: n ids each, on chip unless the caller brings them
     uint16_t* queue = lists ? lists + 2 * (int64_t)t * n : (uint16_t*)after;
     uint16_t* list = queue + n;
-    const int64_t davg = symmetric ? g.m / (n > 0 ? n : 1) : 0;   // 0: no level runs bottom-up
+    // asym: the level's symmetry_sums (nullptr: known to be symmetric); 0: no level runs bottom-up
+    const int64_t davg = !asym || (asym[2] == 0 && asym[3] == 0) ? g.m / (n > 0 ? n : 1) : 0;
     const uint64_t ts = trial_salt(seed, t);
     int64_t wsum = 0;
     for (int32_t v = threadIdx.x; v < n; v += blockDim.x) { state[v] = 0; wsum += g.vw ? g.vw[v] : 1; }
@@ -770,8 +772,14 @@ int initial_partition(Ctx& c, const Level& L, const Params& P, int32_t* part_out
         // (16 trials per row of the grid, which has at most 65,535 rows)
         const bool cuts = !csr_on && m >= kTrialCuts && lab <= cap && T <= 65535 * TC_G;
         auto kernel = csr_on ? k_initpart_chip<true, 1> : (davg >= 32 ? k_initpart_chip<false, 4> : k_initpart_chip<false, 1>);
-        kernel<<<T, threads, smem, c.s>>>(L.g, P.k, P.seed, labels, glists, tcut, tmaxpw, tile, cuts ? 0 : 1,
-                                            P.symmetric ? 1 : 0);
+        // an input that was not checked, or is not symmetric: look at this level (21 us on
+        // 2.7 M entries, where searches without bottom-up levels take 2.9 ms more)
+        int64_t* asym = nullptr;
+        if (davg >= 32 && !P.symmetric) {
+            asym = c.tmp_alloc<int64_t>(5);
+            symmetry_sums(c, L.g, asym);
+        }
+        kernel<<<T, threads, smem, c.s>>>(L.g, P.k, P.seed, labels, glists, tcut, tmaxpw, tile, cuts ? 0 : 1, asym);
         GP_LAUNCHED(c);
         if (cuts) {
             const dim3 grid((unsigned)std::max<int64_t>(1, std::min<int64_t>(c.sm_count * TC_G / T + 1, (n + 15) / 16)),

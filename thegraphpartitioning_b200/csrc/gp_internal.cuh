@@ -218,6 +218,9 @@ int64_t match_level(Ctx& c, const Level& L, int level, const Params& P, int32_t*
 // pairs: matched pairs; coarse.heavy_deg and coarse.item_len are set by the caller
 void contract_level(Ctx& c, Level& fine, Level& coarse, const int32_t* match, int64_t pairs);
 
+// gp_api.cu
+void symmetry_sums(Ctx& c, const DGraph& g, int64_t* sums);
+
 // gp_initpart.cu
 int initial_partition(Ctx& c, const Level& L, const Params& P, int32_t* part_out);
 
